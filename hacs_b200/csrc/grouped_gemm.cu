@@ -28,205 +28,46 @@ namespace {
 
 using namespace limb;
 
-__device__ __forceinline__ void grouped_drain(uint64_t* bar, uint32_t parity, int* err) {
-    int never = 0;
-    mbar_wait(bar, parity, &never, err, DERR_WAIT_DRAIN);
-}
+// The tiles of a table of products, down the columns of each (consecutive
+// tiles share their B tile).
+template <int BN>
+struct ProductTable {
+    const GroupedProblem* __restrict__ probs;
+    const int* __restrict__ tile_prob;
+    int total_arg;
+    const int* __restrict__ d_total;
+
+    // the tile count: a launch argument, or read from device memory (tables built on the device)
+    __device__ __forceinline__ int total() const { return d_total ? *d_total : total_arg; }
+    __device__ __forceinline__ int kblocks(int t) const { return probs[tile_prob[t]].kblocks; }
+    // tile_begin + the tile column is unique: a product has at least as many tiles as columns
+    __device__ __forceinline__ int b_key(int t) const {
+        const GroupedProblem& P = probs[tile_prob[t]];
+        return P.tile_begin + (t - P.tile_begin) / ((P.M + kBM - 1) / kBM);
+    }
+    __device__ __forceinline__ void prefetch_maps() const {}
+    __device__ __forceinline__ TileRef tile(int t) const {
+        const GroupedProblem& P = probs[tile_prob[t]];
+        const int local = t - P.tile_begin, tiles_m = (P.M + kBM - 1) / kBM;
+        const int tn = local / tiles_m, tm = local - tn * tiles_m;
+        return {P.tmA, P.tmB, P.a_row0 + tm * kBM, P.b_col0 + tn * BN, 0, P.kblocks, P.C, P.ldc, P.M, P.N,
+                tm * kBM, tn * BN, P.op, P.tile_begin + tn};
+    }
+};
 
 template <int L, int BN, int KB>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(gemm_threads(L), 1)
     grouped_limb_gemm_kernel(const GroupedProblem* __restrict__ probs, const int* __restrict__ tile_prob,
-                             int total_tiles_arg, const int* __restrict__ d_total, uint32_t p, uint64_t barrett,
-                             int* err) {
-    // the tile count: a launch argument, or read from device memory (tables built on the device)
-    const int total_tiles = d_total ? *d_total : total_tiles_arg;
-    using CF = Cfg<L, BN, KB>;
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t* sA = smem;
-    uint8_t* sB = smem + CF::STAGES * CF::A_BYTES;
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + CF::STAGES * CF::STAGE_BYTES);
-    uint64_t* empty = full + CF::STAGES;
-    uint64_t* acc_full = empty + CF::STAGES;
-    uint64_t* acc_empty = acc_full + 2;
-    uint64_t* drain = acc_empty + 2;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    uint32_t* epi_stage = reinterpret_cast<uint32_t*>(smem + CF::STAGES * CF::STAGE_BYTES + CF::BAR_BYTES);
+                             int total_tiles_arg, const int* __restrict__ d_total, const EpiRed red, int* err) {
+    long_tiles<L, BN, KB>(ProductTable<BN>{probs, tile_prob, total_tiles_arg, d_total}, red, err);
+}
 
-    const int warp = threadIdx.x >> 5;
-    const int lane = threadIdx.x & 31;
-
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < CF::STAGES; ++s) {
-            mbar_init(&full[s], 1);
-            mbar_init(&empty[s], 1);
-        }
-        for (int a = 0; a < 2; ++a) {
-            mbar_init(&acc_full[a], 1);
-            mbar_init(&acc_empty[a], 32 * kEpiWarps);
-        }
-        mbar_init(drain, 1);
-        *abort_flag = 0;
-        fence_mbar_init();
-        fence_proxy_async_smem();
-    }
-    if (warp == 1) {
-        tmem_alloc(tmem_slot, CF::TMEM_COLS);
-        tmem_relinquish();
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
-
-    if (warp == 0) {
-        if (lane == 0) {
-            int it = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
-                const int pi = tile_prob[tile];
-                const GroupedProblem& P = probs[pi];
-                const int local = tile - P.tile_begin;
-                const int tm = local / P.tiles_n, tn = local - tm * P.tiles_n;
-                for (int i = 0; ok && i < L; ++i) {
-                    for (int kb = 0; kb < P.kblocks; ++kb, ++it) {
-                        const int s = it % CF::STAGES;
-                        const uint32_t ph = (it / CF::STAGES) & 1;
-                        if (!mbar_wait(&empty[s], ph ^ 1, abort_flag, err, DERR_WAIT_EMPTY)) {
-                            ok = false;
-                            break;
-                        }
-                        mbar_arrive_expect_tx(&full[s], CF::STAGE_BYTES);
-                        tma_load_3d(sA + s * CF::A_BYTES, P.tmA, &full[s], kb * KB, P.a_row0 + tm * kBM, i);
-                        tma_load_4d(sB + s * CF::B_BYTES, P.tmB, &full[s], kb * KB, P.b_col0 + tn * BN, 0, i);
-                    }
-                }
-            }
-            if (!ok)
-                for (int t = max(0, it - CF::STAGES); t < it; ++t)
-                    grouped_drain(&full[t % CF::STAGES], (t / CF::STAGES) & 1, err);
-        }
-    } else if (warp == 1) {
-        if (lane == 0) {
-            int it = 0, lt = 0;
-            bool ok = true, issued_any = false;
-            for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, ++lt) {
-                const int kblocks = probs[tile_prob[tile]].kblocks;
-                const int a = lt & 1;
-                const uint32_t aph = (lt >> 1) & 1;
-                if (!mbar_wait(&acc_empty[a], aph ^ 1, abort_flag, err, DERR_WAIT_ACCUM_FREE)) {
-                    ok = false;
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t d = tmem_base + a * CF::ACC_STRIDE;
-                for (int i = 0; ok && i < L; ++i) {
-                    for (int kb = 0; kb < kblocks; ++kb, ++it) {
-                        const int s = it % CF::STAGES;
-                        const uint32_t ph = (it / CF::STAGES) & 1;
-                        if (!mbar_wait(&full[s], ph, abort_flag, err, DERR_WAIT_FULL)) {
-                            ok = false;
-                            break;
-                        }
-                        tc_fence_after();
-                        const uint64_t adesc = smem_desc_kmajor<KB>(smem_u32(sA + s * CF::A_BYTES));
-                        const uint64_t bdesc = smem_desc_kmajor<KB>(smem_u32(sB + s * CF::B_BYTES));
-#pragma unroll
-                        for (int kk = 0; kk < KB / 32; ++kk)
-                            mma_u8(d, adesc + 2 * kk, bdesc + 2 * kk, CF::IDESC, (i | kb | kk) != 0);
-                        issued_any = true;
-                        mma_commit(&empty[s]);
-                    }
-                }
-                if (ok) mma_commit(&acc_full[a]);
-            }
-            if (!ok && issued_any) {
-                mma_commit(drain);
-                grouped_drain(drain, 0, err);
-            }
-        }
-    } else {
-        const int q = warp & 3;
-        const uint32_t lane_base = static_cast<uint32_t>(q * 32) << 16;
-        uint32_t (*stage)[17] = reinterpret_cast<uint32_t (*)[17]>(epi_stage + (warp - 2) * 32 * 17);
-        const int chalf = (warp - 2) >> 2;  // the two warps of a lane quarter take alternate 16-column chunks
-        const int half = lane >> 4, col_in = lane & 15;
-        // Add / Sub read C: each lane prefetches its row of this warp's quarter of
-        // a tile into L2 one tile ahead, so the old values come from L2 and the
-        // HBM reads of the next tile overlap this tile's drain
-        auto prefetch_tile = [&](int t) {
-            if (t >= total_tiles) return;
-            const GroupedProblem& Q = probs[tile_prob[t]];
-            if (Q.op == HME_SET) return;
-            const int lq = t - Q.tile_begin;
-            const int qm = lq / Q.tiles_n, qn = lq - qm * Q.tiles_n;
-            const int row = qm * kBM + q * 32 + lane;
-            if (chalf == 0 && row < Q.M) prefetch_l2_span(Q.C + static_cast<size_t>(row) * Q.ldc + qn * BN, min(BN, Q.N - qn * BN));
-        };
-        prefetch_tile(blockIdx.x);
-        int lt = 0;
-        for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++lt) {
-            prefetch_tile(tile + gridDim.x);
-            const int a = lt & 1;
-            const uint32_t aph = (lt >> 1) & 1;
-            if (!mbar_wait(&acc_full[a], aph, abort_flag, err, DERR_WAIT_ACCUM)) break;
-            tc_fence_after();
-            const GroupedProblem& P = probs[tile_prob[tile]];
-            const int local = tile - P.tile_begin;
-            const int tm = local / P.tiles_n, tn = local - tm * P.tiles_n;
-            const int row0 = tm * kBM + q * 32;
-#pragma unroll 1
-            for (int c0 = 16 * chalf; c0 < BN; c0 += 32) {
-                uint32_t v[L][16];
-#pragma unroll
-                for (int j = 0; j < L; ++j)
-                    tmem_ld16(tmem_base + lane_base + a * CF::ACC_STRIDE + j * BN + c0, v[j]);
-                tmem_wait_ld();
-#pragma unroll
-                for (int e = 0; e < 16; ++e) {
-                    uint64_t s = v[0][e];
-                    if (L > 1) s += static_cast<uint64_t>(v[L > 1 ? 1 : 0][e]) << 8;
-                    if (L > 2) s += static_cast<uint64_t>(v[L > 2 ? 2 : 0][e]) << 16;
-                    if (L > 3) s += static_cast<uint64_t>(v[L > 3 ? 3 : 0][e]) << 24;
-                    stage[lane][e] = reduce_u64(s, p, barrett);
-                }
-                __syncwarp();
-                const int col = tn * BN + c0 + col_in;
-                if (col < P.N) {
-                    // all 16 rows' C values in flight at once, then combine and store
-                    const int rlim = min(32, P.M - row0);
-                    uint32_t old[16];
-                    if (P.op != HME_SET) {
-#pragma unroll
-                        for (int t = 0; t < 16; ++t) {
-                            const int rr = half + 2 * t;
-                            old[t] = rr < rlim ? P.C[static_cast<size_t>(row0 + rr) * P.ldc + col] : 0u;
-                        }
-                    }
-#pragma unroll
-                    for (int t = 0; t < 16; ++t) {
-                        const int rr = half + 2 * t;
-                        if (rr >= rlim) break;
-                        uint32_t o = stage[rr][col_in];
-                        if (P.op == HME_ADD) o = mod_add(old[t], o, p);
-                        else if (P.op == HME_SUB) o = mod_sub(old[t], o, p);
-                        P.C[static_cast<size_t>(row0 + rr) * P.ldc + col] = o;
-                    }
-                }
-                __syncwarp();
-            }
-            tc_fence_before();
-            mbar_arrive(&acc_empty[a]);
-        }
-    }
-
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 1) {
-        tc_fence_after();
-        tmem_dealloc(tmem_base, CF::TMEM_COLS);
-    }
+// Every product's K fits one k-block of KB bytes.
+template <int L, int BN, int KB>
+__global__ void __launch_bounds__(gemm_threads(L), 1)
+    grouped_limb_gemm_short_kernel(const GroupedProblem* __restrict__ probs, const int* __restrict__ tile_prob,
+                                   int total_tiles_arg, const int* __restrict__ d_total, const EpiRed red, int* err) {
+    short_tiles<L, BN, KB>(ProductTable<BN>{probs, tile_prob, total_tiles_arg, d_total}, red, err);
 }
 
 template <int L>
@@ -254,17 +95,24 @@ void ensure_grouped_attr() {
     attr.run([](int) {
         HME_CUDA(cudaFuncSetAttribute(grouped_limb_gemm_kernel<L, BN, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       Cfg<L, BN, KB>::SMEM));
+        HME_CUDA(cudaFuncSetAttribute(grouped_limb_gemm_short_kernel<L, BN, KB>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<L, BN, KB>::SMEM));
     });
 }
 
 template <int L, int BN, int KB>
 void launch_grouped(hme_ctx* ctx, const ModParams& mp, const GroupedProblem* d_probs, const int* d_tile_prob,
-                    int total_tiles, const int* d_total = nullptr) {
+                    int total_tiles, uint32_t kmax, const int* d_total = nullptr) {
     using CF = Cfg<L, BN, KB>;
     ensure_grouped_attr<L, BN, KB>();
     const int grid = d_total ? ctx->num_sms : std::min(total_tiles, ctx->num_sms);
-    HME_TIMED(ctx, "grouped_gemm", grouped_limb_gemm_kernel<L, BN, KB><<<grid, kThreads, CF::SMEM, ctx->stream>>>(
-                                       d_probs, d_tile_prob, total_tiles, d_total, mp.p, mp.barrett, ctx->d_err));
+    const EpiRed red = make_epi(mp, kmax);
+    if (kmax <= static_cast<uint32_t>(KB))
+        HME_TIMED(ctx, "grouped_gemm", grouped_limb_gemm_short_kernel<L, BN, KB><<<grid, gemm_threads(L), CF::SMEM, ctx->stream>>>(
+                                           d_probs, d_tile_prob, total_tiles, d_total, red, ctx->d_err));
+    else
+        HME_TIMED(ctx, "grouped_gemm", grouped_limb_gemm_kernel<L, BN, KB><<<grid, gemm_threads(L), CF::SMEM, ctx->stream>>>(
+                                           d_probs, d_tile_prob, total_tiles, d_total, red, ctx->d_err));
     HME_CUDA(cudaGetLastError());
 }
 
@@ -426,14 +274,14 @@ void run_grouped(hme_ctx* ctx, const ModParams& mp, const std::vector<GemmJob>& 
               grouped_split_kernel<L><<<blocks, 256, 0, ctx->stream>>>(d_split, d_block_job, blocks, nullptr));
     HME_CUDA(cudaGetLastError());
     if (KBsel == 32) {
-        if (narrow) launch_grouped<L, BNn, 32>(ctx, mp, d_probs, d_tile_prob, tiles);
-        else launch_grouped<L, BNw, 32>(ctx, mp, d_probs, d_tile_prob, tiles);
+        if (narrow) launch_grouped<L, BNn, 32>(ctx, mp, d_probs, d_tile_prob, tiles, kmax);
+        else launch_grouped<L, BNw, 32>(ctx, mp, d_probs, d_tile_prob, tiles, kmax);
     } else if (KBsel == 64) {
-        if (narrow) launch_grouped<L, BNn, 64>(ctx, mp, d_probs, d_tile_prob, tiles);
-        else launch_grouped<L, BNw, 64>(ctx, mp, d_probs, d_tile_prob, tiles);
+        if (narrow) launch_grouped<L, BNn, 64>(ctx, mp, d_probs, d_tile_prob, tiles, kmax);
+        else launch_grouped<L, BNw, 64>(ctx, mp, d_probs, d_tile_prob, tiles, kmax);
     } else {
-        if (narrow) launch_grouped<L, BNn, kBK>(ctx, mp, d_probs, d_tile_prob, tiles);
-        else launch_grouped<L, BNw, kBK>(ctx, mp, d_probs, d_tile_prob, tiles);
+        if (narrow) launch_grouped<L, BNn, kBK>(ctx, mp, d_probs, d_tile_prob, tiles, kmax);
+        else launch_grouped<L, BNw, kBK>(ctx, mp, d_probs, d_tile_prob, tiles, kmax);
     }
     // the host tables must outlive the asynchronous uploads
     HME_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -447,7 +295,7 @@ void launch_device_tables(hme_ctx* ctx, const ModParams& mp, const GroupedSplitJ
     HME_TIMED(ctx, "grouped_split", grouped_split_kernel<L><<<split_grid, 256, 0, ctx->stream>>>(d_split, d_block_job,
                                                                                               0, d_nblocks));
     HME_CUDA(cudaGetLastError());
-    launch_grouped<L, grouped_bn_wide(L), 32>(ctx, mp, d_probs, d_tile_prob, 0, d_ntiles);
+    launch_grouped<L, grouped_bn_wide(L), 32>(ctx, mp, d_probs, d_tile_prob, 0, 32, d_ntiles);
 }
 
 }  // namespace

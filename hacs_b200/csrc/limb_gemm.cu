@@ -49,236 +49,61 @@ struct GemmArgs {
     int k_begin;  // first k of this chunk (multiple of kBK)
     int kblocks;  // k-blocks of kBK bytes in this chunk
     int op;
-    uint32_t p;
-    uint64_t barrett;
+    EpiRed red;
     int tiles_m, tiles_n, group_m;
     int* err;
 };
 
-__device__ __forceinline__ void tile_coords(int tile, const GemmArgs& g, int& tm, int& tn) {
-    // Grouped raster: group_m tile-rows share the B tiles they stream, so a
-    // wave of CTAs re-reads each K-slice of A and B from L2, not HBM.
-    const int per_group = g.group_m * g.tiles_n;
-    const int grp = tile / per_group;
-    const int first_m = grp * g.group_m;
-    const int gm = min(g.tiles_m - first_m, g.group_m);
-    const int local = tile - grp * per_group;
-    tm = first_m + local % gm;
-    tn = local / gm;
-}
+// The tiles of one product.  Long K: a grouped raster, group_m tile-rows share
+// the B tiles they stream, so a wave of CTAs re-reads each K-slice of A and B
+// from L2, not HBM.  One k-block (COLS): down the columns, so that consecutive
+// tiles share their B tile.
+template <int BN, bool COLS>
+struct OneProduct {
+    const CUtensorMap* tmA;
+    const CUtensorMap* tmB;
+    const GemmArgs& g;
 
-// Time-bounded wait that ignores the abort flag: used while tearing down, to
-// let in-flight copies and MMAs land before shared / tensor memory is released.
-__device__ __forceinline__ void drain_wait(uint64_t* bar, uint32_t parity, int* err) {
-    int never = 0;
-    mbar_wait(bar, parity, &never, err, DERR_WAIT_DRAIN);
-}
+    __device__ __forceinline__ int total() const { return g.tiles_m * g.tiles_n; }
+    __device__ __forceinline__ int kblocks(int) const { return g.kblocks; }
+    __device__ __forceinline__ int b_key(int tile) const { return tile / g.tiles_m; }
+    __device__ __forceinline__ void prefetch_maps() const {
+        if (threadIdx.x == 0) {
+            prefetch_tmap(tmA);
+            prefetch_tmap(tmB);
+        }
+    }
+    __device__ __forceinline__ TileRef tile(int t) const {
+        int tm, tn;
+        if constexpr (COLS) {
+            tn = t / g.tiles_m;
+            tm = t - tn * g.tiles_m;
+        } else {
+            const int per_group = g.group_m * g.tiles_n;
+            const int grp = t / per_group;
+            const int first_m = grp * g.group_m;
+            const int gm = min(g.tiles_m - first_m, g.group_m);
+            const int local = t - grp * per_group;
+            tm = first_m + local % gm;
+            tn = local / gm;
+        }
+        return {tmA, tmB, tm * kBM, tn * BN, g.k_begin, g.kblocks, g.C, g.ldc, g.M, g.N, tm * kBM, tn * BN, g.op, tn};
+    }
+};
 
 template <int L, int BN, int KB = kBK>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(gemm_threads(L), 1)
     limb_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                     const GemmArgs g) {
-    using CF = Cfg<L, BN, KB>;
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t* sA = smem;
-    uint8_t* sB = smem + CF::STAGES * CF::A_BYTES;
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + CF::STAGES * CF::STAGE_BYTES);
-    uint64_t* empty = full + CF::STAGES;
-    uint64_t* acc_full = empty + CF::STAGES;
-    uint64_t* acc_empty = acc_full + 2;
-    uint64_t* drain = acc_empty + 2;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    uint32_t* epi_stage = reinterpret_cast<uint32_t*>(smem + CF::STAGES * CF::STAGE_BYTES + CF::BAR_BYTES);
+                     const __grid_constant__ GemmArgs g) {
+    long_tiles<L, BN, KB>(OneProduct<BN, false>{&tmA, &tmB, g}, g.red, g.err);
+}
 
-    const int warp = threadIdx.x >> 5;
-    const int lane = threadIdx.x & 31;
-    const int total_tiles = g.tiles_m * g.tiles_n;
-
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < CF::STAGES; ++s) {
-            mbar_init(&full[s], 1);
-            mbar_init(&empty[s], 1);
-        }
-        for (int a = 0; a < 2; ++a) {
-            mbar_init(&acc_full[a], 1);
-            mbar_init(&acc_empty[a], 32 * kEpiWarps);
-        }
-        mbar_init(drain, 1);
-        *abort_flag = 0;
-        fence_mbar_init();
-        fence_proxy_async_smem();
-    }
-    if (warp == 1) {
-        tmem_alloc(tmem_slot, CF::TMEM_COLS);
-        tmem_relinquish();
-    }
-    if (warp == 0 && lane == 0) {
-        prefetch_tmap(&tmA);
-        prefetch_tmap(&tmB);
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
-    // the set-up above overlaps the tail of the limb split when this grid is a
-    // programmatic dependent of it; the planes are read only after this point
-    grid_dep_wait();
-
-    if (warp == 0) {
-        // ---------------- TMA producer ----------------
-        if (lane == 0) {
-            int it = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
-                int tm, tn;
-                tile_coords(tile, g, tm, tn);
-                for (int i = 0; ok && i < L; ++i) {
-                    for (int kb = 0; kb < g.kblocks; ++kb, ++it) {
-                        const int s = it % CF::STAGES;
-                        const uint32_t ph = (it / CF::STAGES) & 1;
-                        if (!mbar_wait(&empty[s], ph ^ 1, abort_flag, g.err, DERR_WAIT_EMPTY)) {
-                            ok = false;
-                            break;
-                        }
-                        mbar_arrive_expect_tx(&full[s], CF::STAGE_BYTES);
-                        const int kx = g.k_begin + kb * KB;
-                        tma_load_3d(sA + s * CF::A_BYTES, &tmA, &full[s], kx, tm * kBM, i);
-                        tma_load_4d(sB + s * CF::B_BYTES, &tmB, &full[s], kx, tn * BN, 0, i);
-                    }
-                }
-            }
-            if (!ok) {
-                // let every copy issued into shared memory land before the CTA exits
-                for (int t = max(0, it - CF::STAGES); t < it; ++t)
-                    drain_wait(&full[t % CF::STAGES], (t / CF::STAGES) & 1, g.err);
-            }
-        }
-    } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            int it = 0, lt = 0;
-            bool ok = true, issued_any = false;
-            for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, ++lt) {
-                const int a = lt & 1;
-                const uint32_t aph = (lt >> 1) & 1;
-                if (!mbar_wait(&acc_empty[a], aph ^ 1, abort_flag, g.err, DERR_WAIT_ACCUM_FREE)) {
-                    ok = false;
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t d = tmem_base + a * CF::ACC_STRIDE;
-                for (int i = 0; ok && i < L; ++i) {
-                    for (int kb = 0; kb < g.kblocks; ++kb, ++it) {
-                        const int s = it % CF::STAGES;
-                        const uint32_t ph = (it / CF::STAGES) & 1;
-                        if (!mbar_wait(&full[s], ph, abort_flag, g.err, DERR_WAIT_FULL)) {
-                            ok = false;
-                            break;
-                        }
-                        tc_fence_after();
-                        const uint64_t adesc = smem_desc_kmajor<KB>(smem_u32(sA + s * CF::A_BYTES));
-                        const uint64_t bdesc = smem_desc_kmajor<KB>(smem_u32(sB + s * CF::B_BYTES));
-#pragma unroll
-                        for (int kk = 0; kk < KB / 32; ++kk) {
-                            // +32 bytes along K inside the swizzle atom = +2 in the 16-byte address field
-                            mma_u8(d, adesc + 2 * kk, bdesc + 2 * kk, CF::IDESC, (i | kb | kk) != 0);
-                        }
-                        issued_any = true;
-                        mma_commit(&empty[s]);
-                    }
-                }
-                if (ok) mma_commit(&acc_full[a]);
-            }
-            if (!ok && issued_any) {
-                mma_commit(drain);
-                drain_wait(drain, 0, g.err);
-            }
-        }
-    } else {
-        // ---------------- epilogue: TMEM -> registers -> shared -> C ----------------
-        // Each thread owns one accumulator row (its TMEM lane); the reduced
-        // 16-column chunk goes through a per-warp shared-memory stage so that
-        // C is read and written along rows: two rows x 64 contiguous bytes
-        // per warp instruction instead of 32 rows x 16 bytes.
-        const int q = warp & 3;  // the TMEM lane quarter this warp may read
-        const uint32_t lane_base = static_cast<uint32_t>(q * 32) << 16;
-        uint32_t (*stage)[17] = reinterpret_cast<uint32_t (*)[17]>(epi_stage + (warp - 2) * 32 * 17);
-        const int chalf = (warp - 2) >> 2;  // the two warps of a lane quarter take alternate 16-column chunks
-        const int half = lane >> 4, col_in = lane & 15;
-        // Add / Sub read C: each lane prefetches its row of this warp's quarter of
-        // a tile into L2 one tile ahead (the first tile before its accumulator is
-        // ready), so the old values come from L2 when the drain reads them
-        auto prefetch_tile = [&](int t) {
-            if (g.op == HME_SET || t >= total_tiles) return;
-            int qm, qn;
-            tile_coords(t, g, qm, qn);
-            const int row = qm * kBM + q * 32 + lane;
-            if (chalf == 0 && row < g.M) prefetch_l2_span(g.C + static_cast<size_t>(row) * g.ldc + qn * BN, min(BN, g.N - qn * BN));
-        };
-        prefetch_tile(blockIdx.x);
-        int lt = 0;
-        for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++lt) {
-            prefetch_tile(tile + gridDim.x);
-            const int a = lt & 1;
-            const uint32_t aph = (lt >> 1) & 1;
-            if (!mbar_wait(&acc_full[a], aph, abort_flag, g.err, DERR_WAIT_ACCUM)) break;
-            tc_fence_after();
-            int tm, tn;
-            tile_coords(tile, g, tm, tn);
-            const int row0 = tm * kBM + q * 32;
-#pragma unroll 1
-            for (int c0 = 16 * chalf; c0 < BN; c0 += 32) {
-                uint32_t v[L][16];
-#pragma unroll
-                for (int j = 0; j < L; ++j)
-                    tmem_ld16(tmem_base + lane_base + a * CF::ACC_STRIDE + j * BN + c0, v[j]);
-                tmem_wait_ld();
-#pragma unroll
-                for (int e = 0; e < 16; ++e) {
-                    uint64_t s = v[0][e];
-                    if (L > 1) s += static_cast<uint64_t>(v[L > 1 ? 1 : 0][e]) << 8;
-                    if (L > 2) s += static_cast<uint64_t>(v[L > 2 ? 2 : 0][e]) << 16;
-                    if (L > 3) s += static_cast<uint64_t>(v[L > 3 ? 3 : 0][e]) << 24;
-                    stage[lane][e] = reduce_u64(s, g.p, g.barrett);
-                }
-                __syncwarp();
-                const int col = tn * BN + c0 + col_in;
-                if (col < g.N) {
-                    // all 16 rows' C values in flight at once, then combine and store
-                    const int rlim = min(32, g.M - row0);
-                    uint32_t old[16];
-                    if (g.op != HME_SET) {
-#pragma unroll
-                        for (int t = 0; t < 16; ++t) {
-                            const int rr = half + 2 * t;
-                            old[t] = rr < rlim ? g.C[static_cast<size_t>(row0 + rr) * g.ldc + col] : 0u;
-                        }
-                    }
-#pragma unroll
-                    for (int t = 0; t < 16; ++t) {
-                        const int rr = half + 2 * t;
-                        if (rr >= rlim) break;
-                        uint32_t o = stage[rr][col_in];
-                        if (g.op == HME_ADD) o = mod_add(old[t], o, g.p);
-                        else if (g.op == HME_SUB) o = mod_sub(old[t], o, g.p);
-                        g.C[static_cast<size_t>(row0 + rr) * g.ldc + col] = o;
-                    }
-                }
-                __syncwarp();
-            }
-            tc_fence_before();
-            mbar_arrive(&acc_empty[a]);
-        }
-    }
-
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 1) {
-        tc_fence_after();
-        tmem_dealloc(tmem_base, CF::TMEM_COLS);
-    }
+// One k-block of KB bytes holds K.
+template <int L, int BN, int KB>
+__global__ void __launch_bounds__(gemm_threads(L), 1)
+    limb_gemm_short_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                           const __grid_constant__ GemmArgs g) {
+    short_tiles<L, BN, KB>(OneProduct<BN, true>{&tmA, &tmB, g}, g.red, g.err);
 }
 
 template <int L>
@@ -336,6 +161,8 @@ void launch_gemm(hme_ctx* ctx, const ModParams& mp, uint32_t m, uint32_t n, uint
     attr.run([](int) {
         HME_CUDA(cudaFuncSetAttribute(limb_gemm_kernel<L, BN, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       CF::SMEM));
+        HME_CUDA(cudaFuncSetAttribute(limb_gemm_short_kernel<L, BN, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      CF::SMEM));
     });
     CUtensorMap tmA, tmB;
     {
@@ -357,8 +184,6 @@ void launch_gemm(hme_ctx* ctx, const ModParams& mp, uint32_t m, uint32_t n, uint
     g.ldc = ldc;
     g.M = static_cast<int>(m);
     g.N = static_cast<int>(n);
-    g.p = mp.p;
-    g.barrett = mp.barrett;
     g.tiles_m = static_cast<int>((m + kBM - 1) / kBM);
     g.tiles_n = static_cast<int>((n + BN - 1) / BN);
     g.group_m = 16;
@@ -371,9 +196,10 @@ void launch_gemm(hme_ctx* ctx, const ModParams& mp, uint32_t m, uint32_t n, uint
         g.k_begin = static_cast<int>(kb0);
         g.kblocks = static_cast<int>((kc + KB - 1) / KB);
         g.op = kb0 == 0 ? op : (op == HME_SET ? HME_ADD : op);
+        g.red = make_epi(mp, kc);
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(grid);
-        cfg.blockDim = dim3(kThreads);
+        cfg.blockDim = dim3(gemm_threads(L));
         cfg.dynamicSmemBytes = CF::SMEM;
         cfg.stream = ctx->stream;
         cudaLaunchAttribute attr[1];
@@ -381,7 +207,11 @@ void launch_gemm(hme_ctx* ctx, const ModParams& mp, uint32_t m, uint32_t n, uint
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = (pdl && kb0 == 0 && !ctx->timer.on) ? 1 : 0;
-        HME_TIMED(ctx, "limb_gemm", HME_CUDA(cudaLaunchKernelEx(&cfg, limb_gemm_kernel<L, BN, KB>, tmA, tmB, g)));
+        // one k-block: B stays in shared memory down a column of tiles
+        if (k <= static_cast<uint32_t>(KB))
+            HME_TIMED(ctx, "limb_gemm", HME_CUDA(cudaLaunchKernelEx(&cfg, limb_gemm_short_kernel<L, BN, KB>, tmA, tmB, g)));
+        else
+            HME_TIMED(ctx, "limb_gemm", HME_CUDA(cudaLaunchKernelEx(&cfg, limb_gemm_kernel<L, BN, KB>, tmA, tmB, g)));
     }
 }
 
@@ -723,8 +553,6 @@ void noalloc_gemm(const NoAllocDevice& d, cudaStream_t st, const ModParams& mp, 
     g.ldc = ldc;
     g.M = static_cast<int>(m);
     g.N = static_cast<int>(n);
-    g.p = mp.p;
-    g.barrett = mp.barrett;
     g.tiles_m = static_cast<int>((m + kBM - 1) / kBM);
     g.tiles_n = static_cast<int>((n + BN - 1) / BN);
     g.group_m = 16;
@@ -736,7 +564,8 @@ void noalloc_gemm(const NoAllocDevice& d, cudaStream_t st, const ModParams& mp, 
         g.k_begin = static_cast<int>(kb0);
         g.kblocks = static_cast<int>((kc + kBK - 1) / kBK);
         g.op = kb0 == 0 ? op : (op == HME_SET ? HME_ADD : op);
-        limb_gemm_kernel<L, BN><<<grid, kThreads, CF::SMEM, st>>>(tmA, tmB, g);
+        g.red = make_epi(mp, kc);
+        limb_gemm_kernel<L, BN><<<grid, gemm_threads(L), CF::SMEM, st>>>(tmA, tmB, g);
         HME_CUDA(cudaGetLastError());
     }
 }
