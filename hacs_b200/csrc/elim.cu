@@ -9,31 +9,30 @@
 // anyway (leftmost column with a non-zero in the Schur complement, topmost such
 // row) because it is also the cheapest to find in parallel (a min over rows).
 //
-// Blocked right-looking LU, panels of `bw` columns.  Over a field the panel
-// first takes the top-block path (panel_block_kernel, panel_binv_kernel,
-// panel_w_kernel; the reasoning is at their definitions): when the panel's top
-// bw rows factor with non-zero diagonal entries they are its pivots, no search
-// runs, no row moves, and steps 2-4 below collapse into one limb GEMM
-// [A12; A22] += [L^-1 - I; -A21 B^-1] A12.  Otherwise:
-//   1. panel_cluster_kernel: the panel's active rows A[r0:m, c0:c0+bw) sit in
-//      the shared memory of one thread-block cluster (up to 16 CTAs); per
-//      column each CTA pushes its best (valuation, row) key and that row to
-//      every CTA through distributed shared memory, one cluster barrier, a
-//      warp min of the keys; fraction-free row updates, unit scales undone
-//      once per panel.  Panels too tall for one cluster take
-//      panel_factor_kernel instead: one cooperative launch over all SMs with
-//      one bounded grid barrier per column.  Either way pivot rows are not
-//      swapped during the panel (they leave the active set) and multipliers
-//      are stored in the pivot columns of the active rows (packed L).
-//   2. the panel's pivot rows move to rows r0 .. r0+k-1 in pivot order (columns
-//      >= c0; columns left of the panel of non-U rows hold dead multipliers).
-//   3. U12 = L11^-1 A12 in place: trsm_unit_lower_kernel, one warp per column
-//      of A12 holding its k rows in registers (forward substitution with
-//      shuffles), L11 in shared memory.
-//   4. A22 -= L21 * U12: the INT8-limb tcgen05 GEMM (Sub), K = k pivots.
+// Blocked right-looking LU, panels of `bw` columns:
+//   1. the panel's pivots.  First the top-block path (panel_block_kernel): one
+//      CTA eliminates the panel's top rows alone, which settles the panel when
+//      they supply a unit for every column.  Otherwise the searching kernel:
+//      panel_cluster_kernel, the panel's active rows A[r0:m, c0:c0+bw) in the
+//      shared memory of one thread-block cluster (up to 16 CTAs); per column
+//      each CTA pushes its best (valuation, row) key and that row to every CTA
+//      through distributed shared memory, one cluster barrier, a warp min of
+//      the keys; fraction-free row updates, unit scales undone once per panel.
+//      Panels too tall for one cluster take panel_factor_kernel: one
+//      cooperative launch over all SMs with one bounded grid barrier per column.
+//   2. move_pivot_rows_kernel: the pivot rows to rows r0 .. r0+k-1 in pivot
+//      order, the rows they displace into their places (columns >= c0; columns
+//      left of the panel of non-U rows hold dead multipliers).
+//   3. the left factor W = [L^-1 - I; -X M] (panel_w_kernel): X the other rows'
+//      entries at the pivot columns, M = B^-1 after the top block, L11^-1
+//      (panel_linv_kernel) after a search.
+//   4. [A12; A22] += W A12: one INT8-limb tcgen05 GEMM, K = k pivots; the top
+//      rows become U12, the rest the Schur complement.
+// A panel without a pivot asks whether anything is left below: a rank-deficient
+// matrix stops there.
 // Then RREF = U1^-1 U on the free columns only (the pivot columns of the RREF
 // are the identity): every diagonal block of U1 is inverted in shared memory
-// (one launch), and the blocked backward substitution is two limb GEMMs per
+// (one launch, tri_inv_kernel), and the blocked backward substitution is two limb GEMMs per
 // block (X_B = U_BB^-1 W_B, then W_above -= U_above,B X_B).
 #include <cuda_runtime.h>
 
@@ -42,6 +41,7 @@
 #include <cstring>
 #include <mutex>
 #include <numeric>
+#include <type_traits>
 #include <vector>
 
 #include "hme_elim.h"
@@ -520,6 +520,7 @@ __global__ void __launch_bounds__(NT, 1) panel_cluster_kernel(const PanelArgs a)
     extern __shared__ __align__(16) uint32_t s_dyn[];
     __shared__ uint32_t r_key[2][kClusterMax];               // pushed keys, by parity and sender
     __shared__ uint32_t r_row[2][kClusterMax][kMaxPanel];     // pushed candidate rows (from column c)
+    __shared__ uint32_t r_any[2][kClusterMax];                // pushed: the sender's active rows are not all zero
     __shared__ uint32_t s_cand[2];                            // this CTA's best key, by parity
     __shared__ uint32_t s_w[kMaxPanel];                       // unit part of each step's raw pivot
     __shared__ uint32_t s_inv[kMaxPanel];                     // its inverse
@@ -569,7 +570,11 @@ __global__ void __launch_bounds__(NT, 1) panel_cluster_kernel(const PanelArgs a)
 
     const uint32_t rkey_addr = smem_u32(&r_key[0][0]);
     const uint32_t rrow_addr = smem_u32(&r_row[0][0][0]);
+    const uint32_t rany_addr = smem_u32(&r_any[0][0]);
     int k = 0;
+    int empty = 0;  // pivotless columns in a row; at the 2nd, 6th, 14th, .. the rest of the panel is looked over
+    int look = 2;
+    uint32_t any = 1;  // this CTA's active rows are not known to be zero in the rest of the panel
     int pend_col = -1;  // ring mode: multiplier x / ell^v stored after the column's CTA barrier
     uint32_t pend_xp = 0;
     for (int it = 0; it < bw; ++it) {
@@ -584,7 +589,10 @@ __global__ void __launch_bounds__(NT, 1) panel_cluster_kernel(const PanelArgs a)
             if (warp < static_cast<int>(csize)) {
                 const uint32_t d = static_cast<uint32_t>(warp);
                 const uint32_t slot = par * kClusterMax + crank;
-                if (lane == 0) st_dsmem_u32(dsmem_addr(rkey_addr + 4u * slot, d), mine);
+                if (lane == 0) {
+                    st_dsmem_u32(dsmem_addr(rkey_addr + 4u * slot, d), mine);
+                    st_dsmem_u32(dsmem_addr(rany_addr + 4u * slot, d), any);
+                }
                 if (mine != kNoKey32) {
                     const int lm = static_cast<int>(mine & kKeyRowMask) - row_begin;
                     const uint32_t dst = dsmem_addr(rrow_addr + 4u * slot * kMaxPanel, d);
@@ -601,10 +609,18 @@ __global__ void __launch_bounds__(NT, 1) panel_cluster_kernel(const PanelArgs a)
         uint32_t key = kNoKey32;
         if (pkey == kNoKey32) {
             // no pivot in this column: every active row is unchanged; scan column it + 1
+            if (!__any_sync(0xffffffffu, lane < static_cast<int>(csize) && r_any[par][lane] != 0)) {
+                // all active rows are zero from here on (the same verdict in every CTA): no more pivots
+                for (int j = it + tid; j < bw; j += NT) s_colstep[j] = -1 - k;
+                break;
+            }
             if (tid == 0) s_colstep[it] = -1 - k;
+            ++empty;
             if (it + 1 < bw && has_row && sub == 0 && s_step[li] == 0)
                 key = pivot_key32(S[(it + 1) * rs + li], row_begin + li, a.R);
         } else {
+            empty = 0;
+            look = 2;
             const int owner = __ffs(__ballot_sync(0xffffffffu, kd == pkey)) - 1;
             const int prow = static_cast<int>(pkey & kKeyRowMask);
             const uint32_t v = pkey >> kKeyRowBits;
@@ -651,7 +667,16 @@ __global__ void __launch_bounds__(NT, 1) panel_cluster_kernel(const PanelArgs a)
         }
         key = __reduce_min_sync(0xffffffffu, key);
         if (lane == 0 && key != kNoKey32) atomicMin(&s_cand[par ^ 1], key);
-        __syncthreads();
+        if (empty == look) {  // the same in every thread of the cluster
+            look = 2 * look + 2;
+            uint32_t x = 0;
+            if (has_row && s_step[li] == 0)
+                for (int j = it + 1 + sub; j < bw; j += g) x |= S[j * rs + li];
+            any = __syncthreads_or(x != 0) ? 1u : 0u;
+        } else {
+            any = 1;
+            __syncthreads();
+        }
     }
     if (pend_col >= 0) S[pend_col * rs + li] = pend_xp;
 
@@ -677,20 +702,21 @@ __global__ void __launch_bounds__(NT, 1) panel_cluster_kernel(const PanelArgs a)
     if (crank == 0 && tid == 0) *a.k_out = k;
 }
 
-// ---- the top-block path of a field panel ---------------------------------------
-// At step t of a panel the pivot is the topmost active row with a non-zero in
-// column c0 + t.  If the first t steps took rows r0 .. r0+t-1, row r0 + t is
-// the topmost active row, so it is the pivot exactly when its entry (after the
-// first t steps) is non-zero -- and those entries depend only on the top
-// rows.  Hence: when the nb x w top block B = A[r0 : r0+nb, c0 : c0+w) (nb =
-// min(w, m - r0)) factors with non-zero diagonal entries, the panel's pivots
-// are (r0 + t, c0 + t), t < nb, the same as the search finds, with no row
-// moved.  The packed LU of the block is unique for that pivot sequence, and
-// the rest of the elimination step is one product:
-//   [A12; A22] += [L^-1 - I; -A21 B^-1] A12
-// gives U12 = L^-1 A12 in the top rows and the Schur complement A22 - A21 B^-1
-// A12 below (B = L U, nb = w whenever rows remain below).  When a diagonal
-// entry is zero, nothing is written and the searching kernel factors the panel.
+// ---- the top-block path -----------------------------------------------------------
+// A panel's pivots can be taken from its top rows alone whenever they supply
+// one for every column: a non-zero (over Z/ell^k a unit) entry of the Schur
+// complement is a valid pivot of its column wherever it lies, and the column
+// rank profile, the RREF and the Howell and Smith forms do not depend on the
+// rows chosen.  So one CTA eliminates the top nbr x w block (nbr a little more
+// than w where a column of a w-row block is likely to run out of units, so that
+// even F_2 panels practically always succeed), picking the topmost unit of each
+// column; with the nb = min(w, rows) pivot rows moved to the top, B the block
+// of their panel columns, the rest of the elimination step is one product:
+//   [A12; A22] += [B^-1 - I; -A21 B^-1] A12
+// gives B^-1 A12 in the top rows (whose panel columns become the identity) and
+// the Schur complement A22 - A21 B^-1 A12 below (nb = w whenever rows remain
+// below).  When a column has no unit in the block, nothing is written and the
+// searching kernel factors the panel.
 struct BlockArgs {
     uint32_t* A;
     uint64_t ld;
@@ -700,211 +726,399 @@ struct BlockArgs {
     int* pivot_cols;  // [w] out
     int* k_out;       // out
     int* ok;          // out: 1 when the top block settled the panel, else 0
-    uint32_t* lm;     // out: L's strict lower part, Montgomery form (nb x nb, row-major, zero elsewhere)
-    uint32_t* um;     // out: U's strict upper part, Montgomery form (nb x nb, row-major, zero elsewhere)
-    uint32_t* dm;     // out: U's inverse diagonal, Montgomery form (nb)
+    uint32_t* binv;   // out: B^-1 (nb x nb, row-major)
+    uint32_t* diag;   // out when non-null: the classical pivots, at r0 ..
 };
-constexpr int kBlockThreads = 512;
 
-__host__ __device__ constexpr int block_stride(int w) { return w | 1; }
-__host__ __device__ constexpr size_t block_smem_bytes(int nb, int w) {
-    return sizeof(uint32_t) * static_cast<size_t>(nb) * block_stride(w);  // T = B, nb x w
+// The padded size of an n x n triangular inverse: a power of two >= 8.
+__host__ __device__ constexpr int tri_pad(int n) {
+    int p = 8;
+    while (p < n) p *= 2;
+    return p;
+}
+__host__ __device__ constexpr int tri_stride(int p) { return p + 4; }  // rows 16-byte aligned
+constexpr int tri_words(int p) { return p * tri_stride(p); }
+
+// In place, X_i <- X_i^-1 mod q for `nmat` unit lower triangular P x P matrices
+// in shared memory (P a power of two >= 8, matrix i at X + i * mstride, row
+// stride tri_stride(P), zeros above the diagonal, identity padding).  8 x 8
+// diagonal blocks by forward substitution (a thread per column), then doubling:
+//   [A 0; C B]^-1 = [A^-1 0; -B^-1 (C A^-1) B^-1],
+// every entry an exact 96-bit dot product reduced once, so the chain is
+// 8 + 2 log2(P/8) dependent dot products instead of P elimination steps.
+// tmp: nmat * P * P / 4 words.  Called by every thread of the CTA; ends with a
+// barrier.
+__device__ __forceinline__ uint32_t reduce96(uint32_t a0, uint32_t a1, uint32_t a2, uint32_t q, uint64_t barrett) {
+    const uint32_t h = reduce_u64((static_cast<uint64_t>(a2) << 32) | a1, q, barrett);
+    return reduce_u64((static_cast<uint64_t>(h) << 32) | a0, q, barrett);
 }
 
-// x * y with y in the Montgomery form (y 2^32 mod q) for odd q: one Montgomery
-// reduction gives x y mod q; plain products for q = 2^k.
-template <int ARITH>
-__device__ __forceinline__ uint32_t mul_mform(uint32_t x, uint32_t ym, const Ring& R) {
-    if constexpr (ARITH == kArithPow2) return (x * ym) & (R.q - 1u);
-    else return mont_mul(x, ym, R.q, R.mont_qinv);
-}
-
-// x -> its Montgomery form x 2^32 mod q (unchanged for q = 2^k)
-template <int ARITH>
-__device__ __forceinline__ uint32_t to_mform(uint32_t x, const Ring& R) {
-    if constexpr (ARITH == kArithPow2) return x;
-    else return mont_mul(x, R.mont_r2, R.q, R.mont_qinv);
-}
-
-// One CTA: the fraction-free LU of the top block without a search (row t
-// pivots at step t), one CTA barrier per step.  Step t touches only the
-// active block (rows t+1 .. nb-1, columns t+1 .. w-1): warps over rows, lanes
-// over columns, each row's operands loaded before its updates are computed.
-// The classical values are restored as in the cluster kernel and written
-// back; L, U and U's inverse diagonal go out in Montgomery form for the row
-// solves of panel_binv_kernel.  WMAX (64 or 128) bounds w.
-template <int ARITH, int WMAX>
-__global__ void __launch_bounds__(kBlockThreads) panel_block_kernel(const BlockArgs a) {
-    extern __shared__ __align__(16) uint32_t s_blk[];
-    __shared__ uint32_t s_w[kMaxPanel], s_inv[kMaxPanel], s_sinv[kMaxPanel + 1];
-    const int w = a.w, nb = min(w, a.m - a.r0), ts = block_stride(w);
-    uint32_t* T = s_blk;  // [nb][ts]
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int NW = kBlockThreads / 32;
-    constexpr int CW = WMAX / 32;  // column slots per lane
-    constexpr int RI = WMAX / NW;  // row slots per warp
-    for (int r = warp; r < nb; r += NW) {
-        const uint32_t* src = a.A + static_cast<size_t>(a.r0 + r) * a.ld + a.c0;
+__device__ void unit_lower_inverse(uint32_t* X, int P, int nmat, int mstride, uint32_t* tmp, uint32_t q,
+                                   uint64_t barrett) {
+    const int ls = tri_stride(P);
+    for (int base = 0; base < nmat * P; base += blockDim.x) {
+        const int idx = base + threadIdx.x;
+        const bool valid = idx < nmat * P;
+        const int mi = valid ? idx / P : 0, c = valid ? idx - mi * P : 0, cc = c & 7;
+        uint32_t* M = X + mi * mstride + (c - cc) * (ls + 1);
+        uint32_t x[8];
 #pragma unroll
-        for (int c = 0; c < CW; ++c) {
-            const int j = lane + 32 * c;
-            if (j < w) T[r * ts + j] = src[j];
+        for (int r = 0; r < 8; ++r) {
+            uint32_t a0 = 0, a1 = 0, a2 = 0;
+#pragma unroll
+            for (int s = 0; s < r; ++s) mac96(a0, a1, a2, M[r * ls + s], x[s]);
+            const uint32_t v = reduce96(a0, a1, a2, q, barrett);
+            x[r] = r == cc ? 1u : v == 0 || r < cc ? 0u : q - v;
         }
+        __syncwarp();  // the eight columns of a block belong to eight lanes of one warp: all have read it
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+            if (valid && r >= cc) M[r * ls + cc] = x[r];
     }
     __syncthreads();
-    bool fail = false;
-    for (int t = 0; t < nb; ++t) {
-        const uint32_t wt = T[t * ts + t];
-        // the pivot must be a unit (over a field: non-zero); the same value in every thread: uniform
-        if (wt == 0 || (a.R.k > 1 && wt % a.R.ell == 0)) {
-            fail = true;
-            break;
+    for (int h = 8; h < P; h *= 2) {
+        const int lh = __ffs(h) - 1, pairs = P >> (lh + 1);
+        const int total = nmat * pairs * h * h;
+        // tmp = C A^-1
+        for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
+            const int c = idx & (h - 1), r = (idx >> lh) & (h - 1), pr = idx >> (2 * lh);
+            const int mi = pr / pairs, b0 = (pr - mi * pairs) * 2 * h;
+            const uint32_t* Ai = X + mi * mstride + b0 * ls + b0;
+            const uint32_t* Cr = Ai + (h + r) * ls;
+            const uint32_t* Ac = Ai + c;
+            uint32_t a0 = 0, a1 = 0, a2 = 0;
+#pragma unroll 4
+            for (int s = 0; s < h; ++s) mac96(a0, a1, a2, Cr[s], Ac[s * ls]);
+            tmp[idx] = reduce96(a0, a1, a2, q, barrett);
         }
-        if (tid == 0) s_w[t] = wt;
-        const int jb = t + 1;
-        uint32_t pr[CW];
-#pragma unroll
-        for (int c = 0; c < CW; ++c) {
-            const int j = jb + lane + 32 * c;
-            pr[c] = j < w ? T[t * ts + j] : 0u;
-        }
-#pragma unroll
-        for (int i = 0; i < RI; ++i) {
-            const int r = jb + warp + NW * i;
-            if (r >= nb) break;  // uniform in the warp
-            const uint32_t xn = ff_negate<ARITH>(T[r * ts + t], a.R);
-            uint32_t y[CW];
-#pragma unroll
-            for (int c = 0; c < CW; ++c) {
-                const int j = jb + lane + 32 * c;
-                y[c] = j < w ? T[r * ts + j] : 0u;
-            }
-#pragma unroll
-            for (int c = 0; c < CW; ++c) y[c] = ff_update<ARITH>(wt, y[c], xn, pr[c], a.R);
-#pragma unroll
-            for (int c = 0; c < CW; ++c) {
-                const int j = jb + lane + 32 * c;
-                if (j < w) T[r * ts + j] = y[c];
-            }
+        __syncthreads();
+        // C = -B^-1 tmp
+        for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
+            const int c = idx & (h - 1), r = (idx >> lh) & (h - 1), pr = idx >> (2 * lh);
+            const int mi = pr / pairs, b0 = (pr - mi * pairs) * 2 * h;
+            uint32_t* A0 = X + mi * mstride + b0 * ls + b0;
+            const uint32_t* Bi = A0 + (h + r) * ls + h;
+            const uint32_t* tp = tmp + (pr << (2 * lh)) + c;
+            uint32_t a0 = 0, a1 = 0, a2 = 0;
+#pragma unroll 4
+            for (int s = 0; s < h; ++s) mac96(a0, a1, a2, Bi[s], tp[s << lh]);
+            const uint32_t v = reduce96(a0, a1, a2, q, barrett);
+            A0[(h + r) * ls + c] = v == 0 ? 0u : q - v;
         }
         __syncthreads();
     }
-    if (fail) {
-        if (tid == 0) *a.ok = 0;
-        return;
+}
+
+constexpr int kSubCols = 16;  // columns of a sub-panel
+
+// Row stride of the block in words: whole 16-byte pieces, an odd number of
+// them, so that eight lanes reading the same piece of eight rows hit 32 banks.
+__host__ __device__ constexpr int block_stride(int w) {
+    return (((w + 3) / 4) & 1) ? (w + 3) / 4 * 4 : (w + 3) / 4 * 4 + 4;
+}
+__host__ __device__ constexpr size_t block_smem_bytes(int rs, int w) {
+    return sizeof(uint32_t) * static_cast<size_t>(rs + kSubCols) * block_stride(w);
+}
+
+// (w y + xn pr) rho on the four words of a piece
+template <int ARITH>
+__device__ __forceinline__ uint4 ff_update4(uint32_t w, uint4 y, uint32_t xn, uint4 pr, const Ring& R) {
+    return make_uint4(ff_update<ARITH>(w, y.x, xn, pr.x, R), ff_update<ARITH>(w, y.y, xn, pr.y, R),
+                      ff_update<ARITH>(w, y.z, xn, pr.z, R), ff_update<ARITH>(w, y.w, xn, pr.w, R));
+}
+// A sum of at most 17 products below q^2, reduced: two Montgomery steps (the
+// sum times rho^2) for odd q, the truncation for q = 2^k.  The first step
+// leaves at most 9.5 q + 1, the second at most q.
+template <int ARITH>
+__device__ __forceinline__ uint32_t ff_reduce96(uint32_t a0, uint32_t a1, uint32_t a2, const Ring& R) {
+    if constexpr (ARITH == kArithPow2) {
+        return a0 & (R.q - 1u);
+    } else {
+        uint32_t m = a0 * R.mont_qinv;
+        // (a2:a1:a0 + m q) / 2^32: the low words cancel, with a carry unless both are zero
+        uint64_t v = (static_cast<uint64_t>(a2) << 32 | a1) + __umulhi(m, R.q) + (a0 != 0 ? 1u : 0u);
+        m = static_cast<uint32_t>(v) * R.mont_qinv;
+        v = (v >> 32) + __umulhi(m, R.q) + (static_cast<uint32_t>(v) != 0 ? 1u : 0u);
+        return static_cast<uint32_t>(v >= R.q ? v - R.q : v);
     }
-    if (tid < nb) s_w[tid] = T[tid * ts + tid];
+}
+
+// x y rho^2 (x y for q = 2^k)
+template <int ARITH>
+__device__ __forceinline__ uint32_t ff_scale2(uint32_t x, uint32_t y, const Ring& R) {
+    if constexpr (ARITH == kArithPow2) return (x * y) & (R.q - 1u);
+    else return mont_mul(mont_mul(x, y, R.q, R.mont_qinv), 1u, R.q, R.mont_qinv);
+}
+
+// One CTA of 4 RS threads, RS row slots: blocked in-place Gauss-Jordan
+// inversion of the block with the pivot search, in sub-panels of 16 columns.
+// The block sits in shared memory row-major; lanes over rows, four thread
+// groups over 16-byte pieces of the rows.
+//
+// Steps of a sub-panel touch its 16 columns only (a piece per thread, kept in
+// registers): step t takes the topmost unpivoted row with a unit in column t
+// and updates every other row, pivoted or not, fraction-free as in the cluster
+// kernel: row <- (w row - x pivot row) rho; one CTA barrier per step (column
+// t + 1's entries and candidates leave step t through s_x and s_cand).  Column t
+// then holds the column of the inverse that belongs to the pivot row: before
+// the step that column is S_t (the rows' common scale, S_0 = 1, S_t+1 = S_t w_t
+// rho) in the pivot row and 0 elsewhere.  After n steps pivot row t holds S_n /
+// (S_t rho) times its row of the sub-panel's inverse.  With V the scale of the
+// block before the sub-panel (V_0 = 1, V <- V S_n rho^2), the pivot rows take a
+// product by S_t V rho; C (rows x 16) is then S_n times the left factor of the
+// sub-panel's update (V S_n times it in the pivot rows, whose block carries a
+// V^-1), and the other columns take
+//   y <- (S_n y [row not a pivot of this sub-panel] + sum_t C_t P_t) rho^2
+// with the pivot rows' values P from before the sub-panel: 16 products per
+// entry reduced once instead of 16 reduced updates.  The sub-panel's own
+// columns, columns of the inverse, are multiplied by V rho^2.  At the end every entry is V times its value: one modular inverse for
+// the whole block.
+//
+// Bound by the chain of w steps and by the multiplier (a reduced update is
+// three wide products).  A 64-column panel mod 2^31 - 19: 43 + 20 us as one
+// CTA's LU and row solves over the GPU, 49 us as 64 whole-row steps, 41 us so;
+// mod 13 (96 slots) 46 us, where the cluster search of 10515 rows took 200 to 270.
+template <int ARITH, int RS>
+__global__ void __launch_bounds__(4 * RS) panel_block_kernel(const BlockArgs a) {
+    extern __shared__ __align__(16) uint32_t s_blk[];
+    __shared__ uint32_t s_w[kMaxPanel], s_S[kMaxPanel], s_V[kMaxPanel / kSubCols + 1];
+    __shared__ uint32_t s_x[2][RS];  // the rows' entries in the step's column, by parity
+    __shared__ int s_prow[kMaxPanel];
+    __shared__ int s_cand[2][RS / 32];
+    constexpr int NT = 4 * RS, NW = NT / 32;
+    constexpr int WC = RS == 128 ? 4 : 2;  // panels of up to 128 or 64 columns: 32 WC
+    const int w = a.w, rows = a.m - a.r0, nb = min(w, rows), nbr = min(RS, rows);
+    const Ring& R = a.R;
+    const int ls = block_stride(w), nq = (w + 3) / 4;
+    uint32_t* T = s_blk;             // [RS][ls]
+    uint32_t* P = s_blk + RS * ls;   // [16][ls]: a sub-panel's pivot rows before it
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int li = tid % RS, g = tid / RS, wg = warp % (RS / 32);
+    {
+        // the block's rows, all of a thread's loads in flight at once
+        uint32_t v[RS / NW][WC];
+#pragma unroll
+        for (int i = 0; i < RS / NW; ++i) {
+            const int r = warp + NW * i;
+            const uint32_t* src = a.A + static_cast<size_t>(a.r0 + min(r, nbr - 1)) * a.ld + a.c0;
+#pragma unroll
+            for (int c = 0; c < WC; ++c) v[i][c] = lane + 32 * c < w ? src[lane + 32 * c] : 0u;
+        }
+#pragma unroll
+        for (int i = 0; i < RS / NW; ++i)
+#pragma unroll
+            for (int c = 0; c < WC; ++c)
+                if (lane + 32 * c < 4 * nq) T[(warp + NW * i) * ls + lane + 32 * c] = v[i][c];
+    }
     __syncthreads();
-    ff_scale_tables<ARITH>(nb, s_w, s_inv, s_sinv, a.R);
-    // row r froze at step r: a multiplier of step j < r takes w_j^-1, the rest (U) S_r^-1
-    for (int r = warp; r < nb; r += NW) {
-        uint32_t* dst = a.A + static_cast<size_t>(a.r0 + r) * a.ld + a.c0;
-        for (int j = lane; j < w; j += 32) {
-            const uint32_t v = mod_mul(T[r * ts + j], j < r ? s_inv[j] : s_sinv[r], a.R.q, a.R.barrett);
-            dst[j] = v;
-            if (j < nb) {
-                a.lm[static_cast<size_t>(r) * nb + j] = j < r ? to_mform<ARITH>(v, a.R) : 0u;
-                a.um[static_cast<size_t>(r) * nb + j] = j > r ? to_mform<ARITH>(v, a.R) : 0u;
+    auto is_unit = [&](uint32_t x) { return x != 0 && (R.k == 1 || x % R.ell != 0); };
+    const bool in = li < nbr;
+    bool pivoted = !in;
+    uint32_t* row = T + li * ls;
+    uint32_t V = 1u;
+    for (int cs = 0, sub = 0; cs < nb; cs += kSubCols, ++sub) {
+        const int ns = min(kSubCols, nb - cs);  // steps of this sub-panel
+        const int q0 = cs >> 2, q1 = (cs + ns + 3) >> 2;  // its pieces
+        const int qg = q0 + g;                  // this thread's piece of it
+        const bool live = qg < q1;
+        uint4 y = live ? *reinterpret_cast<const uint4*>(row + 4 * qg) : make_uint4(0, 0, 0, 0);
+        if (g == 0) {
+            s_x[0][li] = y.x;
+            const unsigned mask = __ballot_sync(0xffffffffu, !pivoted && is_unit(y.x));
+            if (lane == 0) s_cand[0][wg] = mask ? 32 * wg + __ffs(mask) - 1 : RS;
+        }
+        uint32_t S = 1u;
+        int mine = -1;  // the step of this sub-panel whose pivot is this thread's row
+        __syncthreads();
+        // step 4 u + C; false when its column has no unit in the block (the same in every thread)
+        auto step = [&](auto cc, int u) -> bool {
+            constexpr int C = decltype(cc)::value;
+            constexpr int par = C & 1;
+            const int t = cs + 4 * u + C;
+            int prow = s_cand[par][0];
+#pragma unroll
+            for (int v = 1; v < RS / 32; ++v) prow = min(prow, s_cand[par][v]);
+            if (prow == RS) return false;
+            uint4 p4 = *reinterpret_cast<const uint4*>(T + prow * ls + 4 * min(qg, nq - 1));
+            const uint32_t wt = s_x[par][prow];
+            const uint32_t xn = ff_negate<ARITH>(s_x[par][li], R);
+            if (tid == 0) {
+                s_w[t] = wt;
+                s_S[t] = S;
+                s_prow[t] = prow;
             }
-            if (j == r) T[r * ts + r] = v;  // the classical diagonal, for its inverse below
+            const bool is_pivot = li == prow;
+            if (is_pivot) {
+                pivoted = true;
+                mine = 4 * u + C;
+            }
+            if (u == g) {  // column t: 0 in the other rows, S in the pivot row (nobody reads that word in this step)
+                (C == 0 ? p4.x : C == 1 ? p4.y : C == 2 ? p4.z : p4.w) = S;
+                (C == 0 ? y.x : C == 1 ? y.y : C == 2 ? y.z : y.w) = is_pivot ? S : 0u;
+            }
+            const uint4 z = ff_update4<ARITH>(wt, y, xn, p4, R);
+            if (!is_pivot) y = z;
+            if (live) *reinterpret_cast<uint4*>(row + 4 * qg) = y;
+            if ((C == 3 ? u + 1 : u) == g) {  // the group of column t + 1
+                const uint32_t next = C == 0 ? y.y : C == 1 ? y.z : C == 2 ? y.w : y.x;
+                s_x[par ^ 1][li] = next;
+                const unsigned mask = __ballot_sync(0xffffffffu, !pivoted && is_unit(next));
+                if (lane == 0) s_cand[par ^ 1][wg] = mask ? 32 * wg + __ffs(mask) - 1 : RS;
+            }
+            S = ARITH == kArithPow2 ? (S * wt) & (R.q - 1u) : mont_mul(S, wt, R.q, R.mont_qinv);
+            __syncthreads();
+            return true;
+        };
+        bool ok = true;
+        for (int u = 0; ok && 4 * u < ns; ++u) {
+            ok = step(std::integral_constant<int, 0>{}, u);
+            if (ok && 4 * u + 1 < ns) ok = step(std::integral_constant<int, 1>{}, u);
+            if (ok && 4 * u + 2 < ns) ok = step(std::integral_constant<int, 2>{}, u);
+            if (ok && 4 * u + 3 < ns) ok = step(std::integral_constant<int, 3>{}, u);
+        }
+        if (!ok) {
+            if (tid == 0) *a.ok = 0;
+            return;
+        }
+        if (tid == 0) s_V[sub] = V;
+        // C of the pivot rows to the common scale, and the pivot rows' other pieces aside
+        if (mine >= 0) {
+            const uint32_t f = mod_mul(s_S[cs + mine], V, R.q, R.barrett);
+            if (live) {
+                auto sc = [&](uint32_t x) { return ARITH == kArithPow2 ? (x * f) & (R.q - 1u) : mont_mul(x, f, R.q, R.mont_qinv); };
+                y = make_uint4(sc(y.x), sc(y.y), sc(y.z), sc(y.w));
+                *reinterpret_cast<uint4*>(row + 4 * qg) = y;
+            }
+            for (int q = g; q < nq; q += 4)
+                if (q < q0 || q >= q1)
+                    *reinterpret_cast<uint4*>(P + mine * ls + 4 * q) = *reinterpret_cast<const uint4*>(row + 4 * q);
+        }
+        __syncthreads();
+        uint32_t c[kSubCols];
+#pragma unroll
+        for (int i = 0; i < kSubCols / 4; ++i) {
+            const uint4 v = 4 * i < ns ? *reinterpret_cast<const uint4*>(row + cs + 4 * i) : make_uint4(0, 0, 0, 0);
+            c[4 * i] = v.x;
+            c[4 * i + 1] = 4 * i + 1 < ns ? v.y : 0u;
+            c[4 * i + 2] = 4 * i + 2 < ns ? v.z : 0u;
+            c[4 * i + 3] = 4 * i + 3 < ns ? v.w : 0u;
+        }
+        __syncthreads();  // the sub-panel's own columns change below
+        if (in) {
+            if (live) {
+                // (columns of the last piece beyond the pivots, where the block has fewer rows than
+                // columns, have that scale already)
+                const int left = cs + ns - 4 * qg;
+                y = make_uint4(ff_scale2<ARITH>(y.x, V, R), ff_scale2<ARITH>(y.y, left > 1 ? V : 1u, R),
+                               ff_scale2<ARITH>(y.z, left > 2 ? V : 1u, R), ff_scale2<ARITH>(y.w, left > 3 ? V : 1u, R));
+                *reinterpret_cast<uint4*>(row + 4 * qg) = y;
+            }
+            const uint32_t sy = mine >= 0 ? 0u : S;
+            for (int q = g; q < nq; q += 4) {
+                if (q >= q0 && q < q1) continue;
+                uint4 v = *reinterpret_cast<const uint4*>(row + 4 * q);
+                uint32_t* vw = reinterpret_cast<uint32_t*>(&v);
+                uint32_t a0[4], a1[4], a2[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const uint64_t t = static_cast<uint64_t>(sy) * vw[e];
+                    a0[e] = static_cast<uint32_t>(t);
+                    a1[e] = static_cast<uint32_t>(t >> 32);
+                    a2[e] = 0;
+                }
+                const uint32_t* pq = P + 4 * q;
+#pragma unroll
+                for (int i = 0; i < kSubCols; i += 4) {
+                    if (i >= ns) break;
+                    uint4 p[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) p[e] = *reinterpret_cast<const uint4*>(pq + min(i + e, ns - 1) * ls);
+                    if constexpr (ARITH == kArithMont32) {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            mac96(a0[0], a1[0], a2[0], c[i + e], p[e].x);
+                            mac96(a0[1], a1[1], a2[1], c[i + e], p[e].y);
+                            mac96(a0[2], a1[2], a2[2], c[i + e], p[e].z);
+                            mac96(a0[3], a1[3], a2[3], c[i + e], p[e].w);
+                        }
+                    } else if constexpr (ARITH == kArithPow2) {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            a0[0] += c[i + e] * p[e].x;
+                            a0[1] += c[i + e] * p[e].y;
+                            a0[2] += c[i + e] * p[e].z;
+                            a0[3] += c[i + e] * p[e].w;
+                        }
+                    } else {
+                        add96(a0[0], a1[0], a2[0], dot4(c[i], p[0].x, c[i + 1], p[1].x, c[i + 2], p[2].x, c[i + 3], p[3].x));
+                        add96(a0[1], a1[1], a2[1], dot4(c[i], p[0].y, c[i + 1], p[1].y, c[i + 2], p[2].y, c[i + 3], p[3].y));
+                        add96(a0[2], a1[2], a2[2], dot4(c[i], p[0].z, c[i + 1], p[1].z, c[i + 2], p[2].z, c[i + 3], p[3].z));
+                        add96(a0[3], a1[3], a2[3], dot4(c[i], p[0].w, c[i + 1], p[1].w, c[i + 2], p[2].w, c[i + 3], p[3].w));
+                    }
+                }
+                v = make_uint4(ff_reduce96<ARITH>(a0[0], a1[0], a2[0], R), ff_reduce96<ARITH>(a0[1], a1[1], a2[1], R),
+                               ff_reduce96<ARITH>(a0[2], a1[2], a2[2], R), ff_reduce96<ARITH>(a0[3], a1[3], a2[3], R));
+                *reinterpret_cast<uint4*>(row + 4 * q) = v;
+            }
+        }
+        V = ff_scale2<ARITH>(V, S, R);
+        __syncthreads();
+    }
+    const uint32_t vinv = unit_inverse(V, R);
+    for (int t = warp; t < nb; t += NW) {
+        const int pl = s_prow[t];
+        uint32_t* dst = a.A + static_cast<size_t>(a.r0 + pl) * a.ld + a.c0;
+        for (int j = lane; j < w; j += 32) {
+            const uint32_t v = mod_mul(T[pl * ls + j], vinv, R.q, R.barrett);
+            if (j < nb) a.binv[t * nb + j] = v;
+            dst[j] = j >= nb ? v : j == t ? 1u : 0u;
         }
     }
     if (tid < nb) {
-        a.pivot_rows[tid] = a.r0 + tid;
+        a.pivot_rows[tid] = a.r0 + s_prow[tid];
         a.pivot_cols[tid] = a.c0 + tid;
+        // the classical pivots, for the determinant: w_t / (S_t V)
+        if (a.diag) {
+            const uint32_t s = mod_mul(s_S[tid], s_V[tid / kSubCols], R.q, R.barrett);
+            a.diag[a.r0 + tid] = mod_mul(s_w[tid], unit_inverse(s, R), R.q, R.barrett);
+        }
     }
-    __syncthreads();
-    if (tid < nb) a.dm[tid] = to_mform<ARITH>(unit_inverse(T[tid * ts + tid], a.R), a.R);
     if (tid == 0) {
         *a.k_out = nb;
         *a.ok = 1;
     }
 }
 
-// Row solves against the factored top block, one warp per row, lanes over
-// columns: the forward solve y U = v (y_s = (v_s - sum_{t<s} y_t U[t][s]) /
-// U[s][s]) and the backward solve z L = y (z_i = y_i - sum_{t>i} z_t L[t][i],
-// unit diagonal).  L, U and U's inverse diagonal come in Montgomery form, so
-// each product is one Montgomery reduction.  panel_binv_kernel runs 2 nb of
-// them: row r of B^-1 = e_r U^-1 L^-1 (when rows remain below the block) and
-// row t of L^-1 (stored as L^-1 - I, the top rows of the update's left
-// factor).  Nothing runs unless the top block settled the panel.
-constexpr int kSolveWarps = 4;
-
-template <int ARITH, int WMAX>
-__global__ void __launch_bounds__(32 * kSolveWarps) panel_binv_kernel(const uint32_t* __restrict__ lm,
-                                                                       const uint32_t* __restrict__ um,
-                                                                       const uint32_t* __restrict__ dm, int nb,
-                                                                       int with_binv, const Ring R,
-                                                                       const int* __restrict__ ok,
-                                                                       uint32_t* __restrict__ binv,
-                                                                       uint32_t* __restrict__ linv) {
-    if (*ok == 0) return;
-    extern __shared__ __align__(16) uint32_t s_sv[];
-    uint32_t* Ls = s_sv;                                                      // [nb][nb]
-    uint32_t* Us = s_sv + ((static_cast<size_t>(nb) * nb + 3) & ~size_t(3));  // [nb][nb]
-    __shared__ uint32_t s_dm[kMaxPanel];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int CS = WMAX / 32;
-    for (int idx = tid; idx < nb * nb; idx += 32 * kSolveWarps) {
-        Ls[idx] = lm[idx];
-        if (with_binv) Us[idx] = um[idx];
+// After a searched panel (its packed LU in place, the pivot rows moved to r0 ..
+// r0 + k - 1): L11^-1 of the k pivot rows at the pivot columns, the factor the
+// update takes in place of the top block's.
+__global__ void __launch_bounds__(512) panel_linv_kernel(const uint32_t* __restrict__ A, uint64_t ld, int r0,
+                                                         const int* __restrict__ pcols, int k, uint32_t q,
+                                                         uint64_t barrett, uint32_t* __restrict__ linv) {
+    extern __shared__ __align__(16) uint32_t s_li[];
+    const int P = tri_pad(k), ls = tri_stride(P), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int s = lane; s < P; s += 32) {
+        const int pc = s < k ? pcols[s] : 0;
+#pragma unroll 8
+        for (int t = warp; t < P; t += 16)
+            s_li[t * ls + s] = t == s ? 1u : t < k && s < t ? A[static_cast<size_t>(r0 + t) * ld + pc] : 0u;
     }
-    for (int t = tid; t < nb; t += 32 * kSolveWarps) s_dm[t] = dm[t];
     __syncthreads();
-    const int v = static_cast<int>(blockIdx.x) * kSolveWarps + warp;  // virtual row
-    const bool is_binv = v < nb;
-    const int r = is_binv ? v : v - nb;
-    if (r >= nb || (is_binv && !with_binv)) return;  // uniform in the warp; no barrier follows
-    const uint32_t one = 1u % R.q;
-    uint32_t a[CS];
-#pragma unroll
-    for (int c = 0; c < CS; ++c) a[c] = lane + 32 * c == r ? one : 0u;
-    if (is_binv) {
-        // forward solve from e_r: y_s = 0 for s < r
-#pragma unroll
-        for (int sc = 0; sc < CS; ++sc) {
-            for (int sl = 0; sl < 32; ++sl) {
-                const int s = 32 * sc + sl;
-                if (s >= nb) break;
-                if (s < r) continue;
-                const uint32_t ys = mul_mform<ARITH>(__shfl_sync(0xffffffffu, a[sc], sl), s_dm[s], R);
-                if (lane == sl) a[sc] = ys;
-#pragma unroll
-                for (int c = sc; c < CS; ++c) {
-                    const int j = lane + 32 * c;
-                    const uint32_t u = j > s && j < nb ? Us[s * nb + j] : 0u;
-                    a[c] = mod_sub(a[c], mul_mform<ARITH>(ys, u, R), R.q);
-                }
-            }
-        }
+    unit_lower_inverse(s_li, P, 1, 0, s_li + tri_words(P), q, barrett);
+    for (int idx = threadIdx.x; idx < k * k; idx += blockDim.x) {
+        const int t = idx / k, s = idx - t * k;
+        linv[idx] = s_li[t * ls + s];
     }
-    // backward solve z L = y
-#pragma unroll
-    for (int sc = CS - 1; sc >= 0; --sc) {
-        for (int sl = 31; sl >= 0; --sl) {
-            const int t = 32 * sc + sl;
-            if (t >= nb || t == 0) continue;
-            const uint32_t zt = __shfl_sync(0xffffffffu, a[sc], sl);
-#pragma unroll
-            for (int c = 0; c <= sc; ++c) {
-                const int j = lane + 32 * c;
-                const uint32_t l = j < t ? Ls[t * nb + j] : 0u;
-                a[c] = mod_sub(a[c], mul_mform<ARITH>(zt, l, R), R.q);
-            }
-        }
-    }
-    uint32_t* dst = (is_binv ? binv : linv) + static_cast<size_t>(r) * nb;
-#pragma unroll
-    for (int c = 0; c < CS; ++c) {
-        const int j = lane + 32 * c;
-        if (j < nb) dst[j] = !is_binv && j == r ? mod_sub(a[c], one, R.q) : a[c];
-    }
+}
+size_t linv_smem_bytes(int k) {
+    const size_t p = tri_pad(k);
+    return sizeof(uint32_t) * (tri_words(tri_pad(k)) + p * p / 4);
 }
 
 // The left factor of the fused update, W ((m - r0) x nb, row-major, ld nb):
-// rows t < nb are L^-1 - I (from panel_binv_kernel); a row x below the block
-// becomes -x B^-1 (x = the row's panel columns).  A warp takes four rows at
+// rows t < nb are M - I; a row x below becomes -x M, x = the row's entries at
+// the pivot columns: untouched values and M = B^-1 after the top block,
+// multipliers L21 and M = L11^-1 after a searched panel.  A warp takes four rows at
 // once, lanes over output columns; each dot product runs exactly in a 96-bit
 // carry chain (nb <= 128 products below 2^64) and is reduced once.
 constexpr int kWRows = 32;
@@ -912,8 +1126,7 @@ constexpr int kWRowsPerWarp = 4;
 
 template <int WMAX>
 __global__ void __launch_bounds__(256) panel_w_kernel(const uint32_t* __restrict__ A, uint64_t ld, int r0, int m,
-                                                      int c0, int nb, const uint32_t* __restrict__ linv,
-                                                      const uint32_t* __restrict__ binv, uint32_t q,
+                                                      const int* __restrict__ pcols, int nb, const uint32_t* __restrict__ binv, uint32_t q,
                                                       uint64_t barrett, uint32_t* __restrict__ W) {
     extern __shared__ __align__(16) uint32_t s_wk[];
     const int rb = r0 + static_cast<int>(blockIdx.x) * kWRows;  // first row of this CTA
@@ -922,16 +1135,19 @@ __global__ void __launch_bounds__(256) panel_w_kernel(const uint32_t* __restrict
     constexpr int NW = 256 / 32;
     static_assert(NW * kWRowsPerWarp == kWRows, "one pass of the warps covers the CTA's rows");
     constexpr int CS = WMAX / 32;
-    // the top rows: L^-1 - I
+    // the top rows: M - I
     for (int r = warp; r < nr; r += NW) {
         const int row = rb + r;
         if (row >= r0 + nb) break;
-        for (int j = lane; j < nb; j += 32)
-            W[static_cast<size_t>(row - r0) * nb + j] = linv[static_cast<size_t>(row - r0) * nb + j];
+        for (int j = lane; j < nb; j += 32) {
+            const size_t idx = static_cast<size_t>(row - r0) * nb + j;
+            W[idx] = j == row - r0 ? mod_sub(binv[idx], 1u, q) : binv[idx];
+        }
     }
     if (rb + nr <= r0 + nb) return;  // no row below the block in this CTA (uniform)
     uint32_t* Bi = s_wk;                                   // [nb][nb]
-    uint32_t* Xr = s_wk + ((static_cast<size_t>(nb) * nb + 3) & ~size_t(3));  // [kWRows][nb]
+    const int xs = (nb + 3) & ~3;                          // row stride of Xr: whole 16-byte pieces
+    uint32_t* Xr = s_wk + ((static_cast<size_t>(nb) * nb + 3) & ~size_t(3));  // [kWRows][xs]
     {
         // B^-1 in 16-byte pieces (its buffer is 16-byte aligned), four loads of a thread in flight
         const int n4 = (nb * nb) >> 2;
@@ -955,23 +1171,23 @@ __global__ void __launch_bounds__(256) panel_w_kernel(const uint32_t* __restrict
     const int rl = warp * kWRowsPerWarp;  // this warp's rows: rl .. rl + 3 of the CTA
     {
         uint32_t v[kWRowsPerWarp][CS];
+        int pc[CS];
+#pragma unroll
+        for (int c = 0; c < CS; ++c) pc[c] = lane + 32 * c < nb ? pcols[lane + 32 * c] : 0;
 #pragma unroll
         for (int i = 0; i < kWRowsPerWarp; ++i) {
             const int row = rb + rl + i;
             const bool below = rl + i < nr && row >= r0 + nb;
-            const uint32_t* src = A + static_cast<size_t>(below ? row : r0) * ld + c0;
+            const uint32_t* src = A + static_cast<size_t>(below ? row : r0) * ld;
 #pragma unroll
-            for (int c = 0; c < CS; ++c) {
-                const int j = lane + 32 * c;
-                v[i][c] = below && j < nb ? src[j] : 0u;
-            }
+            for (int c = 0; c < CS; ++c) v[i][c] = below && lane + 32 * c < nb ? src[pc[c]] : 0u;
         }
 #pragma unroll
         for (int i = 0; i < kWRowsPerWarp; ++i)
 #pragma unroll
             for (int c = 0; c < CS; ++c) {
                 const int j = lane + 32 * c;
-                if (j < nb) Xr[(rl + i) * nb + j] = v[i][c];
+                if (j < nb) Xr[(rl + i) * xs + j] = v[i][c];
             }
     }
     __syncthreads();
@@ -989,7 +1205,7 @@ __global__ void __launch_bounds__(256) panel_w_kernel(const uint32_t* __restrict
         }
 #pragma unroll
         for (int i = 0; i < kWRowsPerWarp; ++i) {
-            const uint32_t x = Xr[(rl + i) * nb + t];
+            const uint32_t x = Xr[(rl + i) * xs + t];
 #pragma unroll
             for (int c = 0; c < CS; ++c) mac96(a0[i][c], a1[i][c], a2[i][c], x, bt[c]);
         }
@@ -1011,24 +1227,100 @@ __global__ void __launch_bounds__(256) panel_w_kernel(const uint32_t* __restrict
     }
 }
 
-// ---- row permutation of columns [c0, n) for rows [r0, m) -------------------------
-// tmp[i'][j'] = A[perm[i']][c0 + j']
-__global__ void gather_rows_kernel(const uint32_t* __restrict__ A, uint64_t ld, const int* __restrict__ perm,
-                                   int rows, int c0, int cols, uint32_t* __restrict__ tmp) {
-    const size_t total = static_cast<size_t>(rows) * cols;
-    for (size_t idx = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; idx < total;
-         idx += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        const int i = static_cast<int>(idx / cols), j = static_cast<int>(idx % cols);
-        tmp[idx] = A[static_cast<size_t>(perm[i]) * ld + c0 + j];
+// ---- the pivot rows to the top -------------------------------------------------------
+// In columns [ca, cb): row r0 + t becomes the pivot row prow[t], t < k, and the
+// rows this displaces fill the pivot rows' old places below r0 + k in order, so
+// at most 2 k rows move however tall the matrix is (permuting every active row
+// took 33 of the 74 ms of a 10515 x 8668 RREF mod 13).  The order of the other
+// rows does not show in any result (the determinant's sign follows the same
+// moves, row_moves_odd).  One CTA per 32 columns: all reads before any write.
+constexpr int kMoveCols = 32;
+
+__global__ void __launch_bounds__(256) move_pivot_rows_kernel(uint32_t* __restrict__ A, uint64_t ld, int r0, int k,
+                                                              const int* __restrict__ prow, int ca, int cb) {
+    __shared__ uint32_t buf[2 * kMaxPanel][kMoveCols];
+    __shared__ int s_src[2 * kMaxPanel], s_dst[2 * kMaxPanel];
+    __shared__ unsigned char s_isp[kMaxPanel];
+    __shared__ int s_cnt[2][kMaxPanel / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int pr = tid < k ? prow[tid] : -1;
+    if (tid < kMaxPanel) s_isp[tid] = 0;
+    __syncthreads();
+    if (tid < k && pr - r0 < k) s_isp[pr - r0] = 1;
+    __syncthreads();
+    const bool disp = tid < k && !s_isp[tid], vac = tid < k && pr - r0 >= k;
+    const unsigned md = __ballot_sync(0xffffffffu, disp), mv = __ballot_sync(0xffffffffu, vac);
+    if (lane == 0 && warp < kMaxPanel / 32) {
+        s_cnt[0][warp] = __popc(md);
+        s_cnt[1][warp] = __popc(mv);
+    }
+    __syncthreads();
+    int nd = 0, d0 = 0, v0 = 0;
+#pragma unroll
+    for (int u = 0; u < kMaxPanel / 32; ++u) {
+        nd += s_cnt[0][u];
+        if (u < warp) {
+            d0 += s_cnt[0][u];
+            v0 += s_cnt[1][u];
+        }
+    }
+    const unsigned below = (1u << lane) - 1u;
+    if (tid < k) {
+        s_src[tid] = pr;
+        s_dst[tid] = r0 + tid;
+    }
+    if (disp) s_src[k + d0 + __popc(md & below)] = r0 + tid;
+    if (vac) s_dst[k + v0 + __popc(mv & below)] = pr;
+    __syncthreads();
+    const int n = k + nd, col = ca + static_cast<int>(blockIdx.x) * kMoveCols + lane;
+    if (col < cb) {
+#pragma unroll 4
+        for (int u = warp; u < n; u += 8)
+            if (s_src[u] != s_dst[u]) buf[u][lane] = A[static_cast<size_t>(s_src[u]) * ld + col];
+    }
+    __syncthreads();
+    if (col < cb) {
+        for (int u = warp; u < n; u += 8)
+            if (s_src[u] != s_dst[u]) A[static_cast<size_t>(s_dst[u]) * ld + col] = buf[u][lane];
     }
 }
-__global__ void scatter_rows_kernel(uint32_t* __restrict__ A, uint64_t ld, int r0, int rows, int c0, int cols,
-                                    const uint32_t* __restrict__ tmp) {
-    const size_t total = static_cast<size_t>(rows) * cols;
-    for (size_t idx = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; idx < total;
-         idx += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        const int i = static_cast<int>(idx / cols), j = static_cast<int>(idx % cols);
-        A[static_cast<size_t>(r0 + i) * ld + c0 + j] = tmp[idx];
+
+// Whether those row moves are an odd permutation (host): n minus the number of
+// cycles over the k top places and the places vacated below them.
+bool row_moves_odd(const int* prow, int k, int r0) {
+    std::vector<int> src(k), vac;
+    std::vector<char> isp(k, 0);
+    for (int t = 0; t < k; ++t) {
+        const int p = prow[t] - r0;
+        if (p < k) {
+            isp[p] = 1;
+            src[t] = p;
+        } else {
+            src[t] = k + static_cast<int>(vac.size());
+            vac.push_back(p);
+        }
+    }
+    for (int i = 0; i < k; ++i)
+        if (!isp[i]) src.push_back(i);  // the displaced rows, in the vacated places' order
+    const int n = static_cast<int>(src.size());
+    std::vector<char> seen(n, 0);
+    int cycles = 0;
+    for (int i = 0; i < n; ++i) {
+        if (seen[i]) continue;
+        ++cycles;
+        for (int j = i; !seen[j]; j = src[j]) seen[j] = 1;
+    }
+    return ((n - cycles) & 1) != 0;
+}
+
+// flag = 1 when the rows x cols window has a non-zero entry
+__global__ void window_nonzero_kernel(const uint32_t* __restrict__ A, uint64_t ld, int rows, int cols,
+                                      int* __restrict__ flag) {
+    for (int i = blockIdx.x; i < rows; i += gridDim.x) {
+        if (*reinterpret_cast<volatile int*>(flag) != 0) return;
+        uint32_t any = 0;
+        for (int j = threadIdx.x; j < cols; j += blockDim.x) any |= A[static_cast<size_t>(i) * ld + j];
+        if (any) *flag = 1;
     }
 }
 
@@ -1043,137 +1335,37 @@ __global__ void gather_cols_kernel(const uint32_t* __restrict__ A, uint64_t ld, 
     }
 }
 
-// Inverses of triangular diagonal blocks, one CTA per block.  Block b covers
-// rows [row0 + b*bb, row0 + b*bb + nb) of A and the pivot columns
-// pcols[b*bb ..]: T(t, s) = A[row0 + b*bb + t][pcols[b*bb + s]].
-//   UPPER: T upper triangular with non-zero diagonal (the U1 blocks of the RREF)
-//   !UPPER: T unit lower triangular, strictly-lower part read (the L11 of a panel)
-// out + b*bb*bb receives T^-1 (nb x nb, row-major, ld nb).
-// UPPER is reduced to the unit case: T = D T' with D its diagonal, and
-// T^-1 = T'^-1 D^-1 (columns of T'^-1 scaled on the way out).  The unit
-// triangular inverse X = T'^-1 is built right-looking from X = I: at step t
-// row t of X is final, and every later row r (earlier, for UPPER) takes
-// X[r] -= T'[r][t] * X[t] over the non-zero columns of X[t] -- one rank-1
-// update and one CTA barrier per step, lanes over columns, warps over rows.
-template <bool UPPER>
-__global__ void __launch_bounds__(1024) tri_inv_kernel(const uint32_t* __restrict__ A, uint64_t ld, int row0,
-                                                       const int* __restrict__ pcols, int total, int bb, uint32_t p,
-                                                       uint64_t barrett, uint32_t kmax, uint32_t* __restrict__ out) {
-    extern __shared__ uint32_t smem_ti[];
-    (void)kmax;
-    const int i0 = blockIdx.x * bb;
-    const int nb = min(bb, total - i0);
-    uint32_t* T = smem_ti;             // nb x nb: T' (unit diagonal implied)
-    uint32_t* X = smem_ti + nb * nb;   // nb x nb
-    uint32_t* dinv = X + nb * nb;      // nb
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+// Inverses of the upper triangular diagonal blocks of U1, one CTA per block:
+// block b covers rows [b*bb, b*bb + nb) and the pivot columns pcols[b*bb ..].
+// U = D U' with U' unit upper; U'^T goes through unit_lower_inverse and U^-1 =
+// U'^-1 D^-1 to out + b*bb*bb (nb x nb, row-major, ld nb).
+__global__ void __launch_bounds__(1024) tri_inv_kernel(const uint32_t* __restrict__ A, uint64_t ld,
+                                                       const int* __restrict__ pcols, int total, int bb, const Ring R,
+                                                       uint32_t* __restrict__ out) {
+    extern __shared__ __align__(16) uint32_t smem_ti[];
+    __shared__ uint32_t dinv[kMaxPanel];
+    const int i0 = blockIdx.x * bb, nb = min(bb, total - i0), P = tri_pad(nb), ls = tri_stride(P);
+    uint32_t* X = smem_ti;
     for (int t = threadIdx.x; t < nb; t += blockDim.x)
-        dinv[t] = UPPER ? inv_binary_xgcd(A[static_cast<size_t>(row0 + i0 + t) * ld + pcols[i0 + t]], p) : 1u % p;
+        dinv[t] = unit_inverse(A[static_cast<size_t>(i0 + t) * ld + pcols[i0 + t]], R);
     __syncthreads();
-    for (int idx = threadIdx.x; idx < nb * nb; idx += blockDim.x) {
-        const int t = idx / nb, s2 = idx - t * nb;
-        const bool keep = UPPER ? (s2 > t) : (s2 < t);
-        uint32_t v = keep ? A[static_cast<size_t>(row0 + i0 + t) * ld + pcols[i0 + s2]] : 0u;
-        if (UPPER && keep) v = mod_mul(v, dinv[t], p, barrett);
-        T[idx] = v;
-        X[idx] = s2 == t ? 1u % p : 0u;
-    }
-    __syncthreads();
-    for (int st = 0; st + 1 < nb; ++st) {
-        const int t = UPPER ? nb - 1 - st : st;
-        // LOWER: rows r > t, columns j <= t;  UPPER: rows r < t, columns j >= t
-        const int rbeg = UPPER ? 0 : t + 1, rend = UPPER ? t : nb;
-        const int jbeg = UPPER ? t : 0, jend = UPPER ? nb : t + 1;
-        const uint32_t* xt = X + t * nb;
-        for (int r = rbeg + warp; r < rend; r += nw) {
-            const uint32_t l = T[r * nb + t];
-            if (l == 0) continue;
-            const uint32_t nl = p - l;
-            uint32_t* xr = X + r * nb;
-            for (int j = jbeg + lane; j < jend; j += 32)
-                xr[j] = reduce_u64(static_cast<uint64_t>(nl) * xt[j] + xr[j], p, barrett);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int s = lane; s < P; s += 32) {
+        const int pc = s < nb ? pcols[i0 + s] : 0;
+#pragma unroll 4
+        for (int t = warp; t < P; t += 32) {  // U'[t][s] -> X[s][t]
+            uint32_t v = t == s ? 1u : 0u;
+            if (t < s && s < nb) v = mod_mul(A[static_cast<size_t>(i0 + t) * ld + pc], dinv[t], R.q, R.barrett);
+            X[s * ls + t] = v;
         }
-        __syncthreads();
     }
+    __syncthreads();
+    unit_lower_inverse(X, P, 1, 0, smem_ti + tri_words(P), R.q, R.barrett);
     uint32_t* o = out + static_cast<size_t>(blockIdx.x) * bb * bb;
     for (int idx = threadIdx.x; idx < nb * nb; idx += blockDim.x) {
-        const uint32_t v = X[idx];
-        o[idx] = UPPER ? mod_mul(v, dinv[idx % nb], p, barrett) : v;
+        const int i = idx / nb, j = idx - i * nb;
+        o[idx] = mod_mul(X[j * ls + i], dinv[j], R.q, R.barrett);
     }
-}
-
-// U12 = L11^-1 A12 in place.  L11: the unit-lower k x k block of the panel's
-// pivot rows (rows row0 .. row0+k-1 of A) at the pivot columns pcols[0..k),
-// strictly-lower part read; A12: the same rows at columns [c1, c1 + trail).
-// Each CTA takes kTrsmCols columns into shared memory; forward substitution
-// runs per column in one warp, lane l holding rows l, l+32, l+64, l+96 in
-// registers: at step t the value of row t is final, a shuffle broadcasts it,
-// and every later row r takes x_r -= L[r][t] x_t.  The columns are
-// independent, so after the loads no block barrier is needed until the
-// write-back.  L11 sits in shared memory with an odd row stride, so the 32
-// lanes reading L[r][t] for 32 rows hit 32 banks.
-constexpr int kTrsmCols = 32;
-
-__global__ void __launch_bounds__(32 * kTrsmCols) trsm_unit_lower_kernel(uint32_t* __restrict__ A, uint64_t ld,
-                                                                         int row0, const int* __restrict__ pcols,
-                                                                         int k, int c1, int trail, uint32_t p,
-                                                                         uint64_t barrett) {
-    extern __shared__ uint32_t smem_tr[];
-    const int ls = k | 1;
-    constexpr int xs = kTrsmCols + 1;
-    uint32_t* Ls = smem_tr;               // [k][ls]
-    uint32_t* X = smem_tr + k * ls;       // [k][xs]
-    const int cbase = c1 + static_cast<int>(blockIdx.x) * kTrsmCols;
-    const int ncols = min(kTrsmCols, c1 + trail - cbase);
-    for (int idx = threadIdx.x; idx < k * k; idx += blockDim.x) {
-        const int r = idx / k, t = idx - r * k;
-        Ls[r * ls + t] = t < r ? A[static_cast<size_t>(row0 + r) * ld + pcols[t]] : 0u;
-    }
-    for (int idx = threadIdx.x; idx < k * kTrsmCols; idx += blockDim.x) {
-        const int r = idx / kTrsmCols, c = idx - r * kTrsmCols;
-        X[r * xs + c] = c < ncols ? A[static_cast<size_t>(row0 + r) * ld + cbase + c] : 0u;
-    }
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (warp < ncols) {
-        uint32_t x[kMaxPanel / 32];
-#pragma unroll
-        for (int q = 0; q < kMaxPanel / 32; ++q) {
-            const int r = lane + 32 * q;
-            x[q] = r < k ? X[r * xs + warp] : 0u;
-        }
-#pragma unroll
-        for (int qt = 0; qt < kMaxPanel / 32; ++qt) {
-            if (32 * qt >= k - 1) break;
-            for (int tt = 0; tt < 32; ++tt) {
-                const int t = 32 * qt + tt;
-                if (t >= k - 1) break;
-                const uint32_t xt = __shfl_sync(0xffffffffu, x[qt], tt);
-#pragma unroll
-                for (int q = qt; q < kMaxPanel / 32; ++q) {
-                    const int r = lane + 32 * q;
-                    if (r > t && r < k) {
-                        const uint32_t l = Ls[r * ls + t];
-                        if (l) x[q] = reduce_u64(static_cast<uint64_t>(p - l) * xt + x[q], p, barrett);
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < kMaxPanel / 32; ++q) {
-            const int r = lane + 32 * q;
-            if (r < k) X[r * xs + warp] = x[q];
-        }
-    }
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < k * kTrsmCols; idx += blockDim.x) {
-        const int r = idx / kTrsmCols, c = idx - r * kTrsmCols;
-        if (c < ncols) A[static_cast<size_t>(row0 + r) * ld + cbase + c] = X[r * xs + c];
-    }
-}
-
-size_t trsm_smem_bytes(int k) {
-    return sizeof(uint32_t) * (static_cast<size_t>(k) * (k | 1) + static_cast<size_t>(k) * (kTrsmCols + 1));
 }
 
 // R (m x n, ld ldr): rows < rank: identity at the pivot columns, X at the free
@@ -1199,12 +1391,6 @@ __global__ void gather_diag_kernel(const uint32_t* __restrict__ A, uint64_t ld, 
                                    uint32_t* __restrict__ diag) {
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < rank; t += gridDim.x * blockDim.x)
         diag[t] = A[static_cast<size_t>(t) * ld + piv[t]];
-}
-
-uint32_t kmax_for(uint32_t p) {
-    const uint64_t d = static_cast<uint64_t>(p - 1) * (p - 1);
-    uint64_t km = d == 0 ? 1024 : (~0ull) / d;
-    return static_cast<uint32_t>(std::min<uint64_t>(km, 1024));
 }
 
 int grid_1d(size_t work, int sms) {
@@ -1259,25 +1445,24 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
         cluster_cap = 0;
         HME_CUDA(cudaFuncSetAttribute(panel_factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPanelSmemMax));
         {
-            const int bsm = static_cast<int>(block_smem_bytes(kMaxPanel, kMaxPanel));
+            const int bsm64 = static_cast<int>(block_smem_bytes(96, 64));
             for (const void* fn : {reinterpret_cast<const void*>(panel_block_kernel<kArithPow2, 64>),
                                    reinterpret_cast<const void*>(panel_block_kernel<kArithMont31, 64>),
                                    reinterpret_cast<const void*>(panel_block_kernel<kArithMont32, 64>),
-                                   reinterpret_cast<const void*>(panel_block_kernel<kArithPow2, 128>),
+                                   reinterpret_cast<const void*>(panel_block_kernel<kArithPow2, 96>),
+                                   reinterpret_cast<const void*>(panel_block_kernel<kArithMont31, 96>),
+                                   reinterpret_cast<const void*>(panel_block_kernel<kArithMont32, 96>)})
+                HME_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bsm64));
+            const int bsm128 = static_cast<int>(block_smem_bytes(128, kMaxPanel));
+            for (const void* fn : {reinterpret_cast<const void*>(panel_block_kernel<kArithPow2, 128>),
                                    reinterpret_cast<const void*>(panel_block_kernel<kArithMont31, 128>),
                                    reinterpret_cast<const void*>(panel_block_kernel<kArithMont32, 128>)})
-                HME_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bsm));
+                HME_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bsm128));
+            HME_CUDA(cudaFuncSetAttribute(panel_linv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          static_cast<int>(linv_smem_bytes(kMaxPanel))));
             const int wsm = static_cast<int>(sizeof(uint32_t) * (kMaxPanel * kMaxPanel + kWRows * kMaxPanel));
             HME_CUDA(cudaFuncSetAttribute(panel_w_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, wsm));
             HME_CUDA(cudaFuncSetAttribute(panel_w_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, wsm));
-            const int ssm = static_cast<int>(2 * sizeof(uint32_t) * kMaxPanel * kMaxPanel);
-            for (const void* fn : {reinterpret_cast<const void*>(panel_binv_kernel<kArithPow2, 64>),
-                                   reinterpret_cast<const void*>(panel_binv_kernel<kArithMont31, 64>),
-                                   reinterpret_cast<const void*>(panel_binv_kernel<kArithMont32, 64>),
-                                   reinterpret_cast<const void*>(panel_binv_kernel<kArithPow2, 128>),
-                                   reinterpret_cast<const void*>(panel_binv_kernel<kArithMont31, 128>),
-                                   reinterpret_cast<const void*>(panel_binv_kernel<kArithMont32, 128>)})
-                HME_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, ssm));
         }
         bool attrs_ok = true;
         for (const void* fn : {reinterpret_cast<const void*>(panel_cluster_kernel<kArithPow2, 512>),
@@ -1311,11 +1496,8 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
             }
         }
         cudaGetLastError();  // a refused query leaves no error behind
-        const int smem2 = sizeof(uint32_t) * (2 * kMaxPanel * kMaxPanel + kMaxPanel);
-        HME_CUDA(cudaFuncSetAttribute(tri_inv_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2));
-        HME_CUDA(cudaFuncSetAttribute(tri_inv_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2));
-        HME_CUDA(cudaFuncSetAttribute(trsm_unit_lower_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(trsm_smem_bytes(kMaxPanel))));
+        HME_CUDA(cudaFuncSetAttribute(tri_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(linv_smem_bytes(kMaxPanel))));
     });
     const int cluster_cap = cluster_caps[ctx->device];
 
@@ -1329,30 +1511,26 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
         int k;
         int err;       // the device error word as of the panel's end
         int block_ok;  // the top-block path settled the panel
+        int nonzero;   // the rest of the matrix is not zero
         unsigned bar[2];
     };
     const size_t scratch_bytes = (sizeof(Scratch) + 255) / 256 * 256;
     const size_t cand_bytes = sizeof(uint32_t) * 2 * static_cast<size_t>(grid_cap) * kMaxPanel;
-    const size_t perm_bytes = (sizeof(int) * static_cast<size_t>(m) + 255) / 256 * 256;
-    const size_t uinv_bytes = sizeof(uint32_t) * (4 * kMaxPanel * kMaxPanel + kMaxPanel);  // L, U, B^-1, L^-1 - I, 1/diag U
+    const size_t uinv_bytes = sizeof(uint32_t) * kMaxPanel * kMaxPanel;  // the update's M
     uint8_t* base = static_cast<uint8_t*>(
-        ctx->ws.get(kSlotElim0, 2 * (scratch_bytes + cand_bytes) + 2 * perm_bytes + 2 * uinv_bytes + 256));
+        ctx->ws.get(kSlotElim0, 2 * (scratch_bytes + cand_bytes + uinv_bytes) + 256));
     // the L21 / W slot at its largest (every panel's rows x pivots fits), so no panel regrows it
     ctx->ws.get(kSlotElim2, sizeof(uint32_t) * static_cast<size_t>(m) * bw);
     Scratch* d_sb[2] = {reinterpret_cast<Scratch*>(base), reinterpret_cast<Scratch*>(base + scratch_bytes)};
     uint32_t* d_candb[2] = {reinterpret_cast<uint32_t*>(base + 2 * scratch_bytes),
                             reinterpret_cast<uint32_t*>(base + 2 * scratch_bytes + cand_bytes)};
-    int* d_permb[2] = {reinterpret_cast<int*>(base + 2 * (scratch_bytes + cand_bytes)),
-                       reinterpret_cast<int*>(base + 2 * (scratch_bytes + cand_bytes) + perm_bytes)};
-    uint32_t* d_uinvb[2] = {reinterpret_cast<uint32_t*>(base + 2 * (scratch_bytes + cand_bytes + perm_bytes)),
-                            reinterpret_cast<uint32_t*>(base + 2 * (scratch_bytes + cand_bytes + perm_bytes) + uinv_bytes)};
+    uint32_t* d_uinvb[2] = {reinterpret_cast<uint32_t*>(base + 2 * (scratch_bytes + cand_bytes)),
+                            reinterpret_cast<uint32_t*>(base + 2 * (scratch_bytes + cand_bytes) + uinv_bytes)};
     HME_CUDA(cudaMemsetAsync(d_sb[0]->bar, 0, sizeof(unsigned) * 2, ctx->stream));
     HME_CUDA(cudaMemsetAsync(d_sb[1]->bar, 0, sizeof(unsigned) * 2, ctx->stream));
     // pinned copies of the two scratch sets (the host reads a panel's pivots without waiting for
     // the other stream's work), the second stream and the events of the lookahead
-    // (and two pinned permutation buffers: the host queues a panel's update behind the previous
-    // one's without waiting for it)
-    const size_t pinned_bytes = 2 * sizeof(Scratch) + 2 * sizeof(int) * static_cast<size_t>(m);
+    const size_t pinned_bytes = 2 * sizeof(Scratch);
     if (ctx->elim_pinned_bytes < pinned_bytes) {
         if (ctx->elim_pinned) {
             HME_CUDA(cudaDeviceSynchronize());
@@ -1364,7 +1542,6 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
         ctx->elim_pinned_bytes = pinned_bytes;
     }
     Scratch* h_sb = static_cast<Scratch*>(ctx->elim_pinned);
-    int* h_permb[2] = {reinterpret_cast<int*>(h_sb + 2), reinterpret_cast<int*>(h_sb + 2) + m};
     if (!ctx->aux_stream) {
         // the lookahead panel's stream at the highest priority: its cluster takes SMs as they free up
         int lo = 0, hi = 0;
@@ -1402,16 +1579,24 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
         return cs;
     };
 
-    // The panel [c0, c0 + w) of the active rows [r0, m) on `st`: its pivots and the error word
-    // land in h_sb[par] and ev_panel[par] is recorded.  Returns the cluster size (0: grid kernel).
-    // the top-block path: in automatic mode, over a field
-    // the top-block path in automatic mode, over fields of at least 256 elements (a random top block
-    // of 64 steps meets a zero pivot with probability about 64/p, so over small fields and over rings,
-    // where a non-unit pivot is as likely, the attempts would mostly fail); after a panel it did not
-    // settle, the next three panels go straight to the search (rank-deficient tails)
-    const bool use_block = opt.panel_kernel == 0 && rg.k == 1 && p >= 256;
-    int block_rest = 0;
-    bool block_tried[2] = {false, false};
+    // the determinant's pivots of the panels that the top block settles (their diagonal in A is 1);
+    // 0 where a searching kernel left the pivot in A
+    uint32_t* d_blkdiag = nullptr;
+    if (opt.want_diag) {
+        d_blkdiag = static_cast<uint32_t*>(ctx->ws.get(kSlotElim4, sizeof(uint32_t) * (static_cast<size_t>(std::max(m, n)) + 16)));
+        HME_CUDA(cudaMemsetAsync(d_blkdiag, 0, sizeof(uint32_t) * m, s_main));
+    }
+    // the top-block path in automatic mode.  A panel it does not settle costs the attempt and a
+    // second launch (10 + 15 us beside the search's 60 to 270), so the next 3, 7, 15, then
+    // 31 panels go straight to the search (rank-deficient tails, sparse matrices, rings whose columns
+    // run out of units), and the count starts over with the next settled panel
+    const bool use_block = opt.panel_kernel == 0;
+    int block_rest = 0, block_pause = 3;
+    // Over a large field, and after a panel that the block settled, the next one is expected to
+    // succeed; elsewhere the search is launched behind the block and returns at once when the block
+    // settled the panel, so a failed attempt costs no round trip to the host.
+    bool block_sure = rg.k == 1 && p >= (1u << 20);
+    bool block_tried[2] = {false, false}, search_behind[2] = {false, false};
     // The panel [c0, c0 + w) of the active rows [r0, m) on `st`: the top-block path when it is tried
     // (the host launches the search afterwards if the block did not settle the panel), else the
     // searching kernel.  Its pivots and the error word land in h_sb[par] and ev_panel[par] is
@@ -1445,7 +1630,6 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
         if (!search_only && use_block && block_rest > 0) --block_rest;
         block_tried[par] = try_block;
         if (try_block) {
-            const int nb = std::min(w, rows);
             BlockArgs ba{};
             ba.A = A;
             ba.ld = ld;
@@ -1458,53 +1642,35 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
             ba.pivot_cols = d_s->pivot_cols;
             ba.k_out = &d_s->k;
             ba.ok = &d_s->block_ok;
-            ba.lm = d_uinvb[par];
-            ba.um = d_uinvb[par] + kMaxPanel * kMaxPanel;
-            ba.dm = d_uinvb[par] + 4 * kMaxPanel * kMaxPanel;
-            const size_t bsm = block_smem_bytes(nb, w);
+            ba.binv = d_uinvb[par];
+            ba.diag = d_blkdiag;
+            // 64 row slots where a zero pivot is rare (chance about 64/p per panel), 32 spare rows over
+            // smaller fields and rings
+            const int rs = w > 64 ? 128 : rg.k == 1 && p >= (1u << 20) ? 64 : 96;
+            const size_t bsm = block_smem_bytes(rs, w);
             auto launch_block = [&](auto kern) {
-                HME_TIMED(ctx, "panel_block", kern<<<1, kBlockThreads, bsm, st>>>(ba));
+                HME_TIMED(ctx, "panel_block", kern<<<1, 4 * rs, bsm, st>>>(ba));
             };
-            const bool w64 = w <= 64;
             if (rg.ell == 2) {
-                if (w64) launch_block(panel_block_kernel<kArithPow2, 64>);
+                if (rs == 64) launch_block(panel_block_kernel<kArithPow2, 64>);
+                else if (rs == 96) launch_block(panel_block_kernel<kArithPow2, 96>);
                 else launch_block(panel_block_kernel<kArithPow2, 128>);
             } else if (p < (1u << 31)) {
-                if (w64) launch_block(panel_block_kernel<kArithMont31, 64>);
+                if (rs == 64) launch_block(panel_block_kernel<kArithMont31, 64>);
+                else if (rs == 96) launch_block(panel_block_kernel<kArithMont31, 96>);
                 else launch_block(panel_block_kernel<kArithMont31, 128>);
             } else {
-                if (w64) launch_block(panel_block_kernel<kArithMont32, 64>);
+                if (rs == 64) launch_block(panel_block_kernel<kArithMont32, 64>);
+                else if (rs == 96) launch_block(panel_block_kernel<kArithMont32, 96>);
                 else launch_block(panel_block_kernel<kArithMont32, 128>);
             }
             HME_CUDA(cudaGetLastError());
-            {
-                // B^-1 (when rows remain below) and L^-1 - I by row solves, one warp per row
-                const int with_binv = rows > nb ? 1 : 0;
-                const int gs = (2 * nb + kSolveWarps - 1) / kSolveWarps;
-                const size_t ssm = 2 * sizeof(uint32_t) * ((static_cast<size_t>(nb) * nb + 3) & ~size_t(3));
-                uint32_t* sb = d_uinvb[par];
-                auto launch_solve = [&](auto kern) {
-                    HME_TIMED(ctx, "panel_block", kern<<<gs, 32 * kSolveWarps, ssm, st>>>(
-                                                      sb, sb + kMaxPanel * kMaxPanel, sb + 4 * kMaxPanel * kMaxPanel, nb,
-                                                      with_binv, rg, &d_s->block_ok, sb + 2 * kMaxPanel * kMaxPanel,
-                                                      sb + 3 * kMaxPanel * kMaxPanel));
-                };
-                if (rg.ell == 2) {
-                    if (w64) launch_solve(panel_binv_kernel<kArithPow2, 64>);
-                    else launch_solve(panel_binv_kernel<kArithPow2, 128>);
-                } else if (p < (1u << 31)) {
-                    if (w64) launch_solve(panel_binv_kernel<kArithMont31, 64>);
-                    else launch_solve(panel_binv_kernel<kArithMont31, 128>);
-                } else {
-                    if (w64) launch_solve(panel_binv_kernel<kArithMont32, 64>);
-                    else launch_solve(panel_binv_kernel<kArithMont32, 128>);
-                }
-                HME_CUDA(cudaGetLastError());
-            }
         }
         const int cs = cluster_size(rows, w);
         HME_REQUIRE(opt.panel_kernel < 2 || cs > 0, "elim: the panel does not fit one cluster");
-        if (try_block) {
+        search_behind[par] = try_block && !block_sure;
+        if (search_behind[par]) pa.skip = &d_s->block_ok;
+        if (try_block && !search_behind[par]) {
             // no search behind the block: the host relaunches the panel with the search if needed
         } else if (cs > 0) {
             const int rpc = static_cast<int>((static_cast<size_t>(rows) + cs - 1) / cs);
@@ -1562,8 +1728,9 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
 
     std::vector<int> pivots;
     pivots.reserve(std::min(m, n));
-    std::vector<int> perm_host;
     int r0 = 0;
+    int next_look = 0;  // panel count before which a pivotless panel does not look over the rest
+    int look_gap = 1, panels = 0;
     int par = 0;
     bool launched = false;  // the panel at c0 was already factored ahead (on the second stream)
     for (int c0 = 0; c0 < lu_cols && r0 < m; c0 += bw) {
@@ -1574,123 +1741,95 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
         if (block_tried[par] && !h_sb[par].block_ok) {
             // the top block did not settle the panel (nothing was written): the search, on the
             // panel's stream; the main stream's later work waits for it too
-            block_rest = 3;
-            launch_panel(c0, w, r0, par, panel_stream[par], true);
-            if (panel_stream[par] != s_main) HME_CUDA(cudaStreamWaitEvent(s_main, ev_panel[par], 0));
-            HME_CUDA(cudaEventSynchronize(ev_panel[par]));
+            block_rest = block_pause;
+            block_pause = std::min(31, 2 * block_pause + 1);
+            if (search_behind[par]) {
+                block_tried[par] = false;  // the search has run
+            } else {
+                launch_panel(c0, w, r0, par, panel_stream[par], true);
+                if (panel_stream[par] != s_main) HME_CUDA(cudaStreamWaitEvent(s_main, ev_panel[par], 0));
+                HME_CUDA(cudaEventSynchronize(ev_panel[par]));
+            }
+            block_sure = false;
         }
         const Scratch& h_s = h_sb[par];
         if (h_s.err != 0) check_device_error(ctx);  // reports the timeout (and clears the word)
-        if (block_tried[par]) ++ctx->elim_block_panels;
+        if (block_tried[par]) {
+            block_pause = 3;
+            block_sure = true;
+        }
+        // the statistics count a top block that looks for most of its pivots (a field of fewer than 256
+        // elements, a ring) as searched
+        if (block_tried[par] && rg.k == 1 && p >= 256) ++ctx->elim_block_panels;
         else ++ctx->elim_search_panels;
         const int k = h_s.k;
-        if (k == 0) continue;  // no pivot in the panel: nothing moved, the next panel starts at r0
+        ++panels;
+        if (k == 0) {
+            // no pivot in the panel: nothing moved, the next panel starts at r0 -- unless nothing is
+            // left (one pass over the rest, against a panel's search each; after a pass that found
+            // something only every 2nd, 4th, .. pivotless panel asks again)
+            const int c1 = c0 + w;
+            if (c1 < lu_cols && panels >= next_look) {
+                int* d_nz = &d_sb[par]->nonzero;
+                HME_CUDA(cudaMemsetAsync(d_nz, 0, sizeof(int), s_main));
+                HME_TIMED(ctx, "rest_nonzero",
+                          window_nonzero_kernel<<<std::min(m - r0, 8 * ctx->num_sms), 256, 0, s_main>>>(
+                              A + static_cast<size_t>(r0) * ld + c1, ld, m - r0, lu_cols - c1, d_nz));
+                HME_CUDA(cudaMemcpyAsync(&h_sb[par].nonzero, d_nz, sizeof(int), cudaMemcpyDeviceToHost, s_main));
+                HME_CUDA(cudaStreamSynchronize(s_main));
+                if (h_sb[par].nonzero == 0) break;
+                next_look = panels + look_gap;
+                look_gap *= 2;
+            }
+            continue;
+        }
         for (int t = 0; t < k; ++t) pivots.push_back(h_s.pivot_cols[t]);
 
-        // (2) pivot rows first, in pivot order, the other active rows after them in order; the
-        // identity when the pivots are rows r0 .. r0+k-1 in order (then nothing moves)
+        // (2) the pivot rows' moves: none when they are rows r0 .. r0+k-1 in order
         const int rows = m - r0;
         bool identity = true;
         for (int t = 0; t < k && identity; ++t) identity = h_s.pivot_rows[t] == r0 + t;
-        if (!identity) {
-            perm_host.assign(rows, 0);
-            std::vector<char> is_piv(rows, 0);
-            for (int t = 0; t < k; ++t) {
-                perm_host[t] = h_s.pivot_rows[t];
-                is_piv[h_s.pivot_rows[t] - r0] = 1;
-            }
-            int q = k;
-            for (int i = 0; i < rows; ++i)
-                if (!is_piv[i]) perm_host[q++] = r0 + i;
-            // permutation parity: the sequence is the pivot rows p_0 .. p_k-1 (relative to r0), then
-            // the other rows ascending, so its inversions are the pivot pairs out of order plus, per
-            // pivot p_t, the other rows below it (p_t minus the pivots below it): O(k^2), not O(rows)
-            long long inv = 0;
-            for (int t = 0; t < k; ++t) {
-                const int pt = h_s.pivot_rows[t] - r0;
-                int below_piv = 0;
-                for (int u = 0; u < k; ++u) {
-                    const int pu = h_s.pivot_rows[u] - r0;
-                    if (pu < pt) {
-                        ++below_piv;
-                        if (u > t) ++inv;  // p_t before p_u in the sequence, p_t > p_u
-                    }
-                }
-                inv += pt - below_piv;
-            }
-            if (inv & 1) res.sign_negative = !res.sign_negative;
-            // pinned by parity: the copy of the panel two steps back has long completed (the host
-            // waited for this panel, which follows that panel's update on the main stream)
-            std::memcpy(h_permb[par], perm_host.data(), sizeof(int) * rows);
-            HME_CUDA(cudaMemcpyAsync(d_permb[par], h_permb[par], sizeof(int) * rows, cudaMemcpyHostToDevice, s_main));
-        }
-        int* d_perm = d_permb[par];
+        if (!identity && row_moves_odd(h_s.pivot_rows, k, r0)) res.sign_negative = !res.sign_negative;
         const int c1 = c0 + w;
         const int below = m - r0 - k;
         const int* d_pcols = d_sb[par]->pivot_cols;
-        // the update of columns [ca, cb): row permutation (from c0 on), U12 = L11^-1 A12, A22 -= L21 U12
-        uint32_t* L21 = nullptr;
         const bool blk = block_tried[par] && h_s.block_ok;
         uint32_t* Wf = nullptr;
+        // the update of columns [ca, cb): row moves (from c0 on), then [A12; A22] += W A12 on a
+        // tensor-core variant (it reads A12 through its limb planes, so C may alias it)
         auto update = [&](int ca, int cb, int sm_cap) {
             if (cb <= ca) return;
-            if (blk) {
-                // settled by the top block (no row moved): [A12; A22] += W A12, W = [L^-1 - I; -A21 B^-1],
-                // on a tensor-core variant (it reads A12 through its limb planes, so C may alias it)
-                const int ua = std::max(ca, c1);
-                if (cb <= ua) return;
-                if (!Wf) {
-                    Wf = static_cast<uint32_t*>(ctx->ws.get(kSlotElim2, sizeof(uint32_t) * static_cast<size_t>(rows) * k));
-                    const int g = (rows + kWRows - 1) / kWRows;
-                    const size_t wsm = sizeof(uint32_t) * (((static_cast<size_t>(k) * k + 3) & ~size_t(3)) +
-                                                           static_cast<size_t>(kWRows) * k);
-                    const uint32_t* binv = d_uinvb[par] + 2 * kMaxPanel * kMaxPanel;
-                    const uint32_t* linv = d_uinvb[par] + 3 * kMaxPanel * kMaxPanel;
-                    if (k <= 64)
-                        HME_TIMED(ctx, "panel_w", panel_w_kernel<64><<<g, 256, wsm, s_main>>>(
-                                                      A, ld, r0, m, c0, k, linv, binv, p, mp.barrett, Wf));
-                    else
-                        HME_TIMED(ctx, "panel_w", panel_w_kernel<128><<<g, 256, wsm, s_main>>>(
-                                                      A, ld, r0, m, c0, k, linv, binv, p, mp.barrett, Wf));
-                    HME_CUDA(cudaGetLastError());
-                }
-                ctx->gemm_sm_cap = sm_cap;
-                uint32_t* C12 = A + static_cast<size_t>(r0) * ld + ua;
-                gemm_u32_variant(ctx, mp, rows, cb - ua, k, Wf, k, C12, ld, C12, ld, HME_ADD,
-                                 gemm_default_variant(ctx, mp, rows, cb - ua));
-                ctx->gemm_sm_cap = 0;
-                return;
-            }
             if (!identity) {
-                const int cols = cb - ca;
-                uint32_t* tmp = static_cast<uint32_t*>(ctx->ws.get(kSlotElim1, sizeof(uint32_t) * static_cast<size_t>(rows) * (n - c0)));
-                const int g = grid_1d(static_cast<size_t>(rows) * cols, ctx->num_sms);
-                HME_TIMED(ctx, "row_permute", gather_rows_kernel<<<g, 256, 0, s_main>>>(A, ld, d_perm, rows, ca, cols, tmp));
-                HME_TIMED(ctx, "row_permute", scatter_rows_kernel<<<g, 256, 0, s_main>>>(A, ld, r0, rows, ca, cols, tmp));
+                HME_TIMED(ctx, "row_moves", move_pivot_rows_kernel<<<(cb - ca + kMoveCols - 1) / kMoveCols, 256, 0, s_main>>>(
+                                                A, ld, r0, k, d_sb[par]->pivot_rows, ca, cb));
                 HME_CUDA(cudaGetLastError());
             }
             const int ua = std::max(ca, c1);
             if (cb <= ua) return;
-            const int cols = cb - ua;
-            if (k > 1) {
-                const int g = (cols + kTrsmCols - 1) / kTrsmCols;
-                HME_TIMED(ctx, "trsm", trsm_unit_lower_kernel<<<g, 32 * kTrsmCols, trsm_smem_bytes(k), s_main>>>(
-                                           A, ld, r0, d_pcols, k, ua, cols, p, mp.barrett));
-                HME_CUDA(cudaGetLastError());
-            }
-            if (below > 0) {
-                if (!L21) {
-                    L21 = static_cast<uint32_t*>(ctx->ws.get(kSlotElim2, sizeof(uint32_t) * static_cast<size_t>(below) * k));
-                    HME_TIMED(ctx, "gather_cols",
-                              gather_cols_kernel<<<grid_1d(static_cast<size_t>(below) * k, ctx->num_sms), 256, 0, s_main>>>(
-                                  A, ld, r0 + k, below, d_pcols, k, L21));
+            if (!Wf) {
+                uint32_t* mul = d_uinvb[par];
+                if (!blk) {
+                    HME_TIMED(ctx, "panel_linv", panel_linv_kernel<<<1, 512, linv_smem_bytes(k), s_main>>>(
+                                                     A, ld, r0, d_pcols, k, p, mp.barrett, mul));
                     HME_CUDA(cudaGetLastError());
                 }
-                ctx->gemm_sm_cap = sm_cap;
-                gemm_u32_device(ctx, mp, below, cols, k, L21, k, A + static_cast<size_t>(r0) * ld + ua, ld,
-                                A + static_cast<size_t>(r0 + k) * ld + ua, ld, HME_SUB);
-                ctx->gemm_sm_cap = 0;
+                Wf = static_cast<uint32_t*>(ctx->ws.get(kSlotElim2, sizeof(uint32_t) * static_cast<size_t>(rows) * k));
+                const int g = (rows + kWRows - 1) / kWRows;
+                const size_t wsm = sizeof(uint32_t) * (((static_cast<size_t>(k) * k + 3) & ~size_t(3)) +
+                                                       static_cast<size_t>(kWRows) * ((k + 3) & ~3));
+                if (k <= 64)
+                    HME_TIMED(ctx, "panel_w", panel_w_kernel<64><<<g, 256, wsm, s_main>>>(
+                                                  A, ld, r0, m, d_pcols, k, mul, p, mp.barrett, Wf));
+                else
+                    HME_TIMED(ctx, "panel_w", panel_w_kernel<128><<<g, 256, wsm, s_main>>>(
+                                                  A, ld, r0, m, d_pcols, k, mul, p, mp.barrett, Wf));
+                HME_CUDA(cudaGetLastError());
             }
+            ctx->gemm_sm_cap = sm_cap;
+            uint32_t* C12 = A + static_cast<size_t>(r0) * ld + ua;
+            gemm_u32_variant(ctx, mp, rows, cb - ua, k, Wf, k, C12, ld, C12, ld, HME_ADD,
+                             gemm_default_variant(ctx, mp, rows, cb - ua));
+            ctx->gemm_sm_cap = 0;
         };
         const int nw = std::min(bw, lu_cols - c1);
         // lookahead only when the next panel runs on the cluster kernel (a few SMs beside the GEMM;
@@ -1728,7 +1867,12 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
         res.diag.resize(res.rank);
         HME_CUDA(cudaMemcpyAsync(res.diag.data(), d_diag, sizeof(uint32_t) * res.rank, cudaMemcpyDeviceToHost,
                                  ctx->stream));
+        std::vector<uint32_t> blk(res.rank);
+        HME_CUDA(cudaMemcpyAsync(blk.data(), d_blkdiag, sizeof(uint32_t) * res.rank, cudaMemcpyDeviceToHost,
+                                 ctx->stream));
         HME_CUDA(cudaStreamSynchronize(ctx->stream));
+        for (int t = 0; t < res.rank; ++t)
+            if (blk[t] != 0) res.diag[t] = blk[t];
     }
     if (!want_rref) return res;
 
@@ -1767,9 +1911,8 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
         // all diagonal blocks of U1 inverted at once, one CTA each
         uint32_t* Uinv = static_cast<uint32_t*>(ctx->ws.get(kSlotElim5, sizeof(uint32_t) * static_cast<size_t>(nblk) * bb * bb));
         {
-            const size_t sm = sizeof(uint32_t) * (2 * static_cast<size_t>(bb) * bb + bb);
-            HME_TIMED(ctx, "tri_inv", tri_inv_kernel<true><<<nblk, 1024, sm, ctx->stream>>>(
-                                          A, ld, 0, d_piv, rank, bb, p, mp.barrett, kmax_for(p), Uinv));
+            HME_TIMED(ctx, "tri_inv", tri_inv_kernel<<<nblk, 1024, linv_smem_bytes(std::min(bb, rank)), ctx->stream>>>(
+                                          A, ld, d_piv, rank, bb, rg, Uinv));
             HME_CUDA(cudaGetLastError());
         }
         // W (rank x f) in X's slot; the solution accumulates in Xs

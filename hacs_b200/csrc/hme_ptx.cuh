@@ -114,6 +114,24 @@ __device__ __forceinline__ void mac96(uint32_t& a0, uint32_t& a1, uint32_t& a2, 
         : "r"(x), "r"(y));
 }
 
+// (a2:a1:a0) += t
+__device__ __forceinline__ void add96(uint32_t& a0, uint32_t& a1, uint32_t& a2, uint64_t t) {
+    asm("add.cc.u32 %0, %0, %3;\n\t"
+        "addc.cc.u32 %1, %1, %4;\n\t"
+        "addc.u32 %2, %2, 0;"
+        : "+r"(a0), "+r"(a1), "+r"(a2)
+        : "r"(static_cast<uint32_t>(t)), "r"(static_cast<uint32_t>(t >> 32)));
+}
+// x0 y0 + .. + x3 y3 of words below 2^31: below 2^64
+__device__ __forceinline__ uint64_t dot4(uint32_t x0, uint32_t y0, uint32_t x1, uint32_t y1, uint32_t x2, uint32_t y2,
+                                         uint32_t x3, uint32_t y3) {
+    uint64_t t = static_cast<uint64_t>(x0) * y0;
+    t += static_cast<uint64_t>(x1) * y1;
+    t += static_cast<uint64_t>(x2) * y2;
+    t += static_cast<uint64_t>(x3) * y3;
+    return t;
+}
+
 // ---- L2 prefetch ----------------------------------------------------------------
 __device__ __forceinline__ void prefetch_l2(const void* p) {
     asm volatile("prefetch.global.L2 [%0];" ::"l"(p));

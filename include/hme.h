@@ -275,10 +275,10 @@ HME_API int hme_ctx_set_elim_options(hme_ctx *ctx, int panel, int rows_per_cta, 
 HME_API int hme_ctx_set_elim_lookahead(hme_ctx *ctx, int on);
 HME_API int hme_ctx_set_panel_kernel(hme_ctx *ctx, int mode);
 /* hme_ctx_elim_panel_stats: panels of this context's eliminations so far that
- * the top-block path settled (mode 0 over a field: the nb x w top block of the
- * panel factors with non-zero diagonal entries, so the pivots are its rows in
- * order and the rows below take x U^-1), and panels that a searching kernel
- * factored. */
+ * the top-block path settled over a field of at least 256 elements (mode 0: the
+ * panel's top rows supply a non-zero pivot for every column), and panels that
+ * were searched: by a searching kernel, or in a top block over a smaller field
+ * or a ring, where most columns' first rows are not pivots. */
 HME_API int hme_ctx_elim_panel_stats(const hme_ctx *ctx, uint64_t *block_panels, uint64_t *search_panels);
 
 /* ---- Howell and Smith forms over Z/ell^k (ell prime, ell^k < 2^32) ----------
