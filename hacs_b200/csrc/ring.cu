@@ -17,10 +17,11 @@
 // divided by ell is the next level.
 //
 // Howell: the blocked device LU with minimal-valuation pivots gives echelon
-// rows with the same row span; the Sec. 13.5 pass (active rows in id order,
-// closure rows appended at the bottom) runs on them in one CTA; the
-// reduce-above runs in blocks of pivots, the floor quotients of the rows above
-// a block by one kernel and their application by one limb GEMM (mod ell^k).
+// rows with the same row span; the Sec. 13.5 pass normalises all of them at
+// once and inserts the non-zero closure rows one column at a time; the
+// reduce-above runs in blocks of pivots, the floor quotients of the rows down
+// to a block's last by one kernel and their application by one limb GEMM (mod
+// ell^k).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -40,7 +41,6 @@ constexpr size_t kHowellLeadSmemMax = 192 * 1024;  // leading-column table of th
 struct RingK {
     uint32_t q, ell, k;
     uint64_t barrett;
-    uint32_t unit_exp;
     uint32_t pw[33];
 };
 
@@ -55,7 +55,6 @@ RingK make_ring(uint32_t ell, uint32_t k) {
     }
     r.q = r.pw[k];
     r.barrett = make_mod(r.q).barrett;
-    r.unit_exp = static_cast<uint32_t>(static_cast<uint64_t>(r.pw[k - 1]) * (ell - 1) - 1);
     return r;
 }
 
@@ -133,131 +132,6 @@ __global__ void any_nonzero_kernel(const uint32_t* __restrict__ A, uint64_t ld, 
         }
 }
 
-// zero the stale multipliers left of each echelon row's pivot column
-__global__ void clean_left_kernel(uint32_t* __restrict__ A, uint64_t ld, int rank, const int* __restrict__ pcols) {
-    for (int i = blockIdx.x; i < rank; i += gridDim.x) {
-        const int c = pcols[i];
-        for (int j = threadIdx.x; j < c; j += blockDim.x) A[static_cast<size_t>(i) * ld + j] = 0;
-    }
-}
-
-// ---- the Sec. 13.5 pass, one CTA ------------------------------------------------------
-// W: row store (capacity cap rows x n, ld), rows [0, r) the echelon rows;
-// closure rows are appended at r, r+1, ...  The active list is the alive rows
-// in id order (echelon rows first, closure rows in creation order), which is
-// the reference's list order, so "topmost" is the smallest id.
-struct PassArgs {
-    uint32_t* W;
-    uint64_t ld;
-    int n, r, cap;
-    RingK R;
-    unsigned char* alive;  // [cap]
-    int* piv_id;           // [n] out: row id of each pivot
-    int* piv_col;          // [n] out
-    int* piv_v;            // [n] out
-    int* h_out;
-    int* nrows_out;        // rows used in the store
-    int* err;
-};
-
-__global__ void __launch_bounds__(kHowellThreads) howell_pass_scan_kernel(const PassArgs a) {
-    __shared__ unsigned long long s_best;
-    __shared__ int s_nel;
-    __shared__ int s_el[kHowellThreads];
-    __shared__ uint32_t s_ui;
-    __shared__ int s_nrows, s_h;
-    __shared__ int s_closure_nz;
-    const RingK& R = a.R;
-    if (threadIdx.x == 0) {
-        s_nrows = a.r;
-        s_h = 0;
-    }
-    for (int i = threadIdx.x; i < a.cap; i += blockDim.x) a.alive[i] = i < a.r ? 1 : 0;
-    __syncthreads();
-    for (int c = 0; c < a.n; ++c) {
-        if (threadIdx.x == 0) s_best = ~0ull;
-        __syncthreads();
-        const int nrows = s_nrows;
-        for (int id = threadIdx.x; id < nrows; id += blockDim.x) {
-            if (!a.alive[id]) continue;
-            const uint32_t x = a.W[static_cast<size_t>(id) * a.ld + c];
-            if (x == 0) continue;
-            const unsigned long long key = (static_cast<unsigned long long>(val_k(x, R)) << 32) | static_cast<unsigned>(id);
-            atomicMin(&s_best, key);
-        }
-        __syncthreads();
-        const unsigned long long best = s_best;
-        if (best == ~0ull) continue;
-        const int pid = static_cast<int>(best & 0xffffffffu);
-        const uint32_t v = static_cast<uint32_t>(best >> 32);
-        uint32_t* P = a.W + static_cast<size_t>(pid) * a.ld;
-        if (threadIdx.x == 0) {
-            a.alive[pid] = 0;
-            s_ui = pow_mod_d(P[c] / R.pw[v], R.unit_exp, R.q, R.barrett);
-            s_nel = 0;
-            s_closure_nz = 0;
-        }
-        __syncthreads();
-        // scale the pivot row so that it leads with ell^v exactly
-        const uint32_t ui = s_ui;
-        for (int j = c + threadIdx.x; j < a.n; j += blockDim.x) P[j] = mod_mul(P[j], ui, R.q, R.barrett);
-        __syncthreads();
-        // the other alive rows with a non-zero in column c, in chunks of the CTA size
-        for (int base = 0; base < nrows; base += blockDim.x) {
-            const int id = base + threadIdx.x;
-            if (id < nrows && a.alive[id] && a.W[static_cast<size_t>(id) * a.ld + c] != 0) {
-                const int slot = atomicAdd(&s_nel, 1);
-                s_el[slot] = id;
-            }
-            __syncthreads();
-            const int nel = s_nel;
-            // one warp per row: R -= (R[c] / ell^v) * P over columns [c, n)
-            const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-            for (int t = warp; t < nel; t += nw) {
-                uint32_t* Rw = a.W + static_cast<size_t>(s_el[t]) * a.ld;
-                const uint32_t f = Rw[c] / R.pw[v];
-                __syncwarp();
-                for (int j = c + lane; j < a.n; j += 32)
-                    Rw[j] = mod_sub(Rw[j], mod_mul(f, P[j], R.q, R.barrett), R.q);
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) s_nel = 0;
-            __syncthreads();
-        }
-        // Howell closure: ell^(k - v) * P, zero in columns <= c, appended at the bottom
-        if (v > 0) {
-            const int nid = s_nrows;
-            if (nid >= a.cap) {
-                if (threadIdx.x == 0) atomicCAS(a.err, 0, 64);  // store exhausted: cannot happen (<= n closures)
-                return;
-            }
-            uint32_t* Z = a.W + static_cast<size_t>(nid) * a.ld;
-            const uint32_t f = R.pw[R.k - v];
-            for (int j = threadIdx.x; j < a.n; j += blockDim.x) {
-                const uint32_t z = j > c ? mod_mul(P[j], f, R.q, R.barrett) : 0u;
-                Z[j] = z;
-                if (z) s_closure_nz = 1;
-            }
-            __syncthreads();
-            if (threadIdx.x == 0 && s_closure_nz) {
-                a.alive[nid] = 1;
-                s_nrows = nid + 1;
-            }
-        }
-        if (threadIdx.x == 0) {
-            a.piv_id[s_h] = pid;
-            a.piv_col[s_h] = c;
-            a.piv_v[s_h] = static_cast<int>(v);
-            ++s_h;
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        *a.h_out = s_h;
-        *a.nrows_out = s_nrows;
-    }
-}
-
 // The inverse of a unit u of Z/ell^k by Newton's iteration x <- x (2 - u x),
 // which doubles the ell-adic precision per step: in 32-bit wraparound from
 // x = u (right to 3 bits) for ell = 2; from the inverse mod ell,
@@ -277,193 +151,291 @@ __device__ __forceinline__ uint32_t ring_unit_inverse(uint32_t u, const RingK& R
     return x;
 }
 
-// The pass with a leading-column table in shared memory.  Every live row's
-// first non-zero column is at least the current column c (eliminating column
-// c' zeroes it in every row that had a non-zero there), so the rows with a
-// non-zero in column c are exactly those whose leading column IS c: the scan
-// per column reads the table, not the store.  A row reduced by the pivot gets
-// its new leading column from the same warp pass that updates it; consumed
-// pivot rows, zero rows and unused slots hold n (never a candidate).  On
-// entry piv_col[0 .. r) holds the echelon rows' pivot columns (their leading
-// columns: the entries left of them are zero).
-__global__ void __launch_bounds__(kHowellThreads) howell_pass_kernel(const PassArgs a) {
-    extern __shared__ int s_lead[];  // [cap]
-    __shared__ unsigned long long s_best;
-    __shared__ int s_nel, s_over;
-    __shared__ int s_el[kHowellThreads];
+// ---- the Sec. 13.5 pass ---------------------------------------------------------------
+// The Howell form needs, for every pivot row P with pivot ell^v, v > 0, its
+// closure ell^(k-v) P (zero in the pivot's column) reduced to zero by the rows
+// below.  The form is unique, so the order is free: all echelon rows are
+// normalised and their closures looked over at once (howell_rows_kernel); only
+// the non-zero closures, and rows they displace, go through the sequential
+// insertion (howell_insert_kernel).  Over a matrix whose closures vanish -- unit
+// pivots, or rows with little right of their pivot -- nothing is sequential
+// (the column-by-column pass took 5.1 ms for a 2048 x 2048 U D V over Z/2^16,
+// 2.5 us a column).
+
+// One CTA per echelon row i (pivot column pcol[i], an arbitrary unit times ell^v
+// there): the stale multipliers left of the pivot to zero, the row scaled to
+// lead with ell^v exactly; piv_id / piv_v of its column; lead[i] = the first
+// non-zero column of its closure or n, counted in *nclose.
+__global__ void __launch_bounds__(256) howell_rows_kernel(uint32_t* __restrict__ W, uint64_t ld, int n,
+                                                          const int* __restrict__ pcol, const RingK R,
+                                                          int* __restrict__ piv_id, int* __restrict__ piv_v,
+                                                          int* __restrict__ lead, int* __restrict__ nclose) {
     __shared__ uint32_t s_ui;
-    __shared__ int s_nrows, s_h, s_zlead;
-    const RingK& R = a.R;
-    const int none = a.n;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int i = threadIdx.x; i < a.cap; i += blockDim.x) s_lead[i] = i < a.r ? a.piv_col[i] : none;
+    __shared__ int s_lead;
+    const int i = blockIdx.x, c = pcol[i];
+    uint32_t* P = W + static_cast<size_t>(i) * ld;
+    const uint32_t x = P[c];
+    const uint32_t v = val_k(x, R);
     if (threadIdx.x == 0) {
-        s_nrows = a.r;
-        s_h = 0;
+        s_ui = ring_unit_inverse(x / R.pw[v], R);
+        s_lead = n;
     }
     __syncthreads();
-    for (int c = 0; c < a.n; ++c) {
+    const uint32_t ui = s_ui, f = R.pw[R.k - v];
+    int first = n;
+    for (int j = threadIdx.x; j < n; j += blockDim.x) {
+        const uint32_t y = j < c ? 0u : mod_mul(P[j], ui, R.q, R.barrett);
+        P[j] = y;
+        if (v > 0 && j > c && first == n && mod_mul(y, f, R.q, R.barrett) != 0) first = j;
+    }
+    if (first < n) atomicMin(&s_lead, first);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        piv_id[c] = i;
+        piv_v[c] = static_cast<int>(v);
+        lead[i] = s_lead;
+        if (s_lead < n) atomicAdd(nclose, 1);
+    }
+}
+
+// The rows of the pass: echelon rows [0, r) in W, closures r, r + 1, .. in Z.
+struct PassArgs {
+    uint32_t* W;
+    uint32_t* Z;
+    uint64_t ld;
+    int n, r, cap;   // cap: rows of the two stores together
+    RingK R;
+    int* piv_id;     // [n] row id of each column's pivot, -1 for none
+    int* piv_v;      // [n]
+    int* lead;       // [cap] work: leading column of every pending row, n for none (used when it does not fit shared memory)
+    const int* first_lead;  // [r] from howell_rows_kernel
+    int* err;
+    __device__ __forceinline__ uint32_t* row(int id) const {
+        return id < r ? W + static_cast<size_t>(id) * ld : Z + static_cast<size_t>(id - r) * ld;
+    }
+};
+
+// Stores the non-zero closures (ids r, r + 1, .. in echelon order; every CTA
+// counts those before its row) and their leading columns.
+__global__ void __launch_bounds__(256) howell_closures_kernel(const PassArgs a, const int* __restrict__ pcol,
+                                                              int* __restrict__ lead_out) {
+    const int i = blockIdx.x;
+    const int z = a.first_lead[i];
+    if (z >= a.n) return;
+    int before = 0;
+    for (int t = threadIdx.x; t < i; t += blockDim.x) before += a.first_lead[t] < a.n ? 1 : 0;
+    __shared__ int s_before;
+    if (threadIdx.x == 0) s_before = 0;
+    __syncthreads();
+    if (before) atomicAdd(&s_before, before);
+    __syncthreads();
+    const int id = a.r + s_before, c = pcol[i];
+    const uint32_t f = a.R.pw[a.R.k - a.piv_v[c]];
+    const uint32_t* P = a.row(i);
+    uint32_t* Z = a.row(id);
+    for (int j = threadIdx.x; j < a.n; j += blockDim.x) Z[j] = j > c ? mod_mul(P[j], f, a.R.q, a.R.barrett) : 0u;
+    if (threadIdx.x == 0) lead_out[s_before] = z;
+}
+
+// The pending rows (the closures) inserted, one CTA.  Each round takes the
+// smallest leading column c of a pending row; all of a column's rows are there
+// when it comes up, so its pivot changes at most once: to the pending row of
+// smallest valuation, if that is smaller than the pivot's.  Then the new
+// pivot is normalised, its closure joins the pending rows, the old pivot row
+// too, and every pending row of the column is reduced by the pivot, a warp
+// each, which gives its next leading column.
+__global__ void __launch_bounds__(kHowellThreads) howell_insert_kernel(const PassArgs a, const int* __restrict__ lead0,
+                                                                       int nclose, int smem_lead) {
+    extern __shared__ int s_tab[];  // [cap] leading columns, when they fit
+    __shared__ unsigned long long s_best;
+    __shared__ int s_nel, s_c, s_nrows, s_zlead;
+    __shared__ int s_el[kHowellThreads];
+    __shared__ uint32_t s_ui;
+    const RingK& R = a.R;
+    int* lead = smem_lead ? s_tab : a.lead;
+    const int none = a.n;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    for (int i = threadIdx.x; i < a.cap; i += blockDim.x) lead[i] = i >= a.r && i < a.r + nclose ? lead0[i - a.r] : none;
+    if (threadIdx.x == 0) {
+        s_nrows = a.r + nclose;
+        s_c = none;
+    }
+    __syncthreads();
+    for (;;) {
+        const int nrows = s_nrows;
+        int c = none;
+        for (int id = threadIdx.x; id < nrows; id += blockDim.x) c = min(c, lead[id]);
+        c = __reduce_min_sync(0xffffffffu, c);
+        if (lane == 0 && c < none) atomicMin(&s_c, c);
         if (threadIdx.x == 0) {
             s_best = ~0ull;
             s_nel = 0;
-            s_over = 0;
-        }
-        __syncthreads();
-        const int nrows = s_nrows;
-        // the candidates: smallest (valuation, id) and the list of all of them
-        for (int id = threadIdx.x; id < nrows; id += blockDim.x) {
-            if (s_lead[id] != c) continue;
-            const uint32_t x = a.W[static_cast<size_t>(id) * a.ld + c];
-            atomicMin(&s_best, (static_cast<unsigned long long>(val_k(x, R)) << 32) | static_cast<unsigned>(id));
-            const int slot = atomicAdd(&s_nel, 1);
-            if (slot < kHowellThreads) s_el[slot] = id;
-            else s_over = 1;
-        }
-        __syncthreads();
-        const unsigned long long best = s_best;
-        if (best == ~0ull) continue;
-        const int pid = static_cast<int>(best & 0xffffffffu);
-        const uint32_t v = static_cast<uint32_t>(best >> 32);
-        uint32_t* P = a.W + static_cast<size_t>(pid) * a.ld;
-        if (threadIdx.x == 0) {
-            s_lead[pid] = none;  // consumed
-            s_ui = ring_unit_inverse(P[c] / R.pw[v], R);
             s_zlead = none;
         }
         __syncthreads();
-        // scale the pivot row so that it leads with ell^v exactly
-        const uint32_t ui = s_ui;
-        for (int j = c + threadIdx.x; j < a.n; j += blockDim.x) P[j] = mod_mul(P[j], ui, R.q, R.barrett);
+        c = s_c;
+        if (c >= none) break;
+        // the column's pending rows: the smallest (valuation, id) of all, a list of up to one CTA-size of them
+        for (int id = threadIdx.x; id < nrows; id += blockDim.x) {
+            if (lead[id] != c) continue;
+            const uint32_t x = a.row(id)[c];
+            atomicMin(&s_best, (static_cast<unsigned long long>(val_k(x, R)) << 32) | static_cast<unsigned>(id));
+            const int slot = atomicAdd(&s_nel, 1);
+            if (slot < kHowellThreads) s_el[slot] = id;
+        }
+        const int old = a.piv_id[c];
+        const uint32_t old_v = old >= 0 ? static_cast<uint32_t>(a.piv_v[c]) : R.k;
         __syncthreads();
-        // R -= (R[c] / ell^v) * P over columns [c, n) for every other candidate,
-        // one warp per row; more than one CTA-size of candidates: rescan
-        for (;;) {
-            const int nel = min(s_nel, kHowellThreads);
-            for (int t = warp; t < nel; t += nw) {
-                const int id = s_el[t];
-                if (id == pid) continue;
-                uint32_t* Rw = a.W + static_cast<size_t>(id) * a.ld;
-                const uint32_t f = Rw[c] / R.pw[v];
-                __syncwarp();
+        const unsigned long long best = s_best;
+        const bool change = static_cast<uint32_t>(best >> 32) < old_v;
+        const int pid = change ? static_cast<int>(best & 0xffffffffu) : old;
+        const uint32_t v = change ? static_cast<uint32_t>(best >> 32) : old_v;
+        uint32_t* P = a.row(pid);
+        int nel = min(s_nel, kHowellThreads);
+        if (change) {
+            if (threadIdx.x == 0) {
+                s_ui = ring_unit_inverse(P[c] / R.pw[v], R);
+                lead[pid] = none;
+            }
+            __syncthreads();
+            const uint32_t ui = s_ui;
+            for (int j = c + threadIdx.x; j < a.n; j += blockDim.x) P[j] = mod_mul(P[j], ui, R.q, R.barrett);
+            __syncthreads();
+            if (v > 0) {  // its closure
+                if (nrows >= a.cap) {
+                    if (threadIdx.x == 0) atomicCAS(a.err, 0, 64);  // store exhausted: cannot happen (one change per column)
+                    return;
+                }
+                uint32_t* Z = a.row(nrows);
+                const uint32_t f = R.pw[R.k - v];
                 int first = none;
-                for (int j = c + lane; j < a.n; j += 32) {
-                    const uint32_t y = mod_sub(Rw[j], mod_mul(f, P[j], R.q, R.barrett), R.q);
-                    Rw[j] = y;
-                    if (y != 0 && first == none) first = j;
+                for (int j = threadIdx.x; j < a.n; j += blockDim.x) {
+                    const uint32_t z = j > c ? mod_mul(P[j], f, R.q, R.barrett) : 0u;
+                    Z[j] = z;
+                    if (z && first == none) first = j;
                 }
                 first = __reduce_min_sync(0xffffffffu, first);
-                if (lane == 0) s_lead[id] = first;
-            }
-            __syncthreads();
-            if (!s_over) break;
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                s_nel = 0;
-                s_over = 0;
-            }
-            __syncthreads();
-            for (int id = threadIdx.x; id < nrows; id += blockDim.x) {
-                if (s_lead[id] != c) continue;
-                const int slot = atomicAdd(&s_nel, 1);
-                if (slot < kHowellThreads) s_el[slot] = id;
-                else s_over = 1;
-            }
-            __syncthreads();
-        }
-        // Howell closure: ell^(k - v) * P, zero in columns <= c, appended at the bottom
-        if (v > 0) {
-            const int nid = s_nrows;
-            if (nid >= a.cap) {
-                if (threadIdx.x == 0) atomicCAS(a.err, 0, 64);  // store exhausted: cannot happen (<= n closures)
-                return;
-            }
-            uint32_t* Z = a.W + static_cast<size_t>(nid) * a.ld;
-            const uint32_t f = R.pw[R.k - v];
-            for (int j = threadIdx.x; j < a.n; j += blockDim.x) {
-                const uint32_t z = j > c ? mod_mul(P[j], f, R.q, R.barrett) : 0u;
-                Z[j] = z;
-                if (z) atomicMin(&s_zlead, j);
-            }
-            __syncthreads();
-            if (threadIdx.x == 0 && s_zlead != none) {
-                s_lead[nid] = s_zlead;
-                s_nrows = nid + 1;
+                if (lane == 0 && first < none) atomicMin(&s_zlead, first);
             }
         }
+        // R -= (R[c] / ell^v) P over columns [c, n): the listed rows and a displaced pivot
+        for (int t = warp; t < nel + (change && old >= 0 ? 1 : 0); t += nw) {
+            const int id = t < nel ? s_el[t] : old;
+            if (id == pid) continue;
+            uint32_t* Rw = a.row(id);
+            const uint32_t f = Rw[c] / R.pw[v];
+            __syncwarp();
+            int first = none;
+            for (int j = c + lane; j < a.n; j += 32) {
+                const uint32_t y = mod_sub(Rw[j], mod_mul(f, P[j], R.q, R.barrett), R.q);
+                Rw[j] = y;
+                if (y != 0 && first == none) first = j;
+            }
+            first = __reduce_min_sync(0xffffffffu, first);
+            if (lane == 0) lead[id] = first;
+        }
+        __syncthreads();
         if (threadIdx.x == 0) {
-            a.piv_id[s_h] = pid;
-            a.piv_col[s_h] = c;
-            a.piv_v[s_h] = static_cast<int>(v);
-            ++s_h;
+            if (change) {
+                a.piv_id[c] = pid;
+                a.piv_v[c] = static_cast<int>(v);
+                if (s_zlead < none) {
+                    lead[nrows] = s_zlead;
+                    s_nrows = nrows + 1;
+                }
+            }
+            s_c = none;
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        *a.h_out = s_h;
-        *a.nrows_out = s_nrows;
+}
+
+// The pivots by column to lists: ids, columns, valuations and their number.
+__global__ void __launch_bounds__(1024) howell_pivots_kernel(const int* __restrict__ piv_id,
+                                                             const int* __restrict__ piv_v, int n,
+                                                             int* __restrict__ ids, int* __restrict__ cols,
+                                                             int* __restrict__ vals, int* __restrict__ count) {
+    __shared__ int s_cnt[32], s_base;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) s_base = 0;
+    __syncthreads();
+    for (int c0 = 0; c0 < n; c0 += 1024) {
+        const int c = c0 + threadIdx.x;
+        const int id = c < n ? piv_id[c] : -1;
+        const unsigned mask = __ballot_sync(0xffffffffu, id >= 0);
+        if (lane == 0) s_cnt[warp] = __popc(mask);
+        __syncthreads();
+        int at = s_base + __popc(mask & ((1u << lane) - 1u)), all = s_base;
+        for (int w = 0; w < 32; ++w) {
+            if (w < warp) at += s_cnt[w];
+            all += s_cnt[w];
+        }
+        if (id >= 0) {
+            ids[at] = id;
+            cols[at] = c;
+            vals[at] = piv_v[c];
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) s_base = all;
+        __syncthreads();
     }
+    if (threadIdx.x == 0) *count = s_base;
 }
 
 // ---- blocked reduce-above --------------------------------------------------------------
-// For the pivot block [t0, t0+b): Q[i][t] (rows i < t0) are the floor quotients
-// of row i against the block's pivots applied in order (each quotient on the
-// canonical residue after the previous ones); one thread per row.
-__global__ void reduce_quotients_kernel(const uint32_t* __restrict__ H, uint64_t ld, int t0, int b,
-                                        const int* __restrict__ pcol, const int* __restrict__ pv, RingK R,
-                                        uint32_t* __restrict__ Q) {
-    __shared__ uint32_t sB[kReduceBlock * kReduceBlock];  // sB[t][t3] = H[t0+t][pcol[t0+t3]]
+// For the pivot block [t0, t0+b): Q[i][t] are the floor quotients of row i <
+// t0 + b against the block's pivots applied in order (each quotient on the
+// canonical residue after the previous ones; inside the block only by the
+// pivots below the row), so that H[0 : t0+b] -= Q H[t0 : t0+b] reduces all of
+// them at once.  A warp per row, two of the block's columns per lane: a pivot
+// costs a shuffle and a compare where the quotient is 0.  (A thread per row with
+// its 64 values in local memory and a separate triangle pass over the block:
+// 36 + 28 us per block of a 2048 x 2048 form; this 7 us.)
+__global__ void __launch_bounds__(256) reduce_quotients_kernel(const uint32_t* __restrict__ H, uint64_t ld, int t0,
+                                                               int b, const int* __restrict__ pcol,
+                                                               const int* __restrict__ pv, RingK R,
+                                                               uint32_t* __restrict__ Q) {
+    __shared__ uint32_t sB[kReduceBlock][kReduceBlock + 1];  // sB[t][t3] = H[t0+t][pcol[t0+t3]]
     __shared__ uint32_t sdiv[kReduceBlock];
-    __shared__ int scol[kReduceBlock];
-    for (int idx = threadIdx.x; idx < b * b; idx += blockDim.x) {
-        const int t = idx / b, t3 = idx % b;
-        sB[idx] = H[static_cast<size_t>(t0 + t) * ld + pcol[t0 + t3]];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int l0 = lane, l1 = lane + 32;
+    const int pc0 = l0 < b ? pcol[t0 + l0] : 0, pc1 = l1 < b ? pcol[t0 + l1] : 0;
+#pragma unroll 4
+    for (int t = warp; t < b; t += 8) {
+        const uint32_t* src = H + static_cast<size_t>(t0 + t) * ld;
+        sB[t][l0] = l0 < b ? src[pc0] : 0u;
+        sB[t][l1] = l1 < b ? src[pc1] : 0u;
     }
-    for (int t = threadIdx.x; t < b; t += blockDim.x) {
-        sdiv[t] = R.pw[pv[t0 + t]];
-        scol[t] = pcol[t0 + t];
-    }
+    for (int t = threadIdx.x; t < b; t += 256) sdiv[t] = R.pw[pv[t0 + t]];
     __syncthreads();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= t0) return;
-    uint32_t vals[kReduceBlock];
-    for (int t = 0; t < b; ++t) vals[t] = H[static_cast<size_t>(i) * ld + scol[t]];
-    for (int t = 0; t < b; ++t) {
-        const uint32_t qt = vals[t] / sdiv[t];
-        Q[static_cast<size_t>(i) * b + t] = qt;
-        if (qt == 0) continue;
-        for (int t3 = t + 1; t3 < b; ++t3)
-            vals[t3] = mod_sub(vals[t3], mod_mul(qt, sB[t * b + t3], R.q, R.barrett), R.q);
+    const int i = static_cast<int>(blockIdx.x) * 8 + warp;
+    if (i >= t0 + b) return;
+    const uint32_t* src = H + static_cast<size_t>(i) * ld;
+    uint32_t v0 = l0 < b ? src[pc0] : 0u, v1 = l1 < b ? src[pc1] : 0u;
+    uint32_t q0 = 0, q1 = 0;
+    for (int t = max(0, i - t0 + 1); t < b; ++t) {
+        const uint32_t x = __shfl_sync(0xffffffffu, t < 32 ? v0 : v1, t & 31);
+        const uint32_t d = sdiv[t];
+        if (x < d) continue;  // the same in every lane
+        const uint32_t qt = x / d;
+        if (t < 32) q0 = lane == t ? qt : q0;
+        else q1 = lane == t - 32 ? qt : q1;
+        if (l0 > t) v0 = mod_sub(v0, mod_mul(qt, sB[t][l0], R.q, R.barrett), R.q);
+        if (l1 > t) v1 = mod_sub(v1, mod_mul(qt, sB[t][l1], R.q, R.barrett), R.q);
     }
+    uint32_t* dst = Q + static_cast<size_t>(i) * b;
+    if (l0 < b) dst[l0] = q0;
+    if (l1 < b) dst[l1] = q1;
 }
 
-// The triangle inside a block: for t = t0+1 .. t0+b-1, rows i in [t0, t) are
-// reduced by pivot row t (one CTA, a warp per row).
-__global__ void reduce_triangle_kernel(uint32_t* __restrict__ H, uint64_t ld, int n, int t0, int b,
-                                       const int* __restrict__ pcol, const int* __restrict__ pv, RingK R) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int t = t0 + 1; t < t0 + b; ++t) {
-        const int ct = pcol[t];
-        const uint32_t div = R.pw[pv[t]];
-        const uint32_t* Pt = H + static_cast<size_t>(t) * ld;
-        for (int i = t0 + warp; i < t; i += nw) {
-            uint32_t* Hi = H + static_cast<size_t>(i) * ld;
-            const uint32_t qv = Hi[ct] / div;
-            __syncwarp();
-            if (qv == 0) continue;
-            for (int j = ct + lane; j < n; j += 32) Hi[j] = mod_sub(Hi[j], mod_mul(qv, Pt[j], R.q, R.barrett), R.q);
-        }
-        __syncthreads();
-    }
-}
-
-// H[i] = W[piv_id[i]]  (h x n)
-__global__ void gather_rows_by_id_kernel(const uint32_t* __restrict__ W, uint64_t ldw, const int* __restrict__ ids,
-                                         int h, int n, uint32_t* __restrict__ H, uint64_t ldh) {
+// H[i] = row ids[i] of the pass's stores (h x n)
+__global__ void gather_rows_by_id_kernel(const PassArgs a, const int* __restrict__ ids, int h, int n,
+                                         uint32_t* __restrict__ H, uint64_t ldh) {
     const size_t total = static_cast<size_t>(h) * n;
     for (size_t idx = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; idx < total;
          idx += static_cast<size_t>(gridDim.x) * blockDim.x) {
         const int i = static_cast<int>(idx / n), j = static_cast<int>(idx % n);
-        H[static_cast<size_t>(i) * ldh + j] = W[static_cast<size_t>(ids[i]) * ldw + j];
+        H[static_cast<size_t>(i) * ldh + j] = a.row(ids[i])[j];
     }
 }
 
@@ -575,8 +547,7 @@ HowellOut howell_device(hme_ctx* ctx, uint32_t ell, uint32_t k, const uint32_t* 
     const RingK R = make_ring(ell, k);
     check_input(ctx, A, lda, m, n, R.q);
     const size_t ld = pad_ld(n);
-    const int cap = std::max(m, 0) + n;  // echelon rows (<= min(m, n)) plus at most one closure row per pivot
-    uint32_t* W = static_cast<uint32_t*>(ctx->ws.get(kSlotRing0, sizeof(uint32_t) * static_cast<size_t>(cap) * ld));
+    uint32_t* W = static_cast<uint32_t*>(ctx->ws.get(kSlotRing0, sizeof(uint32_t) * static_cast<size_t>(m) * ld));
     int* d_map = static_cast<int*>(ctx->ws.get(kSlotRing3, sizeof(int) * (static_cast<size_t>(n) + 16)));
     {
         std::vector<int> identity(n);
@@ -594,47 +565,61 @@ HowellOut howell_device(hme_ctx* ctx, uint32_t ell, uint32_t k, const uint32_t* 
     ElimOptions o = opt;
     const ElimResult lu = elim_device(ctx, make_mod(R.q), W, ld, m, n, false, nullptr, 0, o, &rs);
     const int r = lu.rank;
-    int* d_idx = static_cast<int*>(ctx->ws.get(kSlotRing2, sizeof(int) * (5 * static_cast<size_t>(n) + 64)));
+    if (r == 0) return out;
+    // (2) the Sec. 13.5 pass
+    int* d_idx = static_cast<int*>(ctx->ws.get(kSlotRing2, sizeof(int) * (7 * static_cast<size_t>(n) + 64)));
     int* d_pid = d_idx;
     int* d_pcol = d_idx + n;
     int* d_pv = d_idx + 2 * n;
-    int* d_cnt = d_idx + 3 * n;  // h, nrows
-    unsigned char* alive = static_cast<unsigned char*>(ctx->ws.get(kSlotRing1, static_cast<size_t>(cap) + 64));
-    if (r > 0) {
-        HME_CUDA(cudaMemcpyAsync(d_pcol, lu.pivots.data(), sizeof(int) * r, cudaMemcpyHostToDevice, ctx->stream));
-        HME_TIMED(ctx, "ring_clean", clean_left_kernel<<<std::min(r, ctx->num_sms * 4), 256, 0, ctx->stream>>>(
-                                         W, ld, r, d_pcol));
-    }
-    // rows [r, m) of W are the (zero) Schur complement; the closure rows start at r
-    // (2) the Sec. 13.5 pass
+    int* d_piv_id = d_idx + 3 * n;   // by column
+    int* d_piv_v = d_idx + 4 * n;
+    int* d_lead = d_idx + 5 * n;     // of the echelon rows' closures
+    int* d_lead0 = d_idx + 6 * n;    // of the non-zero closures, in order
+    int* d_cnt = d_idx + 7 * n;      // non-zero closures, pivots
+    HME_CUDA(cudaMemcpyAsync(d_pcol, lu.pivots.data(), sizeof(int) * r, cudaMemcpyHostToDevice, ctx->stream));
+    HME_CUDA(cudaMemsetAsync(d_piv_id, 0xff, sizeof(int) * n, ctx->stream));
+    HME_CUDA(cudaMemsetAsync(d_cnt, 0, 2 * sizeof(int), ctx->stream));
+    HME_TIMED(ctx, "howell_rows", howell_rows_kernel<<<r, 256, 0, ctx->stream>>>(W, ld, n, d_pcol, R, d_piv_id, d_piv_v,
+                                                                                d_lead, d_cnt));
+    HME_CUDA(cudaGetLastError());
+    int nclose = 0;
+    HME_CUDA(cudaMemcpyAsync(&nclose, d_cnt, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    HME_CUDA(cudaStreamSynchronize(ctx->stream));
     PassArgs pa{};
     pa.W = W;
     pa.ld = ld;
     pa.n = n;
     pa.r = r;
-    pa.cap = cap;
     pa.R = R;
-    pa.alive = alive;
-    pa.piv_id = d_pid;
-    pa.piv_col = d_pcol;
-    pa.piv_v = d_pv;
-    pa.h_out = d_cnt;
-    pa.nrows_out = d_cnt + 1;
+    pa.piv_id = d_piv_id;
+    pa.piv_v = d_piv_v;
+    pa.first_lead = d_lead;
     pa.err = ctx->d_err;
-    // the leading-column table in shared memory when it fits, else the store-scanning pass
-    const size_t lead_bytes = sizeof(int) * static_cast<size_t>(cap);
-    if (lead_bytes <= kHowellLeadSmemMax) {
-        HME_CUDA(cudaFuncSetAttribute(howell_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(kHowellLeadSmemMax)));
-        HME_TIMED(ctx, "howell_pass", howell_pass_kernel<<<1, kHowellThreads, lead_bytes, ctx->stream>>>(pa));
-    } else {
-        HME_TIMED(ctx, "howell_pass", howell_pass_scan_kernel<<<1, kHowellThreads, 0, ctx->stream>>>(pa));
+    if (nclose > 0) {
+        // the closures and, per column, at most one more of a new pivot; the leading columns beside them
+        const size_t zrows = static_cast<size_t>(nclose) + n;
+        pa.cap = r + static_cast<int>(zrows);
+        const size_t lead_bytes = sizeof(int) * static_cast<size_t>(pa.cap);
+        pa.Z = static_cast<uint32_t*>(ctx->ws.get(kSlotRing1, sizeof(uint32_t) * zrows * ld + lead_bytes));
+        pa.lead = reinterpret_cast<int*>(pa.Z + zrows * ld);
+        HME_TIMED(ctx, "howell_pass", howell_closures_kernel<<<r, 256, 0, ctx->stream>>>(pa, d_pcol, d_lead0));
+        HME_CUDA(cudaGetLastError());
+        const int in_smem = lead_bytes <= kHowellLeadSmemMax ? 1 : 0;
+        static OncePerDevice attr;
+        attr.run([](int) {
+            HME_CUDA(cudaFuncSetAttribute(howell_insert_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          static_cast<int>(kHowellLeadSmemMax)));
+        });
+        HME_TIMED(ctx, "howell_pass", howell_insert_kernel<<<1, kHowellThreads, in_smem ? lead_bytes : 0, ctx->stream>>>(
+                                          pa, d_lead0, nclose, in_smem));
+        HME_CUDA(cudaGetLastError());
     }
+    HME_TIMED(ctx, "howell_rows", howell_pivots_kernel<<<1, 1024, 0, ctx->stream>>>(d_piv_id, d_piv_v, n, d_pid, d_pcol,
+                                                                                  d_pv, d_cnt + 1));
     HME_CUDA(cudaGetLastError());
-    int hc[2] = {0, 0};
-    HME_CUDA(cudaMemcpyAsync(hc, d_cnt, sizeof(int) * 2, cudaMemcpyDeviceToHost, ctx->stream));
+    int h = 0;
+    HME_CUDA(cudaMemcpyAsync(&h, d_cnt + 1, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     check_device_error(ctx);
-    const int h = hc[0];
     out.pivots.resize(h);
     out.pivot_v.resize(h);
     out.H.assign(static_cast<size_t>(h) * n, 0);
@@ -645,24 +630,21 @@ HowellOut howell_device(hme_ctx* ctx, uint32_t ell, uint32_t k, const uint32_t* 
     const size_t ldh = ld;
     uint32_t* H = static_cast<uint32_t*>(ctx->ws.get(kSlotRing4, sizeof(uint32_t) * static_cast<size_t>(h) * ldh));
     HME_TIMED(ctx, "ring_gather", gather_rows_by_id_kernel<<<grid_for(static_cast<size_t>(h) * n, ctx->num_sms), 256, 0,
-                                                             ctx->stream>>>(W, ld, d_pid, h, n, H, ldh));
+                                                             ctx->stream>>>(pa, d_pid, h, n, H, ldh));
     HME_CUDA(cudaStreamSynchronize(ctx->stream));
     uint32_t* Q = static_cast<uint32_t*>(ctx->ws.get(kSlotRing5, sizeof(uint32_t) * static_cast<size_t>(h) * kReduceBlock));
     const ModParams mq = make_mod(R.q);
     for (int t0 = 0; t0 < h; t0 += kReduceBlock) {
         const int b = std::min(kReduceBlock, h - t0);
         const int c0 = out.pivots[t0];
-        if (t0 > 0) {
-            HME_TIMED(ctx, "reduce_quot", reduce_quotients_kernel<<<(t0 + 127) / 128, 128, 0, ctx->stream>>>(
-                                              H, ldh, t0, b, d_pcol, d_pv, R, Q));
-            HME_CUDA(cudaGetLastError());
-            gemm_u32_device(ctx, mq, t0, n - c0, b, Q, b, H + static_cast<size_t>(t0) * ldh + c0, ldh, H + c0, ldh,
-                            HME_SUB);
-        }
-        if (b > 1)
-            HME_TIMED(ctx, "reduce_tri", reduce_triangle_kernel<<<1, 1024, 0, ctx->stream>>>(H, ldh, n, t0, b, d_pcol,
-                                                                                              d_pv, R));
+        if (t0 + b == 1) continue;
+        HME_TIMED(ctx, "reduce_quot", reduce_quotients_kernel<<<(t0 + b + 7) / 8, 256, 0, ctx->stream>>>(
+                                          H, ldh, t0, b, d_pcol, d_pv, R, Q));
         HME_CUDA(cudaGetLastError());
+        // on a tensor-core variant: the block's own rows are among the reduced ones (C aliases B, which
+        // is read through its limb planes)
+        gemm_u32_variant(ctx, mq, t0 + b, n - c0, b, Q, b, H + static_cast<size_t>(t0) * ldh + c0, ldh, H + c0, ldh,
+                         HME_SUB, gemm_default_variant(ctx, mq, t0 + b, n - c0));
     }
     HME_CUDA(cudaMemcpy2DAsync(out.H.data(), sizeof(uint32_t) * n, H, sizeof(uint32_t) * ldh, sizeof(uint32_t) * n, h,
                                cudaMemcpyDeviceToHost, ctx->stream));
