@@ -403,13 +403,16 @@ class Engine:
         """(H, pivots, pivot_v): the Howell form of rowspan(A) over Z/ell^k."""
         A = _u32(A)
         m, n = A.shape
-        H = np.zeros((max(1, n), max(1, n)), np.uint32)
+        H = np.empty((max(1, n), max(1, n)), np.uint32)  # only the form's rows are written and returned
         piv = np.zeros(max(1, n), np.uint32)
         pv = np.zeros(max(1, n), np.uint32)
         h = C.c_uint32()
         check(self._lib.hme_howell_u32(self._h, ell, k, m, n, _p32(A), max(1, n), _p32(H), max(1, n), _p32(piv),
                                        _p32(pv), C.byref(h)))
-        return H[: h.value, :n].copy(), piv[: h.value].copy(), pv[: h.value].copy()
+        H = H[: h.value, :n]
+        if 2 * h.value < n:  # few rows: not the whole square kept alive
+            H = H.copy()
+        return H, piv[: h.value].copy(), pv[: h.value].copy()
 
     def smith(self, ell: int, k: int, A) -> np.ndarray:
         """Smith valuations sigma (ascending, each < k) of A over Z/ell^k."""

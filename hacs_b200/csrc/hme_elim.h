@@ -38,7 +38,6 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
 namespace hme {
 
 struct HowellOut {
-    std::vector<uint32_t> H;  // h x n, row-major
     std::vector<int> pivots;
     std::vector<int> pivot_v;
 };
@@ -46,8 +45,9 @@ struct HowellOut {
 // Smith valuations (ascending) of A (m x n, device, canonical mod ell^k).
 std::vector<uint32_t> smith_device(hme_ctx* ctx, uint32_t ell, uint32_t k, const uint32_t* A, size_t lda, int m,
                                    int n, const ElimOptions& opt);
-// Howell form of rowspan(A) (m x n, device, canonical mod ell^k).
+// Howell form of rowspan(A) (m x n, device, canonical mod ell^k); its rows go to
+// the host buffer H (room for n rows of ldh words).
 HowellOut howell_device(hme_ctx* ctx, uint32_t ell, uint32_t k, const uint32_t* A, size_t lda, int m, int n,
-                        const ElimOptions& opt);
+                        uint32_t* H, size_t ldh, const ElimOptions& opt);
 
 }  // namespace hme
