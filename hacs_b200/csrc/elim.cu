@@ -12,8 +12,9 @@
 // Blocked right-looking LU, panels of `bw` columns:
 //   1. the panel's pivots.  First the top-block path (panel_block_kernel): one
 //      CTA eliminates the panel's top rows alone, which settles the panel when
-//      they supply a unit for every column.  Otherwise the searching kernel:
-//      panel_cluster_kernel, the panel's active rows A[r0:m, c0:c0+bw) in the
+//      they supply a unit for every column.  Then, where most of the panel's rows
+//      are zero, panel_compact_kernel over the others, in one CTA.  Otherwise the
+//      searching kernel: panel_cluster_kernel, the panel's active rows A[r0:m, c0:c0+bw) in the
 //      shared memory of one thread-block cluster (up to 16 CTAs); per column
 //      each CTA pushes its best (valuation, row) key and that row to every CTA
 //      through distributed shared memory, one cluster barrier, a warp min of
@@ -25,7 +26,7 @@
 //      left of the panel of non-U rows hold dead multipliers).
 //   3. the left factor W = [L^-1 - I; -X M] (panel_w_kernel): X the other rows'
 //      entries at the pivot columns, M = B^-1 after the top block, L11^-1
-//      (panel_linv_kernel) after a search.
+//      (panel_linv_kernel) after a search; the compact kernel has written it.
 //   4. [A12; A22] += W A12: one INT8-limb tcgen05 GEMM, K = k pivots; the top
 //      rows become U12, the rest the Schur complement.
 // A panel without a pivot asks whether anything is left below: a rank-deficient
@@ -177,7 +178,8 @@ struct PanelArgs {
     int* k_out;          // out: pivots found
     unsigned* bar;       // [2]: arrival count, generation
     int* err;
-    const int* skip;     // non-null and non-zero: the panel is settled already (top-block path)
+    const int* skip;     // non-null and non-zero: the panel is settled already (top block, compact rows)
+    int keep;            // pivotless columns left of a pivot are updated too (cluster kernel only)
 };
 
 // Bounded grid-wide barrier for a cooperative launch (all CTAs co-resident).
@@ -526,6 +528,7 @@ __global__ void __launch_bounds__(NT, 1) panel_cluster_kernel(const PanelArgs a)
     __shared__ uint32_t s_inv[kMaxPanel];                     // its inverse
     __shared__ uint32_t s_sinv[kMaxPanel + 1];                // S_t^-1
     __shared__ int s_colstep[kMaxPanel];                      // step t of pivot column c0 + j; else -1 - pivots left of it
+    __shared__ int s_skip[kMaxPanel];                         // keep mode: the pivotless columns so far
 
     // settled by the top-block path: the same in every CTA, before any cluster barrier
     if (a.skip != nullptr && *a.skip != 0) return;
@@ -572,6 +575,7 @@ __global__ void __launch_bounds__(NT, 1) panel_cluster_kernel(const PanelArgs a)
     const uint32_t rrow_addr = smem_u32(&r_row[0][0][0]);
     const uint32_t rany_addr = smem_u32(&r_any[0][0]);
     int k = 0;
+    int nskip = 0;  // pivotless columns so far (keep mode)
     int empty = 0;  // pivotless columns in a row; at the 2nd, 6th, 14th, .. the rest of the panel is looked over
     int look = 2;
     uint32_t any = 1;  // this CTA's active rows are not known to be zero in the rest of the panel
@@ -597,6 +601,8 @@ __global__ void __launch_bounds__(NT, 1) panel_cluster_kernel(const PanelArgs a)
                     const int lm = static_cast<int>(mine & kKeyRowMask) - row_begin;
                     const uint32_t dst = dsmem_addr(rrow_addr + 4u * slot * kMaxPanel, d);
                     for (int j = lane; j < bw - it; j += 32) st_dsmem_u32(dst + 4u * j, S[(it + j) * rs + lm]);
+                    // keep mode: the row's entries of the pivotless columns behind them (they are left of it)
+                    for (int j = lane; j < nskip; j += 32) st_dsmem_u32(dst + 4u * (bw - it + j), S[s_skip[j] * rs + lm]);
                 }
             }
             if (tid == 0) s_cand[par ^ 1] = kNoKey32;  // collects column it + 1's candidate below
@@ -614,7 +620,11 @@ __global__ void __launch_bounds__(NT, 1) panel_cluster_kernel(const PanelArgs a)
                 for (int j = it + tid; j < bw; j += NT) s_colstep[j] = -1 - k;
                 break;
             }
-            if (tid == 0) s_colstep[it] = -1 - k;
+            if (tid == 0) {
+                s_colstep[it] = -1 - k;
+                if (a.keep) s_skip[nskip] = it;  // read after this column's CTA barrier
+            }
+            if (a.keep) ++nskip;
             ++empty;
             if (it + 1 < bw && has_row && sub == 0 && s_step[li] == 0)
                 key = pivot_key32(S[(it + 1) * rs + li], row_begin + li, a.R);
@@ -658,6 +668,10 @@ __global__ void __launch_bounds__(NT, 1) panel_cluster_kernel(const PanelArgs a)
                     sp[sstep] = y1;
                 }
                 if (j < bw) *sp = ff_update<ARITH>(w, *sp, xn, *pp, a.R);
+                for (int u = sub; u < nskip; u += g) {
+                    uint32_t* sk = S + s_skip[u] * rs + li;
+                    *sk = ff_update<ARITH>(w, *sk, xn, prv[bw - it + u], a.R);
+                }
                 if (v != 0 && sub == 0) {
                     pend_col = it;
                     pend_xp = xp;
@@ -690,7 +704,8 @@ __global__ void __launch_bounds__(NT, 1) panel_cluster_kernel(const PanelArgs a)
             // a multiplier of step t < tau: times w_t^-1; any other entry was last
             // scaled by the step before min(tau, pivots left of column j)
             const int t = s_colstep[j];
-            const uint32_t f = t >= 0 ? (t < tau ? s_inv[t] : sc) : s_sinv[min(tau, -1 - t)];
+            // (in keep mode pivotless columns take every step's scale)
+            const uint32_t f = t >= 0 ? (t < tau ? s_inv[t] : sc) : s_sinv[a.keep ? tau : min(tau, -1 - t)];
             S[j * rs + li] = mod_mul(S[j * rs + li], f, a.R.q, a.R.barrett);
         }
     }
@@ -1089,6 +1104,243 @@ __global__ void __launch_bounds__(4 * RS) panel_block_kernel(const BlockArgs a) 
     }
 }
 
+// ---- panels with few non-zero rows ----------------------------------------------------
+// Sparse matrices (boundary-like blocks, U D V products close to diagonal) have
+// panels in which most active rows are zero.  Zero rows never pivot and are
+// never updated, so the search runs on the others alone: panel_rows_kernel
+// lists them (and clears the update's left factor W), and when there are at
+// most kCompactRows of them panel_compact_kernel factors them in one CTA, where
+// a column costs one CTA barrier instead of the cluster's exchange.  It keeps
+// every row operation's effect on the identity as well (in place: the pivot's
+// column of a row holds that row's entry of the inverse of the operations), so W
+// comes out directly, with no triangular inverse and no panel_w_kernel.
+constexpr int kCompactRows = 256;
+
+struct CompactArgs {
+    uint32_t* A;
+    uint64_t ld;
+    int m, r0, c0, w;
+    Ring R;
+    int* list;        // [kCompactRows] rows with a non-zero entry in the panel, in any order
+    int* count;       // their number (counted on beyond the list); 0 between panels
+    int after_block;  // the top block was tried before: nothing to do when it settled the panel
+    int* ok;          // out: 2 when the panel was factored here, else 0 (left alone when the block settled it)
+    int* pivot_rows;  // [w] out
+    int* pivot_cols;  // [w] out
+    int* k_out;       // out
+    uint32_t* W;      // out: (m - r0) x w, row stride ldw, rows in their places after the pivot rows' moves
+    int ldw;
+};
+
+__global__ void __launch_bounds__(256) panel_rows_kernel(const CompactArgs a) {
+    if (a.after_block && *a.ok != 0) return;
+    const int lane = threadIdx.x & 31, row = a.r0 + static_cast<int>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+    if (row >= a.m) return;
+    const uint32_t* src = a.A + static_cast<size_t>(row) * a.ld + a.c0;
+    uint32_t* dst = a.W + static_cast<size_t>(row - a.r0) * a.ldw;
+    uint32_t any = 0;
+#pragma unroll
+    for (int c = 0; c < kMaxPanel / 32; ++c)
+        if (lane + 32 * c < a.w) {
+            any |= src[lane + 32 * c];
+            dst[lane + 32 * c] = 0u;
+        }
+    if (__any_sync(0xffffffffu, any != 0) && lane == 0) {
+        const int at = atomicAdd(a.count, 1);
+        if (at < kCompactRows) a.list[at] = row;
+    }
+}
+
+__host__ __device__ constexpr size_t compact_smem_bytes(int w) {
+    return sizeof(uint32_t) * static_cast<size_t>(w) * (kCompactRows + 1);
+}
+
+// One CTA of 32 warps.  The rows, in row order, sit in shared memory
+// column-major, lanes over rows: rwn = 1, 2, 4 or 8 warps cover them and 32 /
+// rwn groups of warps share the columns.  Pivot rule and fraction-free update
+// are the cluster kernel's, but a step whose column has no other entry updates
+// nothing (and no scale), and every column is updated, pivotless ones left of
+// the pivot too, the pivot's own becoming the inverse's column.
+// A 64-column panel of a 2048 x 2048 U D V over Z/2^16: 41 us and 2 us for the
+// list, against 98 us for the cluster search and 21 us for L11^-1 and W.
+template <int ARITH>
+__global__ void __launch_bounds__(1024, 1) panel_compact_kernel(const CompactArgs a) {
+    extern __shared__ __align__(16) uint32_t s_cmp[];
+    __shared__ uint32_t s_x[2][kCompactRows];
+    __shared__ uint32_t s_key[2][8];
+    __shared__ int s_nz[2][8];
+    __shared__ uint32_t s_S[kMaxPanel + 1], s_Sinv[kMaxPanel + 1];
+    __shared__ int s_prow[kMaxPanel], s_pcol[kMaxPanel], s_colpiv[kMaxPanel];
+    __shared__ int s_row[kCompactRows], s_step[kCompactRows];
+    __shared__ int s_raw[kCompactRows];
+    __shared__ unsigned char s_isp[kMaxPanel];
+    __shared__ int s_vac[kMaxPanel];
+    __shared__ int s_cnt;
+    if (a.after_block && *a.ok != 0) return;
+    const Ring& R = a.R;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, w = a.w;
+    if (tid == 0) {
+        s_cnt = *a.count;
+        *a.count = 0;
+    }
+    __syncthreads();
+    const int cnt = s_cnt;
+    if (cnt > kCompactRows) {
+        if (tid == 0) *a.ok = 0;
+        return;
+    }
+    // the list in row order (ranks by counting)
+    if (tid < cnt) s_raw[tid] = a.list[tid];
+    if (tid < kMaxPanel) s_colpiv[tid] = -1;
+    __syncthreads();
+    if (tid < cnt) {
+        const int mine = s_raw[tid];
+        int rank = 0;
+        for (int u = 0; u < cnt; ++u) rank += s_raw[u] < mine ? 1 : 0;
+        s_row[rank] = mine;
+        s_step[tid] = 0;
+    }
+    __syncthreads();
+    const int rwn = cnt <= 32 ? 1 : cnt <= 64 ? 2 : cnt <= 128 ? 4 : 8;
+    const int G = 32 / rwn, rs = 32 * rwn + 1;
+    uint32_t* S = s_cmp;  // [w][rs]
+#pragma unroll 4
+    for (int r = warp; r < cnt; r += 32) {
+        const uint32_t* src = a.A + static_cast<size_t>(s_row[r]) * a.ld + a.c0;
+#pragma unroll
+        for (int c = 0; c < kMaxPanel / 32; ++c)
+            if (lane + 32 * c < w) S[(lane + 32 * c) * rs + r] = src[lane + 32 * c];
+    }
+    __syncthreads();
+    const int rwi = warp & (rwn - 1), g = warp / rwn, li = 32 * rwi + lane;
+    bool active = li < cnt;  // in the list and not a pivot row yet
+    uint32_t* col = S + li;
+    // column c's entries, smallest (valuation, slot) and non-zeros of the active rows, for step c
+    auto publish = [&](int c) {
+        const uint32_t x = active ? col[c * rs] : 0u;
+        uint32_t key = kNoKey32;
+        if (x != 0) {
+            const uint32_t v = R.k == 1 ? 0u : R.max_v == 0 ? (x % R.ell == 0 ? 1u : 0u) : valuation(x, R, R.max_v);
+            if (v <= R.max_v) key = (v << 16) | static_cast<uint32_t>(li);
+        }
+        key = __reduce_min_sync(0xffffffffu, key);
+        const unsigned nz = __ballot_sync(0xffffffffu, x != 0);
+        s_x[c & 1][li] = x;
+        if (lane == 0) {
+            s_key[c & 1][rwi] = key;
+            s_nz[c & 1][rwi] = __popc(nz);
+        }
+    };
+    if (g == 0) publish(0);
+    uint32_t scale = 1u;
+    int k = 0;
+    __syncthreads();
+    for (int it = 0; it < w; ++it) {
+        const int par = it & 1;
+        uint32_t pk = s_key[par][0];
+        int nz = s_nz[par][0];
+        for (int u = 1; u < rwn; ++u) {
+            pk = min(pk, s_key[par][u]);
+            nz += s_nz[par][u];
+        }
+        if (pk != kNoKey32) {
+            const int prow = static_cast<int>(pk & 0xffffu);
+            const uint32_t v = pk >> 16;
+            const uint32_t wt = div_pw(s_x[par][prow], v, R);
+            if (tid == 0) {
+                s_S[k] = scale;
+                s_prow[k] = prow;
+                s_pcol[k] = it;
+                s_colpiv[it] = k;
+                s_step[prow] = k + 1;
+            }
+            if (li == prow) active = false;
+            if (nz > 1) {
+                if (active) {
+                    const uint32_t xn = ff_negate<ARITH>(div_pw(s_x[par][li], v, R), R);
+                    const uint32_t* pr = S + prow;
+#pragma unroll 4
+                    for (int j = g; j < w; j += G) {
+                        const bool own = j == it;
+                        const uint32_t y = own ? 0u : col[j * rs];
+                        const uint32_t p = own ? scale : pr[j * rs];
+                        col[j * rs] = ff_update<ARITH>(wt, y, xn, p, R);
+                    }
+                }
+                scale = ARITH == kArithPow2 ? (scale * wt) & (R.q - 1u) : mont_mul(scale, wt, R.q, R.mont_qinv);
+            }
+            ++k;
+        }
+        if (it + 1 < w && ((it + 1) & (G - 1)) == g) publish(it + 1);
+        __syncthreads();
+    }
+    // the rows' scales: row of pivot t by S_t, the others by the last
+    if (tid == 0) s_S[k] = scale;
+    __syncthreads();
+    if (tid <= k) s_Sinv[tid] = unit_inverse(s_S[tid], R);
+    // the rows' places after the moves (as move_pivot_rows_kernel makes them)
+    if (tid < kMaxPanel) s_isp[tid] = 0;
+    __syncthreads();
+    if (tid < k && s_row[s_prow[tid]] - a.r0 < k) s_isp[s_row[s_prow[tid]] - a.r0] = 1;
+    if (tid == 0) {
+        int nv = 0;
+        for (int t = 0; t < k; ++t)
+            if (s_row[s_prow[t]] - a.r0 >= k) s_vac[nv++] = s_row[s_prow[t]] - a.r0;
+    }
+    __syncthreads();
+    for (int r = warp; r < cnt; r += 32) {
+        const int st = s_step[r], tau = st ? st - 1 : k;
+        const uint32_t sc = s_Sinv[tau];
+        int pos = st ? st - 1 : s_row[r] - a.r0;
+        if (!st && pos < k) {
+            int rank = 0;
+            for (int i = lane; i < pos; i += 32) rank += s_isp[i] ? 0 : 1;
+            pos = s_vac[__reduce_add_sync(0xffffffffu, rank)];
+        }
+        uint32_t* dst = a.A + static_cast<size_t>(s_row[r]) * a.ld + a.c0;
+        uint32_t* wd = a.W + static_cast<size_t>(pos) * a.ldw;
+        for (int j = lane; j < w; j += 32) {
+            const uint32_t val = mod_mul(S[j * rs + r], sc, R.q, R.barrett);
+            const int t = s_colpiv[j];
+            const bool done = t >= 0 && t < tau;  // eliminated from this row: its entry is the inverse's
+            dst[j] = done ? 0u : val;
+            if (done) wd[t] = val;
+        }
+    }
+    if (tid < k) {
+        a.pivot_rows[tid] = s_row[s_prow[tid]];
+        a.pivot_cols[tid] = a.c0 + s_pcol[tid];
+    }
+    if (tid == 0) {
+        *a.k_out = k;
+        *a.ok = 2;
+    }
+}
+
+// Columns [c0, c0 + w) without pivots (pcols[0 .. k) has them) of rows [row0,
+// row0 + rows) to columns dst, dst + 1, .. of the same rows: a warp per row.
+__global__ void __launch_bounds__(256) append_cols_kernel(uint32_t* __restrict__ A, uint64_t ld, int row0, int rows,
+                                                          int c0, int w, const int* __restrict__ pcols, int k,
+                                                          int dst) {
+    __shared__ int s_at[kMaxPanel];
+    for (int j = threadIdx.x; j < w; j += 256) {
+        int at = j;  // minus the pivot columns before it; -1 for a pivot column
+        for (int t = 0; t < k; ++t) {
+            const int c = pcols[t] - c0;
+            if (c == j) at = INT_MIN / 2;
+            else if (c < j) --at;
+        }
+        s_at[j] = at;
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    for (int i = static_cast<int>(blockIdx.x) * 8 + (threadIdx.x >> 5); i < rows; i += static_cast<int>(gridDim.x) * 8) {
+        uint32_t* row = A + static_cast<size_t>(row0 + i) * ld;
+        for (int j = lane; j < w; j += 32)
+            if (s_at[j] >= 0) row[dst + s_at[j]] = row[c0 + j];
+    }
+}
+
 // After a searched panel (its packed LU in place, the pivot rows moved to r0 ..
 // r0 + k - 1): L11^-1 of the k pivot rows at the pivot columns, the factor the
 // update takes in place of the top block's.
@@ -1397,46 +1649,9 @@ int grid_1d(size_t work, int sms) {
     return static_cast<int>(std::max<size_t>(1, std::min<size_t>((work + 255) / 256, static_cast<size_t>(sms) * 8)));
 }
 
-}  // namespace
-
-// ---------------------------------------------------------------------------------
-ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld, int m, int n, bool want_rref,
-                       uint32_t* R, size_t ldr, const ElimOptions& opt, const RingSpec* ring) {
-    HME_REQUIRE(m >= 0 && n >= 0, "elim: negative shape");
-    HME_REQUIRE(!(want_rref && ring && ring->k > 1), "elim: the RREF is a field-only object");
-    ElimResult res;
-    res.sign_negative = false;
-    if (m == 0 || n == 0) {
-        if (want_rref && m > 0 && n > 0) HME_CUDA(cudaMemsetAsync(R, 0, 1, ctx->stream));
-        return res;
-    }
-    const int bw = std::max(1, std::min<int>(opt.panel > 0 ? opt.panel : 64, kMaxPanel));
-    const uint32_t p = mp.p;
-    // the ring: F_p by default, Z/ell^k with a pivot valuation bound when given
-    Ring rg{};
-    rg.q = p;
-    rg.barrett = mp.barrett;
-    rg.ell = ring ? ring->ell : p;
-    rg.k = ring ? ring->k : 1;
-    rg.max_v = ring ? ring->max_v : 0;
-    {
-        uint64_t pw = 1;
-        for (uint32_t v = 0; v <= rg.k && v < 32; ++v) {
-            rg.pw[v] = static_cast<uint32_t>(pw);
-            pw *= rg.ell;
-        }
-        HME_REQUIRE(static_cast<uint64_t>(rg.pw[rg.k]) == p || rg.k == 1, "elim: modulus is not ell^k");
-        // phi(ell^k) - 1 = ell^(k-1) (ell - 1) - 1
-        rg.unit_exp = static_cast<uint32_t>(static_cast<uint64_t>(rg.pw[rg.k - 1]) * (rg.ell - 1) - 1);
-    }
-    if (p & 1u) {
-        uint32_t x = p;  // p^-1 mod 2^32 by Newton's iteration (x = p is right to 3 bits)
-        for (int i = 0; i < 5; ++i) x *= 2u - p * x;
-        rg.mont_qinv = 0u - x;
-        rg.mont_r2 = static_cast<uint32_t>(((static_cast<unsigned __int128>(1) << 64)) % p);
-    }
-    const int lu_cols = ring && ring->lu_cols > 0 ? std::min(ring->lu_cols, n) : n;
-
+// Kernel attributes, once per device; the largest cluster the panel kernel can be
+// launched with (0: none).
+int setup_kernels(int device) {
     static OncePerDevice attr;
     // per device: the largest cluster the panel kernel can be launched with (0: none)
     static int cluster_caps[OncePerDevice::kMaxDevices] = {};
@@ -1458,6 +1673,11 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
                                    reinterpret_cast<const void*>(panel_block_kernel<kArithMont31, 128>),
                                    reinterpret_cast<const void*>(panel_block_kernel<kArithMont32, 128>)})
                 HME_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bsm128));
+            const int csm = static_cast<int>(compact_smem_bytes(kMaxPanel));
+            for (const void* fn : {reinterpret_cast<const void*>(panel_compact_kernel<kArithPow2>),
+                                   reinterpret_cast<const void*>(panel_compact_kernel<kArithMont31>),
+                                   reinterpret_cast<const void*>(panel_compact_kernel<kArithMont32>)})
+                HME_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, csm));
             HME_CUDA(cudaFuncSetAttribute(panel_linv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           static_cast<int>(linv_smem_bytes(kMaxPanel))));
             const int wsm = static_cast<int>(sizeof(uint32_t) * (kMaxPanel * kMaxPanel + kWRows * kMaxPanel));
@@ -1499,7 +1719,78 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
         HME_CUDA(cudaFuncSetAttribute(tri_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       static_cast<int>(linv_smem_bytes(kMaxPanel))));
     });
-    const int cluster_cap = cluster_caps[ctx->device];
+    return cluster_caps[device];
+}
+
+int panel_width(const ElimOptions& opt) { return std::max(1, std::min<int>(opt.panel > 0 ? opt.panel : 64, kMaxPanel)); }
+
+// The cluster that runs a panel of rows x w: it doubles (up to the largest the
+// device runs) until each CTA holds at most rows_per_cta rows, and further while
+// a slice does not fit; 0 when the panel needs the grid kernel.
+int panel_cluster_size(int rows, int w, int cluster_cap, const ElimOptions& opt) {
+    int cs = 0;
+    if (opt.panel_kernel != 1 && cluster_cap > 0) {
+        const size_t want = static_cast<size_t>(std::max(1, opt.rows_per_cta > 0 ? opt.rows_per_cta : 32));
+        auto rpc_of = [&](int c) { return (static_cast<size_t>(rows) + c - 1) / c; };
+        auto fits = [&](int c) {
+            const size_t rpc = rpc_of(c);
+            return rpc <= static_cast<size_t>(kClusterRowsMax) &&
+                   cluster_smem_bytes(static_cast<int>(rpc), w) <= static_cast<size_t>(kClusterSmemMax);
+        };
+        int c = 1;
+        while (c < cluster_cap && (rpc_of(c) > want || !fits(c))) c *= 2;
+        if (fits(c)) cs = c;
+    }
+    return cs;
+}
+
+}  // namespace
+
+bool elim_can_keep(hme_ctx* ctx, int m, const ElimOptions& opt) {
+    return panel_cluster_size(m, panel_width(opt), setup_kernels(ctx->device), opt) > 0;
+}
+
+// ---------------------------------------------------------------------------------
+ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld, int m, int n, bool want_rref,
+                       uint32_t* R, size_t ldr, const ElimOptions& opt, const RingSpec* ring) {
+    HME_REQUIRE(m >= 0 && n >= 0, "elim: negative shape");
+    HME_REQUIRE(!(want_rref && ring && ring->k > 1), "elim: the RREF is a field-only object");
+    HME_REQUIRE(!(ring && ring->keep_skipped) || (ring->max_v == 0 && ring->lu_cols == 0 && ld >= 2 * static_cast<size_t>(n)),
+                "elim: keep_skipped needs unit pivots, all columns and room for n more");
+    ElimResult res;
+    res.sign_negative = false;
+    if (m == 0 || n == 0) {
+        if (want_rref && m > 0 && n > 0) HME_CUDA(cudaMemsetAsync(R, 0, 1, ctx->stream));
+        return res;
+    }
+    const int bw = panel_width(opt);
+    const uint32_t p = mp.p;
+    // the ring: F_p by default, Z/ell^k with a pivot valuation bound when given
+    Ring rg{};
+    rg.q = p;
+    rg.barrett = mp.barrett;
+    rg.ell = ring ? ring->ell : p;
+    rg.k = ring ? ring->k : 1;
+    rg.max_v = ring ? ring->max_v : 0;
+    {
+        uint64_t pw = 1;
+        for (uint32_t v = 0; v <= rg.k && v < 32; ++v) {
+            rg.pw[v] = static_cast<uint32_t>(pw);
+            pw *= rg.ell;
+        }
+        HME_REQUIRE(static_cast<uint64_t>(rg.pw[rg.k]) == p || rg.k == 1, "elim: modulus is not ell^k");
+        // phi(ell^k) - 1 = ell^(k-1) (ell - 1) - 1
+        rg.unit_exp = static_cast<uint32_t>(static_cast<uint64_t>(rg.pw[rg.k - 1]) * (rg.ell - 1) - 1);
+    }
+    if (p & 1u) {
+        uint32_t x = p;  // p^-1 mod 2^32 by Newton's iteration (x = p is right to 3 bits)
+        for (int i = 0; i < 5; ++i) x *= 2u - p * x;
+        rg.mont_qinv = 0u - x;
+        rg.mont_r2 = static_cast<uint32_t>(((static_cast<unsigned __int128>(1) << 64)) % p);
+    }
+    const int lu_cols = ring && ring->lu_cols > 0 ? std::min(ring->lu_cols, n) : n;
+
+    const int cluster_cap = setup_kernels(ctx->device);
 
     // device scratch: two sets (by panel parity), so that the next panel, factored ahead on the
     // second stream, never writes the pivot lists the current panel's update still reads
@@ -1510,7 +1801,9 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
         int pivot_cols[kMaxPanel];
         int k;
         int err;       // the device error word as of the panel's end
-        int block_ok;  // the top-block path settled the panel
+        int settled;   // 1: by the top block, 2: by the compact kernel, 0: by a searching kernel (or not yet)
+        int count;     // rows listed for the compact kernel
+        int list[kCompactRows];
         int nonzero;   // the rest of the matrix is not zero
         unsigned bar[2];
     };
@@ -1519,15 +1812,19 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
     const size_t uinv_bytes = sizeof(uint32_t) * kMaxPanel * kMaxPanel;  // the update's M
     uint8_t* base = static_cast<uint8_t*>(
         ctx->ws.get(kSlotElim0, 2 * (scratch_bytes + cand_bytes + uinv_bytes) + 256));
-    // the L21 / W slot at its largest (every panel's rows x pivots fits), so no panel regrows it
-    ctx->ws.get(kSlotElim2, sizeof(uint32_t) * static_cast<size_t>(m) * bw);
+    // the update's left factor W at its largest (every panel's rows x pivots fits), and those that the
+    // compact kernel writes ahead of their panel's update
+    uint32_t* d_W = static_cast<uint32_t*>(ctx->ws.get(kSlotElim2, 3 * sizeof(uint32_t) * static_cast<size_t>(m) * bw));
+    uint32_t* d_Wc[2] = {d_W + static_cast<size_t>(m) * bw, d_W + 2 * static_cast<size_t>(m) * bw};
     Scratch* d_sb[2] = {reinterpret_cast<Scratch*>(base), reinterpret_cast<Scratch*>(base + scratch_bytes)};
     uint32_t* d_candb[2] = {reinterpret_cast<uint32_t*>(base + 2 * scratch_bytes),
                             reinterpret_cast<uint32_t*>(base + 2 * scratch_bytes + cand_bytes)};
     uint32_t* d_uinvb[2] = {reinterpret_cast<uint32_t*>(base + 2 * (scratch_bytes + cand_bytes)),
                             reinterpret_cast<uint32_t*>(base + 2 * (scratch_bytes + cand_bytes) + uinv_bytes)};
-    HME_CUDA(cudaMemsetAsync(d_sb[0]->bar, 0, sizeof(unsigned) * 2, ctx->stream));
-    HME_CUDA(cudaMemsetAsync(d_sb[1]->bar, 0, sizeof(unsigned) * 2, ctx->stream));
+    for (Scratch* d_s : d_sb) {
+        HME_CUDA(cudaMemsetAsync(d_s->bar, 0, sizeof(unsigned) * 2, ctx->stream));
+        HME_CUDA(cudaMemsetAsync(&d_s->count, 0, sizeof(int), ctx->stream));
+    }
     // pinned copies of the two scratch sets (the host reads a panel's pivots without waiting for
     // the other stream's work), the second stream and the events of the lookahead
     const size_t pinned_bytes = 2 * sizeof(Scratch);
@@ -1559,25 +1856,8 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
     // per-kernel timer is on (its events assume one stream)
     const bool allow_lookahead = !opt.no_lookahead && !ctx->timer.on;
 
-    // The cluster kernel when the active rows fit the shared memory of one cluster: the cluster
-    // doubles (up to the largest the device runs) until each CTA holds at most rows_per_cta rows,
-    // and further while a slice does not fit.  Returns the cluster size, 0 for the grid kernel.
-    auto cluster_size = [&](int rows, int w) -> int {
-        int cs = 0;
-        if (opt.panel_kernel != 1 && cluster_cap > 0) {
-            const size_t want = static_cast<size_t>(std::max(1, opt.rows_per_cta > 0 ? opt.rows_per_cta : 32));
-            auto rpc_of = [&](int c) { return (static_cast<size_t>(rows) + c - 1) / c; };
-            auto fits = [&](int c) {
-                const size_t rpc = rpc_of(c);
-                return rpc <= static_cast<size_t>(kClusterRowsMax) &&
-                       cluster_smem_bytes(static_cast<int>(rpc), w) <= static_cast<size_t>(kClusterSmemMax);
-            };
-            int c = 1;
-            while (c < cluster_cap && (rpc_of(c) > want || !fits(c))) c *= 2;
-            if (fits(c)) cs = c;
-        }
-        return cs;
-    };
+    // the cluster kernel when the active rows fit the shared memory of one cluster, else the grid kernel (0)
+    auto cluster_size = [&](int rows, int w) { return panel_cluster_size(rows, w, cluster_cap, opt); };
 
     // the determinant's pivots of the panels that the top block settles (their diagonal in A is 1);
     // 0 where a searching kernel left the pivot in A
@@ -1586,24 +1866,36 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
         d_blkdiag = static_cast<uint32_t*>(ctx->ws.get(kSlotElim4, sizeof(uint32_t) * (static_cast<size_t>(std::max(m, n)) + 16)));
         HME_CUDA(cudaMemsetAsync(d_blkdiag, 0, sizeof(uint32_t) * m, s_main));
     }
-    // the top-block path in automatic mode.  A panel it does not settle costs the attempt and a
-    // second launch (10 + 15 us beside the search's 60 to 270), so the next 3, 7, 15, then
-    // 31 panels go straight to the search (rank-deficient tails, sparse matrices, rings whose columns
-    // run out of units), and the count starts over with the next settled panel
-    const bool use_block = opt.panel_kernel == 0;
-    int block_rest = 0, block_pause = 3;
-    // Over a large field, and after a panel that the block settled, the next one is expected to
-    // succeed; elsewhere the search is launched behind the block and returns at once when the block
-    // settled the panel, so a failed attempt costs no round trip to the host.
-    bool block_sure = rg.k == 1 && p >= (1u << 20);
-    bool block_tried[2] = {false, false}, search_behind[2] = {false, false};
-    // The panel [c0, c0 + w) of the active rows [r0, m) on `st`: the top-block path when it is tried
-    // (the host launches the search afterwards if the block did not settle the panel), else the
-    // searching kernel.  Its pivots and the error word land in h_sb[par] and ev_panel[par] is
-    // recorded.  Returns the cluster size the search takes (0: grid kernel), the SMs a GEMM beside
-    // the panel leaves free.
+    // The panel's kernels in automatic mode: the top block, then the compact search of the non-zero
+    // rows, then the search over all rows.  A failed attempt costs 10 us beside the search's 60 to 270,
+    // so after one the next 3, 7, 15, then 31 panels pass over that kernel (the top block: rank-deficient
+    // tails, sparse matrices, rings whose columns run out of units; the compact rows: dense matrices),
+    // and the count starts over with the next panel that it settles.  What is launched behind an
+    // attempt returns at once when the attempt settled the panel, so a failure costs no round trip to
+    // the host; behind an attempt that is expected to succeed -- the kernel's last one did, or it is the
+    // top block over a large field -- nothing is launched, and the host launches the rest if it must.
+    const bool automatic = opt.panel_kernel == 0;
+    struct Attempt {
+        int rest = 0, pause = 3;
+        bool sure = false;
+        void settled() {
+            pause = 3;
+            sure = true;
+        }
+        void failed() {
+            rest = pause;
+            pause = std::min(31, 2 * pause + 1);
+            sure = false;
+        }
+    } block, compact;
+    block.sure = rg.k == 1 && p >= (1u << 20);
+    const bool keep = ring && ring->keep_skipped;
+    bool block_tried[2] = {false, false}, compact_tried[2] = {false, false}, search_run[2] = {false, false};
+    // The panel [c0, c0 + w) of the active rows [r0, m) on `st`, from kernel `from` on (0 the top
+    // block, 1 the compact rows, 2 the search).  Its pivots and the error word land in h_sb[par] and
+    // ev_panel[par] is recorded.  Returns the SMs that a GEMM beside the panel leaves free.
     cudaStream_t panel_stream[2] = {s_main, s_main};
-    auto launch_panel = [&](int c0, int w, int r0, int par, cudaStream_t st, bool search_only) -> int {
+    auto launch_panel = [&](int c0, int w, int r0, int par, cudaStream_t st, int from) -> int {
         Scratch* d_s = d_sb[par];
         const cudaStream_t saved = ctx->stream;
         ctx->stream = st;  // HME_TIMED brackets the launch on the launching stream
@@ -1623,11 +1915,12 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
         pa.k_out = &d_s->k;
         pa.bar = d_s->bar;
         pa.err = ctx->d_err;
+        pa.keep = keep ? 1 : 0;
         const int rows = m - r0;
-        // the top-block path first; the searching kernel below runs only when the block did not
-        // settle the panel
-        const bool try_block = !search_only && use_block && block_rest == 0;
-        if (!search_only && use_block && block_rest > 0) --block_rest;
+        int busy = 0;  // SMs the panel's kernels take
+        bool more = true;  // the kernels after the ones launched so far may be needed
+        const bool try_block = from == 0 && automatic && block.rest == 0;
+        if (from == 0 && block.rest > 0) --block.rest;
         block_tried[par] = try_block;
         if (try_block) {
             BlockArgs ba{};
@@ -1641,7 +1934,7 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
             ba.pivot_rows = d_s->pivot_rows;
             ba.pivot_cols = d_s->pivot_cols;
             ba.k_out = &d_s->k;
-            ba.ok = &d_s->block_ok;
+            ba.ok = &d_s->settled;
             ba.binv = d_uinvb[par];
             ba.diag = d_blkdiag;
             // 64 row slots where a zero pivot is rare (chance about 64/p per panel), 32 spare rows over
@@ -1666,12 +1959,50 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
             }
             HME_CUDA(cudaGetLastError());
         }
+        if (try_block) {
+            more = !block.sure;
+            busy = 1;
+        }
+        const bool try_compact = more && from <= 1 && automatic && compact.rest == 0;
+        if (more && from <= 1 && compact.rest > 0) --compact.rest;
+        compact_tried[par] = try_compact;
+        if (try_compact) {
+            CompactArgs ca{};
+            ca.A = A;
+            ca.ld = ld;
+            ca.m = m;
+            ca.r0 = r0;
+            ca.c0 = c0;
+            ca.w = w;
+            ca.R = rg;
+            ca.list = d_s->list;
+            ca.count = &d_s->count;
+            ca.after_block = try_block ? 1 : 0;
+            ca.ok = &d_s->settled;
+            ca.pivot_rows = d_s->pivot_rows;
+            ca.pivot_cols = d_s->pivot_cols;
+            ca.k_out = &d_s->k;
+            ca.W = d_Wc[par];
+            ca.ldw = bw;
+            HME_TIMED(ctx, "panel_rows", panel_rows_kernel<<<(rows + 7) / 8, 256, 0, st>>>(ca));
+            auto launch_compact = [&](auto kern) {
+                HME_TIMED(ctx, "panel_compact", kern<<<1, 1024, compact_smem_bytes(w), st>>>(ca));
+            };
+            if (rg.ell == 2) launch_compact(panel_compact_kernel<kArithPow2>);
+            else if (p < (1u << 31)) launch_compact(panel_compact_kernel<kArithMont31>);
+            else launch_compact(panel_compact_kernel<kArithMont32>);
+            HME_CUDA(cudaGetLastError());
+            more = !compact.sure;
+            busy = 1;
+        }
         const int cs = cluster_size(rows, w);
         HME_REQUIRE(opt.panel_kernel < 2 || cs > 0, "elim: the panel does not fit one cluster");
-        search_behind[par] = try_block && !block_sure;
-        if (search_behind[par]) pa.skip = &d_s->block_ok;
-        if (try_block && !search_behind[par]) {
-            // no search behind the block: the host relaunches the panel with the search if needed
+        HME_REQUIRE(!keep || cs > 0 || !more, "elim: the panel is too tall for the cluster kernel");
+        search_run[par] = more;
+        if (more) busy = cs;
+        if (try_block || try_compact) pa.skip = &d_s->settled;
+        if (!more) {
+            // the host launches the panel's other kernels if the attempt fails
         } else if (cs > 0) {
             const int rpc = static_cast<int>((static_cast<size_t>(rows) + cs - 1) / cs);
             cudaLaunchConfig_t cfg{};
@@ -1723,11 +2054,21 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
         HME_CUDA(cudaMemcpyAsync(&h_sb[par], d_s, sizeof(Scratch), cudaMemcpyDeviceToHost, st));
         HME_CUDA(cudaEventRecord(ev_panel[par], st));
         ctx->stream = saved;
-        return cs;
+        return busy;
     };
 
     std::vector<int> pivots;
     pivots.reserve(std::min(m, n));
+    // keep mode: the pivotless columns of the panels so far, appended right of the matrix, where the
+    // later updates reach them
+    int app = 0;
+    auto append = [&](int c0, int w, int row0, int par, int k) {
+        if (k == w || row0 >= m) return;
+        HME_TIMED(ctx, "append_cols", append_cols_kernel<<<std::min((m - row0 + 7) / 8, 8 * ctx->num_sms), 256, 0, s_main>>>(
+                                          A, ld, row0, m - row0, c0, w, d_sb[par]->pivot_cols, k, n + app));
+        HME_CUDA(cudaGetLastError());
+        app += w - k;
+    };
     int r0 = 0;
     int next_look = 0;  // panel count before which a pivotless panel does not look over the rest
     int look_gap = 1, panels = 0;
@@ -1735,36 +2076,32 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
     bool launched = false;  // the panel at c0 was already factored ahead (on the second stream)
     for (int c0 = 0; c0 < lu_cols && r0 < m; c0 += bw) {
         const int w = std::min(bw, lu_cols - c0);
-        if (!launched) launch_panel(c0, w, r0, par, s_main, false);
+        if (!launched) launch_panel(c0, w, r0, par, s_main, 0);
         launched = false;
         HME_CUDA(cudaEventSynchronize(ev_panel[par]));
-        if (block_tried[par] && !h_sb[par].block_ok) {
-            // the top block did not settle the panel (nothing was written): the search, on the
-            // panel's stream; the main stream's later work waits for it too
-            block_rest = block_pause;
-            block_pause = std::min(31, 2 * block_pause + 1);
-            if (search_behind[par]) {
-                block_tried[par] = false;  // the search has run
-            } else {
-                launch_panel(c0, w, r0, par, panel_stream[par], true);
-                if (panel_stream[par] != s_main) HME_CUDA(cudaStreamWaitEvent(s_main, ev_panel[par], 0));
-                HME_CUDA(cudaEventSynchronize(ev_panel[par]));
-            }
-            block_sure = false;
+        // what settled the panel: 1 the top block, 2 the compact rows, 0 the search
+        int by = 0;
+        for (;;) {
+            by = block_tried[par] || compact_tried[par] ? h_sb[par].settled : 0;
+            if (block_tried[par]) by == 1 ? block.settled() : block.failed();
+            if (compact_tried[par] && by != 1) by == 2 ? compact.settled() : compact.failed();
+            if (by != 0 || search_run[par]) break;
+            // an attempt that was expected to succeed did not (nothing was written): the panel's other
+            // kernels, on its stream; the main stream's later work waits for them too
+            launch_panel(c0, w, r0, par, panel_stream[par], compact_tried[par] ? 2 : 1);
+            if (panel_stream[par] != s_main) HME_CUDA(cudaStreamWaitEvent(s_main, ev_panel[par], 0));
+            HME_CUDA(cudaEventSynchronize(ev_panel[par]));
         }
         const Scratch& h_s = h_sb[par];
         if (h_s.err != 0) check_device_error(ctx);  // reports the timeout (and clears the word)
-        if (block_tried[par]) {
-            block_pause = 3;
-            block_sure = true;
-        }
         // the statistics count a top block that looks for most of its pivots (a field of fewer than 256
         // elements, a ring) as searched
-        if (block_tried[par] && rg.k == 1 && p >= 256) ++ctx->elim_block_panels;
+        if (by == 1 && rg.k == 1 && p >= 256) ++ctx->elim_block_panels;
         else ++ctx->elim_search_panels;
         const int k = h_s.k;
         ++panels;
         if (k == 0) {
+            if (keep) append(c0, w, r0, par, 0);
             // no pivot in the panel: nothing moved, the next panel starts at r0 -- unless nothing is
             // left (one pass over the rest, against a panel's search each; after a pass that found
             // something only every 2nd, 4th, .. pivotless panel asks again)
@@ -1793,8 +2130,8 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
         const int c1 = c0 + w;
         const int below = m - r0 - k;
         const int* d_pcols = d_sb[par]->pivot_cols;
-        const bool blk = block_tried[par] && h_s.block_ok;
-        uint32_t* Wf = nullptr;
+        uint32_t* Wf = by == 2 ? d_Wc[par] : nullptr;
+        const int ldw = by == 2 ? bw : k;
         // the update of columns [ca, cb): row moves (from c0 on), then [A12; A22] += W A12 on a
         // tensor-core variant (it reads A12 through its limb planes, so C may alias it)
         auto update = [&](int ca, int cb, int sm_cap) {
@@ -1808,12 +2145,12 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
             if (cb <= ua) return;
             if (!Wf) {
                 uint32_t* mul = d_uinvb[par];
-                if (!blk) {
+                if (by == 0) {
                     HME_TIMED(ctx, "panel_linv", panel_linv_kernel<<<1, 512, linv_smem_bytes(k), s_main>>>(
                                                      A, ld, r0, d_pcols, k, p, mp.barrett, mul));
                     HME_CUDA(cudaGetLastError());
                 }
-                Wf = static_cast<uint32_t*>(ctx->ws.get(kSlotElim2, sizeof(uint32_t) * static_cast<size_t>(rows) * k));
+                Wf = d_W;
                 const int g = (rows + kWRows - 1) / kWRows;
                 const size_t wsm = sizeof(uint32_t) * (((static_cast<size_t>(k) * k + 3) & ~size_t(3)) +
                                                        static_cast<size_t>(kWRows) * ((k + 3) & ~3));
@@ -1827,7 +2164,7 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
             }
             ctx->gemm_sm_cap = sm_cap;
             uint32_t* C12 = A + static_cast<size_t>(r0) * ld + ua;
-            gemm_u32_variant(ctx, mp, rows, cb - ua, k, Wf, k, C12, ld, C12, ld, HME_ADD,
+            gemm_u32_variant(ctx, mp, rows, cb - ua, k, Wf, ldw, C12, ld, C12, ld, HME_ADD,
                              gemm_default_variant(ctx, mp, rows, cb - ua));
             ctx->gemm_sm_cap = 0;
         };
@@ -1837,16 +2174,17 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
         const bool next = allow_lookahead && c1 < lu_cols && below > 0 && nw > 0 && cluster_size(below, nw) > 0;
         if (next) {
             // LOOKAHEAD: the next panel's columns first; that panel is factored on the second stream
-            // while the rest of this update runs here, the GEMM leaving the cluster's SMs free
+            // while the rest of this update runs here, the GEMM leaving the panel's SMs free
             update(c0, c1 + nw, 0);
             HME_CUDA(cudaEventRecord(ev_next, s_main));
             HME_CUDA(cudaStreamWaitEvent(s_aux, ev_next, 0));
-            const int cs_next = launch_panel(c1, nw, r0 + k, par ^ 1, s_aux, false);
-            update(c1 + nw, n, cs_next > 0 ? std::max(1, ctx->num_sms - cs_next) : 0);
+            const int busy = launch_panel(c1, nw, r0 + k, par ^ 1, s_aux, 0);
+            update(c1 + nw, n + app, std::max(1, ctx->num_sms - busy));
             launched = true;
         } else {
-            update(c0, n, 0);
+            update(c0, n + app, 0);
         }
+        if (keep) append(c0, w, r0 + k, par, k);
         // the main stream's later work (the next panel's update) follows the lookahead panel
         if (launched) HME_CUDA(cudaStreamWaitEvent(s_main, ev_panel[par ^ 1], 0));
         r0 += k;
@@ -1855,6 +2193,7 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
     HME_CUDA(cudaStreamSynchronize(s_aux));
     res.rank = r0;
     res.pivots = pivots;
+    res.appended = app;
 
     // determinant factors: the U diagonal
     if (opt.want_diag && res.rank > 0) {

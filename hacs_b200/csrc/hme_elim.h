@@ -13,6 +13,7 @@ struct ElimResult {
     std::vector<int> pivots;      // pivot columns, ascending (the column rank profile)
     std::vector<uint32_t> diag;   // U[t][pivots[t]] when ElimOptions::want_diag
     bool sign_negative = false;   // parity of the row permutation applied
+    int appended = 0;             // RingSpec::keep_skipped: pivotless columns right of the matrix
 };
 
 // Elimination over Z/q, q = ell^k (mp.p == q): pivots of valuation <= max_v
@@ -23,6 +24,12 @@ struct RingSpec {
     uint32_t ell = 0, k = 1;
     uint32_t max_v = 0;
     int lu_cols = 0;
+    // max_v = 0 only: a column without a unit pivot is left out but goes on being
+    // updated, as the next column right of the matrix (A has room for them: ld
+    // >= 2 n); ElimResult::appended counts them.  At the end rows [rank, m) at
+    // columns [n, n + appended) are the Schur complement of the pivot columns
+    // (its other columns, if the elimination ended early, are zero).
+    bool keep_skipped = false;
 };
 
 // Factor A (m x n, row-major, ld, device memory; destroyed) and, when
@@ -32,6 +39,10 @@ struct RingSpec {
 // and rows [rank, m) the Schur complement of the factored columns.
 ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld, int m, int n, bool want_rref,
                        uint32_t* R, size_t ldr, const ElimOptions& opt, const RingSpec* ring = nullptr);
+
+// Whether keep_skipped eliminations of m rows run (the tallest panel must fit the
+// cluster kernel under these options).
+bool elim_can_keep(hme_ctx* ctx, int m, const ElimOptions& opt);
 
 }  // namespace hme
 
