@@ -59,7 +59,7 @@ template <int L, int BN, int KB>
 __global__ void __launch_bounds__(gemm_threads(L), 1)
     grouped_limb_gemm_kernel(const GroupedProblem* __restrict__ probs, const int* __restrict__ tile_prob,
                              int total_tiles_arg, const int* __restrict__ d_total, const EpiRed red, int* err) {
-    long_tiles<L, BN, KB>(ProductTable<BN>{probs, tile_prob, total_tiles_arg, d_total}, red, err);
+    long_tiles<L, BN, KB>(ProductTable<BN>{probs, tile_prob, total_tiles_arg, d_total}, ResidueEpilogue<L, BN, KB>{red}, err);
 }
 
 // Every product's K fits one k-block of KB bytes.

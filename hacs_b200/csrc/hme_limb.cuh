@@ -83,8 +83,8 @@ struct EpiRed {
     uint64_t barrett;
 };
 
-// The constants for products whose K (per launch) is at most kc.
-inline EpiRed make_epi(const ModParams& mp, uint64_t kc) {
+// The constants for sums up to `bound` (below 2^64) mod p.
+inline EpiRed make_epi_bound(const ModParams& mp, unsigned __int128 bound) {
     EpiRed r{};
     r.p = mp.p;
     r.barrett = mp.barrett;
@@ -92,10 +92,6 @@ inline EpiRed make_epi(const ModParams& mp, uint64_t kc) {
         r.fast = 1;
         return r;
     }
-    const int L = static_cast<int>(mp.limbs);
-    unsigned __int128 bound = 0;  // the largest s
-    for (int j = 0; j < L; ++j)
-        bound += (static_cast<unsigned __int128>(L) * 255u * 255u * kc) << (8 * j);
     int sb = 0;
     while (sb < 128 && (bound >> sb) != 0) ++sb;
     int b = 0;
@@ -107,6 +103,26 @@ inline EpiRed make_epi(const ModParams& mp, uint64_t kc) {
     r.fast = mp.p < (1u << 31) && r.sh1 <= b - 2 ? 1 : 0;
     return r;
 }
+// The constants for products whose K (per launch) is at most kc.
+inline EpiRed make_epi(const ModParams& mp, uint64_t kc) {
+    unsigned __int128 bound = 0;
+    for (uint32_t j = 0; j < mp.limbs; ++j)
+        bound += (static_cast<unsigned __int128>(mp.limbs) * 255u * 255u * kc) << (8 * j);
+    return make_epi_bound(mp, bound);
+}
+
+template <bool FAST>
+__device__ __forceinline__ uint32_t epi_reduce_u64(uint64_t s, const EpiRed& r) {
+    if constexpr (FAST) {
+        const uint32_t lo = static_cast<uint32_t>(s);
+        const uint32_t hi = __funnelshift_r(lo, static_cast<uint32_t>(s >> 32), r.sh1);
+        const uint32_t q = __umulhi(hi, r.M) >> r.sh2;
+        const uint32_t x = lo - q * r.p;
+        return min(x, x - r.p);
+    } else {
+        return reduce_u64(s, r.p, r.barrett);
+    }
+}
 
 template <int L, bool FAST>
 __device__ __forceinline__ uint32_t epi_reduce(uint32_t v0, uint32_t v1, uint32_t v2, uint32_t v3, const EpiRed& r) {
@@ -114,15 +130,7 @@ __device__ __forceinline__ uint32_t epi_reduce(uint32_t v0, uint32_t v1, uint32_
     if (L > 1) s += static_cast<uint64_t>(v1) * 256u;
     if (L > 2) s += static_cast<uint64_t>(v2) * 65536u;
     if (L > 3) s += static_cast<uint64_t>(v3) * 16777216u;
-    if constexpr (FAST) {
-        const uint32_t lo = static_cast<uint32_t>(s);
-        const uint32_t hi = L == 1 ? lo : __funnelshift_r(lo, static_cast<uint32_t>(s >> 32), r.sh1);
-        const uint32_t q = __umulhi(hi, r.M) >> r.sh2;
-        const uint32_t x = lo - q * r.p;
-        return min(x, x - r.p);
-    } else {
-        return reduce_u64(s, r.p, r.barrett);
-    }
+    return epi_reduce_u64<FAST>(s, r);
 }
 
 // How C and the reduced value combine, one form for the three ops: with old = 0
@@ -356,10 +364,23 @@ __device__ __forceinline__ void epilogue_tiles(const Src& src, int first, int en
     }
 }
 
+// An epilogue of a pipeline: what the epilogue warps do with the accumulators.
+template <int L, int BN, int KB>
+struct ResidueEpilogue {  // residues mod p into C
+    const EpiRed& red;
+    template <class Src>
+    __device__ __forceinline__ void run(const Src& src, int first, int end, int step, int warp, int lane,
+                                        uint32_t tmem_base, uint32_t* epi_stage, uint64_t* acc_full,
+                                        uint64_t* acc_empty, volatile int* abort_flag, int* err) const {
+        epilogue_tiles<L, BN, KB>(src, first, end, step, warp, lane, tmem_base, epi_stage, acc_full, acc_empty,
+                                  abort_flag, red, err);
+    }
+};
+
 // Products of several k-blocks: A and B blocks stream through one ring, tiles
 // are taken with the stride of the grid.
-template <int L, int BN, int KB, class Src>
-__device__ __forceinline__ void long_tiles(const Src& src, const EpiRed& red, int* err) {
+template <int L, int BN, int KB, class Src, class Epi>
+__device__ __forceinline__ void long_tiles(const Src& src, const Epi& epi, int* err) {
     using CF = Cfg<L, BN, KB>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -476,8 +497,8 @@ __device__ __forceinline__ void long_tiles(const Src& src, const EpiRed& red, in
             }
         }
     } else {
-        epilogue_tiles<L, BN, KB>(src, blockIdx.x, total_tiles, gridDim.x, warp, lane, tmem_base, epi_stage, acc_full,
-                                  acc_empty, abort_flag, red, err);
+        epi.run(src, blockIdx.x, total_tiles, gridDim.x, warp, lane, tmem_base, epi_stage, acc_full, acc_empty,
+                abort_flag, err);
     }
 
     tc_fence_before();

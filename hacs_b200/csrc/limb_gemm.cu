@@ -95,7 +95,7 @@ template <int L, int BN, int KB = kBK>
 __global__ void __launch_bounds__(gemm_threads(L), 1)
     limb_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                      const __grid_constant__ GemmArgs g) {
-    long_tiles<L, BN, KB>(OneProduct<BN, false>{&tmA, &tmB, g}, g.red, g.err);
+    long_tiles<L, BN, KB>(OneProduct<BN, false>{&tmA, &tmB, g}, ResidueEpilogue<L, BN, KB>{g.red}, g.err);
 }
 
 // One k-block of KB bytes holds K.
@@ -307,15 +307,14 @@ int gemm_default_variant(const hme_ctx* ctx, const ModParams& mp, uint32_t m, ui
 
 int limb_kp(uint32_t k) { return static_cast<int>((k + kblock_for(k) - 1) / kblock_for(k) * kblock_for(k)); }
 
-void gemm_u32_planes(hme_ctx* ctx, const ModParams& mp, uint32_t m, uint32_t n, uint32_t k, int Kp, uint8_t* pa,
-                     uint64_t a_plane, uint8_t* pb, uint32_t* C, size_t ldc, int op) {
-    const bool narrow = gemm_default_variant(ctx, mp, m, n) == kVariantNarrow;
-    launch_gemm_variant(ctx, mp, narrow, m, n, k, Kp, pa, a_plane, pb, C, ldc, op, true);
-}
-
 void gemm_u32_device(hme_ctx* ctx, const ModParams& mp, uint32_t m, uint32_t n, uint32_t k, const uint32_t* A,
                      size_t lda, const uint32_t* B, size_t ldb, uint32_t* C, size_t ldc, int op) {
     int v = ctx->fixed_variant;
+    if (v < 0 && ctx->sched_policy == 0 && (op == HME_SET || op == HME_ADD || op == HME_SUB) && A && B && C &&
+        lda >= k && ldb >= n && ldc >= n && rns_gemm_u32_pays(mp, m, n, k)) {
+        rns_gemm_u32_device(ctx, mp, m, n, k, A, lda, B, ldb, C, ldc, op);
+        return;
+    }
     if (v < 0) v = sched_variant(ctx, mp, m, n, k);
     gemm_u32_variant(ctx, mp, m, n, k, A, lda, B, ldb, C, ldc, op, v);
 }
