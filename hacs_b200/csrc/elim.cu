@@ -743,6 +743,14 @@ struct BlockArgs {
     int* ok;          // out: 1 when the top block settled the panel, else 0
     uint32_t* binv;   // out: B^-1 (nb x nb, row-major)
     uint32_t* diag;   // out when non-null: the classical pivots, at r0 ..
+    // work may be queued behind this panel before its outcome is known: set to the panel's number when
+    // the host must look at the panel (no pivot somewhere; with in_order, pivot rows that have to move);
+    // a panel launched after that does nothing
+    int* fail;
+    int seq;
+    int in_order;
+    const int* err;   // the context's error word
+    int* err_out;     // its value at the panel's end
 };
 
 // The padded size of an n x n triangular inverse: a power of two >= 8.
@@ -902,6 +910,7 @@ __global__ void __launch_bounds__(4 * RS) panel_block_kernel(const BlockArgs a) 
     __shared__ int s_cand[2][RS / 32];
     constexpr int NT = 4 * RS, NW = NT / 32;
     constexpr int WC = RS == 128 ? 4 : 2;  // panels of up to 128 or 64 columns: 32 WC
+    if (*a.fail != 0) return;
     const int w = a.w, rows = a.m - a.r0, nb = min(w, rows), nbr = min(RS, rows);
     const Ring& R = a.R;
     const int ls = block_stride(w), nq = (w + 3) / 4;
@@ -992,7 +1001,11 @@ __global__ void __launch_bounds__(4 * RS) panel_block_kernel(const BlockArgs a) 
             if (ok && 4 * u + 3 < ns) ok = step(std::integral_constant<int, 3>{}, u);
         }
         if (!ok) {
-            if (tid == 0) *a.ok = 0;
+            if (tid == 0) {
+                *a.ok = 0;
+                *a.fail = a.seq;
+                *a.err_out = *a.err;
+            }
             return;
         }
         if (tid == 0) s_V[sub] = V;
@@ -1098,9 +1111,12 @@ __global__ void __launch_bounds__(4 * RS) panel_block_kernel(const BlockArgs a) 
             a.diag[a.r0 + tid] = mod_mul(s_w[tid], unit_inverse(s, R), R.q, R.barrett);
         }
     }
+    const bool moved = tid < nb && s_prow[tid] != tid;
+    if (__syncthreads_or(moved) && a.in_order && tid == 0) *a.fail = a.seq;
     if (tid == 0) {
         *a.k_out = nb;
         *a.ok = 1;
+        *a.err_out = *a.err;
     }
 }
 
@@ -1379,7 +1395,9 @@ constexpr int kWRowsPerWarp = 4;
 template <int WMAX>
 __global__ void __launch_bounds__(256) panel_w_kernel(const uint32_t* __restrict__ A, uint64_t ld, int r0, int m,
                                                       const int* __restrict__ pcols, int nb, const uint32_t* __restrict__ binv, uint32_t q,
-                                                      uint64_t barrett, uint32_t* __restrict__ W) {
+                                                      uint64_t barrett, const Skip skip,
+                                                      uint32_t* __restrict__ W) {
+    if (skip.stands()) return;
     extern __shared__ __align__(16) uint32_t s_wk[];
     const int rb = r0 + static_cast<int>(blockIdx.x) * kWRows;  // first row of this CTA
     const int nr = min(kWRows, m - rb);
@@ -1489,7 +1507,9 @@ __global__ void __launch_bounds__(256) panel_w_kernel(const uint32_t* __restrict
 constexpr int kMoveCols = 32;
 
 __global__ void __launch_bounds__(256) move_pivot_rows_kernel(uint32_t* __restrict__ A, uint64_t ld, int r0, int k,
-                                                              const int* __restrict__ prow, int ca, int cb) {
+                                                              const int* __restrict__ prow, int ca, int cb,
+                                                              const Skip skip) {
+    if (skip.stands()) return;
     __shared__ uint32_t buf[2 * kMaxPanel][kMoveCols];
     __shared__ int s_src[2 * kMaxPanel], s_dst[2 * kMaxPanel];
     __shared__ unsigned char s_isp[kMaxPanel];
@@ -1792,8 +1812,10 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
 
     const int cluster_cap = setup_kernels(ctx->device);
 
-    // device scratch: two sets (by panel parity), so that the next panel, factored ahead on the
-    // second stream, never writes the pivot lists the current panel's update still reads
+    // device scratch: a ring of four sets, so that panels factored ahead on the second stream, and
+    // queued before the host has seen the ones before them, never write the pivot lists that an
+    // update still reads
+    constexpr int kRing = 4;
     const int grid_cap = std::max(1, std::min(ctx->num_sms, opt.panel_ctas > 0 ? opt.panel_ctas : ctx->num_sms));
     struct Scratch {
         unsigned long long piv_slot[kMaxPanel];
@@ -1803,6 +1825,7 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
         int err;       // the device error word as of the panel's end
         int settled;   // 1: by the top block, 2: by the compact kernel, 0: by a searching kernel (or not yet)
         int count;     // rows listed for the compact kernel
+        int fail;      // ring entry 0 only: queued work stands still (BlockArgs::fail)
         int list[kCompactRows];
         int nonzero;   // the rest of the matrix is not zero
         unsigned bar[2];
@@ -1811,23 +1834,25 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
     const size_t cand_bytes = sizeof(uint32_t) * 2 * static_cast<size_t>(grid_cap) * kMaxPanel;
     const size_t uinv_bytes = sizeof(uint32_t) * kMaxPanel * kMaxPanel;  // the update's M
     uint8_t* base = static_cast<uint8_t*>(
-        ctx->ws.get(kSlotElim0, 2 * (scratch_bytes + cand_bytes + uinv_bytes) + 256));
+        ctx->ws.get(kSlotElim0, kRing * (scratch_bytes + cand_bytes + uinv_bytes) + 256));
     // the update's left factor W at its largest (every panel's rows x pivots fits), and those that the
     // compact kernel writes ahead of their panel's update
-    uint32_t* d_W = static_cast<uint32_t*>(ctx->ws.get(kSlotElim2, 3 * sizeof(uint32_t) * static_cast<size_t>(m) * bw));
-    uint32_t* d_Wc[2] = {d_W + static_cast<size_t>(m) * bw, d_W + 2 * static_cast<size_t>(m) * bw};
-    Scratch* d_sb[2] = {reinterpret_cast<Scratch*>(base), reinterpret_cast<Scratch*>(base + scratch_bytes)};
-    uint32_t* d_candb[2] = {reinterpret_cast<uint32_t*>(base + 2 * scratch_bytes),
-                            reinterpret_cast<uint32_t*>(base + 2 * scratch_bytes + cand_bytes)};
-    uint32_t* d_uinvb[2] = {reinterpret_cast<uint32_t*>(base + 2 * (scratch_bytes + cand_bytes)),
-                            reinterpret_cast<uint32_t*>(base + 2 * (scratch_bytes + cand_bytes) + uinv_bytes)};
-    for (Scratch* d_s : d_sb) {
-        HME_CUDA(cudaMemsetAsync(d_s->bar, 0, sizeof(unsigned) * 2, ctx->stream));
-        HME_CUDA(cudaMemsetAsync(&d_s->count, 0, sizeof(int), ctx->stream));
+    const size_t w_words = static_cast<size_t>(m) * bw;
+    uint32_t* d_W = static_cast<uint32_t*>(ctx->ws.get(kSlotElim2, (1 + kRing) * sizeof(uint32_t) * w_words));
+    Scratch* d_sb[kRing];
+    uint32_t *d_candb[kRing], *d_uinvb[kRing], *d_Wc[kRing];
+    for (int i = 0; i < kRing; ++i) {
+        d_sb[i] = reinterpret_cast<Scratch*>(base + i * scratch_bytes);
+        d_candb[i] = reinterpret_cast<uint32_t*>(base + kRing * scratch_bytes + i * cand_bytes);
+        d_uinvb[i] = reinterpret_cast<uint32_t*>(base + kRing * (scratch_bytes + cand_bytes) + i * uinv_bytes);
+        d_Wc[i] = d_W + (1 + i) * w_words;
+        HME_CUDA(cudaMemsetAsync(d_sb[i]->bar, 0, sizeof(unsigned) * 2, ctx->stream));
+        HME_CUDA(cudaMemsetAsync(&d_sb[i]->count, 0, 2 * sizeof(int), ctx->stream));  // count, fail
     }
-    // pinned copies of the two scratch sets (the host reads a panel's pivots without waiting for
+    int* d_fail = &d_sb[0]->fail;
+    // pinned copies of the scratch sets (the host reads a panel's pivots without waiting for
     // the other stream's work), the second stream and the events of the lookahead
-    const size_t pinned_bytes = 2 * sizeof(Scratch);
+    const size_t pinned_bytes = kRing * sizeof(Scratch);
     if (ctx->elim_pinned_bytes < pinned_bytes) {
         if (ctx->elim_pinned) {
             HME_CUDA(cudaDeviceSynchronize());
@@ -1845,12 +1870,13 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
         HME_CUDA(cudaDeviceGetStreamPriorityRange(&lo, &hi));
         HME_CUDA(cudaStreamCreateWithPriority(&ctx->aux_stream, cudaStreamNonBlocking, hi));
     }
-    while (ctx->elim_ev.size() < 3) {
+    while (ctx->elim_ev.size() < 1 + 2 * kRing) {
         cudaEvent_t e;
         HME_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         ctx->elim_ev.push_back(e);
     }
-    cudaEvent_t ev_next = ctx->elim_ev[0], ev_panel[2] = {ctx->elim_ev[1], ctx->elim_ev[2]};
+    // ev_panel: the panel's kernels are done; ev_host: its results are in pinned memory
+    const cudaEvent_t ev_next = ctx->elim_ev[0], *ev_panel = &ctx->elim_ev[1], *ev_host = &ctx->elim_ev[1 + kRing];
     const cudaStream_t s_main = ctx->stream, s_aux = ctx->aux_stream;
     // lookahead only where it can overlap: the cluster kernel (a few SMs), and not while the
     // per-kernel timer is on (its events assume one stream)
@@ -1890,11 +1916,14 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
     } block, compact;
     block.sure = rg.k == 1 && p >= (1u << 20);
     const bool keep = ring && ring->keep_skipped;
-    bool block_tried[2] = {false, false}, compact_tried[2] = {false, false}, search_run[2] = {false, false};
+    bool block_tried[kRing] = {}, compact_tried[kRing] = {}, search_run[kRing] = {};
+    // a block over a large field finds its pivots in row order almost always: nothing is queued for moves
+    const bool in_order = rg.k == 1 && p >= (1u << 20);
     // The panel [c0, c0 + w) of the active rows [r0, m) on `st`, from kernel `from` on (0 the top
-    // block, 1 the compact rows, 2 the search).  Its pivots and the error word land in h_sb[par] and
-    // ev_panel[par] is recorded.  Returns the SMs that a GEMM beside the panel leaves free.
-    cudaStream_t panel_stream[2] = {s_main, s_main};
+    // block, 1 the compact rows, 2 the search).  Its pivots and the error word land in h_sb[par];
+    // ev_panel[par] and ev_host[par] are recorded.  Returns the SMs that a GEMM beside the panel leaves free.
+    int seq = 0, panel_seq[kRing] = {};  // numbers of the top-block attempts
+    cudaStream_t panel_stream[kRing] = {s_main, s_main, s_main, s_main};
     auto launch_panel = [&](int c0, int w, int r0, int par, cudaStream_t st, int from) -> int {
         Scratch* d_s = d_sb[par];
         const cudaStream_t saved = ctx->stream;
@@ -1937,6 +1966,12 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
             ba.ok = &d_s->settled;
             ba.binv = d_uinvb[par];
             ba.diag = d_blkdiag;
+            ba.fail = d_fail;
+            ba.seq = ++seq;
+            panel_seq[par] = seq;
+            ba.in_order = in_order ? 1 : 0;
+            ba.err = ctx->d_err;
+            ba.err_out = &d_s->err;
             // 64 row slots where a zero pivot is rare (chance about 64/p per panel), 32 spare rows over
             // smaller fields and rings
             const int rs = w > 64 ? 128 : rg.k == 1 && p >= (1u << 20) ? 64 : 96;
@@ -2049,10 +2084,13 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
                       HME_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(panel_factor_kernel), want_grid,
                                                            kPanelThreads, args, dyn, st)));
         }
-        // the panel's error word next to its pivots, then the pivots to pinned memory
-        HME_CUDA(cudaMemcpyAsync(&d_s->err, ctx->d_err, sizeof(int), cudaMemcpyDeviceToDevice, st));
-        HME_CUDA(cudaMemcpyAsync(&h_sb[par], d_s, sizeof(Scratch), cudaMemcpyDeviceToHost, st));
         HME_CUDA(cudaEventRecord(ev_panel[par], st));
+        // the panel's error word next to its pivots (the block kernel has written it), then the pivots to
+        // pinned memory
+        if (try_compact || more)
+            HME_CUDA(cudaMemcpyAsync(&d_s->err, ctx->d_err, sizeof(int), cudaMemcpyDeviceToDevice, st));
+        HME_CUDA(cudaMemcpyAsync(&h_sb[par], d_s, sizeof(Scratch), cudaMemcpyDeviceToHost, st));
+        HME_CUDA(cudaEventRecord(ev_host[par], st));
         ctx->stream = saved;
         return busy;
     };
@@ -2069,43 +2107,174 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
         HME_CUDA(cudaGetLastError());
         app += w - k;
     };
-    int r0 = 0;
+    // One panel's update; `skip` where it is queued before the host knows the panel's outcome.
+    struct Update {
+        int c0, w, r0, k, par, by;
+        bool moves;
+        Skip skip;
+        uint32_t* Wf = nullptr;
+    };
+    // columns [ca, cb): row moves (from c0 on), then [A12; A22] += W A12 on a tensor-core variant (it
+    // reads A12 through its limb planes, so C may alias it)
+    auto update = [&](Update& U, int ca, int cb, int sm_cap) {
+        if (cb <= ca) return;
+        if (U.moves) {
+            HME_TIMED(ctx, "row_moves", move_pivot_rows_kernel<<<(cb - ca + kMoveCols - 1) / kMoveCols, 256, 0, s_main>>>(
+                                            A, ld, U.r0, U.k, d_sb[U.par]->pivot_rows, ca, cb, U.skip));
+            HME_CUDA(cudaGetLastError());
+        }
+        const int ua = std::max(ca, U.c0 + U.w), rows = m - U.r0, k = U.k;
+        if (cb <= ua) return;
+        if (!U.Wf && U.by == 2) U.Wf = d_Wc[U.par];
+        if (!U.Wf) {
+            uint32_t* mul = d_uinvb[U.par];
+            const int* d_pcols = d_sb[U.par]->pivot_cols;
+            if (U.by == 0) {
+                HME_TIMED(ctx, "panel_linv", panel_linv_kernel<<<1, 512, linv_smem_bytes(k), s_main>>>(
+                                                 A, ld, U.r0, d_pcols, k, p, mp.barrett, mul));
+                HME_CUDA(cudaGetLastError());
+            }
+            U.Wf = d_W;
+            const int g = (rows + kWRows - 1) / kWRows;
+            const size_t wsm = sizeof(uint32_t) * (((static_cast<size_t>(k) * k + 3) & ~size_t(3)) +
+                                                   static_cast<size_t>(kWRows) * ((k + 3) & ~3));
+            if (k <= 64)
+                HME_TIMED(ctx, "panel_w", panel_w_kernel<64><<<g, 256, wsm, s_main>>>(
+                                              A, ld, U.r0, m, d_pcols, k, mul, p, mp.barrett, U.skip, U.Wf));
+            else
+                HME_TIMED(ctx, "panel_w", panel_w_kernel<128><<<g, 256, wsm, s_main>>>(
+                                              A, ld, U.r0, m, d_pcols, k, mul, p, mp.barrett, U.skip, U.Wf));
+            HME_CUDA(cudaGetLastError());
+        }
+        ctx->gemm_sm_cap = sm_cap;
+        ctx->gemm_skip = U.skip;
+        uint32_t* C12 = A + static_cast<size_t>(U.r0) * ld + ua;
+        gemm_u32_variant(ctx, mp, rows, cb - ua, k, U.Wf, U.by == 2 ? bw : k, C12, ld, C12, ld, HME_ADD,
+                         gemm_default_variant(ctx, mp, rows, cb - ua));
+        ctx->gemm_sm_cap = 0;
+        ctx->gemm_skip = Skip{};
+    };
+    int r0 = 0, c0 = 0, par = 0;
     int next_look = 0;  // panel count before which a pivotless panel does not look over the rest
     int look_gap = 1, panels = 0;
-    int par = 0;
+    auto next_of = [](int i) { return (i + 1) % kRing; };
+    // lookahead only when the next panel runs on the cluster kernel (a few SMs beside the GEMM; the
+    // cooperative grid kernel would wait for the whole device anyway)
+    auto ahead = [&](int c1, int r1) {
+        return allow_lookahead && c1 < lu_cols && r1 < m && cluster_size(m - r1, std::min(bw, lu_cols - c1)) > 0;
+    };
+    // LOOKAHEAD: the next panel's columns first; that panel is factored on the second stream while the
+    // rest of this update runs here, the GEMM leaving the panel's SMs free; the main stream's later work
+    // (the next panel's update) follows that panel
+    auto update_ahead = [&](Update& U) {
+        const int c1 = U.c0 + U.w, nw = std::min(bw, lu_cols - c1);
+        update(U, U.c0, c1 + nw, 0);
+        HME_CUDA(cudaEventRecord(ev_next, s_main));
+        HME_CUDA(cudaStreamWaitEvent(s_aux, ev_next, 0));
+        const int busy = launch_panel(c1, nw, U.r0 + U.k, next_of(U.par), s_aux, 0);
+        update(U, c1 + nw, n + app, std::max(1, ctx->num_sms - busy));
+        if (keep) append(U.c0, U.w, U.r0 + U.k, U.par, U.k);
+        HME_CUDA(cudaStreamWaitEvent(s_main, ev_panel[next_of(U.par)], 0));
+    };
+    // the host's record of a panel with pivots: its columns, the sign of its row moves, the statistics (a
+    // top block that looks for most of its pivots -- a field of fewer than 256 elements, a ring -- counts
+    // as searched)
+    auto record = [&](const Scratch& h, int row0, int by, bool moves) {
+        if (by == 1 && rg.k == 1 && p >= 256) ++ctx->elim_block_panels;
+        else ++ctx->elim_search_panels;
+        ++panels;
+        for (int t = 0; t < h.k; ++t) pivots.push_back(h.pivot_cols[t]);
+        if (moves && row_moves_odd(h.pivot_rows, h.k, row0)) res.sign_negative = !res.sign_negative;
+    };
+    auto in_place = [](const Scratch& h, int row0) {
+        for (int t = 0; t < h.k; ++t)
+            if (h.pivot_rows[t] != row0 + t) return false;
+        return true;
+    };
+    // Panels whose update, and the panel after them, were queued before the host knew their outcome, at
+    // most two: where the top block is expected to settle the panel, the host only checks up on the panel
+    // before, so that its round trip (about 20 us a panel) is off the chain.  A panel that turns out
+    // otherwise raises the flag that everything queued behind it obeys, and the loop takes it up again.
+    std::vector<Update> queued;
     bool launched = false;  // the panel at c0 was already factored ahead (on the second stream)
-    for (int c0 = 0; c0 < lu_cols && r0 < m; c0 += bw) {
-        const int w = std::min(bw, lu_cols - c0);
-        if (!launched) launch_panel(c0, w, r0, par, s_main, 0);
+    while (true) {
+        const bool more_panels = c0 < lu_cols && r0 < m;
+        const int w = more_panels ? std::min(bw, lu_cols - c0) : 0;
+        bool queue = false;
+        if (more_panels) {
+            if (!launched && queued.empty()) {
+                launch_panel(c0, w, r0, par, s_main, 0);
+                launched = true;
+            }
+            queue = launched && block_tried[par] && !compact_tried[par] && !search_run[par] && m - r0 > w &&
+                    ahead(c0 + w, r0 + w);
+            if (queue) {
+                Update U{c0, w, r0, w, par, 1, !in_order, Skip{d_fail, panel_seq[par]}};
+                update_ahead(U);
+                queued.push_back(U);
+                r0 += w;
+                c0 += w;
+                par = next_of(par);
+            }
+        }
+        // check up on the queued panels: all but the newest, all when nothing more is queued
+        bool undo = false;
+        while (queued.size() > (queue ? 1u : 0u)) {
+            const Update U = queued.front();
+            HME_CUDA(cudaEventSynchronize(ev_host[U.par]));
+            const Scratch& h = h_sb[U.par];
+            if (h.err != 0) check_device_error(ctx);
+            if (h.settled == 1 && (!in_order || in_place(h, U.r0))) {
+                block.settled();
+                record(h, U.r0, 1, !in_order && !in_place(h, U.r0));
+                queued.erase(queued.begin());
+                continue;
+            }
+            // stands still from this panel on: take it up again
+            HME_CUDA(cudaStreamSynchronize(s_main));
+            HME_CUDA(cudaStreamSynchronize(s_aux));
+            HME_CUDA(cudaMemsetAsync(d_fail, 0, sizeof(int), s_main));
+            c0 = U.c0;
+            r0 = U.r0;
+            par = U.par;
+            launched = true;
+            queued.clear();
+            undo = true;
+            break;
+        }
+        if (queue && !undo) continue;
+        if (!(c0 < lu_cols && r0 < m)) break;
+        const int wp = std::min(bw, lu_cols - c0);
+        if (!launched) launch_panel(c0, wp, r0, par, s_main, 0);
         launched = false;
-        HME_CUDA(cudaEventSynchronize(ev_panel[par]));
+        HME_CUDA(cudaEventSynchronize(ev_host[par]));
         // what settled the panel: 1 the top block, 2 the compact rows, 0 the search
         int by = 0;
         for (;;) {
             by = block_tried[par] || compact_tried[par] ? h_sb[par].settled : 0;
-            if (block_tried[par]) by == 1 ? block.settled() : block.failed();
+            if (block_tried[par]) {
+                by == 1 ? block.settled() : block.failed();
+                HME_CUDA(cudaMemsetAsync(d_fail, 0, sizeof(int), s_main));  // nothing is queued behind it
+            }
             if (compact_tried[par] && by != 1) by == 2 ? compact.settled() : compact.failed();
             if (by != 0 || search_run[par]) break;
             // an attempt that was expected to succeed did not (nothing was written): the panel's other
             // kernels, on its stream; the main stream's later work waits for them too
-            launch_panel(c0, w, r0, par, panel_stream[par], compact_tried[par] ? 2 : 1);
+            launch_panel(c0, wp, r0, par, panel_stream[par], compact_tried[par] ? 2 : 1);
             if (panel_stream[par] != s_main) HME_CUDA(cudaStreamWaitEvent(s_main, ev_panel[par], 0));
-            HME_CUDA(cudaEventSynchronize(ev_panel[par]));
+            HME_CUDA(cudaEventSynchronize(ev_host[par]));
         }
         const Scratch& h_s = h_sb[par];
         if (h_s.err != 0) check_device_error(ctx);  // reports the timeout (and clears the word)
-        // the statistics count a top block that looks for most of its pivots (a field of fewer than 256
-        // elements, a ring) as searched
-        if (by == 1 && rg.k == 1 && p >= 256) ++ctx->elim_block_panels;
-        else ++ctx->elim_search_panels;
-        const int k = h_s.k;
-        ++panels;
+        const int k = h_s.k, c1 = c0 + wp;
+        const bool moves = k > 0 && !in_place(h_s, r0);
+        record(h_s, r0, by, moves);
         if (k == 0) {
-            if (keep) append(c0, w, r0, par, 0);
+            if (keep) append(c0, wp, r0, par, 0);
+            c0 = c1;
             // no pivot in the panel: nothing moved, the next panel starts at r0 -- unless nothing is
             // left (one pass over the rest, against a panel's search each; after a pass that found
             // something only every 2nd, 4th, .. pivotless panel asks again)
-            const int c1 = c0 + w;
             if (c1 < lu_cols && panels >= next_look) {
                 int* d_nz = &d_sb[par]->nonzero;
                 HME_CUDA(cudaMemsetAsync(d_nz, 0, sizeof(int), s_main));
@@ -2120,75 +2289,17 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
             }
             continue;
         }
-        for (int t = 0; t < k; ++t) pivots.push_back(h_s.pivot_cols[t]);
-
-        // (2) the pivot rows' moves: none when they are rows r0 .. r0+k-1 in order
-        const int rows = m - r0;
-        bool identity = true;
-        for (int t = 0; t < k && identity; ++t) identity = h_s.pivot_rows[t] == r0 + t;
-        if (!identity && row_moves_odd(h_s.pivot_rows, k, r0)) res.sign_negative = !res.sign_negative;
-        const int c1 = c0 + w;
-        const int below = m - r0 - k;
-        const int* d_pcols = d_sb[par]->pivot_cols;
-        uint32_t* Wf = by == 2 ? d_Wc[par] : nullptr;
-        const int ldw = by == 2 ? bw : k;
-        // the update of columns [ca, cb): row moves (from c0 on), then [A12; A22] += W A12 on a
-        // tensor-core variant (it reads A12 through its limb planes, so C may alias it)
-        auto update = [&](int ca, int cb, int sm_cap) {
-            if (cb <= ca) return;
-            if (!identity) {
-                HME_TIMED(ctx, "row_moves", move_pivot_rows_kernel<<<(cb - ca + kMoveCols - 1) / kMoveCols, 256, 0, s_main>>>(
-                                                A, ld, r0, k, d_sb[par]->pivot_rows, ca, cb));
-                HME_CUDA(cudaGetLastError());
-            }
-            const int ua = std::max(ca, c1);
-            if (cb <= ua) return;
-            if (!Wf) {
-                uint32_t* mul = d_uinvb[par];
-                if (by == 0) {
-                    HME_TIMED(ctx, "panel_linv", panel_linv_kernel<<<1, 512, linv_smem_bytes(k), s_main>>>(
-                                                     A, ld, r0, d_pcols, k, p, mp.barrett, mul));
-                    HME_CUDA(cudaGetLastError());
-                }
-                Wf = d_W;
-                const int g = (rows + kWRows - 1) / kWRows;
-                const size_t wsm = sizeof(uint32_t) * (((static_cast<size_t>(k) * k + 3) & ~size_t(3)) +
-                                                       static_cast<size_t>(kWRows) * ((k + 3) & ~3));
-                if (k <= 64)
-                    HME_TIMED(ctx, "panel_w", panel_w_kernel<64><<<g, 256, wsm, s_main>>>(
-                                                  A, ld, r0, m, d_pcols, k, mul, p, mp.barrett, Wf));
-                else
-                    HME_TIMED(ctx, "panel_w", panel_w_kernel<128><<<g, 256, wsm, s_main>>>(
-                                                  A, ld, r0, m, d_pcols, k, mul, p, mp.barrett, Wf));
-                HME_CUDA(cudaGetLastError());
-            }
-            ctx->gemm_sm_cap = sm_cap;
-            uint32_t* C12 = A + static_cast<size_t>(r0) * ld + ua;
-            gemm_u32_variant(ctx, mp, rows, cb - ua, k, Wf, ldw, C12, ld, C12, ld, HME_ADD,
-                             gemm_default_variant(ctx, mp, rows, cb - ua));
-            ctx->gemm_sm_cap = 0;
-        };
-        const int nw = std::min(bw, lu_cols - c1);
-        // lookahead only when the next panel runs on the cluster kernel (a few SMs beside the GEMM;
-        // the cooperative grid kernel would wait for the whole device anyway)
-        const bool next = allow_lookahead && c1 < lu_cols && below > 0 && nw > 0 && cluster_size(below, nw) > 0;
-        if (next) {
-            // LOOKAHEAD: the next panel's columns first; that panel is factored on the second stream
-            // while the rest of this update runs here, the GEMM leaving the panel's SMs free
-            update(c0, c1 + nw, 0);
-            HME_CUDA(cudaEventRecord(ev_next, s_main));
-            HME_CUDA(cudaStreamWaitEvent(s_aux, ev_next, 0));
-            const int busy = launch_panel(c1, nw, r0 + k, par ^ 1, s_aux, 0);
-            update(c1 + nw, n + app, std::max(1, ctx->num_sms - busy));
+        Update U{c0, wp, r0, k, par, by, moves, Skip{}};
+        if (ahead(c1, r0 + k)) {
+            update_ahead(U);
             launched = true;
         } else {
-            update(c0, n + app, 0);
+            update(U, c0, n + app, 0);
+            if (keep) append(c0, wp, r0 + k, par, k);
         }
-        if (keep) append(c0, w, r0 + k, par, k);
-        // the main stream's later work (the next panel's update) follows the lookahead panel
-        if (launched) HME_CUDA(cudaStreamWaitEvent(s_main, ev_panel[par ^ 1], 0));
         r0 += k;
-        par ^= 1;
+        c0 = c1;
+        par = next_of(par);
     }
     HME_CUDA(cudaStreamSynchronize(s_aux));
     res.rank = r0;

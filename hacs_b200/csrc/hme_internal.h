@@ -89,6 +89,21 @@ struct Workspace {
 }  // namespace hme
 
 namespace hme {
+// Work queued before the host knows whether it is wanted: nothing is done when
+// the device word holds a number from 1 to seq (the first of the queued steps that
+// did not come out as expected; later ones depend on it, earlier ones do not).
+struct Skip {
+    const int* word = nullptr;
+    int seq = 0;
+#ifdef __CUDACC__
+    __device__ __forceinline__ bool stands() const {
+        if (word == nullptr) return false;
+        const int f = *word;
+        return f != 0 && f <= seq;
+    }
+#endif
+};
+
 // Tunables of the device elimination (elim.cu); none of them changes a value.
 struct ElimOptions {
     int panel = 64;         // LU panel width (columns, <= 128)
@@ -137,6 +152,7 @@ struct hme_ctx {
     void* sched_table = nullptr;     // planner decisions by shape class (sched.cu)
     void* sched_rank_table = nullptr;  // the rank rounds' planner decisions by shape class (sched.cu)
     int gemm_sm_cap = 0;             // > 0: persistent GEMM grids use at most this many SMs
+    hme::Skip gemm_skip;             // the tensor-core products stand still as it says
     cudaStream_t aux_stream = nullptr;   // elimination: the lookahead panel's stream (created on first use)
     void* elim_pinned = nullptr;         // elimination: pinned copies of the panel scratch, permutations
     size_t elim_pinned_bytes = 0;

@@ -7,6 +7,7 @@
 #include <cstdint>
 
 #include "../../include/hme.h"
+#include "hme_internal.h"
 #include "hme_mod.h"
 #include "hme_ptx.cuh"
 
@@ -690,6 +691,7 @@ struct SplitArgs {
     bool a_vec;          // A rows 16-byte aligned: vector loads
     uint64_t a_plane;    // bytes between A limb planes (0: M * Kp)
     uint64_t b_plane;    // bytes between B limb planes (0: N * Kp)
+    Skip skip;
 };
 
 template <int L>

@@ -52,6 +52,7 @@ struct GemmArgs {
     EpiRed red;
     int tiles_m, tiles_n, group_m;
     int* err;
+    Skip skip;
 };
 
 // The tiles of one product.  Long K: a grouped raster, group_m tile-rows share
@@ -64,7 +65,7 @@ struct OneProduct {
     const CUtensorMap* tmB;
     const GemmArgs& g;
 
-    __device__ __forceinline__ int total() const { return g.tiles_m * g.tiles_n; }
+    __device__ __forceinline__ int total() const { return g.skip.stands() ? 0 : g.tiles_m * g.tiles_n; }
     __device__ __forceinline__ int kblocks(int) const { return g.kblocks; }
     __device__ __forceinline__ int b_key(int tile) const { return tile / g.tiles_m; }
     __device__ __forceinline__ void prefetch_maps() const {
@@ -110,6 +111,7 @@ template <int L>
 __global__ void __launch_bounds__(256) limb_split_kernel(const SplitArgs s) {
     __shared__ uint32_t tile[64][33];
     grid_dep_launch();  // the GEMM that follows may start its set-up
+    if (s.skip.stands()) return;
     if (static_cast<int>(blockIdx.x) < s.a_blocks)
         split_a_part<L>(s, blockIdx.x);
     else
@@ -188,6 +190,7 @@ void launch_gemm(hme_ctx* ctx, const ModParams& mp, uint32_t m, uint32_t n, uint
     g.tiles_n = static_cast<int>((n + BN - 1) / BN);
     g.group_m = 16;
     g.err = ctx->d_err;
+    g.skip = ctx->gemm_skip;
     const int total = g.tiles_m * g.tiles_n;
     const int grid = std::min(total, ctx->gemm_sm_cap > 0 ? std::min(ctx->gemm_sm_cap, ctx->num_sms) : ctx->num_sms);
     const uint32_t chunk = limb_k_chunk(L);
@@ -246,6 +249,7 @@ void launch_split(hme_ctx* ctx, const ModParams& mp, uint32_t m, uint32_t n, uin
     sa.p = mp.p; sa.barrett = mp.barrett;
     sa.planesA = pa; sa.planesB = pb;
     sa.a_plane = a_plane;
+    sa.skip = ctx->gemm_skip;
     const size_t work = static_cast<size_t>(m) * (Kp / 16);
     sa.a_blocks = do_a ? static_cast<int>(std::min<size_t>((work + 255) / 256, static_cast<size_t>(ctx->num_sms) * 8))
                        : 0;
