@@ -288,35 +288,42 @@ void run_grouped(hme_ctx* ctx, const ModParams& mp, const std::vector<GemmJob>& 
 }
 
 template <int L>
-void launch_device_tables(hme_ctx* ctx, const ModParams& mp, const GroupedSplitJob* d_split, const int* d_block_job,
+void launch_device_tables(hme_ctx* ctx, const ModParams& mp, int kb, const GroupedSplitJob* d_split, const int* d_block_job,
                           const int* d_nblocks, const GroupedProblem* d_probs, const int* d_tile_prob,
                           const int* d_ntiles) {
     const int split_grid = ctx->num_sms * 8;
     HME_TIMED(ctx, "grouped_split", grouped_split_kernel<L><<<split_grid, 256, 0, ctx->stream>>>(d_split, d_block_job,
                                                                                               0, d_nblocks));
     HME_CUDA(cudaGetLastError());
-    launch_grouped<L, grouped_bn_wide(L), 32>(ctx, mp, d_probs, d_tile_prob, 0, 32, d_ntiles);
+    if (kb == 32) launch_grouped<L, grouped_bn_wide(L), 32>(ctx, mp, d_probs, d_tile_prob, 0, 32, d_ntiles);
+    else launch_grouped<L, grouped_bn_wide(L), 64>(ctx, mp, d_probs, d_tile_prob, 0, 64, d_ntiles);
 }
 
 }  // namespace
 
-void grouped_prepare_device_tables(uint32_t limbs) {
+template <int L>
+static void prepare_device_tables(int kb) {
+    if (kb == 32) ensure_grouped_attr<L, grouped_bn_wide(L), 32>();
+    else ensure_grouped_attr<L, grouped_bn_wide(L), 64>();
+}
+
+void grouped_prepare_device_tables(uint32_t limbs, int kb) {
     switch (limbs) {
-        case 1: ensure_grouped_attr<1, grouped_bn_wide(1), 32>(); break;
-        case 2: ensure_grouped_attr<2, grouped_bn_wide(2), 32>(); break;
-        case 3: ensure_grouped_attr<3, grouped_bn_wide(3), 32>(); break;
-        default: ensure_grouped_attr<4, grouped_bn_wide(4), 32>(); break;
+        case 1: prepare_device_tables<1>(kb); break;
+        case 2: prepare_device_tables<2>(kb); break;
+        case 3: prepare_device_tables<3>(kb); break;
+        default: prepare_device_tables<4>(kb); break;
     }
 }
 
-void grouped_launch_device_tables(hme_ctx* ctx, const ModParams& mp, const GroupedSplitJob* d_split,
+void grouped_launch_device_tables(hme_ctx* ctx, const ModParams& mp, int kb, const GroupedSplitJob* d_split,
                                   const int* d_block_job, const int* d_nblocks, const GroupedProblem* d_probs,
                                   const int* d_tile_prob, const int* d_ntiles) {
     switch (mp.limbs) {
-        case 1: launch_device_tables<1>(ctx, mp, d_split, d_block_job, d_nblocks, d_probs, d_tile_prob, d_ntiles); break;
-        case 2: launch_device_tables<2>(ctx, mp, d_split, d_block_job, d_nblocks, d_probs, d_tile_prob, d_ntiles); break;
-        case 3: launch_device_tables<3>(ctx, mp, d_split, d_block_job, d_nblocks, d_probs, d_tile_prob, d_ntiles); break;
-        default: launch_device_tables<4>(ctx, mp, d_split, d_block_job, d_nblocks, d_probs, d_tile_prob, d_ntiles); break;
+        case 1: launch_device_tables<1>(ctx, mp, kb, d_split, d_block_job, d_nblocks, d_probs, d_tile_prob, d_ntiles); break;
+        case 2: launch_device_tables<2>(ctx, mp, kb, d_split, d_block_job, d_nblocks, d_probs, d_tile_prob, d_ntiles); break;
+        case 3: launch_device_tables<3>(ctx, mp, kb, d_split, d_block_job, d_nblocks, d_probs, d_tile_prob, d_ntiles); break;
+        default: launch_device_tables<4>(ctx, mp, kb, d_split, d_block_job, d_nblocks, d_probs, d_tile_prob, d_ntiles); break;
     }
 }
 

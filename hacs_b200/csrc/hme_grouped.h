@@ -38,13 +38,13 @@ struct GroupedSplitJob {
 // The wide tile width of the grouped GEMM for L limbs (L * BN close to 256).
 constexpr int grouped_bn_wide(int L) { return L == 1 ? 256 : L == 2 ? 128 : L == 3 ? 80 : 64; }
 
-// The grouped split + GEMM on tables built on the device (32-byte k-blocks, wide
-// tiles): block and tile counts, the per-block job and per-tile problem indexes
+// The grouped split + GEMM on tables built on the device (one k-block of kb = 32
+// or 64 bytes, wide tiles): block and tile counts, the per-block job and per-tile problem indexes
 // are read from device memory when the kernels run, so the launches have fixed
 // shapes (persistent grids) and can be captured in a CUDA graph.
 // Kernel attributes of those launches, set outside any stream capture.
-void grouped_prepare_device_tables(uint32_t limbs);
-void grouped_launch_device_tables(hme_ctx* ctx, const ModParams& mp, const GroupedSplitJob* d_split,
+void grouped_prepare_device_tables(uint32_t limbs, int kb);
+void grouped_launch_device_tables(hme_ctx* ctx, const ModParams& mp, int kb, const GroupedSplitJob* d_split,
                                   const int* d_block_job, const int* d_nblocks, const GroupedProblem* d_probs,
                                   const int* d_tile_prob, const int* d_ntiles);
 
@@ -77,7 +77,7 @@ struct BatchMatrix {
     uint32_t* A = nullptr;
     size_t ld = 0;
     uint32_t m = 0, n = 0, p = 0;
-    int rank_variant = 0;  // the schedule of its rank rounds (RankVariant)
+    int rank_variant = 0;  // the schedule of its rank rounds (RankVariant, or kRankRule)
 };
 
 // The schedules of a job's rank rounds: the trailing-update variant (the
@@ -86,17 +86,24 @@ struct BatchMatrix {
 // one CTA, with no trailing update; otherwise its rounds take 32 columns).
 // Every schedule computes the same rank; only the time changes.
 enum RankVariant {
-    kRankTensorLast128 = 0,  // grouped limb GEMM, last panel up to 128 columns (the batch rule)
+    kRankTensorLast128 = 0,  // grouped limb GEMM, last panel up to 128 columns
     kRankTensorLast32 = 1,   // grouped limb GEMM, 32-column rounds to the end
     kRankSimtLast128 = 2,    // CUDA-core update, last panel up to 128 columns
     kRankSimtLast32 = 3,     // CUDA-core update, 32-column rounds to the end
     kRankVariants = 4
 };
+// No schedule asked for (the batch rule): rounds of 64 columns (rank_rounds.cu)
+// when no job of the call has one, else kRankTensorLast128 or kRankTensorLast32.
+constexpr int kRankRule = -1;
 inline int rank_variant_last(int v) { return v == kRankTensorLast32 || v == kRankSimtLast32 ? 32 : 128; }
 inline bool rank_variant_simt(int v) { return v == kRankSimtLast128 || v == kRankSimtLast32; }
 
 // ranks[j] = rank of mats[j] over F_p (destroys the matrices).
 void batch_rank_device(hme_ctx* ctx, const std::vector<BatchMatrix>& mats, std::vector<int>& ranks);
+// The same for the jobs of `order`, in rounds of 64 columns: 1 to 1024 rows, at
+// least one column each (rank_rounds.cu).
+void batch_rank_rounds(hme_ctx* ctx, const std::vector<BatchMatrix>& mats, std::vector<int> order,
+                       std::vector<int>& ranks);
 
 // One seeded matrix of the job-stream generator.
 struct GenSpec {

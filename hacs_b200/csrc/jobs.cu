@@ -7,7 +7,8 @@
 // host (elim::column_rank_profile, src/ModArithmetic/DenseElim.h:160-169).
 // Here every phase is one launch over all jobs:
 //   GEMM: the grouped limb GEMM (grouped_gemm.cu), one launch per modulus;
-//   rank: a round-based blocked LU over all jobs at once -- per round, one
+//   rank: under the batch rule rounds of 64 columns (rank_rounds.cu); with
+//     schedules named (or planned), the rounds here: a blocked LU over all jobs at once -- per round, one
 //     CTA per job factors that job's next panel of columns in shared memory,
 //     then batched kernels move the pivot rows up and solve the pivot rows'
 //     trailing block, and ONE grouped limb GEMM per modulus applies every
@@ -567,6 +568,14 @@ __global__ void __launch_bounds__(256, 2) batch_simt_update_kernel(const SolveJo
     cp_async_wait<0>();  // no copy outlives the kernel
 }
 
+// The schedule of a job under the batch rule in a call that names a schedule for
+// another job (the rounds of 64 columns, rank_rounds.cu, have no schedules): the
+// grouped tensor-core limb GEMM as the trailing update, and one
+// last panel of up to 128 columns only for jobs of at most 128 rows -- a taller
+// job's last panel is a long serial chain on one CTA that every job of the round
+// waits for, so its rounds take 32 columns to the end.
+int rank_rule(uint32_t m) { return m <= 128 ? kRankTensorLast128 : kRankTensorLast32; }
+
 size_t a256(size_t x) { return (x + 255) / 256 * 256; }
 
 // ---- device-driven rounds ----------------------------------------------------------------
@@ -834,6 +843,7 @@ void batch_rank_device(hme_ctx* ctx, const std::vector<BatchMatrix>& mats, std::
     ranks.assign(nj_all, 0);
     // jobs taller than one panel CTA holds: the single-matrix elimination
     std::vector<int> order;
+    bool scheduled = false;
     order.reserve(nj_all);
     for (int j = 0; j < nj_all; ++j) {
         const BatchMatrix& M = mats[j];
@@ -846,9 +856,15 @@ void batch_rank_device(hme_ctx* ctx, const std::vector<BatchMatrix>& mats, std::
             ranks[j] = r.rank;
         } else {
             order.push_back(j);
+            scheduled = scheduled || M.rank_variant != kRankRule;
         }
     }
     if (order.empty()) return;
+    // jobs under the batch rule beside scheduled ones run on rank_rule's schedule, in the same rounds
+    if (!scheduled) {
+        batch_rank_rounds(ctx, mats, std::move(order), ranks);
+        return;
+    }
     // modulus groups: jobs sorted by modulus (stable)
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return mats[x].p < mats[y].p; });
     const int nj = static_cast<int>(order.size());
@@ -896,8 +912,9 @@ void batch_rank_device(hme_ctx* ctx, const std::vector<BatchMatrix>& mats, std::
             J.out = i;
             D.active = 1;
             D.group = g;
-            D.last_max = rank_variant_last(M.rank_variant);
-            D.simt = rank_variant_simt(M.rank_variant) ? 1 : 0;
+            const int variant = M.rank_variant == kRankRule ? rank_rule(M.m) : M.rank_variant;
+            D.last_max = rank_variant_last(variant);
+            D.simt = rank_variant_simt(variant) ? 1 : 0;
             if (D.simt) {
                 any_simt = true;
                 simt_cap += static_cast<size_t>(simt_tiles(static_cast<int>(M.m), static_cast<int>(M.n)));
@@ -1106,13 +1123,13 @@ void batch_rank_device(hme_ctx* ctx, const std::vector<BatchMatrix>& mats, std::
         }
         for (int g = 0; g < ng; ++g) {
             const RankGroup& G = groups[g];
-            grouped_launch_device_tables(ctx, make_mod(gmod[g]), d_gsplit + G.begin, G.block_job, G.totals + 1,
+            grouped_launch_device_tables(ctx, make_mod(gmod[g]), kRoundBw, d_gsplit + G.begin, G.block_job, G.totals + 1,
                                          d_gprob + G.begin, G.tile_prob, G.totals);
         }
         if (fork) HME_CUDA(cudaStreamWaitEvent(ctx->stream, ev_join, 0));
         HME_CUDA(cudaGetLastError());
     };
-    for (int g = 0; g < ng; ++g) grouped_prepare_device_tables(make_mod(gmod[g]).limbs);
+    for (int g = 0; g < ng; ++g) grouped_prepare_device_tables(make_mod(gmod[g]).limbs, kRoundBw);
     const int rounds = static_cast<int>((max_n + kRoundBw - 1) / kRoundBw) + 2;
     if (ctx->timer.on) {
         for (int r = 0; r < rounds; ++r) round();
@@ -1233,13 +1250,6 @@ void batch_gemm(hme_ctx* ctx, uint32_t njobs, const hme_job* jobs, const int* va
     }
 }
 
-// The batch rule of the rank rounds (the method without the planner): the
-// grouped tensor-core limb GEMM as the trailing update, and one last panel of
-// up to 128 columns only for jobs of at most 128 rows -- a taller job's last
-// panel is a long serial chain on one CTA that every job of the round waits
-// for, so its rounds take 32 columns to the end.
-int rank_rule(uint32_t m) { return m <= 128 ? kRankTensorLast128 : kRankTensorLast32; }
-
 // The rank phase of a batch.  Every job's rank rounds follow one of the
 // RankVariant schedules: from `rank_variants` when given (-1 = the batch rule),
 // else under the learned policy the planner's decision for the job's shape
@@ -1264,7 +1274,7 @@ void batch_rank(hme_ctx* ctx, uint32_t njobs, const hme_job* jobs, uint32_t* ran
         } else if (ctx->sched_policy == 1 && jobs[t].p >= 2) {
             v = sched_planned_rank_variant(ctx, make_mod(jobs[t].p), jobs[t].m, jobs[t].n, jobs[t].k);
         }
-        mats[t].rank_variant = v < 0 ? rank_rule(jobs[t].m) : v;
+        mats[t].rank_variant = v < 0 ? kRankRule : v;
     }
     std::vector<int> r;
     batch_rank_device(ctx, mats, r);
@@ -1351,7 +1361,7 @@ int hme_autotune_batch_rank(hme_ctx* ctx, uint32_t p, uint32_t m, uint32_t n, ui
         bind(ctx);
         // count products C = A B of the stream's construction (banded sparse operands below density 0.5,
         // dense uniform ones otherwise), so the rounds meet the ranks and pivot patterns such jobs have, and
-        // one anchor: a dense 1024 x 1024 product of full rank on the batch rule, whose rounds run the whole
+        // one anchor: a dense 1024 x 1024 product of full rank on rank_rule's schedule, whose rounds run the whole
         // 34-round sequence as the stream's largest jobs do.  A schedule's cost is its jobs' MARGINAL time
         // beside the anchor (the batch with them minus the anchor alone): what the jobs add to a stream whose
         // rounds run anyway, not the latency of a small batch alone.
@@ -1383,7 +1393,7 @@ int hme_autotune_batch_rank(hme_ctx* ctx, uint32_t p, uint32_t m, uint32_t n, ui
         cudaEvent_t e0, e1;
         HME_CUDA(cudaEventCreate(&e0));
         HME_CUDA(cudaEventCreate(&e1));
-        std::vector<int> var(count + 1, kBatchRule);
+        std::vector<int> var(count + 1, rank_rule(kAnchor));
         std::vector<uint32_t> rk(count + 1), rk0(count + 1);
         // the median time of a batched rank of `nj` jobs starting at jobs[j0] (fresh copies every run)
         auto timed = [&](uint32_t j0, uint32_t nj, bool check) {

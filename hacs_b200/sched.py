@@ -44,9 +44,10 @@ RANK_VARIANT_NAMES = ("tensor/last-128", "tensor/last-32", "simt/last-128", "sim
 
 
 def rank_rule(m) -> np.ndarray:
-    """The rank rounds' batch rule (the method without the planner): schedule 0
+    """The batch rule's choice among the planner's schedules: schedule 0
     (tensor-core update, one last panel of up to 128 columns) for jobs of at most
-    128 rows, else 1 (32-column rounds to the end); as jobs.cu rank_rule."""
+    128 rows, else 1 (32-column rounds to the end); as jobs.cu rank_rule.  (In a
+    call without any schedule the library takes rounds of 64 columns instead.)"""
     return np.where(np.asarray(m) <= 128, 0, 1).astype(np.int32)
 
 _fp = C.POINTER(C.c_float)

@@ -360,8 +360,10 @@ HME_API int hme_gen_jobs_u32_dev(hme_ctx *ctx, uint32_t nmat, const hme_gen_spec
  *   2 the CUDA-core update (a list of 64 x 64 tiles over a persistent grid,
  *     exact dot products), last panel up to 128 columns,
  *   3 the CUDA-core update, 32-column rounds to the end,
- *  -1 the batch rule: 0 for jobs of at most 128 rows, else 1 (a taller job's
- *     last panel is a long serial chain on one CTA that the round waits for).
+ *  -1 the batch rule: rounds of 64 columns when no job of the call has a
+ *     schedule; else 0 for jobs of at most 128 rows and 1 for the others (a
+ *     taller job's last panel is a long serial chain on one CTA that the round
+ *     waits for).
  * rank_variants = NULL takes the context's scheduler (under the learned policy
  * the rank planner's decision per job's shape class, recorded by
  * hme_sched_plan_rank; else the batch rule).  No schedule changes a rank.
@@ -410,7 +412,7 @@ HME_API int hme_autotune_batch(hme_ctx *ctx, uint32_t p, uint32_t m, uint32_t n,
 /* The exhaustive autotuner of the rank rounds: `count` products C = A B of
  * one shape (m <= 1024, p prime) built like the stream's jobs (banded sparse
  * operands when density < 0.5, dense uniform ones otherwise) and one anchor
- * (a dense 1024 x 1024 product of full rank on the batch rule, whose rounds run
+ * (a dense 1024 x 1024 product of full rank on schedule 1, whose rounds run
  * as long as the stream's largest jobs'); the batched rank of fresh copies of
  * them under each rank schedule in turn (hme_batch_rank_u32_dev_sched), and of
  * the anchor alone.  ms[v] = (median time with the jobs on schedule v - median
