@@ -381,7 +381,7 @@ __global__ void gemv_warp_kernel(const uint32_t* __restrict__ A, uint64_t a_rs, 
         if (lane == 0) y[row * y_rs] = apply_op(y[row * y_rs], v, op, p);
     }
 }
-// y op= A x for long rows: a CTA per row at a time (rows striped over a
+// y op= A x for long rows whose length fits no chunk of the kernel below: a CTA per row at a time (rows striped over a
 // persistent grid), its 8 warps splitting the row, four vector loads in flight
 // per thread, the 8 warp sums combined in shared memory.
 template <int V>
@@ -426,6 +426,88 @@ __global__ void __launch_bounds__(256) gemv_block_kernel(const uint32_t* __restr
             y[row * y_rs] = apply_op(y[row * y_rs], s, op, p);
         }
         __syncthreads();
+    }
+}
+
+// y op= A x for long rows: a CTA takes R rows at a time (striped over a
+// persistent grid), its threads splitting the rows.  The bound is the read of A,
+// so a thread keeps 32 words of A in flight while it multiplies the 32 before
+// them, across the rows' reductions too, and its words of x stay in registers
+// (a chunk of 8192 columns, 4096 or 2048 as R goes from 1 to 2 to 4; longer rows
+// take a pass per chunk).  One barrier per R rows: the warps' sums alternate
+// between two sets of words.  mod 2^31 - 19, against a row at a time with four
+// loads in flight: 8192 x 8192 62 -> 49 us (5.4 TB/s of the 6.5 that a copy
+// moves), 20000 x 2048 75 -> 38 us, 16384 x 16384 207 -> 189 us.
+template <int V, int Q, int R>
+__global__ void __launch_bounds__(256, 2) gemv_rows_kernel(const uint32_t* __restrict__ A, uint64_t a_rs, uint64_t a_cs,
+                                                           const uint32_t* __restrict__ x, uint64_t x_rs,
+                                                           uint32_t* __restrict__ y, uint64_t y_rs, uint32_t m,
+                                                           uint32_t k, int op, uint32_t p, uint64_t barrett,
+                                                           uint32_t r64) {
+    __shared__ uint32_t part[2][R][8];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, kv = k / V;
+    const uint64_t step = static_cast<uint64_t>(gridDim.x) * R;
+    int buf = 0;
+    for (uint32_t c0 = 0; c0 < kv; c0 += 256 * Q) {
+        const uint32_t j0 = c0 + tid;
+        VW<V> xv[Q], av[R][Q];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            const uint32_t j = j0 + 256 * q;
+            if (j < kv) {
+                xv[q] = ldv<V>(x + (V == 1 ? j * x_rs : static_cast<uint64_t>(j) * V));
+            } else {
+#pragma unroll
+                for (int c = 0; c < V; ++c) xv[q].v[c] = 0u;
+            }
+        }
+        auto load = [&](uint64_t row0) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const uint32_t* a = A + (row0 + r) * a_rs;
+#pragma unroll
+                for (int q = 0; q < Q; ++q) {
+                    const uint32_t j = j0 + 256 * q;
+                    if (j < kv && row0 + r < m) {
+                        av[r][q] = ldv<V>(a + (V == 1 ? j * a_cs : static_cast<uint64_t>(j) * V));
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < V; ++c) av[r][q].v[c] = 0u;
+                    }
+                }
+            }
+        };
+        const int cop = c0 == 0 || op != HME_SET ? op : HME_ADD;
+        load(static_cast<uint64_t>(blockIdx.x) * R);
+        for (uint64_t row0 = static_cast<uint64_t>(blockIdx.x) * R; row0 < m; row0 += step, buf ^= 1) {
+            VW<V> cur[R][Q];
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int q = 0; q < Q; ++q) cur[r][q] = av[r][q];
+            load(row0 + step);
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                uint64_t lo = 0;
+                uint32_t hi = 0;
+#pragma unroll
+                for (int q = 0; q < Q; ++q)
+#pragma unroll
+                    for (int c = 0; c < V; ++c) mac96(lo, hi, cur[r][q].v[c], xv[q].v[c]);
+                uint32_t v = fold96(lo, hi, p, barrett, r64);
+#pragma unroll
+                for (int off = 16; off > 0; off >>= 1) v = mod_add(v, __shfl_xor_sync(0xffffffffu, v, off), p);
+                if (lane == 0) part[buf][r][warp] = v;
+            }
+            __syncthreads();
+            if (tid < R && row0 + tid < m) {
+                uint32_t s = part[buf][tid][0];
+#pragma unroll
+                for (int w = 1; w < 8; ++w) s = mod_add(s, part[buf][tid][w], p);
+                uint32_t* yr = y + (row0 + tid) * y_rs;
+                *yr = apply_op(*yr, s, cop, p);
+            }
+        }
     }
 }
 
@@ -601,17 +683,40 @@ int hme_gemv_u32_dev(hme_ctx* ctx, uint32_t p, uint32_t m, uint32_t k, const uin
         const bool v4 = a_cs == 1 && x_rs == 1 && k % 4 == 0 && (m == 1 || a_rs % 4 == 0) &&
                         reinterpret_cast<uintptr_t>(A) % 16 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0;
         if ((a_cs == 1 || a_rs != 1) && k >= 2048) {
-            // long rows: a CTA per row, the grid one wave of resident CTAs
-            int per_sm = 1;
-            HME_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                &per_sm, v4 ? gemv_block_kernel<4> : gemv_block_kernel<1>, 256, 0));
-            const int grid = static_cast<int>(std::min<size_t>(m, static_cast<size_t>(std::max(1, per_sm)) * ctx->num_sms));
-            if (v4)
-                HME_TIMED(ctx, "gemv", gemv_block_kernel<4><<<grid, 256, 0, ctx->stream>>>(
-                                           A, a_rs, a_cs, x, x_rs, y, y_rs, m, k, op, p, mp.barrett, r64));
-            else
-                HME_TIMED(ctx, "gemv", gemv_block_kernel<1><<<grid, 256, 0, ctx->stream>>>(
-                                           A, a_rs, a_cs, x, x_rs, y, y_rs, m, k, op, p, mp.barrett, r64));
+            // Long rows: the widest chunk that the row's length fills to eight ninths (a pass costs its whole
+            // chunk: 4096 x 4097 takes 27 us in gemv_block_kernel and 48 us as one half-empty chunk per row),
+            // with several passes only where every CTA has several rows per pass (64 x 20000: 9.8 against
+            // 11.5 us); else the kernel that takes any length.  Single words (unaligned rows) are bound by
+            // instructions, which only the widest chunk has fewer of: 8191 x 8191 144 -> 98 us, but 4096 x 4095
+            // 25 -> 31 us with 16 words a row.
+            auto fits = [&](uint64_t chunk, uint64_t rows) {
+                const uint64_t passes = (k + chunk - 1) / chunk;
+                return 8 * passes * chunk <= 9 * static_cast<uint64_t>(k) &&
+                       (passes == 1 || m >= 8 * rows * static_cast<uint64_t>(ctx->num_sms));
+            };
+            const int rows = fits(8192, 1) ? 1 : v4 && fits(4096, 2) ? 2 : v4 && fits(2048, 4) ? 4 : 0;
+            if (rows != 0) {
+                const int grid = static_cast<int>(std::min<size_t>((static_cast<size_t>(m) + rows - 1) / rows,
+                                                                   static_cast<size_t>(2) * ctx->num_sms));
+                auto kernel = !v4         ? gemv_rows_kernel<1, 32, 1>
+                              : rows == 4 ? gemv_rows_kernel<4, 2, 4>
+                              : rows == 2 ? gemv_rows_kernel<4, 4, 2>
+                                          : gemv_rows_kernel<4, 8, 1>;
+                HME_TIMED(ctx, "gemv", kernel<<<grid, 256, 0, ctx->stream>>>(A, a_rs, a_cs, x, x_rs, y, y_rs, m, k, op,
+                                                                            p, mp.barrett, r64));
+            } else {
+                // the grid one wave of resident CTAs
+                int per_sm = 1;
+                HME_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                    &per_sm, v4 ? gemv_block_kernel<4> : gemv_block_kernel<1>, 256, 0));
+                const int grid = static_cast<int>(std::min<size_t>(m, static_cast<size_t>(std::max(1, per_sm)) * ctx->num_sms));
+                if (v4)
+                    HME_TIMED(ctx, "gemv", gemv_block_kernel<4><<<grid, 256, 0, ctx->stream>>>(
+                                               A, a_rs, a_cs, x, x_rs, y, y_rs, m, k, op, p, mp.barrett, r64));
+                else
+                    HME_TIMED(ctx, "gemv", gemv_block_kernel<1><<<grid, 256, 0, ctx->stream>>>(
+                                               A, a_rs, a_cs, x, x_rs, y, y_rs, m, k, op, p, mp.barrett, r64));
+            }
         } else if (a_cs == 1 || a_rs != 1) {
             const int grid = static_cast<int>(std::min<size_t>((static_cast<size_t>(m) + 7) / 8, ctx->num_sms * 16));
             if (v4)
