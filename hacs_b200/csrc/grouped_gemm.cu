@@ -190,8 +190,7 @@ void run_grouped(hme_ctx* ctx, const ModParams& mp, const std::vector<GemmJob>& 
         s.N = static_cast<int>(j.N);
         s.K = static_cast<int>(j.K);
         s.Kp = Kp;
-        s.p = mp.p;
-        s.barrett = mp.barrett;
+        s.red = make_split_red(mp);
         s.planesA = planes + offA[b] + static_cast<size_t>(row0[t]) * Kp;
         s.planesB = planes + offB[b] + static_cast<size_t>(col0[t]) * Kp;
         s.a_plane = static_cast<uint64_t>(b_rows[b]) * Kp;

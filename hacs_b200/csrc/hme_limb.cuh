@@ -104,6 +104,10 @@ inline EpiRed make_epi_bound(const ModParams& mp, unsigned __int128 bound) {
     r.fast = mp.p < (1u << 31) && r.sh1 <= b - 2 ? 1 : 0;
     return r;
 }
+// The constants for 256 v of the limb split, v below 256^limbs.
+inline EpiRed make_split_red(const ModParams& mp) {
+    return make_epi_bound(mp, static_cast<unsigned __int128>(256) << (8 * mp.limbs));
+}
 // The constants for products whose K (per launch) is at most kc.
 inline EpiRed make_epi(const ModParams& mp, uint64_t kc) {
     unsigned __int128 bound = 0;
@@ -682,8 +686,7 @@ struct SplitArgs {
     const uint32_t* B;
     uint64_t ldb;
     int M, N, K, Kp;
-    uint32_t p;
-    uint64_t barrett;
+    EpiRed red;          // make_split_red
     uint8_t* planesA;
     uint8_t* planesB;
     int a_blocks;        // blocks of the A part
@@ -694,18 +697,65 @@ struct SplitArgs {
     Skip skip;
 };
 
+// idx / kch, in 32 bits where the operand's pieces can be counted in them
+__device__ __forceinline__ int split_row(size_t idx, size_t total, int kch) {
+    return total >> 32 ? static_cast<int>(idx / kch)
+                       : static_cast<int>(static_cast<uint32_t>(idx) / static_cast<uint32_t>(kch));
+}
+
+// Rows that are not 16-byte aligned go four words a thread, so that a warp's loads
+// and stores cover consecutive words (16 a thread would load with a stride of 64
+// bytes); figures at split_b_tile.  The index is divided in 32 bits: with a 64-bit
+// division per four words the 65521 half of 2000 uneven jobs took 726 us, 610 so.
+template <int L>
+__device__ __forceinline__ void split_a_words(const SplitArgs& s, int block) {
+    const int kch = s.Kp >> 2;
+    const size_t total = static_cast<size_t>(s.M) * kch;
+    const size_t plane = s.a_plane ? s.a_plane : static_cast<size_t>(s.M) * s.Kp;
+    const size_t step = static_cast<size_t>(s.a_blocks) * blockDim.x;
+    for (size_t i0 = static_cast<size_t>(block) * blockDim.x + threadIdx.x; i0 < total; i0 += 4 * step) {
+        uint32_t x[4][4];
+        uint8_t* dst[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const size_t idx = i0 + u * step, at = min(idx, total - 1);
+            const int row = split_row(at, total, kch);
+            const int k0 = static_cast<int>(at - static_cast<size_t>(row) * kch) << 2;
+            const uint32_t* src = s.A + static_cast<size_t>(row) * s.lda + k0;
+            dst[u] = s.planesA + static_cast<size_t>(row) * s.Kp + k0;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) x[u][e] = idx < total && k0 + e < s.K ? __ldg(src + e) : 0u;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (i0 + u * step >= total) break;
+#pragma unroll
+            for (int j = 0; j < L; ++j) {
+                uint32_t w = 0;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) w |= ((x[u][e] >> (8 * j)) & 0xffu) << (8 * e);
+                *reinterpret_cast<uint32_t*>(dst[u] + j * plane) = w;
+            }
+        }
+    }
+}
+
 template <int L>
 __device__ __forceinline__ void split_a_part(const SplitArgs& s, int block) {
+    if (!s.a_vec) {
+        split_a_words<L>(s, block);
+        return;
+    }
     const int kch = s.Kp >> 4;
     const size_t total = static_cast<size_t>(s.M) * kch;
     const size_t plane = s.a_plane ? s.a_plane : static_cast<size_t>(s.M) * s.Kp;
     for (size_t idx = static_cast<size_t>(block) * blockDim.x + threadIdx.x; idx < total;
          idx += static_cast<size_t>(s.a_blocks) * blockDim.x) {
-        const int row = static_cast<int>(idx / kch);
+        const int row = split_row(idx, total, kch);
         const int k0 = static_cast<int>(idx - static_cast<size_t>(row) * kch) << 4;
         const uint32_t* src = s.A + static_cast<size_t>(row) * s.lda + k0;
         uint32_t x[16];
-        if (s.a_vec && k0 + 16 <= s.K) {
+        if (k0 + 16 <= s.K) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const uint4 v = __ldg(reinterpret_cast<const uint4*>(src) + q);
@@ -726,8 +776,13 @@ __device__ __forceinline__ void split_a_part(const SplitArgs& s, int block) {
     }
 }
 
-template <int L>
-__device__ __forceinline__ void split_b_part(const SplitArgs& s, int block, uint32_t (*tile)[33]) {
+// Bound by the writes of the L^2 planes as long as 256 v mod p is cheap: one
+// 32-bit multiply-high (epi_reduce_u64) where a 64-bit Barrett step took six wide
+// products.
+// Both parts, mod 2^31 - 19, 1677 x 771 x 1419 (unaligned rows): 13.6 -> 9.5 us;
+// mod 65521, 1024^3 5.1 -> 4.1 us, 8192^3 191 -> 175 us (144 at the copy rate).
+template <int L, bool FAST>
+__device__ __forceinline__ void split_b_tile(const SplitArgs& s, int block, uint32_t (*tile)[33]) {
     const int k0 = (block % s.b_blocks_k) * 64, n0 = (block / s.b_blocks_k) * 32;
     // all eight loads of a thread in flight before the first shared-memory store
     // (blockDim.x == 256: 8 x 256 = the 64 x 32 tile)
@@ -757,7 +812,7 @@ __device__ __forceinline__ void split_b_part(const SplitArgs& s, int block, uint
         uint32_t v = tile[kc * 8 + e][nn];
 #pragma unroll
         for (int i = 0; i < L; ++i) {
-            if (i) v = reduce_u64(static_cast<uint64_t>(v) << 8, s.p, s.barrett);
+            if (i) v = epi_reduce_u64<FAST>(static_cast<uint64_t>(v) << 8, s.red);
 #pragma unroll
             for (int j = 0; j < L; ++j) out[i][j][e >> 2] |= ((v >> (8 * j)) & 0xffu) << (8 * (e & 3));
         }
@@ -769,6 +824,12 @@ __device__ __forceinline__ void split_b_part(const SplitArgs& s, int block, uint
         for (int j = 0; j < L; ++j)
             *reinterpret_cast<uint2*>(s.planesB + (i * L + j) * plane + static_cast<size_t>(n) * s.Kp + kb) =
                 make_uint2(out[i][j][0], out[i][j][1]);
+}
+
+template <int L>
+__device__ __forceinline__ void split_b_part(const SplitArgs& s, int block, uint32_t (*tile)[33]) {
+    if (s.red.fast) split_b_tile<L, true>(s, block, tile);
+    else split_b_tile<L, false>(s, block, tile);
 }
 
 }  // namespace limb

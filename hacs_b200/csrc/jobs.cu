@@ -587,6 +587,7 @@ struct RankGroup {
     uint8_t* planesA;
     uint8_t* planesB;
     uint64_t sum_m, sum_n;
+    limb::EpiRed split_red;
     int bn;                  // grouped GEMM tile width
     int begin, end;
     int* tile_prob;          // per tile: the job (index within the group)
@@ -733,8 +734,7 @@ __global__ void rank_post_kernel(RankDev* __restrict__ devs, int nj, const RankO
             sa.N = ntrail;
             sa.K = k;
             sa.Kp = 32;
-            sa.p = J.p;
-            sa.barrett = J.barrett;
+            sa.red = G.split_red;
             sa.planesA = G.planesA + static_cast<size_t>(D.a_row0) * 32;
             sa.planesB = G.planesB + static_cast<size_t>(D.b_col0) * 32;
             sa.a_plane = G.sum_m * 32;
@@ -945,6 +945,7 @@ void batch_rank_device(hme_ctx* ctx, const std::vector<BatchMatrix>& mats, std::
         G.sum_m = sm;
         G.sum_n = sn;
         G.bn = grouped_bn_wide(L);
+        G.split_red = limb::make_split_red(mp);
         G.begin = gbegin[g];
         G.end = gbegin[g + 1];
         g_planes[g] = plane_bytes;

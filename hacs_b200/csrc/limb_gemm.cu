@@ -246,7 +246,7 @@ void launch_split(hme_ctx* ctx, const ModParams& mp, uint32_t m, uint32_t n, uin
     SplitArgs sa{};
     sa.A = A; sa.lda = lda; sa.B = B; sa.ldb = ldb;
     sa.M = static_cast<int>(m); sa.N = static_cast<int>(n); sa.K = static_cast<int>(k); sa.Kp = Kp;
-    sa.p = mp.p; sa.barrett = mp.barrett;
+    sa.red = make_split_red(mp);
     sa.planesA = pa; sa.planesB = pb;
     sa.a_plane = a_plane;
     sa.skip = ctx->gemm_skip;
@@ -627,7 +627,7 @@ extern "C" HME_API int hme_gemm_u32_dev_noalloc(uint32_t p, uint32_t m, uint32_t
         sa.A = A; sa.lda = lda; sa.B = B; sa.ldb = ldb;
         sa.M = static_cast<int>(m); sa.N = static_cast<int>(n); sa.K = static_cast<int>(k);
         sa.Kp = static_cast<int>(Kp);
-        sa.p = mp.p; sa.barrett = mp.barrett;
+        sa.red = make_split_red(mp);
         sa.planesA = pa; sa.planesB = pb;
         const size_t work = static_cast<size_t>(m) * (Kp / 16);
         sa.a_blocks = static_cast<int>(std::min<size_t>((work + 255) / 256, static_cast<size_t>(d.num_sms) * 8));

@@ -54,6 +54,7 @@ struct RrGroup {
     uint8_t* planesA;
     uint8_t* planesB;
     uint64_t sum_m, sum_n;
+    limb::EpiRed split_red;
     int bn;                  // grouped GEMM tile width
     int begin, end;
     int* tile_prob;          // per tile: the job (index within the group)
@@ -563,8 +564,7 @@ __global__ void rr_post_kernel(RrJob* __restrict__ jobs, int nj, RrMove* __restr
             sa.N = ntrail;
             sa.K = k;
             sa.Kp = kRrW;
-            sa.p = G.p;
-            sa.barrett = G.barrett;
+            sa.red = G.split_red;
             sa.planesA = G.planesA + static_cast<size_t>(J.a_row0) * kRrW;
             sa.planesB = G.planesB + static_cast<size_t>(J.b_col0) * kRrW;
             sa.a_plane = G.sum_m * kRrW;
@@ -731,6 +731,7 @@ void batch_rank_rounds(hme_ctx* ctx, const std::vector<BatchMatrix>& mats, std::
         G.sum_m = sm;
         G.sum_n = sn;
         G.bn = bn;
+        G.split_red = limb::make_split_red(mp);
         G.begin = gbegin[g];
         G.end = gbegin[g + 1];
         g_planes[g] = plane_bytes;
