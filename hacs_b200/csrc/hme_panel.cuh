@@ -111,7 +111,10 @@ __device__ __forceinline__ uint32_t valuation(uint32_t x, const Ring& R, uint32_
     return v;
 }
 
-enum : int { kArithPow2 = 0, kArithMont31 = 1, kArithMont32 = 2 };
+// kArithMont13: q < 2^13, where two products, or a sub-panel's seventeen, sum in
+// one 32-bit word.
+enum : int { kArithPow2 = 0, kArithMont31 = 1, kArithMont32 = 2, kArithMont13 = 3 };
+constexpr uint32_t kMont13Max = 1u << 13;
 
 // x / ell^v for x divisible by ell^v
 __device__ __forceinline__ uint32_t div_pw(uint32_t x, uint32_t v, const Ring& R) {
@@ -130,6 +133,10 @@ template <int ARITH>
 __device__ __forceinline__ uint32_t ff_update(uint32_t w, uint32_t y, uint32_t xn, uint32_t pr, const Ring& R) {
     if constexpr (ARITH == kArithPow2) {
         return (w * y + xn * pr) & (R.q - 1u);
+    } else if constexpr (ARITH == kArithMont13) {
+        const uint32_t t = w * y + xn * pr;  // < 2^27: the low words of t + m q cancel, with a carry unless t = 0
+        const uint32_t r = __umulhi(t * R.mont_qinv, R.q) + (t != 0 ? 1u : 0u);
+        return min(r, r - R.q);
     } else if constexpr (ARITH == kArithMont31) {
         // q < 2^31: both products < 2^62, t < 2^63, t + m q < 2^64
         const uint64_t t = static_cast<uint64_t>(w) * y + static_cast<uint64_t>(xn) * pr;
@@ -222,7 +229,8 @@ __device__ __forceinline__ uint32_t ff_scale2(uint32_t x, uint32_t y, const Ring
 // Bound by the chain of w steps and by the multiplier (a reduced update is
 // three wide products).  A 64-column panel mod 2^31 - 19: 43 + 20 us as one
 // CTA's LU and row solves over the GPU, 49 us as 64 whole-row steps, 41 us so;
-// mod 13 (96 slots) 46 us, where the cluster search of 10515 rows took 200 to 270.
+// mod 13 (96 slots) 46 us with the wide products of kArithMont31 and 42 us with
+// kArithMont13, where the cluster search of 10515 rows took 200 to 270.
 template <int ARITH, int RS>
 __device__ bool block_inverse(const BlockArgs& a, uint32_t* s_blk) {
     __shared__ uint32_t s_w[kMaxPanel], s_S[kMaxPanel], s_V[kMaxPanel / kSubCols + 1];
@@ -367,7 +375,7 @@ __device__ bool block_inverse(const BlockArgs& a, uint32_t* s_blk) {
                 for (int e = 0; e < 4; ++e) {
                     const uint64_t t = static_cast<uint64_t>(sy) * vw[e];
                     a0[e] = static_cast<uint32_t>(t);
-                    a1[e] = static_cast<uint32_t>(t >> 32);
+                    a1[e] = ARITH == kArithMont13 ? 0u : static_cast<uint32_t>(t >> 32);
                     a2[e] = 0;
                 }
                 const uint32_t* pq = P + 4 * q;
@@ -385,7 +393,7 @@ __device__ bool block_inverse(const BlockArgs& a, uint32_t* s_blk) {
                             mac96(a0[2], a1[2], a2[2], c[i + e], p[e].z);
                             mac96(a0[3], a1[3], a2[3], c[i + e], p[e].w);
                         }
-                    } else if constexpr (ARITH == kArithPow2) {
+                    } else if constexpr (ARITH == kArithPow2 || ARITH == kArithMont13) {
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
                             a0[0] += c[i + e] * p[e].x;

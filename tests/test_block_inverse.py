@@ -84,7 +84,7 @@ def _rand(rng, shape, p):
 
 # rows around the row slots (64, 96, 128) and the panel widths, p on both sides of the dispatch's lines
 @pytest.mark.gpu
-@pytest.mark.parametrize("p", [2, 3, 13, 251, 257, 1048573, 1048583, 2147483629, 4294967291])
+@pytest.mark.parametrize("p", [2, 3, 13, 251, 257, 8179, 8191, 8209, 1048573, 1048583, 2147483629, 4294967291])
 @pytest.mark.parametrize("m,n", [(1, 5), (63, 64), (64, 65), (65, 64), (95, 200), (96, 96), (97, 130), (129, 70), (200, 333)])
 def test_block_slots(engine, p, m, n):
     rng = np.random.default_rng(m * 1000 + n + p % 97)
