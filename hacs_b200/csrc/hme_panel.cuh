@@ -70,18 +70,36 @@ __device__ __forceinline__ uint32_t mont_mul(uint32_t x, uint32_t y, uint32_t q,
     return static_cast<uint32_t>(r >= q ? r - q : r);
 }
 
-// u^(q-2) mod q (Fermat) for an odd prime q, left-to-right square and
-// multiply in the Montgomery domain: about 2 log2 q dependent products.
-__device__ __forceinline__ uint32_t inv_fermat(uint32_t u, const Ring& R) {
+// The same for odd q < 2^31: no carry out of 64 bits.
+__device__ __forceinline__ uint32_t mont_mul31(uint32_t x, uint32_t y, uint32_t q, uint32_t qinv) {
+    const uint64_t t = static_cast<uint64_t>(x) * y;
+    const uint32_t mq = static_cast<uint32_t>(t) * qinv;
+    const uint32_t r = static_cast<uint32_t>((t + static_cast<uint64_t>(mq) * q) >> 32);
+    return min(r, r - q);
+}
+
+// u^(q-2) mod q (Fermat) for an odd prime q, two bits of the exponent at a time
+// in the Montgomery domain: about 3/2 log2 q dependent products.
+template <bool BELOW31>
+__device__ __forceinline__ uint32_t inv_fermat_as(uint32_t u, const Ring& R) {
     const uint32_t q = R.q, qi = R.mont_qinv;
-    const uint32_t um = mont_mul(u, R.mont_r2, q, qi);  // u * 2^32 mod q
-    const uint32_t e = q - 2;
-    uint32_t r = um;
-    for (int b = 30 - __clz(e); b >= 0; --b) {
-        r = mont_mul(r, r, q, qi);
-        if ((e >> b) & 1u) r = mont_mul(r, um, q, qi);
+    auto mul = [&](uint32_t x, uint32_t y) { return BELOW31 ? mont_mul31(x, y, q, qi) : mont_mul(x, y, q, qi); };
+    const uint32_t u1 = mul(u, R.mont_r2);  // u * 2^32 mod q
+    const uint32_t u2 = mul(u1, u1), u3 = mul(u2, u1);
+    const uint32_t e = q - 2;  // >= 1
+    int b = (31 - __clz(e)) & ~1;
+    uint32_t d = (e >> b) & 3u;
+    uint32_t r = d == 1 ? u1 : d == 2 ? u2 : u3;
+    for (b -= 2; b >= 0; b -= 2) {
+        r = mul(r, r);
+        r = mul(r, r);
+        d = (e >> b) & 3u;
+        if (d) r = mul(r, d == 1 ? u1 : d == 2 ? u2 : u3);
     }
-    return mont_mul(r, 1u, q, qi);  // out of the Montgomery domain
+    return mul(r, 1u);  // out of the Montgomery domain
+}
+__device__ __forceinline__ uint32_t inv_fermat(uint32_t u, const Ring& R) {
+    return R.q < (1u << 31) ? inv_fermat_as<true>(u, R) : inv_fermat_as<false>(u, R);
 }
 
 __device__ __forceinline__ uint32_t unit_inverse(uint32_t u, const Ring& R) {
@@ -195,11 +213,18 @@ __device__ __forceinline__ uint32_t ff_reduce96(uint32_t a0, uint32_t a1, uint32
     }
 }
 
+// x y rho (x y for q = 2^k)
+template <int ARITH>
+__device__ __forceinline__ uint32_t ff_mul(uint32_t x, uint32_t y, const Ring& R) {
+    if constexpr (ARITH == kArithPow2) return (x * y) & (R.q - 1u);
+    else if constexpr (ARITH == kArithMont32) return mont_mul(x, y, R.q, R.mont_qinv);
+    else return mont_mul31(x, y, R.q, R.mont_qinv);
+}
 // x y rho^2 (x y for q = 2^k)
 template <int ARITH>
 __device__ __forceinline__ uint32_t ff_scale2(uint32_t x, uint32_t y, const Ring& R) {
     if constexpr (ARITH == kArithPow2) return (x * y) & (R.q - 1u);
-    else return mont_mul(mont_mul(x, y, R.q, R.mont_qinv), 1u, R.q, R.mont_qinv);
+    else return ff_mul<ARITH>(ff_mul<ARITH>(x, y, R), 1u, R);
 }
 
 // One CTA of 4 RS threads, RS row slots: blocked in-place Gauss-Jordan
@@ -228,12 +253,15 @@ __device__ __forceinline__ uint32_t ff_scale2(uint32_t x, uint32_t y, const Ring
 //
 // Bound by the chain of w steps and by the multiplier (a reduced update is
 // three wide products).  A 64-column panel mod 2^31 - 19: 43 + 20 us as one
-// CTA's LU and row solves over the GPU, 49 us as 64 whole-row steps, 41 us so;
-// mod 13 (96 slots) 46 us with the wide products of kArithMont31 and 42 us with
+// CTA's LU and row solves over the GPU, 49 us as 64 whole-row steps, 37 us so
+// (cycles: 16 steps of a sub-panel 9700, its update 6000, four times; the inverse
+// and the write 10300 before one warp inverted, two exponent bits at a time, and the
+// write took Montgomery products);
+// mod 13 (96 slots) 46 us with the wide products of kArithMont31 and 40 us with
 // kArithMont13, where the cluster search of 10515 rows took 200 to 270.
 template <int ARITH, int RS>
 __device__ bool block_inverse(const BlockArgs& a, uint32_t* s_blk) {
-    __shared__ uint32_t s_w[kMaxPanel], s_S[kMaxPanel], s_V[kMaxPanel / kSubCols + 1];
+    __shared__ uint32_t s_w[kMaxPanel], s_S[kMaxPanel], s_V[kMaxPanel / kSubCols + 2];  // the last word: the scale's inverse
     __shared__ uint32_t s_x[2][RS];  // the rows' entries in the step's column, by parity
     __shared__ int s_prow[kMaxPanel];
     __shared__ int s_cand[2][RS / 32];
@@ -317,7 +345,7 @@ __device__ bool block_inverse(const BlockArgs& a, uint32_t* s_blk) {
                 const unsigned mask = __ballot_sync(0xffffffffu, !pivoted && is_unit(next));
                 if (lane == 0) s_cand[par ^ 1][wg] = mask ? 32 * wg + __ffs(mask) - 1 : RS;
             }
-            S = ARITH == kArithPow2 ? (S * wt) & (R.q - 1u) : mont_mul(S, wt, R.q, R.mont_qinv);
+            S = ff_mul<ARITH>(S, wt, R);
             __syncthreads();
             return true;
         };
@@ -337,7 +365,7 @@ __device__ bool block_inverse(const BlockArgs& a, uint32_t* s_blk) {
         if (mine >= 0) {
             const uint32_t f = mod_mul(s_S[cs + mine], V, R.q, R.barrett);
             if (live) {
-                auto sc = [&](uint32_t x) { return ARITH == kArithPow2 ? (x * f) & (R.q - 1u) : mont_mul(x, f, R.q, R.mont_qinv); };
+                auto sc = [&](uint32_t x) { return ff_mul<ARITH>(x, f, R); };
                 y = make_uint4(sc(y.x), sc(y.y), sc(y.z), sc(y.w));
                 *reinterpret_cast<uint4*>(row + 4 * qg) = y;
             }
@@ -416,12 +444,23 @@ __device__ bool block_inverse(const BlockArgs& a, uint32_t* s_blk) {
         V = ff_scale2<ARITH>(V, S, R);
         __syncthreads();
     }
-    const uint32_t vinv = unit_inverse(V, R);
+    // one warp inverts the scale (the chain's latency; all of them would queue at the multiplier), times
+    // 2^32 for the Montgomery products below
+    if (warp == 0) {
+        const uint32_t vinv = unit_inverse(V, R);
+        if (lane == 0) s_V[kMaxPanel / kSubCols + 1] = ARITH == kArithPow2 ? vinv : ff_mul<ARITH>(vinv, R.mont_r2, R);
+    }
+    __syncthreads();
+    const uint32_t vinv = s_V[kMaxPanel / kSubCols + 1];
+#pragma unroll 4
     for (int t = warp; t < nb; t += NW) {
         const int pl = s_prow[t];
         uint32_t* dst = a.A + static_cast<size_t>(a.r0 + pl) * a.ld + a.c0;
-        for (int j = lane; j < w; j += 32) {
-            const uint32_t v = mod_mul(T[pl * ls + j], vinv, R.q, R.barrett);
+#pragma unroll
+        for (int c = 0; c < WC; ++c) {
+            const int j = lane + 32 * c;
+            if (j >= w) break;
+            const uint32_t v = ff_mul<ARITH>(T[pl * ls + j], vinv, R);
             if (j < nb) a.binv[t * nb + j] = v;
             dst[j] = j >= nb ? v : j == t ? 1u : 0u;
         }
