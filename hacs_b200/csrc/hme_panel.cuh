@@ -253,15 +253,16 @@ __device__ __forceinline__ uint32_t ff_scale2(uint32_t x, uint32_t y, const Ring
 //
 // Bound by the chain of w steps and by the multiplier (a reduced update is
 // three wide products).  A 64-column panel mod 2^31 - 19: 43 + 20 us as one
-// CTA's LU and row solves over the GPU, 49 us as 64 whole-row steps, 37 us so
-// (cycles: 16 steps of a sub-panel 9700, its update 6000, four times; the inverse
+// CTA's LU and row solves over the GPU, 49 us as 64 whole-row steps, 35 us so
+// (cycles: 16 steps of a sub-panel 9700, its update 6000, four times, while every warp
+// kept the running scale in step; the inverse
 // and the write 10300 before one warp inverted, two exponent bits at a time, and the
 // write took Montgomery products);
 // mod 13 (96 slots) 46 us with the wide products of kArithMont31 and 40 us with
 // kArithMont13, where the cluster search of 10515 rows took 200 to 270.
 template <int ARITH, int RS>
 __device__ bool block_inverse(const BlockArgs& a, uint32_t* s_blk) {
-    __shared__ uint32_t s_w[kMaxPanel], s_S[kMaxPanel], s_V[kMaxPanel / kSubCols + 2];  // the last word: the scale's inverse
+    __shared__ uint32_t s_w[kMaxPanel], s_S[kMaxPanel + 1], s_V[kMaxPanel / kSubCols + 2];  // the last word: the scale's inverse
     __shared__ uint32_t s_x[2][RS];  // the rows' entries in the step's column, by parity
     __shared__ int s_prow[kMaxPanel];
     __shared__ int s_cand[2][RS / 32];
@@ -307,7 +308,7 @@ __device__ bool block_inverse(const BlockArgs& a, uint32_t* s_blk) {
             const unsigned mask = __ballot_sync(0xffffffffu, !pivoted && is_unit(y.x));
             if (lane == 0) s_cand[0][wg] = mask ? 32 * wg + __ffs(mask) - 1 : RS;
         }
-        uint32_t S = 1u;
+        if (tid == 0) s_S[cs] = 1u;
         int mine = -1;  // the step of this sub-panel whose pivot is this thread's row
         __syncthreads();
         // step 4 u + C; false when its column has no unit in the block (the same in every thread)
@@ -320,11 +321,10 @@ __device__ bool block_inverse(const BlockArgs& a, uint32_t* s_blk) {
             for (int v = 1; v < RS / 32; ++v) prow = min(prow, s_cand[par][v]);
             if (prow == RS) return false;
             uint4 p4 = *reinterpret_cast<const uint4*>(T + prow * ls + 4 * min(qg, nq - 1));
-            const uint32_t wt = s_x[par][prow];
+            const uint32_t wt = s_x[par][prow], S = s_S[t];
             const uint32_t xn = ff_negate<ARITH>(s_x[par][li], R);
             if (tid == 0) {
                 s_w[t] = wt;
-                s_S[t] = S;
                 s_prow[t] = prow;
             }
             const bool is_pivot = li == prow;
@@ -345,7 +345,10 @@ __device__ bool block_inverse(const BlockArgs& a, uint32_t* s_blk) {
                 const unsigned mask = __ballot_sync(0xffffffffu, !pivoted && is_unit(next));
                 if (lane == 0) s_cand[par ^ 1][wg] = mask ? 32 * wg + __ffs(mask) - 1 : RS;
             }
-            S = ff_mul<ARITH>(S, wt, R);
+            if (warp == 0) {
+                const uint32_t Sn = ff_mul<ARITH>(S, wt, R);
+                if (lane == 0) s_S[t + 1] = Sn;
+            }
             __syncthreads();
             return true;
         };
@@ -360,6 +363,7 @@ __device__ bool block_inverse(const BlockArgs& a, uint32_t* s_blk) {
             if (tid == 0) *a.ok = 0;
             return false;
         }
+        const uint32_t S = s_S[cs + ns];
         if (tid == 0) s_V[sub] = V;
         // C of the pivot rows to the common scale, and the pivot rows' other pieces aside
         if (mine >= 0) {
