@@ -31,6 +31,22 @@ void* Workspace::get(int slot, size_t bytes) {
     return ptr[slot];
 }
 
+bool Workspace::holds(int slot, size_t bytes, cudaStream_t stream) {
+    if (size[slot] >= bytes) return true;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return false;
+    }
+    try {
+        get(slot, bytes);
+        return true;
+    } catch (const Error&) {
+        cudaGetLastError();  // the failed allocation's
+        return false;
+    }
+}
+
 void Workspace::release() {
     for (int s = 0; s < kSlots; ++s) {
         if (ptr[s]) cudaFree(ptr[s]);

@@ -584,15 +584,20 @@ bool rns_gemm_u32_pays(const ModParams& mp, uint32_t m, uint32_t n, uint32_t k) 
     return rns < 0.95 * limb;
 }
 
-// C op= A*B mod p, u32 entries, p < 2^32, device pointers, on ctx->stream.
-void rns_gemm_u32_device(hme_ctx* ctx, const ModParams& mp, uint32_t m, uint32_t n, uint32_t k, const uint32_t* A,
+// C op= A*B mod p, u32 entries, p < 2^32, device pointers, on ctx->stream; false, with nothing done, when its
+// planes (up to twice the limb product's) cannot be had.
+bool rns_gemm_u32_device(hme_ctx* ctx, const ModParams& mp, uint32_t m, uint32_t n, uint32_t k, const uint32_t* A,
                          size_t lda, const uint32_t* B, size_t ldb, uint32_t* C, size_t ldc, int op) {
     const RnsPlan P = make_plan(mp.p, k, 4);
     const int Kp = limb_kp(k);
     const size_t pbytes = align256(static_cast<size_t>(P.t) * n * Kp);
-    uint8_t* pa = static_cast<uint8_t*>(ctx->ws.get(kSlotPlanesA, static_cast<size_t>(P.t) * m * Kp));
-    uint8_t* pb = static_cast<uint8_t*>(ctx->ws.get(kSlotPlanesB, pbytes + static_cast<size_t>(P.t) * m * ((n + 31) / 32 * 32)));
+    const size_t need_a = static_cast<size_t>(P.t) * m * Kp;
+    const size_t need_b = pbytes + static_cast<size_t>(P.t) * m * ((n + 31) / 32 * 32);
+    if (!ctx->ws.holds(kSlotPlanesA, need_a, ctx->stream) || !ctx->ws.holds(kSlotPlanesB, need_b, ctx->stream)) return false;
+    uint8_t* pa = static_cast<uint8_t*>(ctx->ws.get(kSlotPlanesA, need_a));
+    uint8_t* pb = static_cast<uint8_t*>(ctx->ws.get(kSlotPlanesB, need_b));
     rns_gemm(ctx, P, m, n, k, A, lda, B, ldb, C, ldc, op, pa, pb, pb + pbytes);
+    return true;
 }
 
 }  // namespace hme

@@ -101,8 +101,9 @@ inline bool rank_variant_simt(int v) { return v == kRankSimtLast128 || v == kRan
 // ranks[j] = rank of mats[j] over F_p (destroys the matrices).
 void batch_rank_device(hme_ctx* ctx, const std::vector<BatchMatrix>& mats, std::vector<int>& ranks);
 // The same for the jobs of `order`, in rounds of 64 columns: 1 to 1024 rows, at
-// least one column each (rank_rounds.cu).
-void batch_rank_rounds(hme_ctx* ctx, const std::vector<BatchMatrix>& mats, std::vector<int> order,
+// least one column each (rank_rounds.cu); false, with nothing done, when its
+// buffers (up to 1.4 times the schedules') cannot be had.
+bool batch_rank_rounds(hme_ctx* ctx, const std::vector<BatchMatrix>& mats, std::vector<int> order,
                        std::vector<int>& ranks);
 
 // One seeded matrix of the job-stream generator.

@@ -83,6 +83,9 @@ struct Workspace {
     bool retain = false;
     std::vector<void*> retired;
     void* get(int slot, size_t bytes);
+    // Whether the slot holds `bytes`, grown if need be; false during a capture that would have to allocate and
+    // when the memory cannot be had: for methods with a cheaper one to fall back on.
+    bool holds(int slot, size_t bytes, cudaStream_t stream);
     void release();
 };
 
@@ -264,7 +267,7 @@ int limb_kp(uint32_t k);
 // The product over the 8-bit residue system (gemm_u64.cu), and whether it beats
 // the limb product.
 bool rns_gemm_u32_pays(const ModParams& mp, uint32_t m, uint32_t n, uint32_t k);
-void rns_gemm_u32_device(hme_ctx* ctx, const ModParams& mp, uint32_t m, uint32_t n, uint32_t k, const uint32_t* A,
+bool rns_gemm_u32_device(hme_ctx* ctx, const ModParams& mp, uint32_t m, uint32_t n, uint32_t k, const uint32_t* A,
                          size_t lda, const uint32_t* B, size_t ldb, uint32_t* C, size_t ldc, int op);
 // C op= A*B mod 2^32 (native wraparound u32 arithmetic, any u32 words) on the
 // same limb-split + tcgen05 kernels: with the modulus constants p = 0 and

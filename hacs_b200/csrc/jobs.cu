@@ -861,10 +861,7 @@ void batch_rank_device(hme_ctx* ctx, const std::vector<BatchMatrix>& mats, std::
     }
     if (order.empty()) return;
     // jobs under the batch rule beside scheduled ones run on rank_rule's schedule, in the same rounds
-    if (!scheduled) {
-        batch_rank_rounds(ctx, mats, std::move(order), ranks);
-        return;
-    }
+    if (!scheduled && batch_rank_rounds(ctx, mats, order, ranks)) return;
     // modulus groups: jobs sorted by modulus (stable)
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return mats[x].p < mats[y].p; });
     const int nj = static_cast<int>(order.size());

@@ -315,10 +315,9 @@ void gemm_u32_device(hme_ctx* ctx, const ModParams& mp, uint32_t m, uint32_t n, 
                      size_t lda, const uint32_t* B, size_t ldb, uint32_t* C, size_t ldc, int op) {
     int v = ctx->fixed_variant;
     if (v < 0 && ctx->sched_policy == 0 && (op == HME_SET || op == HME_ADD || op == HME_SUB) && A && B && C &&
-        lda >= k && ldb >= n && ldc >= n && rns_gemm_u32_pays(mp, m, n, k)) {
-        rns_gemm_u32_device(ctx, mp, m, n, k, A, lda, B, ldb, C, ldc, op);
+        lda >= k && ldb >= n && ldc >= n && rns_gemm_u32_pays(mp, m, n, k) &&
+        rns_gemm_u32_device(ctx, mp, m, n, k, A, lda, B, ldb, C, ldc, op))
         return;
-    }
     if (v < 0) v = sched_variant(ctx, mp, m, n, k);
     gemm_u32_variant(ctx, mp, m, n, k, A, lda, B, ldb, C, ldc, op, v);
 }

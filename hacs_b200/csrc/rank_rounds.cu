@@ -670,7 +670,7 @@ size_t general_smem(int rows, int w) { return sizeof(uint32_t) * static_cast<siz
 
 }  // namespace
 
-void batch_rank_rounds(hme_ctx* ctx, const std::vector<BatchMatrix>& mats, std::vector<int> order,
+bool batch_rank_rounds(hme_ctx* ctx, const std::vector<BatchMatrix>& mats, std::vector<int> order,
                        std::vector<int>& ranks) {
     // modulus groups: jobs sorted by modulus (stable)
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return mats[x].p < mats[y].p; });
@@ -756,6 +756,9 @@ void batch_rank_rounds(hme_ctx* ctx, const std::vector<BatchMatrix>& mats, std::
         o_tp[g] = take(sizeof(int) * g_tiles[g]);
         o_bj[g] = take(sizeof(int) * g_blocks[g]);
     }
+    if (!ctx->ws.holds(kSlotJobs1, tb, ctx->stream) || !ctx->ws.holds(kSlotJobs4, buf_bytes, ctx->stream) ||
+        !ctx->ws.holds(kSlotJobs0, plane_bytes, ctx->stream))
+        return false;
     uint8_t* tables = static_cast<uint8_t*>(ctx->ws.get(kSlotJobs1, tb));
     uint8_t* bufs = static_cast<uint8_t*>(ctx->ws.get(kSlotJobs4, buf_bytes));
     uint8_t* planes = static_cast<uint8_t*>(ctx->ws.get(kSlotJobs0, plane_bytes));
@@ -925,6 +928,7 @@ void batch_rank_rounds(hme_ctx* ctx, const std::vector<BatchMatrix>& mats, std::
     check_device_error(ctx);
     HME_CUDA(cudaMemcpy(jobs.data(), d_jobs, sizeof(RrJob) * nj, cudaMemcpyDeviceToHost));
     for (int i = 0; i < nj; ++i) ranks[order[i]] = jobs[i].r0;
+    return true;
 }
 
 }  // namespace hme

@@ -61,3 +61,31 @@ def test_u32_long_k(engine, p, m, n, k):
             assert (buf[:, n:] == 7).all()
     finally:
         engine.use_own_stream()
+
+
+def test_captured_product_without_room_for_the_residue_planes():
+    """A context warmed with limb products only: a capture cannot grow the planes to what the residue system
+    takes, so the captured product takes the limb route; outside the capture it may take the other.  Both agree."""
+    import torch
+
+    import hacs_b200
+    from hacs_b200 import _lib
+
+    p, n = 2147483629, 3072
+    s = torch.cuda.Stream()
+    with hacs_b200.Engine(0) as eng, torch.cuda.stream(s):
+        eng.use_torch_stream()
+        A, B = (torch.randint(0, p, (n, n), dtype=torch.int32, device="cuda") for _ in range(2))
+        C = [torch.zeros((n, n), dtype=torch.int32, device="cuda") for _ in range(3)]
+        assert _lib.lib().hme_ctx_set_gemm_variant(eng._h, 0) == 0
+        eng.gemm_dev(p, A, B, C[0])
+        assert _lib.lib().hme_ctx_set_gemm_variant(eng._h, -1) == 0
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=s):
+            eng.gemm_dev(p, A, B, C[1])
+        graph.replay()
+        torch.cuda.synchronize()
+        eng.gemm_dev(p, A, B, C[2])
+        torch.cuda.synchronize()
+        assert torch.equal(C[0], C[1]) and torch.equal(C[0], C[2])
