@@ -442,8 +442,9 @@ def extra_rref(eng, reps=3):
     eng.rref_dev(p, A)
     eng.sync()
     b1, s1 = eng.elim_panel_stats()
-    kern = kernel_breakdown(eng, ["panel_block", "panel_w", "panel_factor", "limb_split", "limb_gemm", "trsm", "row_permute",
-                                  "tri_inv", "gather_cols", "assemble_rref", "gather", "copy"])
+    kern = kernel_breakdown(eng, ["panel_block", "panel_rows", "panel_compact", "panel_factor", "panel_linv",
+                                  "panel_w", "row_moves", "limb_split", "limb_gemm", "tri_inv", "gather_cols",
+                                  "assemble_rref", "gather", "copy"])
     eng.set_timing(False)
     lu = n * n * r - (n + n) * r * r / 2 + r ** 3 / 3
     back = r * r * (n - r) / 2
@@ -943,7 +944,8 @@ def run_case(args):
         stream_once()
         eng.sync()
         names = ("grouped_gemm", "grouped_split", "batch_panel", "batch_simt_update", "batch_trsm",
-                 "batch_permute", "batch_gather", "rank_post", "rank_plan", "limb_gemm", "simt_gemm")
+                 "batch_permute", "batch_gather", "rank_block", "rank_general", "rank_moves", "rank_apply",
+                 "rank_post", "rank_plan", "limb_gemm", "simt_gemm")
         out["kernels_ms"] = {k: round(eng.kernel_time(k)[0], 3) for k in names if eng.kernel_time(k)[1]}
         eng.set_timing(False)
         print(json.dumps(default=_json, obj=out), flush=True)
