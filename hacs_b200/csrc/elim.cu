@@ -33,7 +33,7 @@
 // matrix stops there.
 // Then RREF = U1^-1 U on the free columns only (the pivot columns of the RREF
 // are the identity): every diagonal block of U1 is inverted in shared memory
-// (one launch, tri_inv_kernel), and the blocked backward substitution is two limb GEMMs per
+// (one launch, tri_inv_kernel), many blocks are joined by pairs (pair_blocks_kernel), and the blocked backward substitution is two limb GEMMs per
 // block (X_B = U_BB^-1 W_B, then W_above -= U_above,B X_B).
 #include <cuda_runtime.h>
 
@@ -46,6 +46,7 @@
 #include <vector>
 
 #include "hme_elim.h"
+#include "hme_grouped.h"
 #include "hme_internal.h"
 #include "hme_panel.cuh"
 #include "hme_ptx.cuh"
@@ -1240,6 +1241,32 @@ __global__ void __launch_bounds__(1024) tri_inv_kernel(const uint32_t* __restric
     }
 }
 
+// Neighbouring diagonal blocks of U1 as one: [B1 U12; 0 B2]^-1 = [I1, -I1 U12 I2;
+// 0, I2].  Each step of the substitution is four or five launches in a chain (about
+// 25 us), so half as many steps pay for the two products of all pairs at once (about
+// 25 us of kernels and two table uploads): RREF 4096 x 4096 of rank 3900 mod 2^31 - 19
+// 4.84 ms with blocks of 128, 4.58 with pairs, 4.52 with pairs of pairs; 10515 x 8668
+// mod 13 18.05, 17.18 and 16.83 ms.  Below kPairBlocks blocks a level costs what it
+// saves, and one more would save four steps of the former.  This kernel lays out the
+// pairs: V (its blocks' inverses, 0 elsewhere, ld = the pair's size) and U12.
+constexpr int kPairBlocks = 8, kPairFrom = 256;  // pairs of blocks of 128 and 256
+
+__global__ void __launch_bounds__(256) pair_blocks_kernel(const uint32_t* __restrict__ A, uint64_t ld,
+                                                          const int* __restrict__ pcols, int rank, int bb,
+                                                          const uint32_t* __restrict__ Uinv, uint32_t* __restrict__ V,
+                                                          uint32_t* __restrict__ U12) {
+    const int i0 = static_cast<int>(blockIdx.x) * 2 * bb, nb = min(2 * bb, rank - i0), n1 = min(bb, nb), n2 = nb - n1;
+    const uint32_t* I1 = Uinv + static_cast<size_t>(2 * blockIdx.x) * bb * bb;
+    const uint32_t* I2 = I1 + static_cast<size_t>(bb) * bb;
+    uint32_t* v = V + static_cast<size_t>(blockIdx.x) * 4 * bb * bb;
+    uint32_t* u = U12 + static_cast<size_t>(blockIdx.x) * bb * bb;
+    for (int r = blockIdx.y; r < nb; r += gridDim.y)
+        for (int c = threadIdx.x; c < nb; c += 256) {
+            v[r * nb + c] = r < n1 ? (c < n1 ? I1[r * n1 + c] : 0u) : c < n1 ? 0u : I2[(r - n1) * n2 + c - n1];
+            if (r < n1 && c >= n1) u[r * n2 + c - n1] = A[static_cast<size_t>(i0 + r) * ld + pcols[i0 + c]];
+        }
+}
+
 // R (m x n, ld ldr): rows < rank: identity at the pivot columns, X at the free
 // columns; rows >= rank: zero.
 __global__ void assemble_rref_kernel(uint32_t* __restrict__ R, uint64_t ldr, int m, int n, int rank,
@@ -1959,14 +1986,59 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
                   gather_cols_kernel<<<grid_1d(static_cast<size_t>(rank) * f, ctx->num_sms), 256, 0, ctx->stream>>>(
                       A, ld, 0, rank, d_cols, f, X));
         HME_CUDA(cudaGetLastError());
-        const int bb = std::max(16, std::min(opt.back_block > 0 ? opt.back_block : 128, 128));
-        const int nblk = (rank + bb - 1) / bb;
+        int bb = std::max(16, std::min(opt.back_block > 0 ? opt.back_block : 128, 128));
+        int nblk = (rank + bb - 1) / bb;
         // all diagonal blocks of U1 inverted at once, one CTA each
-        uint32_t* Uinv = static_cast<uint32_t*>(ctx->ws.get(kSlotElim5, sizeof(uint32_t) * static_cast<size_t>(nblk) * bb * bb));
+        // words of the blocks, then per level of pairs V, U12 and T
+        const auto paired = [](int b, int blocks) { return b >= 128 && b <= kPairFrom && blocks >= kPairBlocks; };
+        size_t words = static_cast<size_t>(nblk) * bb * bb;
+        for (int b = bb, k = nblk; paired(b, k); b *= 2) {
+            k = (k + 1) / 2;
+            words += 6 * static_cast<size_t>(k) * b * b;
+        }
+        uint32_t* Uinv = static_cast<uint32_t*>(ctx->ws.get(kSlotElim5, sizeof(uint32_t) * words));
         {
             HME_TIMED(ctx, "tri_inv", tri_inv_kernel<<<nblk, 1024, linv_smem_bytes(std::min(bb, rank)), ctx->stream>>>(
                                           A, ld, d_piv, rank, bb, rg, Uinv));
             HME_CUDA(cudaGetLastError());
+        }
+        uint32_t* next = Uinv + static_cast<size_t>(nblk) * bb * bb;
+        while (paired(bb, nblk)) {
+            const int pairs = (nblk + 1) / 2;
+            const size_t bsq = static_cast<size_t>(bb) * bb;
+            uint32_t* V = next;
+            uint32_t* U12 = V + 4 * bsq * pairs;
+            uint32_t* T = U12 + bsq * pairs;
+            next = T + bsq * pairs;
+            HME_TIMED(ctx, "tri_inv", pair_blocks_kernel<<<dim3(pairs, 16), 256, 0, ctx->stream>>>(A, ld, d_piv, rank, bb,
+                                                                                                  Uinv, V, U12));
+            HME_CUDA(cudaGetLastError());
+            std::vector<GemmJob> first, second;
+            for (int j = 0; j < pairs; ++j) {
+                const uint32_t nb = static_cast<uint32_t>(std::min(2 * bb, rank - 2 * j * bb)), n1 = std::min<uint32_t>(bb, nb);
+                if (nb == n1) continue;
+                GemmJob g;
+                g.M = n1;
+                g.N = g.K = nb - n1;
+                g.A = U12 + bsq * j;
+                g.B = Uinv + bsq * (2 * j + 1);
+                g.C = T + bsq * j;
+                g.lda = g.ldb = g.ldc = nb - n1;
+                first.push_back(g);
+                g.K = n1;
+                g.A = Uinv + bsq * (2 * j);
+                g.lda = n1;
+                g.B = T + bsq * j;
+                g.C = V + 4 * bsq * j + n1;
+                g.ldc = nb;
+                g.op = HME_SUB;
+                second.push_back(g);
+            }
+            grouped_gemm_u32_device(ctx, mp, first);
+            grouped_gemm_u32_device(ctx, mp, second);
+            Uinv = V;
+            bb *= 2;
+            nblk = pairs;
         }
         // W (rank x f) in X's slot; the solution accumulates in Xs
         uint32_t* Xs = static_cast<uint32_t*>(ctx->ws.get(kSlotElim6, sizeof(uint32_t) * static_cast<size_t>(rank) * f));
