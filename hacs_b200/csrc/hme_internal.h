@@ -24,12 +24,16 @@ struct Error : std::runtime_error {
 
 void set_last_error(const std::string& msg);
 
+// (The runtime keeps a failed call's error for the next cudaGetLastError, which the check behind a later
+// call's kernel launch would report as its own: it is taken out here.)
 #define HME_CUDA(call)                                                                                  \
     do {                                                                                                \
         cudaError_t e_ = (call);                                                                        \
-        if (e_ != cudaSuccess)                                                                          \
+        if (e_ != cudaSuccess) {                                                                        \
+            cudaGetLastError();                                                                         \
             throw ::hme::Error(e_ == cudaErrorMemoryAllocation ? HME_ENOMEM : HME_ECUDA,                \
                                std::string(#call) + ": " + cudaGetErrorString(e_));                     \
+        }                                                                                               \
     } while (0)
 
 #define HME_REQUIRE(cond, msg)                                        \
