@@ -1374,6 +1374,26 @@ int setup_kernels(int device) {
     return cluster_caps[device];
 }
 
+// The SMs and the skip word of the context's products while this lives, an
+// exception's way out included: the word lies in the elimination's scratch, and a
+// later product that read it would stand still or read freed memory.
+class ProductSettings {
+  public:
+    ProductSettings(hme_ctx* ctx, int sm_cap, const Skip& skip) : ctx_(ctx) {
+        ctx->gemm_sm_cap = sm_cap;
+        ctx->gemm_skip = skip;
+    }
+    ~ProductSettings() {
+        ctx_->gemm_sm_cap = 0;
+        ctx_->gemm_skip = Skip{};
+    }
+    ProductSettings(const ProductSettings&) = delete;
+    ProductSettings& operator=(const ProductSettings&) = delete;
+
+  private:
+    hme_ctx* ctx_;
+};
+
 int panel_width(const ElimOptions& opt) { return std::max(1, std::min<int>(opt.panel > 0 ? opt.panel : 64, kMaxPanel)); }
 
 // The cluster that runs a panel of rows x w: it doubles (up to the largest the
@@ -1776,13 +1796,10 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
                                                                      U.skip, U.Wf));
             HME_CUDA(cudaGetLastError());
         }
-        ctx->gemm_sm_cap = sm_cap;
-        ctx->gemm_skip = U.skip;
+        const ProductSettings settings(ctx, sm_cap, U.skip);
         uint32_t* C12 = A + static_cast<size_t>(U.r0) * ld + ua;
         gemm_u32_variant(ctx, mp, rows, cb - ua, k, U.Wf, U.by == 2 ? bw : k, C12, ld, C12, ld, HME_ADD,
                          gemm_default_variant(ctx, mp, rows, cb - ua));
-        ctx->gemm_sm_cap = 0;
-        ctx->gemm_skip = Skip{};
     };
     int r0 = 0, c0 = 0, par = 0;
     int next_look = 0;  // panel count before which a pivotless panel does not look over the rest

@@ -48,3 +48,24 @@ def test_call_after_a_failed_allocation(eng):
         eng.gemm_dev(P31, A, B, C)
     assert e.value.code == _lib.HME_ENOMEM
     assert _product_is_right(eng)
+
+
+def test_product_after_an_elimination_that_ran_out_of_memory(eng):
+    """The update right of a panel of 65 x 160 000 000 takes 164 GB of planes, with the panel's update queued
+    before its outcome is known; the zero in the corner makes the panel raise the flag that queued work obeys."""
+    import torch
+
+    if torch.cuda.mem_get_info()[0] < 50 << 30:
+        pytest.skip("needs 45 GB of device memory")
+    A = torch.zeros((65, 160_000_000), dtype=torch.int32, device="cuda")
+    A[:, :64].random_(1, P31)
+    A[0, 0] = 0
+    with pytest.raises(_lib.HmeError) as e:
+        eng.rref_dev(P31, A)
+    assert e.value.code == _lib.HME_ENOMEM
+    del A
+    assert _product_is_right(eng)
+    B = np.random.default_rng(3).integers(0, P31, (150, 170), dtype=np.uint64).astype(np.uint32)
+    R, piv = eng.rref(P31, B)
+    wR, wpiv = O.rref(P31, B)
+    assert np.array_equal(R, wR) and list(piv) == list(wpiv)
