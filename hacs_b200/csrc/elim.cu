@@ -40,6 +40,7 @@
 #include <algorithm>
 #include <climits>
 #include <cstring>
+#include <exception>
 #include <mutex>
 #include <numeric>
 #include <type_traits>
@@ -1394,6 +1395,28 @@ class ProductSettings {
     hme_ctx* ctx_;
 };
 
+// On an exception's way out of an elimination: the context's stream as the caller
+// set it, and nothing of the elimination in flight on it or on the second stream
+// (the caller may free the matrix, and the next elimination takes the same scratch).
+class FailureDrain {
+  public:
+    explicit FailureDrain(hme_ctx* ctx) : ctx_(ctx), stream_(ctx->stream), exceptions_(std::uncaught_exceptions()) {}
+    ~FailureDrain() {
+        if (std::uncaught_exceptions() == exceptions_) return;
+        ctx_->stream = stream_;
+        cudaStreamSynchronize(ctx_->aux_stream);
+        cudaStreamSynchronize(stream_);
+        cudaGetLastError();
+    }
+    FailureDrain(const FailureDrain&) = delete;
+    FailureDrain& operator=(const FailureDrain&) = delete;
+
+  private:
+    hme_ctx* ctx_;
+    cudaStream_t stream_;
+    int exceptions_;
+};
+
 int panel_width(const ElimOptions& opt) { return std::max(1, std::min<int>(opt.panel > 0 ? opt.panel : 64, kMaxPanel)); }
 
 // The cluster that runs a panel of rows x w: it doubles (up to the largest the
@@ -1530,6 +1553,7 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
     // ev_panel: the panel's kernels are done; ev_host: its results are in pinned memory
     const cudaEvent_t ev_next = ctx->elim_ev[0], *ev_panel = &ctx->elim_ev[1], *ev_host = &ctx->elim_ev[1 + kRing];
     const cudaStream_t s_main = ctx->stream, s_aux = ctx->aux_stream;
+    const FailureDrain drain(ctx);
     // lookahead only where it can overlap: the cluster kernel (a few SMs), and not while the
     // per-kernel timer is on (its events assume one stream)
     const bool allow_lookahead = !opt.no_lookahead && !ctx->timer.on;

@@ -69,3 +69,21 @@ def test_product_after_an_elimination_that_ran_out_of_memory(eng):
     R, piv = eng.rref(P31, B)
     wR, wpiv = O.rref(P31, B)
     assert np.array_equal(R, wR) and list(piv) == list(wpiv)
+
+
+def test_matrix_is_free_once_its_elimination_has_failed(eng):
+    """The panel after the first was launched ahead on a second stream when the update failed: once the call has
+    returned its error, nothing writes the matrix any more."""
+    import torch
+
+    if torch.cuda.mem_get_info()[0] < 50 << 30:
+        pytest.skip("needs 45 GB of device memory")
+    A = torch.zeros((65, 160_000_000), dtype=torch.int32, device="cuda")
+    for _ in range(3):
+        A[:, :256].random_(1, P31)
+        with pytest.raises(_lib.HmeError) as e:
+            eng.rref_dev(P31, A)
+        assert e.value.code == _lib.HME_ENOMEM
+        A[:, :256] = 7
+        torch.cuda.synchronize()
+        assert bool((A[:, :256] == 7).all())
