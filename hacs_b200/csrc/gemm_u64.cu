@@ -452,14 +452,25 @@ RnsPlan make_plan(uint64_t p, uint32_t k, int bytes) {
     return P;
 }
 
+// The largest first row of a plane: TMA coordinates are signed 32-bit numbers, and the stacked planes of one
+// launch put row r of plane t at t m + r.
+constexpr uint32_t kMaxPlaneRows = (1u << 31) - 256;
+
+// One launch over moduli [t0, t0 + moduli) and a chunk of K after another.
 template <int BN, int KB>
-void launch_rns_gemm(hme_ctx* ctx, uint32_t m, uint32_t n, uint32_t k, int Kp, uint8_t* pa, uint8_t* pb, uint8_t* Y,
-                     int Np, const RnsPlan& P) {
+void launch_rns_run(hme_ctx* ctx, uint32_t m, uint32_t n, uint32_t k, int Kp, uint8_t* pa, uint8_t* pb, uint8_t* Y,
+                    int Np, const RnsPlan& plan, int t0, int moduli) {
     using CF = Cfg<1, BN, KB>;
-    static OncePerDevice attr;
-    attr.run([](int) {
-        HME_CUDA(cudaFuncSetAttribute(rns_gemm_kernel<BN, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, CF::SMEM));
-    });
+    RnsPlan P = plan;  // the run's moduli first
+    P.t = moduli;
+    for (int t = 0; t < moduli; ++t) {
+        P.m[t] = plan.m[t0 + t];
+        P.red[t] = plan.red[t0 + t];
+        P.sh[t] = plan.sh[t0 + t];
+    }
+    pa += static_cast<size_t>(t0) * m * Kp;
+    pb += static_cast<size_t>(t0) * n * Kp;
+    Y += static_cast<size_t>(t0) * m * Np;
     CUtensorMap tmA, tmB;
     {
         const cuuint64_t dims[3] = {static_cast<cuuint64_t>(Kp), static_cast<cuuint64_t>(m) * P.t, 1};
@@ -489,13 +500,27 @@ void launch_rns_gemm(hme_ctx* ctx, uint32_t m, uint32_t n, uint32_t k, int Kp, u
         at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = at;
-        cfg.numAttrs = k0 == 0 && !ctx->timer.on ? 1 : 0;
+        cfg.numAttrs = t0 == 0 && k0 == 0 && !ctx->timer.on ? 1 : 0;
         HME_TIMED(ctx, "limb_gemm",
                   HME_CUDA(cudaLaunchKernelEx(&cfg, rns_gemm_kernel<BN, KB>, tmA, tmB, static_cast<int>(m),
                                               static_cast<int>(n), static_cast<int>(k0),
                                               static_cast<int>((kc + KB - 1) / KB), Y, Np, k0 == 0 ? 0 : 1, ctx->d_err,
                                               P)));
     }
+}
+
+template <int BN, int KB>
+void launch_rns_gemm(hme_ctx* ctx, uint32_t m, uint32_t n, uint32_t k, int Kp, uint8_t* pa, uint8_t* pb, uint8_t* Y,
+                     int Np, const RnsPlan& P) {
+    static OncePerDevice attr;
+    attr.run([](int) {
+        HME_CUDA(cudaFuncSetAttribute(rns_gemm_kernel<BN, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      Cfg<1, BN, KB>::SMEM));
+    });
+    // all moduli in one launch, unless their planes' rows pass the coordinates (8 x 200 000 000 mod 2^40 - 87)
+    const int run = static_cast<int>(std::min<uint32_t>(P.t, kMaxPlaneRows / std::max(m, n)));
+    for (int t0 = 0; t0 < P.t; t0 += run)
+        launch_rns_run<BN, KB>(ctx, m, n, k, Kp, pa, pb, Y, Np, P, t0, std::min(run, P.t - t0));
 }
 
 // C op= A*B mod p over the residue system; pa, pb, Y: the planes' buffers.
@@ -542,6 +567,7 @@ void gemm_u64_device(hme_ctx* ctx, uint64_t p, uint32_t m, uint32_t n, uint32_t 
         return;
     }
     HME_REQUIRE(A && B && lda >= k && ldb >= n, "gemm_u64: bad A / B");
+    HME_REQUIRE(std::max({m, n, k}) <= kMaxPlaneRows, "gemm_u64: dimension too large");
     const int sms = ctx->num_sms;
     if (p < (uint64_t(1) << 32)) {
         uint32_t* a32 = static_cast<uint32_t*>(ctx->ws.get(kSlotRns0, 4ull * m * k));
