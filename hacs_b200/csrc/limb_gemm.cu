@@ -311,12 +311,26 @@ int gemm_default_variant(const hme_ctx* ctx, const ModParams& mp, uint32_t m, ui
 
 int limb_kp(uint32_t k) { return static_cast<int>((k + kblock_for(k) - 1) / kblock_for(k) * kblock_for(k)); }
 
+namespace {
+
+// What every product asks of its arguments; false when there is nothing to compute.
+bool check_product(const ModParams& mp, uint32_t m, uint32_t n, uint32_t k, size_t ldc, int op) {
+    HME_REQUIRE(op == HME_SET || op == HME_ADD || op == HME_SUB, "gemm: op must be HME_SET, HME_ADD or HME_SUB");
+    HME_REQUIRE(mp.p >= 2, "gemm: modulus must be >= 2");
+    HME_REQUIRE(m < (1u << 30) && n < (1u << 30) && k < (1u << 30), "gemm: dimension too large");
+    if (m == 0 || n == 0) return false;
+    HME_REQUIRE(ldc >= n, "gemm: ldc < n");
+    return true;
+}
+
+}  // namespace
+
 void gemm_u32_device(hme_ctx* ctx, const ModParams& mp, uint32_t m, uint32_t n, uint32_t k, const uint32_t* A,
                      size_t lda, const uint32_t* B, size_t ldb, uint32_t* C, size_t ldc, int op) {
+    if (!check_product(mp, m, n, k, ldc, op)) return;
     int v = ctx->fixed_variant;
-    if (v < 0 && ctx->sched_policy == 0 && (op == HME_SET || op == HME_ADD || op == HME_SUB) && A && B && C &&
-        lda >= k && ldb >= n && ldc >= n && rns_gemm_u32_pays(mp, m, n, k) &&
-        rns_gemm_u32_device(ctx, mp, m, n, k, A, lda, B, ldb, C, ldc, op))
+    if (v < 0 && ctx->sched_policy == 0 && k > 0 && A && B && C && lda >= k && ldb >= n &&
+        rns_gemm_u32_pays(mp, m, n, k) && rns_gemm_u32_device(ctx, mp, m, n, k, A, lda, B, ldb, C, ldc, op))
         return;
     if (v < 0) v = sched_variant(ctx, mp, m, n, k);
     gemm_u32_variant(ctx, mp, m, n, k, A, lda, B, ldb, C, ldc, op, v);
@@ -324,12 +338,8 @@ void gemm_u32_device(hme_ctx* ctx, const ModParams& mp, uint32_t m, uint32_t n, 
 
 void gemm_u32_variant(hme_ctx* ctx, const ModParams& mp, uint32_t m, uint32_t n, uint32_t k, const uint32_t* A,
                       size_t lda, const uint32_t* B, size_t ldb, uint32_t* C, size_t ldc, int op, int variant) {
-    HME_REQUIRE(op == HME_SET || op == HME_ADD || op == HME_SUB, "gemm: op must be HME_SET, HME_ADD or HME_SUB");
     HME_REQUIRE(variant >= 0 && variant < kGemmVariants, "gemm: unknown variant");
-    HME_REQUIRE(mp.p >= 2, "gemm: modulus must be >= 2");
-    HME_REQUIRE(m < (1u << 30) && n < (1u << 30) && k < (1u << 30), "gemm: dimension too large");
-    if (m == 0 || n == 0) return;
-    HME_REQUIRE(ldc >= n, "gemm: ldc < n");
+    if (!check_product(mp, m, n, k, ldc, op)) return;
     if (k == 0) {
         if (op == HME_SET) {
             HME_TIMED(ctx, "fill_zero",

@@ -38,3 +38,41 @@ def test_planes_beyond_a_32_bit_coordinate(p, wide):
         for c0 in range(0, n, 20_000_000):
             s = slice(c0, min(n, c0 + 20_000_000))
             assert torch.equal(C[0, s].to(torch.int64), B[0, s].to(torch.int64) * a % p), c0
+
+
+@pytest.mark.parametrize("m,n,k", [(0, 4096, 4096), (4096, 0, 4096), (0, 0, 4096)])
+def test_empty_product_touches_nothing(m, n, k):
+    """No rows (or columns) and non-null pointers: C is left alone, as by every other modulus and size."""
+    import torch
+
+    L = _lib.lib()
+    A = torch.ones((1, 4096), dtype=torch.int32, device="cuda")
+    B = torch.ones((4096, 4096), dtype=torch.int32, device="cuda")
+    C = torch.full((8, 4096), 7, dtype=torch.int32, device="cuda")
+    with hacs_b200.Engine(0) as eng:
+        eng.use_torch_stream()
+        for p in (65521, P31):
+            for op in (hacs_b200.SET, hacs_b200.ADD, hacs_b200.SUB):
+                assert L.hme_gemm_u32_dev(eng._h, p, m, n, k, A.data_ptr(), 4096, B.data_ptr(), 4096, C.data_ptr(),
+                                          4096, op) == _lib.HME_OK
+            assert L.hme_schur_update_u32_dev(eng._h, p, m, n, k, A.data_ptr(), 4096, B.data_ptr(), 4096,
+                                              C.data_ptr(), 4096) == _lib.HME_OK
+        torch.cuda.synchronize()
+    assert bool((C == 7).all())
+
+
+def test_refused_products_stay_refused():
+    """A side of 2^30 or more, a leading dimension below the row, an unknown op: HME_EINVAL before anything runs.
+    (The pointers are never followed.)"""
+    import torch
+
+    L = _lib.lib()
+    t = torch.ones(64, dtype=torch.int32, device="cuda").data_ptr()
+    with hacs_b200.Engine(0) as eng:
+        for m, n, k, lda, ldb, ldc, op in ((1, 1, 1 << 30, 1 << 30, 1, 1, 0), (1, 1 << 30, 1, 1, 1 << 30, 1 << 30, 0),
+                                           (1 << 30, 1, 1, 1, 1, 1, 0), (64, 64, 8192, 8191, 64, 64, 0),
+                                           (64, 64, 8192, 8192, 63, 64, 0), (64, 64, 8192, 8192, 64, 63, 0),
+                                           (64, 64, 8192, 8192, 64, 64, 3)):
+            assert L.hme_gemm_u32_dev(eng._h, P31, m, n, k, t, lda, t, ldb, t, ldc, op) == _lib.HME_EINVAL
+        assert L.hme_gemm_u64_dev(eng._h, (1 << 61) - 1, 1, (1 << 32) - 1, 1, t, 1, t, (1 << 32) - 1, t, (1 << 32) - 1,
+                                  0) == _lib.HME_EINVAL
