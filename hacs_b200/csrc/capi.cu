@@ -16,6 +16,11 @@ thread_local std::string g_last_error;
 
 void set_last_error(const std::string& msg) { g_last_error = msg; }
 
+namespace {
+// growth with headroom, so that a sequence of slightly larger calls does not reallocate every time
+size_t with_headroom(size_t bytes) { return bytes + bytes / 8; }
+}  // namespace
+
 void* Workspace::get(int slot, size_t bytes) {
     if (bytes == 0) bytes = 16;
     if (size[slot] < bytes) {
@@ -23,28 +28,43 @@ void* Workspace::get(int slot, size_t bytes) {
         else if (ptr[slot]) HME_CUDA(cudaFree(ptr[slot]));
         ptr[slot] = nullptr;
         size[slot] = 0;
-        // grow with headroom so a sequence of slightly larger calls does not reallocate every time
-        const size_t want = bytes + bytes / 8;
+        const size_t want = with_headroom(bytes);
         HME_CUDA(cudaMalloc(&ptr[slot], want));
         size[slot] = want;
     }
     return ptr[slot];
 }
 
-bool Workspace::holds(int slot, size_t bytes, cudaStream_t stream) {
-    if (size[slot] >= bytes) return true;
+bool Workspace::holds(std::initializer_list<Need> needs, cudaStream_t stream) {
+    struct Grown {
+        int slot;
+        size_t size;
+        void* ptr;
+    };
+    std::vector<Grown> grown;
+    for (const Need& n : needs)
+        if (size[n.slot] < n.bytes) grown.push_back({n.slot, with_headroom(n.bytes), nullptr});
+    if (grown.empty()) return true;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
         return false;
     }
-    try {
-        get(slot, bytes);
-        return true;
-    } catch (const Error&) {
+    bool all = true;
+    for (Grown& g : grown) all = all && cudaMalloc(&g.ptr, g.size) == cudaSuccess;
+    if (!all) {
+        for (const Grown& g : grown)
+            if (g.ptr) cudaFree(g.ptr);
         cudaGetLastError();  // the failed allocation's
         return false;
     }
+    for (const Grown& g : grown) {
+        if (ptr[g.slot] && retain) retired.push_back(ptr[g.slot]);
+        else if (ptr[g.slot]) cudaFree(ptr[g.slot]);
+        ptr[g.slot] = g.ptr;
+        size[g.slot] = g.size;
+    }
+    return true;
 }
 
 void Workspace::release() {

@@ -619,7 +619,7 @@ bool rns_gemm_u32_device(hme_ctx* ctx, const ModParams& mp, uint32_t m, uint32_t
     const size_t pbytes = align256(static_cast<size_t>(P.t) * n * Kp);
     const size_t need_a = static_cast<size_t>(P.t) * m * Kp;
     const size_t need_b = pbytes + static_cast<size_t>(P.t) * m * ((n + 31) / 32 * 32);
-    if (!ctx->ws.holds(kSlotPlanesA, need_a, ctx->stream) || !ctx->ws.holds(kSlotPlanesB, need_b, ctx->stream)) return false;
+    if (!ctx->ws.holds({{kSlotPlanesA, need_a}, {kSlotPlanesB, need_b}}, ctx->stream)) return false;
     uint8_t* pa = static_cast<uint8_t*>(ctx->ws.get(kSlotPlanesA, need_a));
     uint8_t* pb = static_cast<uint8_t*>(ctx->ws.get(kSlotPlanesB, need_b));
     rns_gemm(ctx, P, m, n, k, A, lda, B, ldb, C, ldc, op, pa, pb, pb + pbytes);

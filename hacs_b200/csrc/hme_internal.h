@@ -5,6 +5,7 @@
 
 #include <atomic>
 #include <cstdint>
+#include <initializer_list>
 #include <mutex>
 #include <new>
 #include <stdexcept>
@@ -87,9 +88,14 @@ struct Workspace {
     bool retain = false;
     std::vector<void*> retired;
     void* get(int slot, size_t bytes);
-    // Whether the slot holds `bytes`, grown if need be; false during a capture that would have to allocate and
-    // when the memory cannot be had: for methods with a cheaper one to fall back on.
-    bool holds(int slot, size_t bytes, cudaStream_t stream);
+    // Whether the slots hold their bytes, grown if need be; false, with every slot as it was, during a capture
+    // that would have to allocate and when the memory cannot be had beside what the slots hold now: for methods
+    // with a cheaper one to fall back on, which then finds the memory that it would have found.
+    struct Need {
+        int slot;
+        size_t bytes;
+    };
+    bool holds(std::initializer_list<Need> needs, cudaStream_t stream);
     void release();
 };
 

@@ -756,9 +756,7 @@ bool batch_rank_rounds(hme_ctx* ctx, const std::vector<BatchMatrix>& mats, std::
         o_tp[g] = take(sizeof(int) * g_tiles[g]);
         o_bj[g] = take(sizeof(int) * g_blocks[g]);
     }
-    if (!ctx->ws.holds(kSlotJobs1, tb, ctx->stream) || !ctx->ws.holds(kSlotJobs4, buf_bytes, ctx->stream) ||
-        !ctx->ws.holds(kSlotJobs0, plane_bytes, ctx->stream))
-        return false;
+    if (!ctx->ws.holds({{kSlotJobs1, tb}, {kSlotJobs4, buf_bytes}, {kSlotJobs0, plane_bytes}}, ctx->stream)) return false;
     uint8_t* tables = static_cast<uint8_t*>(ctx->ws.get(kSlotJobs1, tb));
     uint8_t* bufs = static_cast<uint8_t*>(ctx->ws.get(kSlotJobs4, buf_bytes));
     uint8_t* planes = static_cast<uint8_t*>(ctx->ws.get(kSlotJobs0, plane_bytes));

@@ -87,3 +87,60 @@ def test_matrix_is_free_once_its_elimination_has_failed(eng):
         A[:, :256] = 7
         torch.cuda.synchronize()
         assert bool((A[:, :256] == 7).all())
+
+
+def _fill(free):
+    """Device memory taken up to `free` bytes."""
+    import torch
+
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    return torch.empty(torch.cuda.mem_get_info()[0] - free, dtype=torch.uint8, device="cuda")
+
+
+@pytest.mark.parametrize("held", [False, True])
+def test_product_beside_full_memory_takes_the_smaller_planes(eng, held):
+    """8192^3 mod 2^31 - 19, u = 64 MiB a byte plane, an eighth of headroom on every buffer: the residue system's
+    planes take 11.25 u + 22.5 u, the limbs' 4.5 u + 18 u.  With 26 u free, or with the limbs' planes held and
+    20 u free, the first does not fit in whole, and the second has to find what it needs."""
+    import torch
+
+    n, u = 8192, 8192 * 8192
+    L = _lib.lib()
+    A, B = (torch.randint(0, P31, (n, n), dtype=torch.int32, device="cuda") for _ in range(2))
+    C, want = torch.zeros_like(A), torch.zeros_like(A)
+    with hacs_b200.Engine(0) as ref:
+        ref.use_torch_stream()
+        ref.gemm_dev(P31, A, B, want)
+        torch.cuda.synchronize()
+    if held:
+        assert L.hme_ctx_set_gemm_variant(eng._h, 0) == 0
+        eng.gemm_dev(P31, A, B, C)
+        assert L.hme_ctx_set_gemm_variant(eng._h, -1) == 0
+        C.zero_()
+    rest = _fill(20 * u if held else 26 * u)
+    try:
+        eng.gemm_dev(P31, A, B, C)
+        torch.cuda.synchronize()
+    finally:
+        del rest
+    assert torch.equal(C, want)
+
+
+def test_ranks_beside_full_memory_take_the_smaller_rounds(eng):
+    """10000 ranks of 256 x 64 mod 2^31 - 19: rounds of 64 columns take 66.5 + 131 KB a job, rounds of 32 columns
+    53 + 65.5 KB (and about 1 KB of tables), an eighth more with headroom.  With 126 KB a job (and the eighth)
+    free, between the second and the first one's buffers beside the second one's planes."""
+    import torch
+
+    jobs, m, n = 10000, 256, 64
+    C = torch.randint(0, P31, (jobs, m, n), dtype=torch.int32, device="cuda")
+    C[::3, :, 5] = C[::3, :, 4]
+    eng.use_own_stream()
+    torch.cuda.synchronize()
+    rest = _fill(int(jobs * 126_000 * 1.125))
+    try:
+        ranks = eng.batch_rank_dev([dict(A=None, B=None, C=C[t], p=P31) for t in range(jobs)])
+    finally:
+        del rest
+    assert (ranks[::3] == n - 1).all() and (ranks[1::3] == n).all() and (ranks[2::3] == n).all()
