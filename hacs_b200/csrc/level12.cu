@@ -680,57 +680,71 @@ int hme_gemv_u32_dev(hme_ctx* ctx, uint32_t p, uint32_t m, uint32_t k, const uin
         bind(ctx);
         const ModParams mp = make_mod(p);
         const uint32_t r64 = r64_of(p);
-        const bool v4 = a_cs == 1 && x_rs == 1 && k % 4 == 0 && (m == 1 || a_rs % 4 == 0) &&
-                        reinterpret_cast<uintptr_t>(A) % 16 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0;
-        if ((a_cs == 1 || a_rs != 1) && k >= 2048) {
-            // Long rows: the widest chunk that the row's length fills to eight ninths (a pass costs its whole
-            // chunk: 4096 x 4097 takes 27 us in gemv_block_kernel and 48 us as one half-empty chunk per row),
-            // with several passes only where every CTA has several rows per pass (64 x 20000: 9.8 against
-            // 11.5 us); else the kernel that takes any length.  Single words (unaligned rows) are bound by
-            // instructions, which only the widest chunk has fewer of: 8191 x 8191 144 -> 98 us, but 4096 x 4095
-            // 25 -> 31 us with 16 words a row.
-            auto fits = [&](uint64_t chunk, uint64_t rows) {
-                const uint64_t passes = (k + chunk - 1) / chunk;
-                return 8 * passes * chunk <= 9 * static_cast<uint64_t>(k) &&
-                       (passes == 1 || m >= 8 * rows * static_cast<uint64_t>(ctx->num_sms));
-            };
-            const int rows = fits(8192, 1) ? 1 : v4 && fits(4096, 2) ? 2 : v4 && fits(2048, 4) ? 4 : 0;
-            if (rows != 0) {
-                const int grid = static_cast<int>(std::min<size_t>((static_cast<size_t>(m) + rows - 1) / rows,
-                                                                   static_cast<size_t>(2) * ctx->num_sms));
-                auto kernel = !v4         ? gemv_rows_kernel<1, 32, 1>
-                              : rows == 4 ? gemv_rows_kernel<4, 2, 4>
-                              : rows == 2 ? gemv_rows_kernel<4, 4, 2>
-                                          : gemv_rows_kernel<4, 8, 1>;
-                HME_TIMED(ctx, "gemv", kernel<<<grid, 256, 0, ctx->stream>>>(A, a_rs, a_cs, x, x_rs, y, y_rs, m, k, op,
-                                                                            p, mp.barrett, r64));
-            } else {
-                // the grid one wave of resident CTAs
-                int per_sm = 1;
-                HME_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                    &per_sm, v4 ? gemv_block_kernel<4> : gemv_block_kernel<1>, 256, 0));
-                const int grid = static_cast<int>(std::min<size_t>(m, static_cast<size_t>(std::max(1, per_sm)) * ctx->num_sms));
+        auto piece = [&](uint32_t m, uint32_t k, const uint32_t* A, const uint32_t* x, uint32_t* y, int op) {
+            const bool v4 = a_cs == 1 && x_rs == 1 && k % 4 == 0 && (m == 1 || a_rs % 4 == 0) &&
+                            reinterpret_cast<uintptr_t>(A) % 16 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0;
+            if ((a_cs == 1 || a_rs != 1) && k >= 2048) {
+                // Long rows: the widest chunk that the row's length fills to eight ninths (a pass costs its whole
+                // chunk: 4096 x 4097 takes 27 us in gemv_block_kernel and 48 us as one half-empty chunk per row),
+                // with several passes only where every CTA has several rows per pass (64 x 20000: 9.8 against
+                // 11.5 us); else the kernel that takes any length.  Single words (unaligned rows) are bound by
+                // instructions, which only the widest chunk has fewer of: 8191 x 8191 144 -> 98 us, but 4096 x 4095
+                // 25 -> 31 us with 16 words a row.
+                auto fits = [&](uint64_t chunk, uint64_t rows) {
+                    const uint64_t passes = (k + chunk - 1) / chunk;
+                    return 8 * passes * chunk <= 9 * static_cast<uint64_t>(k) &&
+                           (passes == 1 || m >= 8 * rows * static_cast<uint64_t>(ctx->num_sms));
+                };
+                const int rows = fits(8192, 1) ? 1 : v4 && fits(4096, 2) ? 2 : v4 && fits(2048, 4) ? 4 : 0;
+                if (rows != 0) {
+                    const int grid = static_cast<int>(std::min<size_t>((static_cast<size_t>(m) + rows - 1) / rows,
+                                                                       static_cast<size_t>(2) * ctx->num_sms));
+                    auto kernel = !v4         ? gemv_rows_kernel<1, 32, 1>
+                                  : rows == 4 ? gemv_rows_kernel<4, 2, 4>
+                                  : rows == 2 ? gemv_rows_kernel<4, 4, 2>
+                                              : gemv_rows_kernel<4, 8, 1>;
+                    HME_TIMED(ctx, "gemv", kernel<<<grid, 256, 0, ctx->stream>>>(A, a_rs, a_cs, x, x_rs, y, y_rs, m, k, op,
+                                                                                p, mp.barrett, r64));
+                } else {
+                    // the grid one wave of resident CTAs
+                    int per_sm = 1;
+                    HME_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                        &per_sm, v4 ? gemv_block_kernel<4> : gemv_block_kernel<1>, 256, 0));
+                    const int grid = static_cast<int>(std::min<size_t>(m, static_cast<size_t>(std::max(1, per_sm)) * ctx->num_sms));
+                    if (v4)
+                        HME_TIMED(ctx, "gemv", gemv_block_kernel<4><<<grid, 256, 0, ctx->stream>>>(
+                                                   A, a_rs, a_cs, x, x_rs, y, y_rs, m, k, op, p, mp.barrett, r64));
+                    else
+                        HME_TIMED(ctx, "gemv", gemv_block_kernel<1><<<grid, 256, 0, ctx->stream>>>(
+                                                   A, a_rs, a_cs, x, x_rs, y, y_rs, m, k, op, p, mp.barrett, r64));
+                }
+            } else if (a_cs == 1 || a_rs != 1) {
+                const int grid = static_cast<int>(std::min<size_t>((static_cast<size_t>(m) + 7) / 8, ctx->num_sms * 16));
                 if (v4)
-                    HME_TIMED(ctx, "gemv", gemv_block_kernel<4><<<grid, 256, 0, ctx->stream>>>(
+                    HME_TIMED(ctx, "gemv", gemv_warp_kernel<4><<<grid, 256, 0, ctx->stream>>>(
                                                A, a_rs, a_cs, x, x_rs, y, y_rs, m, k, op, p, mp.barrett, r64));
                 else
-                    HME_TIMED(ctx, "gemv", gemv_block_kernel<1><<<grid, 256, 0, ctx->stream>>>(
+                    HME_TIMED(ctx, "gemv", gemv_warp_kernel<1><<<grid, 256, 0, ctx->stream>>>(
                                                A, a_rs, a_cs, x, x_rs, y, y_rs, m, k, op, p, mp.barrett, r64));
+            } else {
+                const int grid = static_cast<int>(std::min<size_t>((static_cast<size_t>(m) + 255) / 256, ctx->num_sms * 8));
+                HME_TIMED(ctx, "gemv", gemv_thread_kernel<<<grid, 256, 0, ctx->stream>>>(A, a_rs, a_cs, x, x_rs, y, y_rs, m,
+                                                                                       k, op, p, mp.barrett, r64));
             }
-        } else if (a_cs == 1 || a_rs != 1) {
-            const int grid = static_cast<int>(std::min<size_t>((static_cast<size_t>(m) + 7) / 8, ctx->num_sms * 16));
-            if (v4)
-                HME_TIMED(ctx, "gemv", gemv_warp_kernel<4><<<grid, 256, 0, ctx->stream>>>(
-                                           A, a_rs, a_cs, x, x_rs, y, y_rs, m, k, op, p, mp.barrett, r64));
-            else
-                HME_TIMED(ctx, "gemv", gemv_warp_kernel<1><<<grid, 256, 0, ctx->stream>>>(
-                                           A, a_rs, a_cs, x, x_rs, y, y_rs, m, k, op, p, mp.barrett, r64));
-        } else {
-            const int grid = static_cast<int>(std::min<size_t>((static_cast<size_t>(m) + 255) / 256, ctx->num_sms * 8));
-            HME_TIMED(ctx, "gemv", gemv_thread_kernel<<<grid, 256, 0, ctx->stream>>>(A, a_rs, a_cs, x, x_rs, y, y_rs, m,
-                                                                                   k, op, p, mp.barrett, r64));
+            HME_CUDA(cudaGetLastError());
+        };
+        // The kernels count rows and columns in 32 bits and step past the end by up to a grid or a chunk: they
+        // take at most 2^30 of each at once (a view of stride 0 has 2^32 - 1 columns for nothing).
+        constexpr uint64_t kMost = uint64_t(1) << 30;
+        for (uint64_t i0 = 0; i0 < m; i0 += kMost) {
+            uint64_t k0 = 0;
+            do {
+                piece(static_cast<uint32_t>(std::min(kMost, m - i0)), static_cast<uint32_t>(std::min(kMost, k - k0)),
+                      A + i0 * a_rs + k0 * a_cs, x + k0 * x_rs, y + i0 * y_rs,
+                      k0 == 0 || op != HME_SET ? op : HME_ADD);
+                k0 += kMost;
+            } while (k0 < k);
         }
-        HME_CUDA(cudaGetLastError());
     });
 }
 

@@ -76,3 +76,36 @@ def test_refused_products_stay_refused():
             assert L.hme_gemm_u32_dev(eng._h, P31, m, n, k, t, lda, t, ldb, t, ldc, op) == _lib.HME_EINVAL
         assert L.hme_gemm_u64_dev(eng._h, (1 << 61) - 1, 1, (1 << 32) - 1, 1, t, 1, t, (1 << 32) - 1, t, (1 << 32) - 1,
                                   0) == _lib.HME_EINVAL
+
+
+def test_matrix_vector_product_of_the_longest_rows():
+    """Rows of 2^30 + 5 columns (the first beyond one piece), rows of 2^32 - 1 columns and 2^32 - 1 rows: the
+    latter two as views of stride 0."""
+    import torch
+
+    L, most = _lib.lib(), (1 << 32) - 1
+    _room(24)
+    with hacs_b200.Engine(0) as eng:
+        eng.use_torch_stream()
+
+        def gemv(p, m, k, A, a_rs, a_cs, x, x_rs, y, op):
+            assert L.hme_gemv_u32_dev(eng._h, p, m, k, A.data_ptr(), a_rs, a_cs, x.data_ptr(), x_rs, y.data_ptr(), 1,
+                                      op) == _lib.HME_OK
+            torch.cuda.synchronize()
+
+        k, p = (1 << 30) + 5, 65521
+        x, A = (torch.empty(k, dtype=torch.int32, device="cuda").random_(0, p) for _ in range(2))
+        dot = sum(int((A[c:c + (1 << 28)].to(torch.int64) * x[c:c + (1 << 28)]).sum()) for c in range(0, k, 1 << 28))
+        for op, want in ((hacs_b200.SET, dot), (hacs_b200.ADD, 11 + dot), (hacs_b200.SUB, 11 - dot)):
+            y = torch.full((1,), 11, dtype=torch.int32, device="cuda")
+            gemv(p, 1, k, A, k, 1, x, 1, y, op)
+            assert int(y[0]) == want % p
+        del x, A
+        torch.cuda.empty_cache()
+        a, b = (torch.full((1,), v, dtype=torch.int32, device="cuda") for v in (P31 - 1, 123456789))
+        y = torch.full((3,), 11, dtype=torch.int32, device="cuda")
+        gemv(P31, 3, most, a, 0, 0, b, 0, y, hacs_b200.SUB)
+        assert y.tolist() == [(11 - (P31 - 1) * 123456789 * most) % P31] * 3
+        y = torch.full((most,), 11, dtype=torch.int32, device="cuda")
+        gemv(P31, most, 1, a, 0, 1, b, 1, y, hacs_b200.SET)
+        assert bool((y == (P31 - 1) * 123456789 % P31).all())
