@@ -44,3 +44,16 @@ def test_thousands_of_pending_rows(engine):
     A[: n - 2, n - 2] = 1 + np.arange(n - 2) % 7
     A[: n - 2, n - 1] = np.arange(n - 2) % 8
     _same(engine, ell, k, A)
+
+
+@pytest.mark.parametrize("ell,k", [(2, 16), (2, 31), (3, 10)])
+def test_pivots_that_change(engine, ell, k):
+    """Triangular with random valuations on the diagonal: most echelon pivots are displaced by the closures of
+    the columns before them, and their own closures with them."""
+    n, q = 160, ell ** k
+    rng = np.random.default_rng(k)
+    A = np.triu(rng.integers(0, q, (n, n), dtype=np.uint64))
+    A[np.arange(n), np.arange(n)] = np.array([ell ** int(e) for e in rng.integers(0, k, n)], np.uint64)
+    _same(engine, ell, k, A.astype(np.uint32))
+    A[:, 10::7] = A[:, 10::7] * ell % q  # no unit in these columns
+    _same(engine, ell, k, A.astype(np.uint32))
