@@ -726,7 +726,12 @@ __global__ void __launch_bounds__(4 * RS) panel_block_kernel(const BlockArgs a, 
 // every row operation's effect on the identity as well (in place: the pivot's
 // column of a row holds that row's entry of the inverse of the operations), so W
 // comes out directly, with no triangular inverse and no panel_w_kernel.
-constexpr int kCompactRows = 256;
+// More listed rows than two a column meet in most columns, and one CTA updates them
+// all in every step: 26 panels of a banded 3000 x 2000 matrix mod 65521 (200 wide, 4
+// entries a row) with up to 256 listed rows took 196 us each, against 104 us in
+// the cluster search and 20 us for L11^-1 and W; the RREF 8.1 ms with a list of 256
+// rows, 6.35 ms with 128, 6.9 ms by searches alone.
+constexpr int kCompactRows = 128;
 
 struct CompactArgs {
     uint32_t* A;
@@ -768,7 +773,7 @@ __host__ __device__ constexpr size_t compact_smem_bytes(int w) {
 }
 
 // One CTA of 32 warps.  The rows, in row order, sit in shared memory
-// column-major, lanes over rows: rwn = 1, 2, 4 or 8 warps cover them and 32 /
+// column-major, lanes over rows: rwn = 1, 2 or 4 warps cover them and 32 /
 // rwn groups of warps share the columns.  Pivot rule and fraction-free update
 // are the cluster kernel's, but a step whose column has no other entry updates
 // nothing (and no scale), and every column is updated, pivotless ones left of
@@ -779,8 +784,8 @@ template <int ARITH>
 __global__ void __launch_bounds__(1024, 1) panel_compact_kernel(const CompactArgs a) {
     extern __shared__ __align__(16) uint32_t s_cmp[];
     __shared__ uint32_t s_x[2][kCompactRows];
-    __shared__ uint32_t s_key[2][8];
-    __shared__ int s_nz[2][8];
+    __shared__ uint32_t s_key[2][kCompactRows / 32];
+    __shared__ int s_nz[2][kCompactRows / 32];
     __shared__ uint32_t s_S[kMaxPanel + 1], s_Sinv[kMaxPanel + 1];
     __shared__ int s_prow[kMaxPanel], s_pcol[kMaxPanel], s_colpiv[kMaxPanel];
     __shared__ int s_row[kCompactRows], s_step[kCompactRows];
@@ -813,7 +818,7 @@ __global__ void __launch_bounds__(1024, 1) panel_compact_kernel(const CompactArg
         s_step[tid] = 0;
     }
     __syncthreads();
-    const int rwn = cnt <= 32 ? 1 : cnt <= 64 ? 2 : cnt <= 128 ? 4 : 8;
+    const int rwn = cnt <= 32 ? 1 : cnt <= 64 ? 2 : 4;
     const int G = 32 / rwn, rs = 32 * rwn + 1;
     uint32_t* S = s_cmp;  // [w][rs]
 #pragma unroll 4

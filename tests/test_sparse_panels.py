@@ -88,3 +88,17 @@ def test_dense_levels(engine, ell, k, mode):
             assert np.array_equal(engine.smith(ell, k, M), O.smith(ell, k, M))
     finally:
         engine.set_panel_kernel(0)
+
+
+@pytest.mark.parametrize("rows", [31, 32, 33, 64, 65, 127, 128, 129])
+def test_the_edges_of_the_list(engine, rows):
+    """Panels whose non-zero rows fill the compact kernel's warps, or its list, or one row more."""
+    rng = np.random.default_rng(rows)
+    for p in (2, 13, 65521, 2147483629):
+        A = np.zeros((400, 200), np.uint32)
+        A[np.sort(rng.permutation(400)[:rows])] = rng.integers(0, p, (rows, 200))
+        A[:, 70:120] = 0
+        A[rng.permutation(400)[: rows // 2], 80] = 1
+        R1, p1 = engine.rref(p, A)
+        R2, p2 = O.rref(p, A)
+        assert np.array_equal(p1, p2) and np.array_equal(R1, R2)
