@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(NT, 1) panel_cluster_kernel(const PanelArgs a)
     extern __shared__ __align__(16) uint32_t s_dyn[];
     __shared__ uint32_t r_key[2][kClusterMax];               // pushed keys, by parity and sender
     __shared__ uint32_t r_row[2][kClusterMax][kMaxPanel];     // pushed candidate rows (from column c)
-    __shared__ uint32_t r_any[2][kClusterMax];                // pushed: the sender's active rows are not all zero
+    __shared__ uint32_t r_any[2][kClusterMax];                // pushed: the sender's active rows may have a pivot
     __shared__ uint32_t s_cand[2];                            // this CTA's best key, by parity
     __shared__ uint32_t s_w[kMaxPanel];                       // unit part of each step's raw pivot
     __shared__ uint32_t s_inv[kMaxPanel];                     // its inverse
@@ -455,7 +455,7 @@ __global__ void __launch_bounds__(NT, 1) panel_cluster_kernel(const PanelArgs a)
     int nskip = 0;  // pivotless columns so far (keep mode)
     int empty = 0;  // pivotless columns in a row; at the 2nd, 6th, 14th, .. the rest of the panel is looked over
     int look = 2;
-    uint32_t any = 1;  // this CTA's active rows are not known to be zero in the rest of the panel
+    uint32_t any = 1;  // this CTA's active rows are not known to have no pivot in the rest of the panel
     int pend_col = -1;  // ring mode: multiplier x / ell^v stored after the column's CTA barrier
     uint32_t pend_xp = 0;
     for (int it = 0; it < bw; ++it) {
@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(NT, 1) panel_cluster_kernel(const PanelArgs a)
         if (pkey == kNoKey32) {
             // no pivot in this column: every active row is unchanged; scan column it + 1
             if (!__any_sync(0xffffffffu, lane < static_cast<int>(csize) && r_any[par][lane] != 0)) {
-                // all active rows are zero from here on (the same verdict in every CTA): no more pivots
+                // no active row has a pivot from here on (the same verdict in every CTA)
                 for (int j = it + tid; j < bw; j += NT) s_colstep[j] = -1 - k;
                 break;
             }
@@ -560,10 +560,12 @@ __global__ void __launch_bounds__(NT, 1) panel_cluster_kernel(const PanelArgs a)
         if (lane == 0 && key != kNoKey32) atomicMin(&s_cand[par ^ 1], key);
         if (empty == look) {  // the same in every thread of the cluster
             look = 2 * look + 2;
-            uint32_t x = 0;
+            // (entries that cannot be pivots stay so while there is none: over a ring with unit pivots
+            // the rest of a level is seldom zero)
+            bool x = false;
             if (has_row && s_step[li] == 0)
-                for (int j = it + 1 + sub; j < bw; j += g) x |= S[j * rs + li];
-            any = __syncthreads_or(x != 0) ? 1u : 0u;
+                for (int j = it + 1 + sub; j < bw; j += g) x |= pivot_key32(S[j * rs + li], 0, a.R) != kNoKey32;
+            any = __syncthreads_or(x) ? 1u : 0u;
         } else {
             any = 1;
             __syncthreads();
@@ -1192,14 +1194,23 @@ bool row_moves_odd(const int* prow, int k, int r0) {
     return ((n - cycles) & 1) != 0;
 }
 
-// flag = 1 when the rows x cols window has a non-zero entry
-__global__ void window_nonzero_kernel(const uint32_t* __restrict__ A, uint64_t ld, int rows, int cols,
-                                      int* __restrict__ flag) {
+// flags |= 1 when the rows x cols window has a non-zero entry, |= 2 when one can be
+// a pivot.  A warp that has seen both leaves as one; one store per warp and row, and
+// none of a bit that is set (every thread storing its own took 33 us on 1024 x 1024
+// non-zero entries).
+__global__ void __launch_bounds__(256) window_look_kernel(const uint32_t* __restrict__ A, uint64_t ld, int rows,
+                                                          int cols, const Ring R, int* __restrict__ flags) {
+    const int lane = threadIdx.x & 31;
     for (int i = blockIdx.x; i < rows; i += gridDim.x) {
-        if (*reinterpret_cast<volatile int*>(flag) != 0) return;
-        uint32_t any = 0;
-        for (int j = threadIdx.x; j < cols; j += blockDim.x) any |= A[static_cast<size_t>(i) * ld + j];
-        if (any) *flag = 1;
+        const int seen = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile int*>(flags), 0);
+        if (seen == 3) return;
+        int f = 0;
+        for (int j = threadIdx.x; j < cols; j += blockDim.x) {
+            const uint32_t x = A[static_cast<size_t>(i) * ld + j];
+            if (x != 0) f |= pivot_key32(x, 0, R) != kNoKey32 ? 3 : 1;
+        }
+        f = __reduce_or_sync(0xffffffffu, f);
+        if (lane == 0 && (f & ~seen) != 0) atomicOr(flags, f);
     }
 }
 
@@ -1507,7 +1518,7 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
         int count;     // rows listed for the compact kernel
         int fail;      // ring entry 0 only: queued work stands still (BlockArgs::fail)
         int list[kCompactRows];
-        int nonzero;   // the rest of the matrix is not zero
+        int rest;      // what the rest of the matrix holds (window_look_kernel)
         unsigned bar[2];
     };
     const size_t scratch_bytes = (sizeof(Scratch) + 255) / 256 * 256;
@@ -1948,18 +1959,24 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
         if (k == 0) {
             if (keep) append(c0, wp, r0, par, 0);
             c0 = c1;
-            // no pivot in the panel: nothing moved, the next panel starts at r0 -- unless nothing is
-            // left (one pass over the rest, against a panel's search each; after a pass that found
-            // something only every 2nd, 4th, .. pivotless panel asks again)
+            // no pivot in the panel: nothing moved, the next panel starts at r0 -- unless there is none in
+            // the rest (one pass over it, against a panel's search each; after a pass that found one only
+            // every 2nd, 4th, .. pivotless panel asks again).  Rows of Z/2^31 scaled by random powers of 2,
+            // 1024 x 1024: Smith 35.3 ms asking whether the rest was zero, 7.6 ms asking for units.
             if (c1 < lu_cols && panels >= next_look) {
-                int* d_nz = &d_sb[par]->nonzero;
-                HME_CUDA(cudaMemsetAsync(d_nz, 0, sizeof(int), s_main));
+                int* d_rest = &d_sb[par]->rest;
+                HME_CUDA(cudaMemsetAsync(d_rest, 0, sizeof(int), s_main));
                 HME_TIMED(ctx, "rest_nonzero",
-                          window_nonzero_kernel<<<std::min(m - r0, 8 * ctx->num_sms), 256, 0, s_main>>>(
-                              A + static_cast<size_t>(r0) * ld + c1, ld, m - r0, lu_cols - c1, d_nz));
-                HME_CUDA(cudaMemcpyAsync(&h_sb[par].nonzero, d_nz, sizeof(int), cudaMemcpyDeviceToHost, s_main));
+                          window_look_kernel<<<std::min(m - r0, 8 * ctx->num_sms), 256, 0, s_main>>>(
+                              A + static_cast<size_t>(r0) * ld + c1, ld, m - r0, lu_cols - c1, rg, d_rest));
+                HME_CUDA(cudaGetLastError());
+                HME_CUDA(cudaMemcpyAsync(&h_sb[par].rest, d_rest, sizeof(int), cudaMemcpyDeviceToHost, s_main));
                 HME_CUDA(cudaStreamSynchronize(s_main));
-                if (h_sb[par].nonzero == 0) break;
+                if ((h_sb[par].rest & 2) == 0) {
+                    if (keep && h_sb[par].rest != 0)  // its columns are left out too
+                        for (int c = c1; c < n; c += kMaxPanel) append(c, std::min(kMaxPanel, n - c), r0, par, 0);
+                    break;
+                }
                 next_look = panels + look_gap;
                 look_gap *= 2;
             }

@@ -28,7 +28,7 @@ struct RingSpec {
     // updated, as the next column right of the matrix (A has room for them: ld
     // >= 2 n); ElimResult::appended counts them.  At the end rows [rank, m) at
     // columns [n, n + appended) are the Schur complement of the pivot columns
-    // (its other columns, if the elimination ended early, are zero).
+    // (without columns at its end that are zero, if the elimination ended early).
     bool keep_skipped = false;
 };
 

@@ -102,3 +102,23 @@ def test_the_edges_of_the_list(engine, rows):
         R1, p1 = engine.rref(p, A)
         R2, p2 = O.rref(p, A)
         assert np.array_equal(p1, p2) and np.array_equal(R1, R2)
+
+
+@pytest.mark.parametrize("ell,k", [(2, 4), (2, 31), (3, 10)])
+@pytest.mark.parametrize("m,n", [(130, 300), (300, 200), (200, 400)])
+def test_levels_that_end_early(engine, ell, k, m, n):
+    """Level matrices whose units are all in the first columns, the rest of them multiples of ell or zero (the
+    elimination ends when no unit is left, and the rest is the next level's), or in a few late ones."""
+    q = ell ** k
+    rng = np.random.default_rng(m + n + k)
+    A = rng.integers(0, q, (m, n), dtype=np.uint64)
+    rows = (np.uint64(ell) ** rng.integers(0, k, m).astype(np.uint64))[:, None]
+    late = A.copy()
+    late[:, : n - 20] *= np.uint64(ell)
+    zero = A * rows % np.uint64(q)
+    zero[:, 100:] = 0
+    first = A * np.uint64(ell)
+    first[:, :30] = A[:, :30]
+    for M in (A * rows, zero, late, first, late * rows):
+        M = (M % np.uint64(q)).astype(np.uint32)
+        assert np.array_equal(engine.smith(ell, k, M), O.smith(ell, k, M))
