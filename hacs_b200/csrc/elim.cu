@@ -1526,17 +1526,19 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
     const size_t uinv_bytes = sizeof(uint32_t) * kMaxPanel * kMaxPanel;  // the update's M
     uint8_t* base = static_cast<uint8_t*>(
         ctx->ws.get(kSlotElim0, kRing * (scratch_bytes + cand_bytes + uinv_bytes) + 256));
-    // the update's left factor W at its largest (every panel's rows x pivots fits), and those that the
-    // compact kernel writes ahead of their panel's update
-    const size_t w_words = static_cast<size_t>(m) * bw;
-    uint32_t* d_W = static_cast<uint32_t*>(ctx->ws.get(kSlotElim2, (1 + kRing) * sizeof(uint32_t) * w_words));
+    // the update's left factor W at its largest, for panels in turn: the compact kernel writes its panel's
+    // while the update before reads its own, and a panel is launched after the last update but one
+    static_assert(kRing % 2 == 0, "neighbouring panels alternate between the two");
+    const int ldw = std::min(bw, lu_cols);
+    const size_t w_words = static_cast<size_t>(m) * ldw;
+    uint32_t* d_W = static_cast<uint32_t*>(ctx->ws.get(kSlotElim2, 2 * sizeof(uint32_t) * w_words));
     Scratch* d_sb[kRing];
-    uint32_t *d_candb[kRing], *d_uinvb[kRing], *d_Wc[kRing];
+    uint32_t *d_candb[kRing], *d_uinvb[kRing], *d_Wb[kRing];
     for (int i = 0; i < kRing; ++i) {
         d_sb[i] = reinterpret_cast<Scratch*>(base + i * scratch_bytes);
         d_candb[i] = reinterpret_cast<uint32_t*>(base + kRing * scratch_bytes + i * cand_bytes);
         d_uinvb[i] = reinterpret_cast<uint32_t*>(base + kRing * (scratch_bytes + cand_bytes) + i * uinv_bytes);
-        d_Wc[i] = d_W + (1 + i) * w_words;
+        d_Wb[i] = d_W + (i & 1) * w_words;
         HME_CUDA(cudaMemsetAsync(d_sb[i]->bar, 0, sizeof(unsigned) * 2, ctx->stream));
         HME_CUDA(cudaMemsetAsync(&d_sb[i]->count, 0, 2 * sizeof(int), ctx->stream));  // count, fail
     }
@@ -1708,8 +1710,8 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
             ca.pivot_rows = d_s->pivot_rows;
             ca.pivot_cols = d_s->pivot_cols;
             ca.k_out = &d_s->k;
-            ca.W = d_Wc[par];
-            ca.ldw = bw;
+            ca.W = d_Wb[par];
+            ca.ldw = ldw;
             HME_TIMED(ctx, "panel_rows", panel_rows_kernel<<<(rows + 7) / 8, 256, 0, st>>>(ca));
             auto launch_compact = [&](auto kern) {
                 HME_TIMED(ctx, "panel_compact", kern<<<1, 1024, compact_smem_bytes(w), st>>>(ca));
@@ -1816,7 +1818,7 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
         }
         const int ua = std::max(ca, U.c0 + U.w), rows = m - U.r0, k = U.k;
         if (cb <= ua) return;
-        if (!U.Wf && U.by == 2) U.Wf = d_Wc[U.par];
+        if (!U.Wf && U.by == 2) U.Wf = d_Wb[U.par];
         if (!U.Wf) {
             uint32_t* mul = d_uinvb[U.par];
             const int* d_pcols = d_sb[U.par]->pivot_cols;
@@ -1825,7 +1827,7 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
                                                  A, ld, U.r0, d_pcols, k, p, mp.barrett, mul));
                 HME_CUDA(cudaGetLastError());
             }
-            U.Wf = d_W;
+            U.Wf = d_Wb[U.par];
             const int g = (rows + kWRows - 1) / kWRows;
             const size_t wsm = sizeof(uint32_t) * (((static_cast<size_t>(k) * k + 3) & ~size_t(3)) +
                                                    static_cast<size_t>(kWRows) * ((k + 3) & ~3));
@@ -1838,7 +1840,7 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
         }
         const ProductSettings settings(ctx, sm_cap, U.skip);
         uint32_t* C12 = A + static_cast<size_t>(U.r0) * ld + ua;
-        gemm_u32_variant(ctx, mp, rows, cb - ua, k, U.Wf, U.by == 2 ? bw : k, C12, ld, C12, ld, HME_ADD,
+        gemm_u32_variant(ctx, mp, rows, cb - ua, k, U.Wf, U.by == 2 ? ldw : k, C12, ld, C12, ld, HME_ADD,
                          gemm_default_variant(ctx, mp, rows, cb - ua));
     };
     int r0 = 0, c0 = 0, par = 0;
