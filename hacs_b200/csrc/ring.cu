@@ -121,18 +121,21 @@ __global__ void gather_div_kernel(const uint32_t* __restrict__ src, uint64_t lds
     }
 }
 
-// flags |= 1 when an entry is non-zero, |= 2 when one is a unit (not divisible by ell)
+// flags |= 1 when an entry is non-zero, |= 2 when one is a unit (not divisible by
+// ell).  A warp leaves as one: its lanes may read the flags at different times, and
+// the reduction below names all of them.
 __global__ void __launch_bounds__(256) level_flags_kernel(const uint32_t* __restrict__ A, uint64_t ld, int m, int n,
                                                           uint32_t ell, int* __restrict__ flags) {
     for (int i = blockIdx.x; i < m; i += gridDim.x) {
-        if (*reinterpret_cast<volatile int*>(flags) == 3) return;
+        const int seen = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile int*>(flags), 0);
+        if (seen == 3) return;
         int f = 0;
         for (int j = threadIdx.x; j < n; j += blockDim.x) {
             const uint32_t x = A[static_cast<size_t>(i) * ld + j];
             if (x != 0) f |= x % ell != 0 ? 3 : 1;
         }
         f = __reduce_or_sync(0xffffffffu, f);
-        if ((threadIdx.x & 31) == 0 && f != 0) atomicOr(flags, f);
+        if ((threadIdx.x & 31) == 0 && (f & ~seen) != 0) atomicOr(flags, f);
     }
 }
 

@@ -122,3 +122,17 @@ def test_levels_that_end_early(engine, ell, k, m, n):
     for M in (A * rows, zero, late, first, late * rows):
         M = (M % np.uint64(q)).astype(np.uint32)
         assert np.array_equal(engine.smith(ell, k, M), O.smith(ell, k, M))
+
+
+@pytest.mark.parametrize("ell,k", [(2, 8), (3, 5)])
+def test_level_flags_of_many_rows(engine, ell, k):
+    """More rows than the look over a level has CTAs: zero, then multiples of ell, then one unit at the end; and
+    each of them everywhere."""
+    m, n, q = 3000, 40, ell ** k
+    rng = np.random.default_rng(k)
+    unit = np.zeros((m, n), np.uint32)
+    unit[m // 3:] = rng.integers(0, q // ell, (m - m // 3, n)) * ell
+    unit[m - 1, n - 1] = 1
+    dense = rng.integers(0, q, (m, n), dtype=np.uint64).astype(np.uint32)
+    for M in (unit, np.where(unit == 1, 0, unit), dense, np.zeros((m, n), np.uint32)):
+        assert np.array_equal(engine.smith(ell, k, M), O.smith(ell, k, M))
