@@ -65,30 +65,31 @@ struct Cfg {
 //  - the reduction takes one 32-bit multiply-high: hi = s >> sh1 (32 bits),
 //    q = (hi * M >> 32) >> sh2 with M = floor(2^(31+b)/p), b the bit length of
 //    p, sh1 the bits of s's bound beyond 32, sh2 = b - 1 - sh1.  q is at most
-//    floor(s/p) and misses it by at most 2^sh1/p + 2^-(31+b) s <= 2^(sh1+2-b)
+//    floor(s/p) and misses it by less than 2^sh1/p + 2^-(31+b) s <= 2^(sh1+2-b)
 //    before the floor, so with sh1 <= b - 2 the rest s - q p is below 2p, and
 //    with p < 2^31 it fits a word and one unsigned min(r, r - p) finishes it.
 //    p = 0 (the wraparound mode) has M = 0: the truncation to 32 bits.  Every
-//    other modulus takes the 64-bit Barrett step;
+//    other modulus has sh1 <= b (at most 2^31 255-bounded products per limb, L
+//    limbs below 256^L): the rest, below 3p, in 64 bits and two corrections (with
+//    a 64-bit Barrett step, six wide products, 3000 x 3000 x 256 mod 2^32 - 17
+//    takes 48 us, 45 so);
 //  - C moves in 16-byte pieces where its rows are 16-byte aligned, and a
 //    chunk's old values are loaded one chunk ahead of their use.
 // Per output 73 -> 33 instructions for four limbs.  Adding an 8192 x 8192 x 64
 // product to C (82 us of C at the copy rate; with short_tiles below, the limb
 // split included): p = 13 244 -> 133 us, 65521 256 -> 132, 2^24 - 3 293 -> 167,
-// 2^31 - 19 293 -> 148, 2^32 - 5 294 -> 205.
+// 2^31 - 19 293 -> 144, 2^32 - 5 294 -> 197.
 struct EpiRed {
     uint32_t p;
     uint32_t M;
     int sh1, sh2;
     int fast;
-    uint64_t barrett;
 };
 
 // The constants for sums up to `bound` (below 2^64) mod p.
 inline EpiRed make_epi_bound(const ModParams& mp, unsigned __int128 bound) {
     EpiRed r{};
     r.p = mp.p;
-    r.barrett = mp.barrett;
     if (mp.p == 0) {
         r.fast = 1;
         return r;
@@ -99,6 +100,7 @@ inline EpiRed make_epi_bound(const ModParams& mp, unsigned __int128 bound) {
     while (b < 32 && (mp.p >> b) != 0) ++b;
     r.sh1 = sb > 32 ? sb - 32 : 0;
     r.sh2 = b - 1 - r.sh1;
+    HME_REQUIRE(r.sh2 >= 0, "gemm: sums too large for the reduction");
     const unsigned __int128 m = (static_cast<unsigned __int128>(1) << (31 + b)) / mp.p;
     r.M = m >> 32 ? 0xffffffffu : static_cast<uint32_t>(m);
     r.fast = mp.p < (1u << 31) && r.sh1 <= b - 2 ? 1 : 0;
@@ -118,14 +120,17 @@ inline EpiRed make_epi(const ModParams& mp, uint64_t kc) {
 
 template <bool FAST>
 __device__ __forceinline__ uint32_t epi_reduce_u64(uint64_t s, const EpiRed& r) {
+    const uint32_t lo = static_cast<uint32_t>(s);
+    const uint32_t hi = __funnelshift_r(lo, static_cast<uint32_t>(s >> 32), r.sh1);
+    const uint32_t q = __umulhi(hi, r.M) >> r.sh2;
     if constexpr (FAST) {
-        const uint32_t lo = static_cast<uint32_t>(s);
-        const uint32_t hi = __funnelshift_r(lo, static_cast<uint32_t>(s >> 32), r.sh1);
-        const uint32_t q = __umulhi(hi, r.M) >> r.sh2;
         const uint32_t x = lo - q * r.p;
         return min(x, x - r.p);
     } else {
-        return reduce_u64(s, r.p, r.barrett);
+        const uint64_t x = s - static_cast<uint64_t>(q) * r.p;
+        const uint32_t xl = static_cast<uint32_t>(x);
+        const uint32_t y = (x >> 32) != 0 || xl >= r.p ? xl - r.p : xl;
+        return min(y, y - r.p);  // p >= 2^31: y < p already, and y - p wraps above it
     }
 }
 
@@ -142,9 +147,10 @@ __device__ __forceinline__ uint32_t epi_reduce(uint32_t v0, uint32_t v1, uint32_
 // for Set, old + (x ^ flip) + bias is old + x, or old + p - x for Sub, below 2p.
 struct EpiOp {
     uint32_t flip, bias;
+    bool set;
 };
 __device__ __forceinline__ EpiOp epi_op(int op, const EpiRed& r) {
-    return op == HME_SUB ? EpiOp{0xffffffffu, r.p + 1u} : EpiOp{0u, 0u};
+    return op == HME_SUB ? EpiOp{0xffffffffu, r.p + 1u, false} : EpiOp{0u, 0u, op == HME_SET};
 }
 
 template <bool FAST>
@@ -153,6 +159,7 @@ __device__ __forceinline__ uint32_t epi_combine(uint32_t old, uint32_t x, const 
         const uint32_t t = old + (x ^ o.flip) + o.bias;
         return min(t, t - r.p);
     } else {
+        if (o.set) return x;
         return o.flip ? mod_sub(old, x, r.p) : mod_add(old, x, r.p);
     }
 }
