@@ -723,23 +723,27 @@ __global__ void __launch_bounds__(4 * RS) panel_block_kernel(const BlockArgs a, 
 // panels in which most active rows are zero.  Zero rows never pivot and are
 // never updated, so the search runs on the others alone: panel_rows_kernel
 // lists them (and clears the update's left factor W), and when there are at
-// most kCompactRows of them panel_compact_kernel factors them in one CTA, where
+// most kCompactMost of them panel_compact_kernel factors them in one CTA, where
 // a column costs one CTA barrier instead of the cluster's exchange.  It keeps
 // every row operation's effect on the identity as well (in place: the pivot's
 // column of a row holds that row's entry of the inverse of the operations), so W
 // comes out directly, with no triangular inverse and no panel_w_kernel.
+constexpr int kCompactRows = 256;
 // More listed rows than two a column meet in most columns, and one CTA updates them
 // all in every step: 26 panels of a banded 3000 x 2000 matrix mod 65521 (200 wide, 4
 // entries a row) with up to 256 listed rows took 196 us each, against 104 us in
-// the cluster search and 20 us for L11^-1 and W; the RREF 8.1 ms with a list of 256
-// rows, 6.35 ms with 128, 6.9 ms by searches alone.
-constexpr int kCompactRows = 128;
+// the cluster search and 20 us for L11^-1 and W; the RREF 8.1 ms with up to 256
+// rows, 6.35 ms with 128, 6.9 ms by searches alone.  An argument of the kernel: with
+// the limit compiled in, its steps come out slower (a panel of the 2048 x 2048 U D V
+// over Z/3^10 44 us against 37.5).
+constexpr int kCompactMost = 128;
 
 struct CompactArgs {
     uint32_t* A;
     uint64_t ld;
     int m, r0, c0, w;
     Ring R;
+    int most;         // listed rows to take, at most kCompactRows
     int* list;        // [kCompactRows] rows with a non-zero entry in the panel, in any order
     int* count;       // their number (counted on beyond the list); 0 between panels
     int after_block;  // the top block was tried before: nothing to do when it settled the panel
@@ -775,7 +779,7 @@ __host__ __device__ constexpr size_t compact_smem_bytes(int w) {
 }
 
 // One CTA of 32 warps.  The rows, in row order, sit in shared memory
-// column-major, lanes over rows: rwn = 1, 2 or 4 warps cover them and 32 /
+// column-major, lanes over rows: rwn = 1, 2, 4 or 8 warps cover them and 32 /
 // rwn groups of warps share the columns.  Pivot rule and fraction-free update
 // are the cluster kernel's, but a step whose column has no other entry updates
 // nothing (and no scale), and every column is updated, pivotless ones left of
@@ -804,7 +808,7 @@ __global__ void __launch_bounds__(1024, 1) panel_compact_kernel(const CompactArg
     }
     __syncthreads();
     const int cnt = s_cnt;
-    if (cnt > kCompactRows) {
+    if (cnt > min(a.most, kCompactRows)) {
         if (tid == 0) *a.ok = 0;
         return;
     }
@@ -820,7 +824,7 @@ __global__ void __launch_bounds__(1024, 1) panel_compact_kernel(const CompactArg
         s_step[tid] = 0;
     }
     __syncthreads();
-    const int rwn = cnt <= 32 ? 1 : cnt <= 64 ? 2 : 4;
+    const int rwn = cnt <= 32 ? 1 : cnt <= 64 ? 2 : cnt <= 128 ? 4 : 8;
     const int G = 32 / rwn, rs = 32 * rwn + 1;
     uint32_t* S = s_cmp;  // [w][rs]
 #pragma unroll 4
@@ -1703,6 +1707,7 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
             ca.c0 = c0;
             ca.w = w;
             ca.R = rg;
+            ca.most = kCompactMost;
             ca.list = d_s->list;
             ca.count = &d_s->count;
             ca.after_block = try_block ? 1 : 0;
