@@ -1592,26 +1592,30 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
     }
     // The panel's kernels in automatic mode: the top block, then the compact search of the non-zero
     // rows, then the search over all rows.  A failed attempt costs 10 us beside the search's 60 to 270,
-    // so after one the next 3, 7, 15, then 31 panels pass over that kernel (the top block: rank-deficient
-    // tails, sparse matrices, rings whose columns run out of units; the compact rows: dense matrices),
-    // and the count starts over with the next panel that it settles.  What is launched behind an
+    // so after one the next 3, then 7 panels pass over the top block (rank-deficient tails, sparse
+    // matrices, rings whose columns run out of units), the next 3, 7, 15, then 31 over the compact rows
+    // (dense matrices), and the count starts over with the next panel that it settles.  (A matrix that
+    // fills up halfway is back on the top block after 7 panels at most: 2000 x 2000 mod 65521, 1000
+    // columns of 4 entries and 1000 dense ones, 5.46 ms with pauses of up to 31 panels, 4.65 with 7,
+    // and 32 searches 5.2.)  What is launched behind an
     // attempt returns at once when the attempt settled the panel, so a failure costs no round trip to
     // the host; behind an attempt that is expected to succeed -- the kernel's last one did, or it is the
     // top block over a large field -- nothing is launched, and the host launches the rest if it must.
     const bool automatic = opt.panel_kernel == 0;
     struct Attempt {
-        int rest = 0, pause = 3;
+        int most, rest = 0, pause = 3;
         bool sure = false;
+        explicit Attempt(int longest_pause) : most(longest_pause) {}
         void settled() {
             pause = 3;
             sure = true;
         }
         void failed() {
             rest = pause;
-            pause = std::min(31, 2 * pause + 1);
+            pause = std::min(most, 2 * pause + 1);
             sure = false;
         }
-    } block, compact;
+    } block(7), compact(31);
     block.sure = rg.k == 1 && p >= (1u << 20);
     const bool keep = ring && ring->keep_skipped;
     bool block_tried[kRing] = {}, compact_tried[kRing] = {}, search_run[kRing] = {};
