@@ -1496,8 +1496,6 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
             pw *= rg.ell;
         }
         HME_REQUIRE(static_cast<uint64_t>(rg.pw[rg.k]) == p || rg.k == 1, "elim: modulus is not ell^k");
-        // phi(ell^k) - 1 = ell^(k-1) (ell - 1) - 1
-        rg.unit_exp = static_cast<uint32_t>(static_cast<uint64_t>(rg.pw[rg.k - 1]) * (rg.ell - 1) - 1);
     }
     if (p & 1u) {
         uint32_t x = p;  // p^-1 mod 2^32 by Newton's iteration (x = p is right to 3 bits)

@@ -597,16 +597,16 @@ void gemm_u64_device(hme_ctx* ctx, uint64_t p, uint32_t m, uint32_t n, uint32_t 
 // ones (p = 2^31 - 19, limbs / residue system): 64 x 64 x 8192 83 / 36, 300 x 300
 // x 8000 95 / 52, 2048^3 128 / 121, 4096^3 829 / 664, 1024^3 26 / 38, 4096 x 4096
 // x 1024 220 / 264, 1677 x 771 x 1419 52 / 53.
-bool rns_gemm_u32_pays(const ModParams& mp, uint32_t m, uint32_t n, uint32_t k) {
+bool rns_gemm_u32_pays(const ModParams& mp, uint32_t m, uint32_t n, uint32_t k, int sms) {
     if (mp.limbs < 4) return false;  // 9 moduli against 9 limb products below 2^24
     const double mk = static_cast<double>(m) * k, kn = static_cast<double>(k) * n, mn = static_cast<double>(m) * n;
     const double kb = (k + 127) / 128, tm = (m + kBM - 1) / kBM;
     const double bits = std::log2(static_cast<double>(k)) + 2 * std::log2(static_cast<double>(mp.p)) + 3;
     const double t = std::ceil(bits / 7.93);
-    const bool narrow = 4 * tm * ((n + 63) / 64) < 3 * 148.0;
+    const bool narrow = 4 * tm * ((n + 63) / 64) < 3.0 * sms;
     const double lt = tm * ((n + (narrow ? 31 : 63)) / (narrow ? 32 : 64)), rt = t * tm * ((n + 255) / 256);
-    const double limb = 6 + (8 * mk + 20 * kn) / 4.5e6 + std::ceil(lt / 148) * (4 * kb * (narrow ? 0.27 : 0.38) + 2);
-    const double rns = 14 + (mk + kn) * t * 3.5e-7 + std::ceil(rt / 148) * (kb * 0.38 + 1.5) + mn * t * 4.0e-7;
+    const double limb = 6 + (8 * mk + 20 * kn) / 4.5e6 + std::ceil(lt / sms) * (4 * kb * (narrow ? 0.27 : 0.38) + 2);
+    const double rns = 14 + (mk + kn) * t * 3.5e-7 + std::ceil(rt / sms) * (kb * 0.38 + 1.5) + mn * t * 4.0e-7;
     return rns < 0.95 * limb;
 }
 

@@ -238,6 +238,9 @@ void run_grouped(hme_ctx* ctx, const ModParams& mp, const std::vector<GemmJob>& 
         }
     }
     std::vector<GroupedProblem> probs(nj);
+    auto tiles_of = [&](const GemmJob& j) {
+        return static_cast<int>((j.M + kBM - 1) / kBM) * static_cast<int>((j.N + BN - 1) / BN);
+    };
     int tiles = 0;
     for (int t = 0; t < nj; ++t) {
         const GemmJob& j = jobs[t];
@@ -250,18 +253,17 @@ void run_grouped(hme_ctx* ctx, const ModParams& mp, const std::vector<GemmJob>& 
         P.N = static_cast<int>(j.N);
         P.kblocks = kp_of[t] / KBsel;
         P.op = j.op;
-        P.tiles_n = static_cast<int>((j.N + BN - 1) / BN);
         P.tile_begin = tiles;
         P.a_row0 = row0[t];
         P.b_col0 = col0[t];
-        tiles += static_cast<int>((j.M + kBM - 1) / kBM) * P.tiles_n;
+        tiles += tiles_of(j);
     }
     HME_CUDA(cudaMemcpyAsync(d_maps, maps.data(), maps_bytes, cudaMemcpyHostToDevice, ctx->stream));
     HME_CUDA(cudaMemcpyAsync(d_probs, probs.data(), probs_bytes, cudaMemcpyHostToDevice, ctx->stream));
     HME_CUDA(cudaMemcpyAsync(d_split, split.data(), split_bytes, cudaMemcpyHostToDevice, ctx->stream));
     std::vector<int> index(total_tiles + static_cast<size_t>(blocks));
     for (int t = 0; t < nj; ++t) {
-        const int nt = static_cast<int>((jobs[t].M + kBM - 1) / kBM) * probs[t].tiles_n;
+        const int nt = tiles_of(jobs[t]);
         std::fill(index.begin() + probs[t].tile_begin, index.begin() + probs[t].tile_begin + nt, t);
         const int nbk = split[t].s.a_blocks + split[t].b_blocks;
         std::fill(index.begin() + total_tiles + split[t].block_begin,

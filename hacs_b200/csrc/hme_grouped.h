@@ -23,7 +23,6 @@ struct GroupedProblem {
     int M, N;
     int kblocks;
     int op;
-    int tiles_n;
     int tile_begin;
     int a_row0, b_col0;
 };

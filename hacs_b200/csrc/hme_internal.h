@@ -276,7 +276,7 @@ void simt_gemm_u32_device(hme_ctx* ctx, const ModParams& mp, uint32_t m, uint32_
 int limb_kp(uint32_t k);
 // The product over the 8-bit residue system (gemm_u64.cu), and whether it beats
 // the limb product.
-bool rns_gemm_u32_pays(const ModParams& mp, uint32_t m, uint32_t n, uint32_t k);
+bool rns_gemm_u32_pays(const ModParams& mp, uint32_t m, uint32_t n, uint32_t k, int sms);
 bool rns_gemm_u32_device(hme_ctx* ctx, const ModParams& mp, uint32_t m, uint32_t n, uint32_t k, const uint32_t* A,
                          size_t lda, const uint32_t* B, size_t ldb, uint32_t* C, size_t ldc, int op);
 // C op= A*B mod 2^32 (native wraparound u32 arithmetic, any u32 words) on the

@@ -841,10 +841,8 @@ __device__ __forceinline__ void split_b_part(const SplitArgs& s, int block, uint
 
 }  // namespace limb
 
-// Host: encode a tiled uint8 TMA descriptor with 128-byte swizzle (limb planes).
-void encode_tma_u8(CUtensorMap* map, void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides,
-                   const cuuint32_t* box);
-// The same with the swizzle matching a k-block of kb bytes (128, 64 or 32).
+// Host: encode a tiled uint8 TMA descriptor (limb planes) with the swizzle matching a k-block of kb bytes (128,
+// 64 or 32).
 void encode_tma_u8_kb(CUtensorMap* map, void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides,
                       const cuuint32_t* box, int kb);
 

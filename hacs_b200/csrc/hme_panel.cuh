@@ -53,7 +53,6 @@ struct Ring {
     uint32_t q;          // modulus
     uint64_t barrett;    // floor(2^64 / q)
     uint32_t ell, k;
-    uint32_t unit_exp;   // phi(q) - 1: u^unit_exp is the inverse of a unit u
     uint32_t max_v;      // pivots of valuation <= max_v only (0: unit pivots)
     uint32_t mont_qinv;  // q odd: -q^-1 mod 2^32 (Montgomery reduction)
     uint32_t mont_r2;    // q odd: 2^64 mod q

@@ -24,7 +24,6 @@ enum DeviceErr : int {
     DERR_WAIT_ACCUM = 3,      // epilogue waited too long for an accumulator
     DERR_WAIT_ACCUM_FREE = 4, // MMA issuer waited too long for a drained accumulator
     DERR_WAIT_DRAIN = 5,      // tear-down wait for in-flight copies / MMAs ran out
-    DERR_TMEM_ADDR = 6,       // tensor-memory allocation returned an unusable address
     DERR_GRID_BARRIER = 7,    // a cooperative kernel's grid barrier waited too long
     DERR_LAUNCH_SHAPE = 8,    // a kernel found its launch shape outside what it supports and did nothing
 };
@@ -263,22 +262,10 @@ __device__ __forceinline__ void tmem_wait_ld() {
 
 // ---- descriptors --------------------------------------------------------------------------
 // Shared-memory matrix descriptor for a K-major operand written by TMA with
-// 128-byte swizzle: rows of 128 bytes, 8-row atoms 1024 bytes apart (SBO),
-// LBO unused for swizzled K-major layouts (encoded 1), version 1 (sm_100),
-// layout type 2 = SWIZZLE_128B.  The tile base must be 1024-byte aligned.
-__device__ __forceinline__ uint64_t smem_desc_k128(uint32_t smem_addr) {
-    uint64_t d = 0;
-    d |= static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4);
-    d |= static_cast<uint64_t>(1) << 16;
-    d |= static_cast<uint64_t>(1024 >> 4) << 32;
-    d |= static_cast<uint64_t>(1) << 46;
-    d |= static_cast<uint64_t>(2) << 61;
-    return d;
-}
-// The same for a K-major operand written by TMA with KB-byte swizzle (KB = 128,
-// 64 or 32): rows of KB bytes, 8-row atoms 8*KB bytes apart, layout type 2
-// (SWIZZLE_128B), 4 (SWIZZLE_64B) or 6 (SWIZZLE_32B).  Tile base aligned to the
-// atom (8*KB bytes).
+// KB-byte swizzle (KB = 128, 64 or 32): rows of KB bytes, 8-row atoms 8*KB bytes
+// apart (SBO), LBO unused for swizzled K-major layouts (encoded 1), version 1
+// (sm_100), layout type 2 (SWIZZLE_128B), 4 (SWIZZLE_64B) or 6 (SWIZZLE_32B).
+// Tile base aligned to the atom (8*KB bytes).
 template <int KB>
 __device__ __forceinline__ uint64_t smem_desc_kmajor(uint32_t smem_addr) {
     static_assert(KB == 128 || KB == 64 || KB == 32, "swizzle width");

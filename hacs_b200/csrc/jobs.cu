@@ -720,10 +720,9 @@ __global__ void rank_post_kernel(RankDev* __restrict__ devs, int nj, const RankO
             gp.N = ntrail;
             gp.kblocks = 1;
             gp.op = HME_SUB;
-            gp.tiles_n = (ntrail + G.bn - 1) / G.bn;
             gp.a_row0 = D.a_row0;
             gp.b_col0 = D.b_col0;
-            tiles[j] = ((below + limb::kBM - 1) / limb::kBM) * gp.tiles_n;
+            tiles[j] = ((below + limb::kBM - 1) / limb::kBM) * ((ntrail + G.bn - 1) / G.bn);
             GroupedSplitJob& gs = gsplit[j];
             limb::SplitArgs& sa = gs.s;
             sa.A = D.L21;

@@ -227,10 +227,6 @@ __global__ void fill_zero_kernel(uint32_t* C, uint64_t ldc, int m, int n) {
 
 }  // namespace
 
-void encode_tma_u8(CUtensorMap* map, void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides,
-                   const cuuint32_t* box) {
-    encode_u8(map, base, rank, dims, strides, box);
-}
 void encode_tma_u8_kb(CUtensorMap* map, void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides,
                       const cuuint32_t* box, int kb) {
     encode_u8(map, base, rank, dims, strides, box, kb);
@@ -330,7 +326,7 @@ void gemm_u32_device(hme_ctx* ctx, const ModParams& mp, uint32_t m, uint32_t n, 
     if (!check_product(mp, m, n, k, ldc, op)) return;
     int v = ctx->fixed_variant;
     if (v < 0 && ctx->sched_policy == 0 && k > 0 && A && B && C && lda >= k && ldb >= n &&
-        rns_gemm_u32_pays(mp, m, n, k) && rns_gemm_u32_device(ctx, mp, m, n, k, A, lda, B, ldb, C, ldc, op))
+        rns_gemm_u32_pays(mp, m, n, k, ctx->num_sms) && rns_gemm_u32_device(ctx, mp, m, n, k, A, lda, B, ldb, C, ldc, op))
         return;
     if (v < 0) v = sched_variant(ctx, mp, m, n, k);
     gemm_u32_variant(ctx, mp, m, n, k, A, lda, B, ldb, C, ldc, op, v);

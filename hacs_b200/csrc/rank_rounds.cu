@@ -74,7 +74,6 @@ __device__ __forceinline__ panel::Ring rr_ring(const RrGroup& G) {
     R.barrett = G.barrett;
     R.ell = G.p;
     R.k = 1;
-    R.unit_exp = G.p - 2;
     R.max_v = 0;
     R.mont_qinv = G.mont_qinv;
     R.mont_r2 = G.mont_r2;
@@ -182,7 +181,7 @@ __global__ void __launch_bounds__(NT, NT == 1024 ? 1 : 2) rr_general_kernel(RrJo
     extern __shared__ __align__(16) uint32_t S[];  // [w][rs]
     __shared__ uint32_t s_x[2][MAXR];
     __shared__ int s_key[2][NRW], s_nz[2][NRW];
-    __shared__ uint32_t s_S[W + 1], s_Sinv[W + 1];
+    __shared__ uint32_t s_inv;
     __shared__ int s_prow[W], s_colpiv[W], s_vac[W];
     __shared__ unsigned char s_isp[W];
     __shared__ int s_row[MAXR], s_step[MAXR], s_pos[MAXR];
@@ -278,7 +277,6 @@ __global__ void __launch_bounds__(NT, NT == 1024 ? 1 : 2) rr_general_kernel(RrJo
             if (pk != NONE) {
                 const uint32_t wt = s_x[par][pk];
                 if (tid == 0) {
-                    s_S[k] = scale;
                     s_prow[k] = pk;
                     s_colpiv[it] = k;
                     s_step[pk] = k + 1;
@@ -312,10 +310,9 @@ __global__ void __launch_bounds__(NT, NT == 1024 ? 1 : 2) rr_general_kernel(RrJo
             if (k == w && cnt == rows && rows > w) J.dense = 1;
         }
         if (k == 0 || J.c0 + w >= J.n || rows == k) continue;  // nothing to update
-        if (tid == 0) s_S[k] = scale;
         if (tid < W) s_isp[tid] = 0;
         __syncthreads();
-        if (tid <= k) s_Sinv[tid] = unit_inverse(s_S[tid], R);
+        if (tid == 0) s_inv = unit_inverse(scale, R);  // the rows below the pivots have the last scale
         // the listed rows' places: pivots in order; the others behind them (listed rows move), or where
         // they are but for those that a pivot row displaces (all rows)
         if constexpr (!TALL) {
@@ -354,7 +351,7 @@ __global__ void __launch_bounds__(NT, NT == 1024 ? 1 : 2) rr_general_kernel(RrJo
             if (lane == 0 && pos < (TALL ? k : cnt)) J.rows[pos] = J.r0 + s_row[r];
             if (pos < k) continue;
             uint32_t* wd = J.F + static_cast<size_t>(pos - k) * W;
-            const uint32_t sc = s_Sinv[k];
+            const uint32_t sc = s_inv;
             for (int c = lane; c < w; c += 32) {
                 const int t = s_colpiv[c];
                 if (t >= 0) wd[t] = mod_mul(S[c * rs + r], sc, R.q, R.barrett);
@@ -550,10 +547,9 @@ __global__ void rr_post_kernel(RrJob* __restrict__ jobs, int nj, RrMove* __restr
             gp.N = ntrail;
             gp.kblocks = 1;
             gp.op = J.kind == 1 ? HME_SUB : HME_ADD;
-            gp.tiles_n = (ntrail + G.bn - 1) / G.bn;
             gp.a_row0 = J.a_row0;
             gp.b_col0 = J.b_col0;
-            tiles[j] = ((below + limb::kBM - 1) / limb::kBM) * gp.tiles_n;
+            tiles[j] = ((below + limb::kBM - 1) / limb::kBM) * ((ntrail + G.bn - 1) / G.bn);
             GroupedSplitJob& gs = gsplit[j];
             limb::SplitArgs& sa = gs.s;
             sa.A = J.kind == 1 ? J.A + static_cast<size_t>(J.r0 + k) * J.ld + J.c0 : J.F;
