@@ -1520,7 +1520,7 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
         int err;       // the device error word as of the panel's end
         int settled;   // 1: by the top block, 2: by the compact kernel, 0: by a searching kernel (or not yet)
         int count;     // rows listed for the compact kernel
-        int fail;      // ring entry 0 only: queued work stands still (BlockArgs::fail)
+        int fail;      // ring entry 0 only: queued work stands still (BlockQueue::fail)
         int list[kCompactRows];
         int rest;      // what the rest of the matrix holds (window_look_kernel)
         unsigned bar[2];

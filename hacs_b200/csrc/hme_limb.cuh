@@ -69,8 +69,8 @@ struct Cfg {
 //    before the floor, so with sh1 <= b - 2 the rest s - q p is below 2p, and
 //    with p < 2^31 it fits a word and one unsigned min(r, r - p) finishes it.
 //    p = 0 (the wraparound mode) has M = 0: the truncation to 32 bits.  Every
-//    other modulus has sh1 <= b (at most 2^31 255-bounded products per limb, L
-//    limbs below 256^L): the rest, below 3p, in 64 bits and two corrections (with
+//    other modulus has sh1 <= b - 1 (a limb's sums stay below 2^31, and 256^(L-1)
+//    < p): the rest, below 3p, in 64 bits and two corrections (with
 //    a 64-bit Barrett step, six wide products, 3000 x 3000 x 256 mod 2^32 - 17
 //    takes 48 us, 45 so);
 //  - C moves in 16-byte pieces where its rows are 16-byte aligned, and a

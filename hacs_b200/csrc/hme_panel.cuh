@@ -1,5 +1,5 @@
 // Panel arithmetic and the top-block inversion, shared by the single-matrix
-// elimination (elim.cu) and the batched ranks (jobs.cu).
+// elimination (elim.cu) and the batched ranks (rank_rounds.cu).
 #pragma once
 #include <cuda_runtime.h>
 

@@ -13,20 +13,22 @@
 // output columns the L matrices D_j sit side by side in one accumulator of
 // L*BN columns, so a CTA runs ONE integer GEMM of 128 x (L*BN) x (L*K) on the
 // tensor cores (tcgen05.mma kind::i8, M=128, N=L*BN, K=32 per instruction),
-// then recombines sum_j 256^j D_j in u64 and reduces once (Barrett, the
-// ModCtx<uint32_t>::reduce_u64 rule).  Exactness: every D_j is a sum of at
+// then recombines sum_j 256^j D_j in u64 and reduces once (a quotient by one 32-bit
+// multiply-high, hme_limb.cuh).  Exactness: every D_j is a sum of at
 // most L*K_chunk products below 255^2, and K is cut into chunks with
 // L * 255^2 * K_chunk < 2^31 (later chunks accumulate with Add).
 //
 // Layout in HBM (workspace): A limb planes [i][m][k] (L x M x Kp bytes) and
 // B planes [i][j][n][k] (L x L x N x Kp bytes), K contiguous (K-major for both
-// tensor-core operands), Kp = K rounded up to 16 bytes for TMA strides.
+// tensor-core operands), Kp = K rounded up to whole k-blocks of 32, 64 or
+// 128 bytes (16 in the allocation-free entry point).
 //
-// Kernel: persistent, one CTA per SM, 10 warps: warp 0 issues TMA loads
-// (128-byte swizzle, each CTA loads its own tiles), warp 1 owns tensor memory and issues the
-// MMAs, warps 2-9 (two per TMEM lane quarter, alternate 16-column chunks)
-// drain the double-buffered accumulator (2 x L*BN columns of
-// TMEM) into C while the next tile's MMAs run.
+// Kernel: persistent, one CTA per SM, 18 warps for one or four limbs and 10 for two
+// or three: warp 0 issues TMA loads (a swizzle row of KB bytes, each CTA loads its
+// own tiles), warp 1 owns tensor memory and issues the MMAs, the others (four or
+// two per TMEM lane quarter, taking its 16-column chunks in turn) drain the
+// double-buffered accumulator (2 x L*BN columns of TMEM) into C while the next
+// tile's MMAs run.
 #include <cuda.h>
 #include <cuda_runtime.h>
 

@@ -87,7 +87,16 @@ HME_API const char *hme_version(void);
  * p <= 2^16, 3 for p <= 2^24, 4 otherwise), the limb products run on the
  * tensor cores with exact int32 accumulation over K chunks with
  * L * 255 * 255 * K_chunk < 2^31, and the epilogue recombines and reduces.
- * Bit-exact with engine::kernels::gemm<uint32_t>.
+ * Device workspace: L m Kp + L^2 n Kp bytes of planes, Kp = k rounded up to 32,
+ * 64 or a multiple of 128, and an eighth more.  hme_gemm_u32_dev takes a large
+ * product at 25 to 32 bits over the residue system of hme_gemm_u64 where its
+ * cost rule says that this is faster (t = 8 to 12 moduli; t (m + n) Kp + t m n
+ * bytes; without them, or under a capture that would have to allocate them, the
+ * limb product runs) -- not under a fixed variant or the learned policy, whose
+ * choices are among the limb product's schedules, nor with host pointers, where
+ * the product is split by rows behind the copies.
+ * Bit-exact with engine::kernels::gemm<uint32_t> for canonical entries (< p);
+ * the result of entries that are not reduced is unspecified.
  *
  * hme_gemm_u32: host pointers.  Replaces the GPU micro-bench hook
  *   micro::GpuHooks::gemm (src/ModArithmetic/PerformanceSmokeValidation.h:158-165,
@@ -107,11 +116,13 @@ HME_API int hme_gemm_u32_dev(hme_ctx *ctx, uint32_t p, uint32_t m, uint32_t n, u
  * and B must be canonical (< p).  Bit-exact with engine::kernels::gemm
  * <uint64_t> (src/ModArithmetic/Kernels.h:178-185) and the device u64 regime
  * engine::cuda::gemm<uint64_t> (src/Cuda/cuda_kernels.cu:151-163, 365-381).
- * Method: p < 2^32 runs the u32 limb GEMM directly; larger p runs t limb GEMMs
- * modulo primes below 2^16 (t chosen so that their product exceeds
- * 4 k (p-1)^2) and reconstructs each entry by the Chinese remainder theorem,
- * reduced mod p once (Montgomery for odd p < 2^63).  Device workspace:
- * t (2 m Kp + 4 n Kp + 4 m n) bytes, Kp = k rounded up to 32, 64 or a multiple of 128, t <= 12
+ * Method: p < 2^32 runs the u32 GEMM directly; larger p runs one int8 product
+ * modulo each of t pairwise coprime moduli of 8 bits (t chosen so that their
+ * product exceeds 4 k (p-1)^2; 18 for p = 2^61 - 1 and k = 2048, at most 22)
+ * and reconstructs each entry by the Chinese remainder theorem, reduced mod p
+ * once (Montgomery for odd p < 2^63).  Sides up to 2^31 - 256.  Device
+ * workspace: t ((m + n) Kp + m n') bytes, Kp = k rounded up to 32, 64 or a
+ * multiple of 128, n' = n rounded up to 32
  * (p < 2^32: 4 (mk + kn + mn) bytes plus the u32 GEMM's planes).
  * hme_gemm_u64: host pointers (synchronous); hme_gemm_u64_dev: device
  * pointers, asynchronous on the context's stream. */
@@ -366,7 +377,10 @@ HME_API int hme_gen_jobs_u32_dev(hme_ctx *ctx, uint32_t nmat, const hme_gen_spec
  *     waits for).
  * rank_variants = NULL takes the context's scheduler (under the learned policy
  * the rank planner's decision per job's shape class, recorded by
- * hme_sched_plan_rank; else the batch rule).  No schedule changes a rank.
+ * hme_sched_plan_rank; else the batch rule).  No schedule changes a rank.  The
+ * planner and the autotuner choose among 0..3 only, and one scheduled job takes
+ * its call off the rounds of 64 columns: a mixed stream of 50 000 jobs runs at
+ * 61 k jobs/s under a plan of the ranks and at 126 k under the batch rule.
  * hme_batch_gemm_rank_u32_dev_sched: the GEMM phase under gemm_variants (as
  * hme_batch_gemm_u32_dev_plan), then the rank phase under rank_variants. */
 HME_API int hme_batch_rank_u32_dev_sched(hme_ctx *ctx, uint32_t njobs, const hme_job *jobs, const int *rank_variants,
