@@ -1596,10 +1596,9 @@ ElimResult elim_device(hme_ctx* ctx, const ModParams& mp, uint32_t* A, size_t ld
     // matrices, rings whose columns run out of units), the next 3, 7, 15, then 31 over the compact rows
     // (dense matrices), and the count starts over with the next panel that it settles.  (A matrix that
     // fills up halfway is back on the top block after 7 panels at most: 2000 x 2000 mod 65521, 1000
-    // columns of 4 entries and 1000 dense ones, 5.46 ms with pauses of up to 31 panels, 4.65 with 7,
-    // and 32 searches 5.2.)  What is launched behind an
-    // attempt returns at once when the attempt settled the panel, so a failure costs no round trip to
-    // the host; behind an attempt that is expected to succeed -- the kernel's last one did, or it is the
+    // columns of 4 entries and 1000 dense ones, 5.46 ms with pauses of up to 31 panels, 4.65 with 7.)
+    // What is launched behind an attempt returns at once when the attempt settled the panel, so a
+    // failure costs no round trip to the host; behind an attempt that is expected to succeed -- the kernel's last one did, or it is the
     // top block over a large field -- nothing is launched, and the host launches the rest if it must.
     const bool automatic = opt.panel_kernel == 0;
     struct Attempt {
